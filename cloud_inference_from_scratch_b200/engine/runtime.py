@@ -74,3 +74,4 @@ class Runtime:
         # kernels that keep scratch memory by the token make it for the largest step at first use, so that
         # it need not grow once a captured graph holds its address
         self.ops.max_rows = self.workspace.max_rows
+        self.ops.max_requests = int(max_requests)

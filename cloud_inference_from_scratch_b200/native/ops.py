@@ -49,6 +49,7 @@ LATENT_PROMPT_KEYS = 1 << 17
 LATENT_PROMPT_BYTES = 1 << 28
 
 
+
 class _Lib:
     """A loaded library whose entry points return 0 or set ``cie_last_error``."""
 
@@ -93,6 +94,7 @@ class Ops:
         self.error_word = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.launches = 0
         self.max_rows = 0             # most tokens of a step, if the runtime knows (0: not known)
+        self.max_requests = 0         # most requests of a step, likewise
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
 
         v, i, f = c_void_p, c_int, c_float
@@ -1327,6 +1329,10 @@ class Ops:
             self._delta_stream = lib.function(
                 "cie_delta_stream", [v, i, i, i, i, i, v, i, v, v, v, v, i, v, v, v, v, i, i, i, i, i, v, v])
             lib.handle.cie_delta_stream_floats.restype = ctypes.c_longlong
+            self._delta_chunked = lib.function(
+                "cie_delta_chunked", [v, i, i, i, i, i, v, i, v, v, v, v, i, v, v, v, v, v, v, i, i, i, i, i, v, v])
+            lib.handle.cie_delta_chunk_floats.restype = ctypes.c_longlong
+            self.delta_chunk_tokens = int(lib.handle.cie_delta_chunk_tokens())
             self.delta_max_dim = int(lib.handle.cie_delta_max_dim())
             self.delta_stream_max_dim = int(lib.handle.cie_delta_stream_max_dim())
             self._delta_lib = lib
@@ -1343,19 +1349,51 @@ class Ops:
         self.launches += 1
         self._tanh_rows(_ptr(x), x.stride(0), _ptr(out), out.shape[0], out.shape[1], self._code_of(out), self.stream)
 
+    def plan_delta(self, host: Any, heads: int, dim: int) -> dict[str, Any]:
+        """Work lists of the generalized delta rule's chunked form (see ``plan_lightning``), for steps that it
+        serves faster than a walk token by token."""
+        self._load_delta()
+        if host.num_single == host.num_requests or dim > self.delta_stream_max_dim:
+            return {}
+        # us on a B200 for heads padded to P: the walk follows its longest portion (2,048 tokens, P = 64: 1,790; P = 128:
+        # 3,945) until its blocks fill the device (32 portions of 64 tokens, 32 heads of 64: 187; 16 of 128: 360); the
+        # chunks cost what there are of them (the same four steps: 246, 515, 257, 612) and two launches
+        pad = 32 if dim <= 32 else 64 if dim <= 64 else 128
+        lengths = host.query_lens
+        walk = max(0.0135 * pad * int(lengths.max()), 7e-7 * pad * pad * heads * int(lengths.sum()))
+        if walk <= 17 + 2.75e-5 * pad * pad * heads * int((-(-lengths // self.delta_chunk_tokens)).sum()):
+            return {}
+        return self._plan_chunks(host, self.delta_chunk_tokens)
+
     def delta_scan(self, proj: Any, offsets: tuple[int, int, int, int], decay: Any, decay_bias: Any,
-                   removal_bias: Any, out: Any, state: Any, ctx: Any, heads: int, dim: int) -> None:
+                   removal_bias: Any, out: Any, state: Any, ctx: Any, heads: int, dim: int,
+                   plan: dict[str, Any] | None = None) -> None:
         """Runs the generalized delta rule over every request's new tokens from the state in its slot
         (``state``: float32 [slots, heads, dim, dim]).  ``proj`` float32 rows hold r, k, v and the
         removal projection from the columns ``offsets``; ``decay`` float32 [T, heads * dim] is the decay
         projection; both biases are added here; ``out`` float32 [T, heads * dim].  A step of single tokens
         runs one kernel that works the rates out as it goes; a step with prompt portions (eight tokens a
         request or more on average) first works out, for all tokens at once, what the recurrence reads
-        and then streams it through a ring of copies: the same additions in the same order."""
+        and then streams it through a ring of copies: the same additions in the same order.  With ``plan``
+        (``plan_delta``, on the device) the step runs in chunks: what a chunk does to any state in parallel, then a
+        walk over each request's chunks."""
         self._flush()
         self._load_delta()
         r_off, k_off, v_off, a_off = offsets
         tokens = proj.shape[0]
+        if plan:
+            chunks = plan["chunk_row"].shape[0]
+            floats = self._delta_lib.handle.cie_delta_chunk_floats
+            most = -(-max(tokens, self.max_rows) // self.delta_chunk_tokens) + max(ctx.num_requests, self.max_requests)
+            cells = self.scratch(f"delta.cells.{heads}x{dim}", int(floats(chunks, heads, dim)),
+                                 reserve=int(floats(max(chunks, most), heads, dim)))
+            self.launches += 2
+            self._delta_chunked(_ptr(proj), proj.stride(0), r_off, k_off, v_off, a_off, _ptr(decay), decay.stride(0),
+                                _ptr(decay_bias), _ptr(removal_bias), _ptr(cells), _ptr(out), out.stride(0), _ptr(state),
+                                _ptr(plan["chunk_row"]), _ptr(plan["chunk_count"]), _ptr(plan["request_chunk_start"]),
+                                _ptr(ctx.slots), _ptr(ctx.request_active), chunks, ctx.num_requests, heads, dim,
+                                state.shape[0], _ptr(self.error_word), self.stream)
+            return
         if (tokens >= 8 * ctx.num_requests and dim <= self.delta_stream_max_dim
                 and os.environ.get("CIE_DELTA_STREAM", "1") != "0"):
             floats = self._delta_lib.handle.cie_delta_stream_floats

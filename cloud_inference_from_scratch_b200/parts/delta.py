@@ -37,6 +37,14 @@ class GeneralDelta(Mixer):
         self.names = {key: key for key in ("r", "k", "v", "g", "a", "a.b", "w1", "w2", "w0", "norm", "o")}
         self.names.update(names or {})
 
+    @property
+    def plan_key(self):
+        return ("delta.chunks", self.num_heads, self.head_dim)
+
+    def plan(self, host, cache):
+        """Chunk work lists for a step with prompt portions (one list serves every layer of these sizes)."""
+        return self.runtime.ops.plan_delta(host, self.num_heads, self.head_dim)
+
     def state_spec(self) -> StateSpec:
         return StateSpec((self.num_heads, self.head_dim, self.head_dim), "float32")
 
@@ -83,7 +91,8 @@ class GeneralDelta(Mixer):
         ops.linear(squashed, self.w_decay, None, decay)
         mixed = rt.workspace.get("delta.o", tokens, width, f32)
         ops.delta_scan(proj, (0, width, 2 * width, 4 * width), decay, self.decay_bias, self.removal_bias, mixed,
-                       binding.state, ctx, self.num_heads, self.head_dim)
+                       binding.state, ctx, self.num_heads, self.head_dim,
+                       plan=getattr(ctx, "extras", {}).get(self.plan_key) or None)
         gated = rt.workspace.get("delta.gated", tokens, width, rt.dtype)
         ops.group_gate_norm(mixed, proj[:, 3 * width:4 * width], self.gain, self.eps, gated, self.num_heads)
         update = rt.workspace.get("mixer.update32", tokens, self.hidden_size, f32)

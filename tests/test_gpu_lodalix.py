@@ -510,6 +510,46 @@ def test_delta_rule_in_one_kernel_and_in_two_kernels_agree(monkeypatch, dim):
     close(seen[0][1], seen[1][1], "float32", scale=float(seen[1][1].abs().max()))
 
 
+@pytest.mark.parametrize("lengths", [[1], [31, 1, 32, 33], [70, 5, 96]])
+@pytest.mark.parametrize("dim", [1, 7, 32, 33, 64, 100, 128])
+def test_delta_rule_in_chunks(dim, lengths):
+    """Chunks that are whole, that hold one token and that end short, heads at the edges of the padded sizes, from states
+    that are not zero, beside a request that only pads; decays at both ends of their range.  A value is a sum of a few
+    hundred float32 products of numbers of its own size: 1e-5 of the largest one is 100 roundings."""
+    rt = runtime("float32")
+    heads, count = 3, len(lengths)
+    width, tokens = heads * dim, sum(lengths)
+    proj, decay = rand(tokens, 5 * width + 2, seed=1), rand(tokens, width, seed=2, scale=6.0)
+    w0, a0 = rand(width, seed=3, scale=3.0), rand(width, seed=4)
+    starts = np.cumsum([0, *lengths]).astype(np.int32)
+    active = [0 if r == 1 else 1 for r in range(count)]
+    ctx = SimpleNamespace(query_start=torch.from_numpy(starts).cuda(), num_requests=count,
+                          slots=torch.arange(count, 0, -1, dtype=torch.int32).cuda(),
+                          request_active=torch.tensor(active, dtype=torch.int32).cuda())
+    host = SimpleNamespace(query_start=starts, query_lens=np.asarray(lengths, dtype=np.int32))
+    rt.ops.require_delta()
+    plan = {key: torch.from_numpy(value).cuda() for key, value in rt.ops._plan_chunks(host, rt.ops.delta_chunk_tokens).items()}
+    before = rand(count + 2, heads, dim, dim, seed=5, scale=0.3)
+    state = before.clone().cuda()
+    out = torch.full((tokens + 1, width), 7.0).cuda()
+    rt.ops.delta_scan(proj.cuda(), (2 * width, 0, 4 * width + 2, width), decay.cuda(), w0.cuda(), a0.cuda(), out[:tokens], state,
+                      ctx, heads, dim, plan=plan)
+    rt.ops.check_errors()
+    assert float((out[tokens] - 7.0).abs().max()) == 0
+    assert torch.equal(state[0].cpu(), before[0]) and torch.equal(state[-1].cpu(), before[-1])      # other slots untouched
+    for r in range(count):
+        rows = proj[starts[r]:starts[r + 1]].double()
+        shape = (-1, heads, dim)
+        k, a, rr, v = (rows[:, o:o + width].view(shape) for o in (0, width, 2 * width, 4 * width + 2))
+        w = torch.exp(-np.exp(-0.5) * torch.sigmoid(decay[starts[r]:starts[r + 1]].double() + w0.double())).view(shape)
+        want, after = plain.delta_recurrence(rr, k, v, w, torch.sigmoid(a.reshape(-1, width) + a0.double()).view(shape),
+                                             before[count - r].double())
+        got = out[starts[r]:starts[r + 1]].view(shape).double().cpu()
+        assert float((got - want).abs().max()) <= 1e-5 * float(want.abs().max())
+        held = after if active[r] else before[count - r].double()
+        assert float((state[count - r].double().cpu() - held).abs().max()) <= 1e-5 * float(after.abs().max())
+
+
 def test_delta_rule_unlearns_along_its_key():
     """With removal rate 1 and no decay, writing a key a second time REPLACES what it held: the
     first value is gone and the read gives the second."""
