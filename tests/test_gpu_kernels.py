@@ -167,6 +167,24 @@ def test_gemm_simt_any_shape(ops, dtype, m):
                                rtol=2e-5, atol=2e-5)
 
 
+@pytest.mark.parametrize("n,k", [(1, 4), (129, 36), (300, 100), (2050, 132), (19000, 32)])
+def test_gemm_float32_tiles_add_in_the_order_of_the_general_kernel(ops, n, k):
+    """Row and column counts around the tiles' edges; the general kernel is reached by operands that are not aligned."""
+    item = ops[torch.float32]
+    bias = rand(n, seed=3)
+    for m in (1, 8, 9, 16, 17, 40, 65, 129, 300):
+        x, w = rand(m * k + 4, seed=m), rand(n * k + 4, scale=0.1, seed=m + 1)
+        results = []
+        for shift in (0, 1):
+            rows, weights = torch.zeros_like(x), torch.zeros_like(w)
+            rows[shift:shift + m * k], weights[shift:shift + n * k] = x[:m * k], w[:n * k]
+            out = torch.full((m + 1, n), 7.0).cuda()
+            item._gemm_simt(rows[shift:].data_ptr(), weights[shift:].data_ptr(), bias.data_ptr(), out.data_ptr(), m, n, k,
+                            0, 0, 0, item.stream)
+            results.append(out)
+        assert torch.equal(results[0], results[1]) and float((results[0][m] - 7.0).abs().max()) == 0
+
+
 def test_gemm_float32_rows_do_not_depend_on_the_batch(ops):
     item = ops[torch.float32]
     x, w = rand(70, 300, seed=8), rand(200, 300, scale=0.1, seed=9)
