@@ -31,7 +31,7 @@ COMMON_FLAGS = (
     "-Xcompiler", "-fPIC", "-shared",
 )
 
-_loaded: dict[str, ctypes.CDLL] = {}
+_loaded: dict[tuple, ctypes.CDLL] = {}
 _lock = threading.Lock()
 
 
@@ -120,11 +120,11 @@ def load_library(
     source: str, defines: dict[str, object] | None = None, extra_flags: tuple[str, ...] = ()
 ) -> ctypes.CDLL:
     """Builds (if needed) and loads ``csrc/<source>``; one handle per (source, defines)."""
-    target, define_flags = library_path(source, defines)
-    key = str(target)
+    key = (source, tuple(sorted((name, str(value)) for name, value in (defines or {}).items())))
     with _lock:
         if key in _loaded:
             return _loaded[key]
+        target, define_flags = library_path(source, defines)
         if not target.exists():
             _compile(source, target, define_flags, extra_flags)
         try:
