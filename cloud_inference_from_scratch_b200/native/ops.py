@@ -227,8 +227,8 @@ class Ops:
                             gates: Any = None) -> None:
         """Attention with the options of ``attention_generic`` (a value size of its own, distance
         penalties, a soft cap, kept first keys, sinks, a gate per head), softmax weights float32 throughout.  bfloat16
-        prompt portions whose key and value heads are multiples of 16 run on the tensor cores (mma.sync; the
-        weights enter the value product as two bfloat16 terms); single tokens, the 32-bit path and every other
+        prompt portions whose key and value heads are multiples of 16 run on the tensor cores (tcgen05 for heads of 64 or
+        128 alike, else mma.sync; the weights enter the value product as two bfloat16 terms); single tokens, the 32-bit path and every other
         shape run on the kernel whose heads of a group share the keys, or on one warp per (token, head)."""
         fast = (self._tensor_attention.get(max(head_dim, value_dim))
                 if head_dim % 16 == 0 and value_dim % 16 == 0 and self.code == BF16 else None)
@@ -250,17 +250,24 @@ class Ops:
 
     def require_attention(self, head_dim: int) -> None:
         """Builds, at model set-up, the attention kernels a head size needs."""
-        self.require_portion_attention(head_dim)
-        if head_dim in self._tensor_attention:
-            self._tensor_attention[head_dim].load_prompt_kernel()
+        held = self._tensor_kernels(head_dim)
+        if held is not None:
+            held.load_prompt_kernel()
 
     def require_portion_attention(self, head_dim: int) -> None:
-        """The same for a layer with options of ``attention_penalised``, which the tcgen05 prompt kernel does not take."""
-        if self.code == BF16:
-            from . import tensor_attention
+        """The same for a layer with options of ``attention_penalised``, which have a tcgen05 prompt kernel of their own."""
+        held = self._tensor_kernels(head_dim)
+        if held is not None:
+            held.load_options_kernel()
 
-            if head_dim not in self._tensor_attention and tensor_attention.supports(head_dim):
-                self._tensor_attention[head_dim] = tensor_attention.TensorAttention(self, head_dim)
+    def _tensor_kernels(self, head_dim: int) -> Any:
+        if self.code != BF16:
+            return None
+        from . import tensor_attention
+
+        if head_dim not in self._tensor_attention and tensor_attention.supports(head_dim):
+            self._tensor_attention[head_dim] = tensor_attention.TensorAttention(self, head_dim)
+        return self._tensor_attention.get(head_dim)
 
     def plan_attention(self, host: Any, group: int) -> dict[str, Any]:
         """Integer work lists the attention kernels want in a step's metadata (may be empty)."""

@@ -5,7 +5,8 @@ csrc/attention_prefill_tc.cu), one build per head size.
 with numpy; it rides in the step's single metadata copy).  ``run`` picks the kernels: requests
 that bring exactly one token (they lead the batch) go to the split-key decode kernel; the
 others to the tcgen05 prefill kernel where it exists (head size 64 or 128, no window, pages of a
-multiple of 16 tokens), else to the mma.sync prefill kernel.  A mixed step therefore launches
+multiple of 16 tokens), else to the mma.sync prefill kernel; layers with options of their own have a tcgen05 kernel
+(csrc/attention_options_tc.cu) for the same sizes.  A mixed step therefore launches
 two attention kernels, each on its own rows.
 """
 
@@ -139,6 +140,19 @@ class TensorAttention:
 
         self.use_tma = 0 if os.environ.get("CIE_DECODE_TMA", "1") == "0" else 1
         self._prefill_tc = None
+        self._prompt_options = None
+
+    def load_options_kernel(self) -> None:
+        """Prompt portions of layers with options (``run_portions``) on tcgen05 where that kernel exists: key and value
+        heads of 64 or 128."""
+        from .ops import _Lib
+
+        v, i, f = c_void_p, c_int, c_float
+        if self._prompt_options is None and self.head_dim in (64, 128):
+            lib = _Lib(load_library("attention_options_tc.cu", {"HEAD_DIM": self.head_dim}))
+            self._prompt_options = lib.function(
+                "cie_attention_prompt_options",
+                [v, i, v, i, v, v, v, i, i, v, v, i, v, v, v, i, i, i, i, f, i, v, v, i, v, f, v, v, i, v, v])
 
     def load_prompt_kernel(self) -> None:
         """Prompt portions on tcgen05 where the kernel exists: head size 64 or 128, no window, pages of a multiple
@@ -338,8 +352,8 @@ class TensorAttention:
                      window: int, plan: dict[str, Any] | None, distance: Any, split_weights: bool,
                      keep_first: int = 0, sinks: Any = None, softcap: float = 0.0, slopes: Any = None,
                      gates: Any = None, key_dim: int | None = None, value_dim: int | None = None) -> None:
-        """The prompt portions of a step (every request after the leading single tokens) on the
-        mma.sync kernel, with the options the other kernels do not have: a distance penalty
+        """The prompt portions of a step (every request after the leading single tokens), on tcgen05 (key and value
+        heads of 64 or 128 alike, pages of a multiple of 16 tokens, split weights) or on the mma.sync kernel, with the options the other kernels do not have: a distance penalty
         (``distance``: float32 vectors r1, r2 per query head), softmax weights that enter the value
         product as two bfloat16 terms, a request's first ``keep_first`` keys visible behind the window, a
         sink term per query head in the softmax denominator (``sinks``: float32 [q_heads]), a soft cap on the scores,
@@ -355,6 +369,23 @@ class TensorAttention:
         ops._flush()
         ops.launches += 1
         r1, r2 = distance if distance is not None else (None, None)
+        # tables of up to 64 keys hold one tile of the mma.sync kernel, which is set up in less (64 tokens, 16 heads of 128:
+        # 14.7 us against 17.7; from 100 keys on the tcgen05 kernel is ahead)
+        if (self._prompt_options is not None and split_weights and kv.page_size % 16 == 0
+                and table.shape[1] * kv.page_size > 64
+                and (key_dim or self.head_dim) == (value_dim or self.head_dim) == self.head_dim
+                and qkv.shape[1] % 8 == 0 and out.shape[1] % 8 == 0
+                and (qkv.data_ptr() | out.data_ptr() | kv.k.data_ptr() | kv.v.data_ptr()) % 16 == 0):
+            pointer = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+            self._prompt_options(qkv.data_ptr(), qkv.shape[1], out.data_ptr(), out.shape[1], kv.k.data_ptr(),
+                                 kv.v.data_ptr(), table.data_ptr(), table.shape[1], kv.num_pages,
+                                 plan["tile_request"].data_ptr(), plan["tile_q0"].data_ptr(),
+                                 plan["tile_request"].shape[0], ctx.context_lens.data_ptr(), ctx.query_lens.data_ptr(),
+                                 ctx.query_start.data_ptr(), q_heads, kv_heads, kv.page_size, heads_per_tile(group),
+                                 scale, window, pointer(r1), pointer(r2), int(keep_first), pointer(sinks), float(softcap),
+                                 pointer(slopes), pointer(gates), 0 if gates is None else gates.stride(0),
+                                 ops.error_word.data_ptr(), ops.stream)
+            return
         self._prefill_ex(qkv.data_ptr(), qkv.shape[1], out.data_ptr(), out.shape[1], kv.k.data_ptr(),
                          kv.v.data_ptr(), table.data_ptr(), table.shape[1], kv.num_pages,
                          plan["tile_request"].data_ptr(), plan["tile_q0"].data_ptr(),

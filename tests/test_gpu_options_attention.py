@@ -1,0 +1,129 @@
+"""The tcgen05 kernel for prompt portions with options (windows, kept keys, penalties, caps, slopes, sinks, gates), against
+plain attention in 64 bits and against the mma.sync kernel, which computes the same for other sizes."""
+
+import math
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+OPTIONS = [
+    dict(),
+    dict(window=64, penalty=True),
+    dict(window=130, keep=3, sink=True),
+    dict(window=257, keep=140, gates=True, slopes=True),
+    dict(cap=5.0, sink=True, gates=True),
+    dict(window=1, keep=20),
+    dict(negative=True),
+]
+
+
+def rand(*shape, seed, scale=1.0):
+    generator = torch.Generator().manual_seed(seed)
+    return torch.randn(*shape, generator=generator) * scale
+
+
+def oracle(q, k, v, position, group, scale, o, heads):
+    """One token's rows [heads, dim] over keys [.., kv, dim] of positions 0 .. position."""
+    out = torch.empty(heads, v.shape[2], dtype=torch.float64)
+    gap = position - torch.arange(position + 1, dtype=torch.float64)
+    seen = torch.ones(position + 1, dtype=torch.bool)
+    if o.window:
+        seen = (gap < o.window) | (torch.arange(position + 1) < o.keep)
+    for h in range(heads):
+        s = (k[:position + 1, h // group] @ q[h]) * scale
+        if o.cap:
+            s = o.cap * torch.tanh(s / o.cap)
+        if o.slopes is not None:
+            s = s - o.slopes[h] * gap
+        if o.penalty is not None:
+            s = s - o.penalty[0][h] * torch.log1p(o.penalty[1][h] * gap)
+        s = s.masked_fill(~seen, -math.inf)
+        if o.sinks is not None:
+            s = torch.cat([s, o.sinks[h].double().view(1)])
+        out[h] = torch.softmax(s, 0)[:position + 1] @ v[:position + 1, h // group]
+    return out
+
+
+@pytest.mark.parametrize("dim,kv_heads,group,page", [(128, 2, 8, 16), (64, 1, 3, 48), (128, 1, 1, 256), (64, 2, 16, 128)])
+@pytest.mark.parametrize("option", range(len(OPTIONS)))
+def test_portions_with_options(option, dim, kv_heads, group, page):
+    """Requests that begin, that go on over a long context, that end at and beside tile edges, and a single token in
+    front; pages in descending order for some requests and in a row for others, gone where a window has left them behind.  A
+    weight enters as two bfloat16 terms and the result is rounded once: 2^-9 of a row's largest value, and as much again
+    for the exponentials' own error under the largest scores."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+    from cloud_inference_from_scratch_b200.native.tensor_attention import plan_tiles
+
+    ops = Runtime("cuda:0", "bfloat16").ops
+    ops.require_portion_attention(dim)
+    fast = ops._tensor_attention[dim]
+    assert fast._prompt_options is not None
+    asked = OPTIONS[option]
+    heads = kv_heads * group
+    lengths, contexts = [1, 40, 17, 2, 129], [5, 0, 300, 126, 511]
+    count, tokens = len(lengths), sum(lengths)
+    scale = (-1 if asked.get("negative") else 1) * dim ** -0.5
+    o = SimpleNamespace(window=asked.get("window", 0), keep=asked.get("keep", 0), cap=asked.get("cap", 0.0), slopes=None,
+                        penalty=None, sinks=None, gates=None)
+    if asked.get("slopes"):
+        o.slopes = torch.tensor([2.0 ** (-8.0 * (h + 1) / heads) for h in range(heads)])
+    if asked.get("penalty"):
+        o.penalty = (rand(heads, seed=1).abs(), rand(heads, seed=2).abs())
+    if asked.get("sink"):
+        o.sinks = rand(heads, seed=3)
+    if asked.get("gates"):
+        o.gates = rand(tokens, heads + 1, seed=4)
+    width = -(-max(c + n for c, n in zip(contexts, lengths)) // page)
+    table = torch.full((count, width), -1, dtype=torch.int32)
+    pools = [torch.full((count * width, kv_heads, page, dim), 100.0).bfloat16() for _ in range(2)]      # nobody's pages
+    keys, values = [], []
+    for r in range(count):
+        total = contexts[r] + lengths[r]
+        k, v = rand(total, kv_heads, dim, seed=10 + r, scale=1.5).bfloat16(), rand(total, kv_heads, dim, seed=20 + r).bfloat16()
+        keys.append(k.double()), values.append(v.double())
+        lowest = max(0, contexts[r] - o.window + 1) if o.window else 0
+        for index in range(-(-total // page)):
+            if (index + 1) * page <= lowest and index * page >= o.keep:
+                continue                                        # behind the window
+            table[r, index] = r * width + (index if r % 2 else width - 1 - index)
+            rows = slice(index * page, min((index + 1) * page, total))
+            for pool, source in zip(pools, (k, v)):
+                pool[table[r, index], :, :rows.stop - rows.start] = source[rows].transpose(0, 1)
+    q = rand(tokens, heads * dim, seed=6, scale=1.5).bfloat16()
+    starts = np.cumsum([0, *lengths]).astype(np.int32)
+    lens = np.asarray(lengths, dtype=np.int32)
+    as_int = lambda numbers: torch.tensor(numbers, dtype=torch.int32).cuda()  # noqa: E731
+    pools = [pool.cuda() for pool in pools]
+    kv = SimpleNamespace(group=0, k=pools[0], v=pools[1], num_pages=count * width, page_size=page)
+    ctx = SimpleNamespace(block_tables=[table.cuda()], context_lens=as_int(contexts), query_lens=as_int(lengths),
+                          query_start=torch.from_numpy(starts).cuda(), num_single=1, num_requests=count)
+    plan = {name: torch.from_numpy(array).cuda() for name, array in plan_tiles(lens, group, skip=1).items()}
+    device = lambda t: None if t is None else t.cuda()  # noqa: E731
+    gates, sinks, slopes = device(o.gates), device(o.sinks), device(o.slopes)
+    penalty = None if o.penalty is None else tuple(device(t) for t in o.penalty)
+    results = []
+    for kernel in (fast._prompt_options, None):
+        held, fast._prompt_options = fast._prompt_options, kernel
+        out = torch.full((tokens, heads * dim), 7.0, dtype=torch.bfloat16).cuda()
+        fast.run_portions(q.cuda(), out, ctx, kv, heads, kv_heads, scale, o.window, plan, penalty, True, keep_first=o.keep,
+                          sinks=sinks, softcap=o.cap, slopes=slopes, gates=None if gates is None else gates[:, 1:])
+        fast._prompt_options = held
+        ops.check_errors()
+        results.append(out.float().cpu())
+    assert float((results[0][0] - 7.0).abs().max()) == 0        # the single token is another kernel's
+    row = 0
+    for r in range(count):
+        for t in range(lengths[r]):
+            if r > 0 and (t < 2 or t > lengths[r] - 3 or t % 16 in (0, 15)):
+                want = oracle(q[row].double().view(heads, dim), keys[r], values[r], contexts[r] + t, group, scale, o, heads)
+                if o.gates is not None:
+                    want = want * torch.sigmoid(o.gates[row, 1:].double()).view(-1, 1)
+                got = results[0][row].view(heads, dim).double()
+                bound = 2.0 ** -8 * float(want.abs().max()) + 1e-6
+                assert float((got - want).abs().max()) <= bound, (r, t)
+            row += 1
+    assert torch.allclose(results[0], results[1], rtol=2.0 ** -7, atol=2.0 ** -8)
