@@ -24,6 +24,7 @@
 //
 // A request's result depends on its own tokens and state only: the batch and the slot change nothing, the cut
 // of a prompt into portions only the order of additions.
+#include "chunk_outputs.cuh"
 #include "common.cuh"
 
 CIE_DEFINE_LAST_ERROR()
@@ -240,15 +241,18 @@ gla_chunk_state_kernel(GlaRows in, float* __restrict__ chunk_state, float* __res
   }
 }
 
-// (2) grid: (requests, heads, blocks over dim * vdim)
+// (2) grid: (requests, heads, blocks over dim * vdim / V).  A thread walks V neighbouring cells of a state row: 16-byte
+// pieces where rows are whole ones (V = 4), and one decay for all of them.
+template <int V>
 __global__ void gla_chunk_prefix_kernel(float* __restrict__ chunk_state, const float* __restrict__ chunk_decay,
                                         float* __restrict__ state, const int* __restrict__ request_chunk_start,
                                         const int* __restrict__ slots, const int* __restrict__ request_active,
                                         int heads, int dim, int vdim, int max_slots, int* err) {
+  struct __align__(4 * V) Cells { float v[V]; };
   pdl_wait();
   pdl_trigger();
   const int request = blockIdx.x, head = blockIdx.y;
-  const int e = blockIdx.z * blockDim.x + threadIdx.x;
+  const int e = (blockIdx.z * blockDim.x + threadIdx.x) * V;
   if (e >= dim * vdim) return;
   const int slot = slots[request];
   if (slot < 0 || slot >= max_slots) {
@@ -256,8 +260,8 @@ __global__ void gla_chunk_prefix_kernel(float* __restrict__ chunk_state, const f
     return;
   }
   const int d = e / vdim;
-  float* cell = state + ((size_t)slot * heads + head) * dim * vdim + e;
-  float s = *cell;
+  Cells* cell = reinterpret_cast<Cells*>(state + ((size_t)slot * heads + head) * dim * vdim + e);
+  Cells s = *cell;
   const size_t stride = (size_t)heads * dim * vdim, decay_stride = (size_t)heads * dim;
   const int last = request_chunk_start[request + 1];
   // eight chunks at a time: their sums are asked for together, before the first store, so that the walk waits
@@ -266,18 +270,21 @@ __global__ void gla_chunk_prefix_kernel(float* __restrict__ chunk_state, const f
   for (int chunk = request_chunk_start[request]; chunk < last; chunk += kBatch) {
     float* u = chunk_state + ((size_t)chunk * heads + head) * dim * vdim + e;
     const float* b = chunk_decay + ((size_t)chunk * heads + head) * dim + d;
-    float gained[kBatch], power[kBatch];
+    Cells gained[kBatch];
+    float power[kBatch];
 #pragma unroll
     for (int x = 0; x < kBatch; ++x) {
-      const bool in = chunk + x < last;
-      gained[x] = in ? u[x * stride] : 0.f;
-      power[x] = in ? b[x * decay_stride] : 1.f;
+      if (chunk + x < last) {
+        gained[x] = *reinterpret_cast<const Cells*>(u + x * stride);
+        power[x] = b[x * decay_stride];
+      }
     }
 #pragma unroll
     for (int x = 0; x < kBatch; ++x) {
       if (chunk + x < last) {
-        u[x * stride] = s;
-        s = fmaf(power[x], s, gained[x]);
+        *reinterpret_cast<Cells*>(u + x * stride) = s;
+#pragma unroll
+        for (int c = 0; c < V; ++c) s.v[c] = fmaf(power[x], s.v[c], gained[x].v[c]);
       }
     }
   }
@@ -285,112 +292,81 @@ __global__ void gla_chunk_prefix_kernel(float* __restrict__ chunk_state, const f
 }
 
 // (3) outputs of a chunk from the state before it and the chunk's own tokens
-__global__ void __launch_bounds__(kScanWarps * 32)
+__global__ void __launch_bounds__(kOutThreads)
 gla_chunk_output_kernel(GlaRows in, float* __restrict__ out, int out_stride, const float* __restrict__ chunk_state,
                         const int* __restrict__ chunk_row, const int* __restrict__ chunk_count, int heads, int dim,
                         int vdim) {
+  static_assert(kChunk == kOutTokens, "chunks of the outputs' size");
   extern __shared__ __align__(16) float smem[];
-  const int ld = dim + 1;                         // rows that lanes walk side by side are padded by one element
-  float* q_s = smem;                              // [kChunk][dim]
-  float* v_s = q_s + kChunk * dim;                // [kChunk][vdim]
-  float* k_s = v_s + kChunk * vdim;               // [kChunk][dim + 1]
-  float* b_s = k_s + kChunk * ld;                 // [kChunk][dim + 1]
-  float* a_s = b_s + kChunk * ld;                 // [kChunk][kChunk]
+  const int ld = pad4(dim), vld = pad4(vdim);
+  float* q_s = smem;                              // [kChunk][ld]
+  float* k_s = q_s + kChunk * ld;
+  float* b_s = k_s + kChunk * ld;
+  float* v_s = b_s + kChunk * ld;                 // [kChunk][vld]
+  float* a_s = v_s + kChunk * vld;                // [kChunk][kOutWeights]
   pdl_wait();
   pdl_trigger();
   const int chunk = blockIdx.x, head = blockIdx.y;
   const int row0 = chunk_row[chunk], n = chunk_count[chunk];
-  stage_rows(q_s, dim, in.proj, in.proj_stride, row0, n, in.q_off + head * dim, dim, in.q_scale);
+  const StateRing ring{a_s + kChunk * kOutWeights, chunk_state + ((size_t)chunk * heads + head) * dim * vdim, dim, vdim};
+  ring.issue(0);
+  stage_rows(q_s, ld, in.proj, in.proj_stride, row0, n, in.q_off + head * dim, dim, in.q_scale);
   stage_rows(k_s, ld, in.proj, in.proj_stride, row0, n, in.k_off + head * dim, dim, 1.f);
-  stage_rows(v_s, vdim, in.proj, in.proj_stride, row0, n, in.v_off + head * vdim, vdim, 1.f);
+  stage_rows(v_s, vld, in.proj, in.proj_stride, row0, n, in.v_off + head * vdim, vdim, 1.f);
   // the sums in units of log 2: every exponential below is one exp2
   stage_rows(b_s, ld, in.z, in.z_stride, row0, n, head * dim, dim, 1.4426950408889634f);
-  __syncthreads();
-  // a[i][j] = sum_d q_i[d] k_j[d] exp(b_i[d] - b_j[d]) for j <= i.  Only those pairs are dealt out: pair p is
-  // (i, j) with p = i (i + 1) / 2 + j, so neighbouring lanes mostly share i and walk neighbouring rows j
-  const int pairs = n * (n + 1) / 2;
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    int i = (int)((sqrtf(8.f * (float)p + 1.f) - 1.f) * 0.5f);
-    while (i * (i + 1) / 2 > p) --i;
-    while ((i + 1) * (i + 2) / 2 <= p) ++i;
-    const int j = p - i * (i + 1) / 2;
-    const float* qi = q_s + i * dim;
-    const float* bi = b_s + i * ld;
-    const float* kj = k_s + j * ld;
-    const float* bj = b_s + j * ld;
-    float dot = 0.f, dot2 = 0.f;       // two chains
-    int x = 0;
-    for (; x + 2 <= dim; x += 2) {
-      dot = fmaf(qi[x] * kj[x], exp2f(bi[x] - bj[x]), dot);
-      dot2 = fmaf(qi[x + 1] * kj[x + 1], exp2f(bi[x + 1] - bj[x + 1]), dot2);
+  if (ld != dim)
+    for (int e = threadIdx.x; e < kChunk * (ld - dim); e += kOutThreads) {
+      const int at = e / (ld - dim) * ld + dim + e % (ld - dim);
+      q_s[at] = k_s[at] = b_s[at] = 0.f;
     }
-    if (x < dim) dot = fmaf(qi[x] * kj[x], exp2f(bi[x] - bj[x]), dot);
-    a_s[i * kChunk + j] = dot + dot2;
+  __syncthreads();
+  // a[i][j] = sum_d q_i[d] k_j[d] exp(b_i[d] - b_j[d]) for j <= i: eight lanes share two rows i and two rows j, a lane the
+  // 16-byte pieces lane, lane + 8, ..; one load from shared memory for two products and one exponential
+  const int lane8 = threadIdx.x & 7, blocks = (n + 1) / 2;
+  for (int p = threadIdx.x >> 3; p < blocks * (blocks + 1) / 2; p += kOutThreads / 8) {
+    int bi = (int)((sqrtf(8.f * (float)p + 1.f) - 1.f) * 0.5f);
+    while (bi * (bi + 1) / 2 > p) --bi;
+    while ((bi + 1) * (bi + 2) / 2 <= p) ++bi;
+    const int i = 2 * bi, j = 2 * (p - bi * (bi + 1) / 2);
+    float dot[2][2] = {};
+    for (int x = lane8 * 4; x < ld; x += 32) {
+      float q[2][4], bq[2][4], k[2][4], bk[2][4];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        *reinterpret_cast<float4*>(q[r]) = *reinterpret_cast<const float4*>(q_s + (i + r) * ld + x);
+        *reinterpret_cast<float4*>(bq[r]) = *reinterpret_cast<const float4*>(b_s + (i + r) * ld + x);
+        *reinterpret_cast<float4*>(k[r]) = *reinterpret_cast<const float4*>(k_s + (j + r) * ld + x);
+        *reinterpret_cast<float4*>(bk[r]) = *reinterpret_cast<const float4*>(b_s + (j + r) * ld + x);
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int y = 0; y < 4; ++y) dot[r][c] = fmaf(q[r][y] * k[c][y], exp2f(bq[r][y] - bk[c][y]), dot[r][c]);
+    }
+    const unsigned mine = 0xffu << (threadIdx.x & 24);      // the eight lanes: others of the warp may have no block left
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        float total = dot[r][c];
+        total += __shfl_xor_sync(mine, total, 1);
+        total += __shfl_xor_sync(mine, total, 2);
+        total += __shfl_xor_sync(mine, total, 4);
+        if (lane8 == 0 && j + c <= i + r) a_s[(j + c) * kOutWeights + i + r] = total;
+      }
   }
   __syncthreads();
   // what the carried state is read with: q_i * exp(b_i)
-  for (int e = threadIdx.x; e < n * dim; e += blockDim.x) {
-    const int i = e / dim, x = e % dim;
-    q_s[e] *= exp2f(b_s[i * ld + x]);
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float* before = chunk_state + ((size_t)chunk * heads + head) * dim * vdim;
-  // a warp takes tokens warp, warp + 8, ...; a lane the value columns lane, lane + 32, ...
-  constexpr int kTokens = kChunk / kScanWarps;
-  float acc[kTokens][kChunkCols] = {};
-  const int dim4 = dim % 4 == 0 ? dim : 0;       // four state rows a step where the q rows allow 16-byte loads
-  for (int x = 0; x < dim4; x += 4) {
-    float sv[4][kChunkCols];
-#pragma unroll
-    for (int y = 0; y < 4; ++y)
-#pragma unroll
-      for (int c = 0; c < kChunkCols; ++c) sv[y][c] = lane + 32 * c < vdim ? before[(size_t)(x + y) * vdim + lane + 32 * c] : 0.f;
-#pragma unroll
-    for (int t = 0; t < kTokens; ++t) {
-      const int i = warp + kScanWarps * t;
-      const float4 q4 = i < n ? *reinterpret_cast<const float4*>(q_s + i * dim + x) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int c = 0; c < kChunkCols; ++c) {
-        acc[t][c] = fmaf(q4.x, sv[0][c], acc[t][c]);
-        acc[t][c] = fmaf(q4.y, sv[1][c], acc[t][c]);
-        acc[t][c] = fmaf(q4.z, sv[2][c], acc[t][c]);
-        acc[t][c] = fmaf(q4.w, sv[3][c], acc[t][c]);
-      }
-    }
-  }
-  for (int x = dim4; x < dim; ++x) {
-    float sv[kChunkCols];
-#pragma unroll
-    for (int c = 0; c < kChunkCols; ++c) sv[c] = lane + 32 * c < vdim ? before[(size_t)x * vdim + lane + 32 * c] : 0.f;
-#pragma unroll
-    for (int t = 0; t < kTokens; ++t) {
-      const int i = warp + kScanWarps * t;
-      const float qv = i < n ? q_s[i * dim + x] : 0.f;
-#pragma unroll
-      for (int c = 0; c < kChunkCols; ++c) acc[t][c] = fmaf(qv, sv[c], acc[t][c]);
-    }
-  }
-  for (int j = 0; j < n; ++j) {
-    float vv[kChunkCols];
-#pragma unroll
-    for (int c = 0; c < kChunkCols; ++c) vv[c] = lane + 32 * c < vdim ? v_s[j * vdim + lane + 32 * c] : 0.f;
-#pragma unroll
-    for (int t = 0; t < kTokens; ++t) {
-      const int i = warp + kScanWarps * t;
-      const float av = (i < n && j <= i) ? a_s[i * kChunk + j] : 0.f;
-#pragma unroll
-      for (int c = 0; c < kChunkCols; ++c) acc[t][c] = fmaf(av, vv[c], acc[t][c]);
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < kTokens; ++t) {
-    const int i = warp + kScanWarps * t;
-    if (i >= n) continue;
-#pragma unroll
-    for (int c = 0; c < kChunkCols; ++c)
-      if (lane + 32 * c < vdim) out[(size_t)(row0 + i) * out_stride + head * vdim + lane + 32 * c] = acc[t][c];
-  }
+  for (int e = threadIdx.x; e < n * ld; e += kOutThreads) q_s[e] *= exp2f(b_s[e]);
+  // (chunk_outputs meets before it reads)
+  float* dst = out + (size_t)row0 * out_stride + head * vdim;
+  const bool wide = vdim % 4 == 0 && out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+  chunk_outputs(ring, q_s, ld, a_s, v_s, [&](int t, int c, const float4& o) {
+    if (t < n) store4(dst + (size_t)t * out_stride, c, vdim, o, wide);
+  });
 }
 
 }  // namespace cie
@@ -441,25 +417,33 @@ extern "C" int cie_gla_chunked(const float* proj, int proj_stride, int q_off, in
     CIE_FAIL("gla_chunked: key / value sizes %d / %d are above %d", dim, vdim, kChunkDim);
   cudaStream_t s = (cudaStream_t)stream;
   const size_t smem1 = (size_t)kChunk * (dim + vdim) * sizeof(float);
-  const size_t smem3 = (size_t)kChunk * (dim + vdim + 2 * (dim + 1) + kChunk) * sizeof(float);
+  const size_t smem3 = ((size_t)kChunk * (3 * pad4(dim) + pad4(vdim) + kOutWeights) + out_ring_floats(vdim)) * sizeof(float);
   static bool raised = false;
   if (!raised) {
     if (cudaFuncSetAttribute(gla_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
-        cudaFuncSetAttribute(gla_chunk_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024) != cudaSuccess)
+        cudaFuncSetAttribute(gla_chunk_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 104 * 1024) != cudaSuccess)
       CIE_FAIL("gla_chunked: cannot raise the shared memory limit");
     raised = true;
   }
   dim3 grid(chunks, heads), block(kScanWarps * 32);
-  dim3 grid2(requests, heads, (dim * vdim + 255) / 256);
+  // a state row of whole 16-byte pieces is walked in them
+  const bool pieces = vdim % 4 == 0 && ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(chunk_state)) & 15) == 0;
+  const int cells = pieces ? dim * vdim / 4 : dim * vdim;
+  dim3 grid2(requests, heads, (cells + 127) / 128);
   int sum_threads = 32;
   while (sum_threads < dim) sum_threads <<= 1;
   CIE_LAUNCH("gla_decay_sums", gla_decay_sums_kernel, grid, dim3(sum_threads), 0, s, z, z_stride, z_bias, inv_tau,
              chunk_row, chunk_count, dim);
   CIE_LAUNCH("gla_chunk_state", gla_chunk_state_kernel, grid, block, smem1, s, in, chunk_state, chunk_decay, chunk_row,
              chunk_count, heads, dim, vdim);
-  CIE_LAUNCH("gla_chunk_prefix", gla_chunk_prefix_kernel, grid2, dim3(256), 0, s, chunk_state,
-             (const float*)chunk_decay, state, request_chunk_start, slots, request_active, heads, dim, vdim,
-             max_slots, err);
+  if (pieces)
+    CIE_LAUNCH("gla_chunk_prefix", gla_chunk_prefix_kernel<4>, grid2, dim3(128), 0, s, chunk_state,
+               (const float*)chunk_decay, state, request_chunk_start, slots, request_active, heads, dim, vdim,
+               max_slots, err);
+  else
+    CIE_LAUNCH("gla_chunk_prefix", gla_chunk_prefix_kernel<1>, grid2, dim3(128), 0, s, chunk_state,
+               (const float*)chunk_decay, state, request_chunk_start, slots, request_active, heads, dim, vdim,
+               max_slots, err);
   CIE_LAUNCH("gla_chunk_output", gla_chunk_output_kernel, grid, block, smem3, s, in, out, out_stride,
              (const float*)chunk_state, chunk_row, chunk_count, heads, dim, vdim);
   return 0;

@@ -27,6 +27,7 @@
 // A last kernel divides every head of a scan's output by its own root mean square, multiplies by a gain
 // (one number per column, or a vector of a head's size shared by the heads) and by sigmoid or SiLU of a
 // gate, and rounds once.
+#include "chunk_outputs.cuh"
 #include "common.cuh"
 
 CIE_DEFINE_LAST_ERROR()
@@ -903,24 +904,35 @@ struct RowsOf {
   int stride, col0, head_col;
 };
 
+// Rows of q and k are `key_row(dim)` floats long: the rows that a load of eight lanes meets then lie in different banks.
+__host__ __device__ __forceinline__ int key_row(int dim) { return pad4(dim) % 8 == 0 ? pad4(dim) + 4 : pad4(dim); }
+static size_t chunk_output_smem(int dim, int vdim) {
+  return ((size_t)kMemChunk * (2 * key_row(dim) + pad4(vdim) + kOutWeights) + out_ring_floats(vdim)) * sizeof(float);
+}
+
 template <bool kMemory>
-__global__ void __launch_bounds__(kMemWarps * 32)
+__global__ void __launch_bounds__(kOutThreads)
 chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
                     const float* __restrict__ gates, const float* __restrict__ chunk_sums,
                     float* __restrict__ out, int out_stride, const int* __restrict__ chunk_row,
                     const int* __restrict__ chunk_count, int heads, int dim, int vdim) {
+  static_assert(kMemChunk == kOutTokens && kMemWarps * 32 == kOutThreads, "chunks of the outputs' size");
   extern __shared__ __align__(16) float smem[];
-  const int kd = dim + 1;                         // k rows are padded by one element: lanes run over keys
-  float* q_s = smem;                              // [kMemChunk][dim]
-  float* v_s = q_s + kMemChunk * dim;             // [kMemChunk][vdim]
-  float* a_s = v_s + kMemChunk * vdim;            // [kMemChunk][kMemChunk]
-  float* k_s = a_s + kMemChunk * kMemChunk;       // [kMemChunk][dim + 1]
-  __shared__ float gi_s[kMemChunk], gb_s[kMemChunk], gm_s[kMemChunk];
+  const int ld = key_row(dim), padded = pad4(dim), vld = pad4(vdim);
+  float* q_s = smem;                              // [kMemChunk][ld]
+  float* k_s = q_s + kMemChunk * ld;
+  float* v_s = k_s + kMemChunk * ld;              // [kMemChunk][vld]
+  float* a_s = v_s + kMemChunk * vld;             // [kMemChunk][kOutWeights]
+  __shared__ float gi_s[kMemChunk], gb_s[kMemChunk], gm_s[kMemChunk], below_s[kMemChunk];
   __shared__ float m_before;
   pdl_wait();
   pdl_trigger();
   const int chunk = blockIdx.x, head = blockIdx.y;
   const int row0 = chunk_row[chunk], n = chunk_count[chunk];
+  const size_t cells = (size_t)dim * vdim + (kMemory ? dim : 0);
+  const float* before = chunk_sums + ((size_t)chunk * heads + head) * cells;
+  const StateRing ring{a_s + kMemChunk * kOutWeights, before, dim, vdim};
+  ring.issue(0);
   if (threadIdx.x < n) {
     const float4 g = *reinterpret_cast<const float4*>(gates + ((size_t)(row0 + threadIdx.x) * heads + head) * kMemGates);
     gi_s[threadIdx.x] = g.x;
@@ -928,120 +940,76 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
     gm_s[threadIdx.x] = g.z;
     if (threadIdx.x == 0) m_before = g.w;
   }
-  stage_rows(q_s, dim, q_rows.base + head * q_rows.head_base, q_rows.stride, row0, n, q_rows.col0 + head * q_rows.head_col,
+  stage_rows(q_s, ld, q_rows.base + head * q_rows.head_base, q_rows.stride, row0, n, q_rows.col0 + head * q_rows.head_col,
              dim, [&](int) { return q_scale; });
-  stage_rows(k_s, kd, k_rows.base + head * k_rows.head_base, k_rows.stride, row0, n, k_rows.col0 + head * k_rows.head_col,
+  stage_rows(k_s, ld, k_rows.base + head * k_rows.head_base, k_rows.stride, row0, n, k_rows.col0 + head * k_rows.head_col,
              dim, [](int) { return 1.f; });
-  stage_rows(v_s, vdim, v_rows.base + head * v_rows.head_base, v_rows.stride, row0, n, v_rows.col0 + head * v_rows.head_col,
+  stage_rows(v_s, vld, v_rows.base + head * v_rows.head_base, v_rows.stride, row0, n, v_rows.col0 + head * v_rows.head_col,
              vdim, [](int) { return 1.f; });
+  if (padded != dim)
+    for (int e = threadIdx.x; e < kMemChunk * (padded - dim); e += kOutThreads) {
+      const int at = e / (padded - dim) * ld + dim + e % (padded - dim);
+      q_s[at] = k_s[at] = 0.f;
+    }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   {
-    // a warp takes four tokens that follow each other, a lane a key: a key's numbers are read once for four products
-    constexpr int kQ = kMemChunk / kMemWarps;
-    const int i0 = warp * kQ, j = lane;
-    float dot[kQ] = {};
-    if (i0 < n && j < n && j < i0 + kQ) {
-      const int whole = dim % 4 == 0 ? dim : 0;
-      for (int x = 0; x < whole; x += 4) {
-        const float k0 = k_s[j * kd + x], k1 = k_s[j * kd + x + 1], k2 = k_s[j * kd + x + 2], k3 = k_s[j * kd + x + 3];
+    // the weights: a warp takes four tokens t, four lanes share four tokens s and take every fourth 16-byte piece
+    const int t0 = warp * 4, s0 = (lane >> 2) * 4, part = lane & 3;
+    float dot[4][4] = {};
+    if (s0 <= t0 + 3) {
+      for (int x = part * 4; x < padded; x += 16) {
+        float4 qv[4];
 #pragma unroll
-        for (int t = 0; t < kQ; ++t) {
-          if (i0 + t >= n) break;
-          const float4 q4 = *reinterpret_cast<const float4*>(q_s + (i0 + t) * dim + x);
-          dot[t] = fmaf(q4.x, k0, dot[t]);
-          dot[t] = fmaf(q4.y, k1, dot[t]);
-          dot[t] = fmaf(q4.z, k2, dot[t]);
-          dot[t] = fmaf(q4.w, k3, dot[t]);
+        for (int i = 0; i < 4; ++i) qv[i] = *reinterpret_cast<const float4*>(q_s + (t0 + i) * ld + x);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 kv = *reinterpret_cast<const float4*>(k_s + (s0 + j) * ld + x);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            dot[i][j] = fmaf(qv[i].x, kv.x, dot[i][j]);
+            dot[i][j] = fmaf(qv[i].y, kv.y, dot[i][j]);
+            dot[i][j] = fmaf(qv[i].z, kv.z, dot[i][j]);
+            dot[i][j] = fmaf(qv[i].w, kv.w, dot[i][j]);
+          }
         }
       }
-      for (int x = whole; x < dim; ++x) {
-        const float kx = k_s[j * kd + x];
+    }
 #pragma unroll
-        for (int t = 0; t < kQ; ++t)
-          if (i0 + t < n) dot[t] = fmaf(q_s[(i0 + t) * dim + x], kx, dot[t]);
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float total = dot[i][j];
+        total += __shfl_xor_sync(0xffffffffu, total, 1);
+        total += __shfl_xor_sync(0xffffffffu, total, 2);
+        const int t = t0 + i, s = s0 + j;
+        if (part == j && t < n && s <= t)
+          a_s[s * kOutWeights + t] = total * expf(gb_s[t] - gb_s[s] + gi_s[s] - gm_s[t]);
       }
-    }
-#pragma unroll
-    for (int t = 0; t < kQ; ++t) {
-      const int i = i0 + t;
-      a_s[i * kMemChunk + j] = (i < n && j <= i) ? dot[t] * expf(gb_s[i] - gb_s[j] + gi_s[j] - gm_s[i]) : 0.f;
-    }
   }
   __syncthreads();
-  const size_t cells = (size_t)dim * vdim + (kMemory ? dim : 0);
-  const float* before = chunk_sums + ((size_t)chunk * heads + head) * cells;
-  const float* n_before = before + (size_t)dim * vdim;
-  // a warp takes tokens warp, warp + 8, ...; a lane the value columns lane, lane + 32, ...
-  constexpr int kTokens = kMemChunk / kMemWarps;
-  float carried[kTokens], below[kTokens];
-#pragma unroll
-  for (int t = 0; t < kTokens; ++t) {
-    const int i = warp + kMemWarps * t;
-    carried[t] = 0.f;
-    below[t] = 1.f;
-    if (i >= n) continue;
-    carried[t] = expf(gb_s[i] + m_before - gm_s[i]);
-    if (!kMemory) continue;
-    float nq = 0.f;
-    for (int x = lane; x < dim; x += 32) nq = fmaf(n_before[x], q_s[i * dim + x], nq);
-    nq = warp_sum(nq) * carried[t] + warp_sum(lane <= i ? a_s[i * kMemChunk + lane] : 0.f);
-    below[t] = fmaxf(fabsf(nq), expf(-gm_s[i])) + 1e-6f;
-  }
-  float inter[kTokens][kMemCols] = {}, intra[kTokens][kMemCols] = {};
-  const int dim4 = dim % 4 == 0 ? dim : 0;       // four state rows a step where the q rows allow 16-byte loads
-  for (int x = 0; x < dim4; x += 4) {
-    float sv[4][kMemCols];
-#pragma unroll
-    for (int y = 0; y < 4; ++y)
-#pragma unroll
-      for (int c = 0; c < kMemCols; ++c) sv[y][c] = lane + 32 * c < vdim ? before[(size_t)(x + y) * vdim + lane + 32 * c] : 0.f;
-#pragma unroll
-    for (int t = 0; t < kTokens; ++t) {
-      const int i = warp + kMemWarps * t;
-      const float4 q4 = i < n ? *reinterpret_cast<const float4*>(q_s + i * dim + x) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int c = 0; c < kMemCols; ++c) {
-        inter[t][c] = fmaf(q4.x, sv[0][c], inter[t][c]);
-        inter[t][c] = fmaf(q4.y, sv[1][c], inter[t][c]);
-        inter[t][c] = fmaf(q4.z, sv[2][c], inter[t][c]);
-        inter[t][c] = fmaf(q4.w, sv[3][c], inter[t][c]);
-      }
+  // what the carried state is read with; the matrix memory's denominators
+  for (int t = warp; t < n; t += kMemWarps) {
+    const float carried = expf(gb_s[t] + m_before - gm_s[t]);
+    if (kMemory) {
+      float nq = 0.f;
+      for (int x = lane; x < dim; x += 32) nq = fmaf(before[(size_t)dim * vdim + x], q_s[t * ld + x], nq);
+      nq = warp_sum(nq) * carried + warp_sum(lane <= t ? a_s[lane * kOutWeights + t] : 0.f);
+      if (lane == 0) below_s[t] = fmaxf(fabsf(nq), expf(-gm_s[t])) + 1e-6f;
     }
+    for (int x = lane; x < padded; x += 32) q_s[t * ld + x] *= carried;
   }
-  for (int x = dim4; x < dim; ++x) {
-    float sv[kMemCols];
-#pragma unroll
-    for (int c = 0; c < kMemCols; ++c) sv[c] = lane + 32 * c < vdim ? before[(size_t)x * vdim + lane + 32 * c] : 0.f;
-#pragma unroll
-    for (int t = 0; t < kTokens; ++t) {
-      const int i = warp + kMemWarps * t;
-      const float qv = i < n ? q_s[i * dim + x] : 0.f;
-#pragma unroll
-      for (int c = 0; c < kMemCols; ++c) inter[t][c] = fmaf(qv, sv[c], inter[t][c]);
+  // (chunk_outputs meets before it reads)
+  float* dst = out + (size_t)row0 * out_stride + head * vdim;
+  const bool wide = vdim % 4 == 0 && out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+  chunk_outputs(ring, q_s, ld, a_s, v_s, [&](int t, int c, float4 o) {
+    if (t >= n) return;
+    if (kMemory) {
+      const float below = below_s[t];
+      o = make_float4(o.x / below, o.y / below, o.z / below, o.w / below);
     }
-  }
-  for (int j = 0; j < n; ++j) {
-    float vv[kMemCols];
-#pragma unroll
-    for (int c = 0; c < kMemCols; ++c) vv[c] = lane + 32 * c < vdim ? v_s[j * vdim + lane + 32 * c] : 0.f;
-#pragma unroll
-    for (int t = 0; t < kTokens; ++t) {
-      const int i = warp + kMemWarps * t;
-      const float av = (i < n && j <= i) ? a_s[i * kMemChunk + j] : 0.f;
-#pragma unroll
-      for (int c = 0; c < kMemCols; ++c) intra[t][c] = fmaf(av, vv[c], intra[t][c]);
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < kTokens; ++t) {
-    const int i = warp + kMemWarps * t;
-    if (i >= n) continue;
-#pragma unroll
-    for (int c = 0; c < kMemCols; ++c)
-      if (lane + 32 * c < vdim)
-        out[(size_t)(row0 + i) * out_stride + head * vdim + lane + 32 * c] = fmaf(carried[t], inter[t][c], intra[t][c]) / below[t];
-  }
+    store4(dst + (size_t)t * out_stride, c, vdim, o, wide);
+  });
 }
 
 // ---------------------------------------------------------------- gated delta rule over prompt portions, in chunks
@@ -1363,7 +1331,7 @@ extern "C" int cie_mlstm_chunked(const float* proj, int proj_stride, int q_off, 
   float* gates = scratch;
   float* sums = scratch + (size_t)tokens * heads * kMemGates;
   const size_t smem2 = (size_t)kMemChunk * (dim + vdim) * sizeof(float);
-  const size_t smem4 = (size_t)kMemChunk * (2 * dim + 1 + vdim + kMemChunk) * sizeof(float);
+  const size_t smem4 = chunk_output_smem(dim, vdim);
   if (smem4 > 48 * 1024 && cudaFuncSetAttribute(chunk_output_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 (int)smem4) != cudaSuccess)
     CIE_FAIL("mlstm_chunked: cannot reserve %zu bytes of shared memory", smem4);
@@ -1415,7 +1383,7 @@ extern "C" int cie_gated_delta_chunked(const float* conv, int conv_stride, int q
   const size_t smem2 = (size_t)(kMemChunk * (vdim + P + 1) + 2 * kMemChunk * (kMemChunk + 1)) * sizeof(float);
   const size_t smem3 = (size_t)(2 * (2 * kMemChunk * P + kMemChunk * kWalkColumns + kMemChunk * kMemGates) +
                                 (kWalkWarps + 1) * kMemChunk * kWalkColumns) * sizeof(float);
-  const size_t smem4 = (size_t)kMemChunk * (2 * dim + 1 + vdim + kMemChunk) * sizeof(float);
+  const size_t smem4 = chunk_output_smem(dim, vdim);
   if (cudaFuncSetAttribute(delta_chunk_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess ||
       cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) != cudaSuccess ||
       cudaFuncSetAttribute(chunk_output_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4) != cudaSuccess)
