@@ -17,6 +17,7 @@
 // A request's result depends on its own tokens and state only: the batch, the cut of a prompt into
 // portions and the slot do not change the order of a single addition.
 #include "common.cuh"
+#include "head_gate.cuh"
 
 CIE_DEFINE_LAST_ERROR()
 
@@ -624,26 +625,6 @@ delta_walk_kernel(const float* __restrict__ cells, float* __restrict__ out, int 
     }
 }
 
-// out[t, g * size + i] = gain[g * size + i] * o[t, g, i] / sqrt(mean_i(o[t, g, :]^2) + eps) * sigmoid(gate[t, g * size + i])
-// grid (tokens, groups), one warp.
-template <typename T>
-__global__ void __launch_bounds__(32)
-group_gate_norm_kernel(const float* __restrict__ o, int o_stride, const float* __restrict__ gate, int gate_stride,
-                       const float* __restrict__ gain, T* __restrict__ out, int out_stride, int size, float eps) {
-  pdl_wait();
-  pdl_trigger();
-  const int t = blockIdx.x, g = blockIdx.y, lane = threadIdx.x;
-  const float* row = o + (size_t)t * o_stride + (size_t)g * size;
-  float sq = 0.f;
-  for (int i = lane; i < size; i += 32) sq = fmaf(row[i], row[i], sq);
-  const float inv = rsqrtf(warp_sum(sq) / (float)size + eps);
-  for (int i = lane; i < size; i += 32) {
-    const int c = g * size + i;
-    const float z = gate[(size_t)t * gate_stride + c];
-    out[(size_t)t * out_stride + c] = from_float<T>(gain[c] * (row[i] * inv) * sigmoid_f(z));
-  }
-}
-
 }  // namespace cie
 
 #define DISPATCH_DTYPE(code, name, ...)                              \
@@ -773,9 +754,11 @@ extern "C" int cie_group_gate_norm(const float* o, int o_stride, const float* ga
   using namespace cie;
   if (tokens <= 0 || groups <= 0) return 0;
   if (groups > 65535) CIE_FAIL("group_gate_norm: too many groups");
-  DISPATCH_DTYPE(dtype, "group_gate_norm", {
-    CIE_LAUNCH("group_gate_norm", group_gate_norm_kernel<T>, dim3(tokens, groups), dim3(32), 0, (cudaStream_t)stream,
-               o, o_stride, gate, gate_stride, gain, (T*)out, out_stride, size, eps);
-  })
+  const HeadGate a{o, o_stride, nullptr, gate, gate_stride, gain, 0, 0, out_stride, groups, size, eps};
+  cudaError_t status;
+  if (dtype == kFloat32) status = launch_head_gate(a, (float*)out, tokens, (cudaStream_t)stream);
+  else if (dtype == kBFloat16) status = launch_head_gate(a, (__nv_bfloat16*)out, tokens, (cudaStream_t)stream);
+  else CIE_FAIL("group_gate_norm: unknown dtype code %d", dtype);
+  if (status != cudaSuccess) CIE_FAIL("group_gate_norm: launch failed: %s", cudaGetErrorString(status));
   return 0;
 }

@@ -29,6 +29,7 @@
 // gate, and rounds once.
 #include "chunk_outputs.cuh"
 #include "common.cuh"
+#include "head_gate.cuh"
 
 CIE_DEFINE_LAST_ERROR()
 
@@ -1512,15 +1513,11 @@ extern "C" int cie_head_norm_gate(const float* o, int o_stride, const float* den
   if (tokens <= 0 || groups <= 0) return 0;
   if (groups > 65535) CIE_FAIL("head_norm_gate: too many heads");
   if (act < 0 || act > 1) CIE_FAIL("head_norm_gate: unknown gate activation %d", act);
-  if (dtype == kFloat32) {
-    CIE_LAUNCH("head_norm_gate", head_norm_gate_kernel<float>, dim3(tokens, groups), dim3(32), 0, (cudaStream_t)stream,
-               o, o_stride, denominators, gate, gate_stride, gain, gain_shared, act, (float*)out, out_stride, size, eps);
-  } else if (dtype == kBFloat16) {
-    CIE_LAUNCH("head_norm_gate", head_norm_gate_kernel<__nv_bfloat16>, dim3(tokens, groups), dim3(32), 0,
-               (cudaStream_t)stream, o, o_stride, denominators, gate, gate_stride, gain, gain_shared, act, (__nv_bfloat16*)out,
-               out_stride, size, eps);
-  } else {
-    CIE_FAIL("head_norm_gate: unknown dtype code %d", dtype);
-  }
+  const HeadGate a{o, o_stride, denominators, gate, gate_stride, gain, gain_shared, act, out_stride, groups, size, eps};
+  cudaError_t status;
+  if (dtype == kFloat32) status = launch_head_gate(a, (float*)out, tokens, (cudaStream_t)stream);
+  else if (dtype == kBFloat16) status = launch_head_gate(a, (__nv_bfloat16*)out, tokens, (cudaStream_t)stream);
+  else CIE_FAIL("head_norm_gate: unknown dtype code %d", dtype);
+  if (status != cudaSuccess) CIE_FAIL("head_norm_gate: launch failed: %s", cudaGetErrorString(status));
   return 0;
 }
