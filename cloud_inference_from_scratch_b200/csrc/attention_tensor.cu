@@ -753,13 +753,72 @@ struct SplitArgs {
   float scale_log2;
   int window;
   int* err;
+  // options (kOptions builds; per query head, nullptr or 0: none): what the prompt kernel's PrefillArgs say of them
+  const float* r1;
+  const float* r2;
+  const float* sinks;
+  float cap;
+  const float* slopes;
+  const float* gates;       // row b of gate_stride floats
+  int gate_stride;
 };
+
+// What a head's sum of weighted values is multiplied with: m its maximum (log2 units), sum its denominator; sinks and gates
+// of the heads, the latter of the request's row (kOptions).
+template <bool kOptions>
+__device__ __forceinline__ float split_inverse(const float* sinks, const float* gates, int head, float m, float sum) {
+  if constexpr (kOptions) {
+    float keep = 1.f;
+    if (sinks) {
+      const float sink = sinks[head] * kLog2eF, top = fmaxf(m, sink);
+      keep = m == -INFINITY ? 0.f : exp2f(m - top);
+      sum = sum * keep + exp2f(sink - top);
+    }
+    const float inv = sum > 0.f ? keep / sum : 0.f;
+    return gates ? inv / (1.f + expf(-gates[head])) : inv;
+  } else {
+    return sum > 0.f ? 1.f / sum : 0.f;
+  }
+}
+
+// The value product with the float32 weights whole: three bfloat16 terms a weight hold its 24 bits (what one rounding
+// leaves is the next one's input).
+template <int NB, bool SW>
+__device__ __forceinline__ void accumulate_whole(const float (&p)[NB * 2][4], const bf16* v_tile, float (&o)[NTILES_D][4], int lane) {
+  const int mi = lane >> 3, r = lane & 7;
+#pragma unroll
+  for (int kb = 0; kb < NB; ++kb) {
+    uint32_t term[3][4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      float p0 = p[2 * kb + (x >> 1)][2 * (x & 1)], p1 = p[2 * kb + (x >> 1)][2 * (x & 1) + 1];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        term[i][x] = pack_bf16(p0, p1);
+        p0 -= __bfloat162float(__float2bfloat16_rn(p0));
+        p1 -= __bfloat162float(__float2bfloat16_rn(p1));
+      }
+    }
+#pragma unroll
+    for (int db = 0; db < KSTEPS; ++db) {
+      uint32_t b[4];
+      ldsm_x4_trans(b, tile_ptr<SW>(v_tile, kb * 16 + (mi & 1) * 8 + r, db * 16 + (mi >> 1) * 8));
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        mma_bf16(o[2 * db], term[i], b[0], b[1]);
+        mma_bf16(o[2 * db + 1], term[i], b[2], b[3]);
+      }
+    }
+  }
+}
 
 // The CTA that drew a unit's last ticket adds up the unit's shares: every thread takes four columns
 // of one head row, asks for the maxima, sums and outputs of eight shares at one time and merges
 // them with a running maximum (in the order of the shares, so the result does not depend on who
 // came last).
-__device__ __noinline__ void merge_shares(const float* unit_shares, int count, bf16* out_rows, int rows, int tid) {
+template <bool kOptions>
+__device__ __noinline__ void merge_shares(const float* sinks, const float* gates, int head0, const float* unit_shares,
+                                          int count, bf16* out_rows, int rows, int tid) {
   for (int idx = tid; idx < rows * (D / 4); idx += SPLIT_WARPS * 32) {
     const int r = idx / (D / 4), c4 = idx % (D / 4);
     const float* row = unit_shares + r * SPLIT_SHARE_ROW;
@@ -789,7 +848,7 @@ __device__ __noinline__ void merge_shares(const float* unit_shares, int count, b
       }
       m_run = m_new;
     }
-    const float inv = sum > 0.f ? 1.f / sum : 0.f;
+    const float inv = split_inverse<kOptions>(sinks, gates, head0 + r, m_run, sum);
     uint2 packed;
     packed.x = pack_bf16(acc.x * inv, acc.y * inv);
     packed.y = pack_bf16(acc.z * inv, acc.w * inv);
@@ -813,7 +872,8 @@ __device__ __forceinline__ void split_mark(int point) {
 #define SPLIT_MARK(point)
 #endif
 
-template <bool kCluster>
+// kOptions: penalties, a cap, slopes, sinks and gates, and softmax weights that enter the value product whole.
+template <bool kCluster, bool kOptions>
 __global__ void __launch_bounds__(SPLIT_WARPS * 32)
 decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                     const SplitArgs a) {
@@ -953,6 +1013,18 @@ decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
   for (int i = 0; i < NTILES_D; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   const int t4 = lane & 3;
+  // the two head rows of this thread (kOptions), as in the prompt kernel
+  float row_r1[2] = {0.f, 0.f}, row_r2[2] = {0.f, 0.f}, row_slope[2] = {0.f, 0.f};
+  const float cap_log2 = kOptions ? a.cap * kLog2eF : 0.f, to_exponent = kOptions && a.cap > 0.f ? 2.f / a.cap : 0.f;
+  if constexpr (kOptions) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = h0 + (lane >> 2) + h * 8, head = kvh * a.group + r;
+      if (r >= a.group) continue;
+      if (a.r1) { row_r1[h] = a.r1[head]; row_r2[h] = a.r2[head]; }
+      if (a.slopes) row_slope[h] = a.slopes[head] * kLog2eF;
+    }
+  }
 
   // A copy that did not arrive in time has set the error bit.  Before the CTA gives up the shared
   // memory that copies still in flight target, every one of them gets one more bounded wait: the
@@ -976,7 +1048,20 @@ decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
       const bf16* v_tile = k_tile + SPLIT_WARPS * SPLIT_BLOCK;
       float s[DN / 8][4];
       scores<DN / 16, true>(q_frag, k_tile, s, lane);
-      if (k0 >= first && k0 + DN <= end) {
+      if constexpr (kOptions) {
+#pragma unroll
+        for (int i = 0; i < DN / 8; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int key = k0 + i * 8 + 2 * t4 + (e & 1);
+            const float gap = (float)(length - 1 - key);
+            float score = s[i][e] * a.scale_log2;
+            if (a.cap > 0.f) score = fmaf(-2.f * cap_log2, __fdividef(1.f, exp2f(score * to_exponent) + 1.f), cap_log2);
+            score = fmaf(-row_slope[e >> 1], gap, score);
+            if (a.r1) score = fmaf(-row_r1[e >> 1], log2f(fmaf(row_r2[e >> 1], fmaxf(gap, 0.f), 1.f)), score);
+            s[i][e] = (key >= first && key < end) ? score : -INFINITY;
+          }
+      } else if (k0 >= first && k0 + DN <= end) {
 #pragma unroll
         for (int i = 0; i < DN / 8; ++i)
 #pragma unroll
@@ -992,7 +1077,8 @@ decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
       }
       if (a.group - h0 <= 8) softmax_update<DN / 8, 1>(s, m, l, o);
       else softmax_update<DN / 8, 2>(s, m, l, o);
-      accumulate<DN / 16, true>(s, v_tile, o, lane);
+      if constexpr (kOptions) accumulate_whole<DN / 16, true>(s, v_tile, o, lane);
+      else accumulate<DN / 16, true>(s, v_tile, o, lane);
     }
     if (it + stages < tiles) {
       // everybody is done with the stage (and agrees on whether its copies arrived) before it is refilled
@@ -1055,6 +1141,7 @@ decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
   float* cluster_share = unit_shares + (size_t)cluster_index * SPLIT_SHARE;
   bf16* out_rows = a.out + (size_t)request * a.out_stride + (size_t)(kvh * a.group + h0) * D;
   const bool exchange = kCluster && peers > 1;
+  const float* gates = kOptions && a.gates ? a.gates + (size_t)request * a.gate_stride : nullptr;
   // the rows this CTA owns, from itself: [rows_per_owner][SPLIT_SHARE_ROW] behind the warps' blocks
   float* own_s = merge_s + SPLIT_WARPS * 16 * D;
   if (exchange) cluster_wait();   // every CTA of the cluster has set its inbox up (they said so when they started)
@@ -1092,7 +1179,7 @@ decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
         if (c4 == 0) push_f2(map_to_rank(theirs + D, owner), m_all, sum, bar);
       }
     } else if (clusters_used == 1) {   // the request is this CTA's alone: the output itself
-      const float inv = sum > 0.f ? 1.f / sum : 0.f;
+      const float inv = split_inverse<kOptions>(a.sinks, gates, kvh * a.group + h0 + r, m_all, sum);
       uint2 packed;
       packed.x = pack_bf16(acc.x * inv, acc.y * inv);
       packed.y = pack_bf16(acc.z * inv, acc.w * inv);
@@ -1130,7 +1217,7 @@ decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
         m_all = m_new;
       }
       if (clusters_used == 1) {
-        const float inv = sum > 0.f ? 1.f / sum : 0.f;
+        const float inv = split_inverse<kOptions>(a.sinks, gates, kvh * a.group + h0 + r, m_all, sum);
         uint2 packed;
         packed.x = pack_bf16(acc.x * inv, acc.y * inv);
         packed.y = pack_bf16(acc.z * inv, acc.w * inv);
@@ -1160,7 +1247,7 @@ decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
   SPLIT_MARK(6);
   if (!last_s) return;
   __threadfence();
-  merge_shares(unit_shares, clusters_used, out_rows, live_rows, tid);
+  merge_shares<kOptions>(a.sinks, gates, kvh * a.group + h0, unit_shares, clusters_used, out_rows, live_rows, tid);
   if (tid == 0) a.tickets[unit] = 0;   // ready for the next launch
   SPLIT_MARK(7);
 }
@@ -1348,12 +1435,12 @@ extern "C" int cie_attention_decode(const void* q, int q_stride, void* out, int 
 template <bool kCluster>
 static int split_ctas_per_sm(int stages, int cluster, int rows) {
   const size_t smem = split_smem(stages, cluster, rows);
-  if (cudaFuncSetAttribute(decode_split_kernel<kCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  if (cudaFuncSetAttribute((decode_split_kernel<kCluster, false>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   int ctas = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, decode_split_kernel<kCluster>, SPLIT_WARPS * 32, smem) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, (decode_split_kernel<kCluster, false>), SPLIT_WARPS * 32, smem) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
@@ -1373,8 +1460,8 @@ extern "C" int cie_attention_decode_split_clusters(int stages, int cluster, int 
   if (D % 64 || stages < SPLIT_MIN_STAGES || stages > SPLIT_MAX_STAGES || rows < 1 || rows > 16) return 0;
   if (cluster != 2 && cluster != 4 && cluster != 8 && cluster != 16) return 0;
   const size_t smem = split_smem(stages, cluster, rows);
-  if (cudaFuncSetAttribute(decode_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      (cluster > 8 && cudaFuncSetAttribute(decode_split_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+  if (cudaFuncSetAttribute((decode_split_kernel<true, false>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      (cluster > 8 && cudaFuncSetAttribute((decode_split_kernel<true, false>), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
     cudaGetLastError();
     return -1;
   }
@@ -1390,7 +1477,7 @@ extern "C" int cie_attention_decode_split_clusters(int stages, int cluster, int 
   config.attrs = &attribute;
   config.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, decode_split_kernel<true>, &config) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, (decode_split_kernel<true, false>), &config) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
@@ -1414,12 +1501,64 @@ extern "C" int cie_attention_decode_split_trace(void* buffer) {
 // int per unit, zero before the first launch (the kernel leaves them zero).  Needs pages of a power
 // of two >= 16 tokens, a head size that is a multiple of 64 and 16-byte-aligned pools (the caller
 // checks and takes the other decode kernel where that does not hold).
-extern "C" int cie_attention_decode_split(const void* q, int q_stride, void* out, int out_stride,
-                                          const void* k_pool, const void* v_pool, const int* table,
-                                          int table_width, int num_pages, const int* context_lens,
-                                          int requests, int q_heads, int kv_heads, int page_size,
-                                          int splits, int min_keys, int stages, int cluster, float* shares,
-                                          int* tickets, float scale, int window, int* err, void* stream) {
+// Options (all null or 0: none; they take a build of their own): see SplitArgs.
+template <bool kOptions>
+static int launch_split(const CUtensorMap& k_map, const CUtensorMap& v_map, const SplitArgs& a, int requests, cudaStream_t stream) {
+  const int cluster = a.cluster;
+  const size_t smem = split_smem(a.stages, cluster, a.group < 16 ? a.group : 16);
+  static size_t configured[2] = {0, 0};
+  const int variant = cluster > 1 ? 1 : 0;
+  if (smem > configured[variant]) {
+    cudaError_t status = variant
+        ? cudaFuncSetAttribute((decode_split_kernel<true, kOptions>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+        : cudaFuncSetAttribute((decode_split_kernel<false, kOptions>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (status != cudaSuccess) CIE_FAIL("attention_decode_split: shared memory %zu: %s", smem, cudaGetErrorString(status));
+    configured[variant] = smem;
+  }
+  if (cluster > 8) {
+    // clusters of more than 8 CTAs need the kernel's consent
+    static bool allowed = false;
+    if (!allowed) {
+      cudaError_t status = cudaFuncSetAttribute((decode_split_kernel<true, kOptions>), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (status != cudaSuccess) CIE_FAIL("attention_decode_split: clusters of %d: %s", cluster, cudaGetErrorString(status));
+      allowed = true;
+    }
+  }
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(a.pools.kv_heads * a.head_chunks, requests, a.splits);
+  config.blockDim = dim3(SPLIT_WARPS * 32);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2];
+  int count = 0;
+  if (cluster > 1) {
+    attributes[count].id = cudaLaunchAttributeClusterDimension;
+    attributes[count].val.clusterDim.x = 1;
+    attributes[count].val.clusterDim.y = 1;
+    attributes[count].val.clusterDim.z = cluster;
+    ++count;
+  }
+  if (pdl_enabled()) {
+    attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[count].val.programmaticStreamSerializationAllowed = 1;
+    ++count;
+  }
+  config.attrs = attributes;
+  config.numAttrs = count;
+  cudaError_t status = cluster > 1 ? cudaLaunchKernelEx(&config, decode_split_kernel<true, kOptions>, k_map, v_map, a)
+                                   : cudaLaunchKernelEx(&config, decode_split_kernel<false, kOptions>, k_map, v_map, a);
+  if (status != cudaSuccess) CIE_FAIL("attention_decode_split: launch failed: %s", cudaGetErrorString(status));
+  return 0;
+}
+
+extern "C" int cie_attention_decode_split_options(const void* q, int q_stride, void* out, int out_stride,
+                                                  const void* k_pool, const void* v_pool, const int* table,
+                                                  int table_width, int num_pages, const int* context_lens,
+                                                  int requests, int q_heads, int kv_heads, int page_size,
+                                                  int splits, int min_keys, int stages, int cluster, float* shares,
+                                                  int* tickets, float scale, int window, const float* r1, const float* r2,
+                                                  const float* sinks, float cap, const float* slopes, const float* gates,
+                                                  int gate_stride, int options, int* err, void* stream) {
   if (requests <= 0) return 0;
   if (kv_heads < 1 || q_heads % kv_heads) CIE_FAIL("attention_decode_split: %d query heads over %d kv heads", q_heads, kv_heads);
   if (splits < 1 || splits > SPLIT_MAX) CIE_FAIL("attention_decode_split: 1 to %d CTAs per request, got %d", SPLIT_MAX, splits);
@@ -1445,55 +1584,27 @@ extern "C" int cie_attention_decode_split(const void* q, int q_stride, void* out
   a.page_shift = page_shift; a.splits = splits; a.min_keys = min_keys; a.stages = stages; a.cluster = cluster;
   a.shares = shares; a.tickets = tickets;
   a.scale_log2 = scale * kLog2e; a.window = window; a.err = err;
+  a.r1 = r1; a.r2 = r2; a.sinks = sinks; a.cap = cap; a.slopes = slopes; a.gates = gates; a.gate_stride = gate_stride;
+  if ((r1 == nullptr) != (r2 == nullptr)) CIE_FAIL("attention_decode_split: a penalty needs both vectors");
   CUtensorMap k_map = {}, v_map = {};
   const long long rows = (long long)num_pages * kv_heads * page_size;
   const bool mapped = kBlockCopies
       ? bw::tensor_map_bf16_row_blocks(k_pool, rows, D, 16, &k_map) && bw::tensor_map_bf16_row_blocks(v_pool, rows, D, 16, &v_map)
       : bw::tensor_map_bf16(k_pool, rows, D, 16, &k_map) && bw::tensor_map_bf16(v_pool, rows, D, 16, &v_map);
   if (!mapped) CIE_FAIL("attention_decode_split: cuTensorMapEncodeTiled failed");
-  const size_t smem = split_smem(stages, cluster, a.group < 16 ? a.group : 16);
-  static size_t configured[2] = {0, 0};
-  const int variant = cluster > 1 ? 1 : 0;
-  if (smem > configured[variant]) {
-    cudaError_t status = variant
-        ? cudaFuncSetAttribute(decode_split_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-        : cudaFuncSetAttribute(decode_split_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (status != cudaSuccess) CIE_FAIL("attention_decode_split: shared memory %zu: %s", smem, cudaGetErrorString(status));
-    configured[variant] = smem;
-  }
-  if (cluster > 8) {
-    // clusters of more than 8 CTAs need the kernel's consent
-    static bool allowed = false;
-    if (!allowed) {
-      cudaError_t status = cudaFuncSetAttribute(decode_split_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (status != cudaSuccess) CIE_FAIL("attention_decode_split: clusters of %d: %s", cluster, cudaGetErrorString(status));
-      allowed = true;
-    }
-  }
   if (requests > 65535) CIE_FAIL("attention_decode_split: at most 65535 requests a launch, got %d", requests);
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(kv_heads * a.head_chunks, requests, splits);
-  config.blockDim = dim3(SPLIT_WARPS * 32);
-  config.dynamicSmemBytes = smem;
-  config.stream = (cudaStream_t)stream;
-  cudaLaunchAttribute attributes[2];
-  int count = 0;
-  if (cluster > 1) {
-    attributes[count].id = cudaLaunchAttributeClusterDimension;
-    attributes[count].val.clusterDim.x = 1;
-    attributes[count].val.clusterDim.y = 1;
-    attributes[count].val.clusterDim.z = cluster;
-    ++count;
-  }
-  if (pdl_enabled()) {
-    attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attributes[count].val.programmaticStreamSerializationAllowed = 1;
-    ++count;
-  }
-  config.attrs = attributes;
-  config.numAttrs = count;
-  cudaError_t status = cluster > 1 ? cudaLaunchKernelEx(&config, decode_split_kernel<true>, k_map, v_map, a)
-                                   : cudaLaunchKernelEx(&config, decode_split_kernel<false>, k_map, v_map, a);
-  if (status != cudaSuccess) CIE_FAIL("attention_decode_split: launch failed: %s", cudaGetErrorString(status));
-  return 0;
+  return options ? launch_split<true>(k_map, v_map, a, requests, (cudaStream_t)stream)
+                 : launch_split<false>(k_map, v_map, a, requests, (cudaStream_t)stream);
+}
+
+extern "C" int cie_attention_decode_split(const void* q, int q_stride, void* out, int out_stride,
+                                          const void* k_pool, const void* v_pool, const int* table,
+                                          int table_width, int num_pages, const int* context_lens,
+                                          int requests, int q_heads, int kv_heads, int page_size,
+                                          int splits, int min_keys, int stages, int cluster, float* shares,
+                                          int* tickets, float scale, int window, int* err, void* stream) {
+  return cie_attention_decode_split_options(q, q_stride, out, out_stride, k_pool, v_pool, table, table_width, num_pages,
+                                            context_lens, requests, q_heads, kv_heads, page_size, splits, min_keys, stages,
+                                            cluster, shares, tickets, scale, window, nullptr, nullptr, nullptr, 0.f, nullptr,
+                                            nullptr, 0, 0, err, stream);
 }

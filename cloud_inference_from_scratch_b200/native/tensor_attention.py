@@ -116,6 +116,10 @@ class TensorAttention:
                 "cie_attention_decode_split",
                 [v, i, v, i, v, v, v, i, i, v, i, i, i, i, i, i, i, i, v, v, f, i, v, v],
             )
+            self._decode_split_options = lib.function(
+                "cie_attention_decode_split_options",
+                [v, i, v, i, v, v, v, i, i, v, i, i, i, i, i, i, i, i, v, v, f, i, v, v, v, f, v, v, i, i, v, v],
+            )
             self.split_max = int(lib.handle.cie_attention_decode_split_max())
             self.split_tile = int(lib.handle.cie_attention_decode_split_tile())
             per_sm = lib.handle.cie_attention_decode_split_ctas_per_sm
@@ -312,6 +316,49 @@ class TensorAttention:
         by_keys = max_keys // (splits * MIN_KEYS_PER_CHUNKED_CTA)
         return max(1, min(by_sms, by_keys, MAX_CHUNKS))
 
+    def splits_decode(self, kv: Any) -> bool:
+        """Whether the split decode kernel takes these pages."""
+        page = kv.page_size
+        return bool(self._decode_split is not None and page >= 16 and page & (page - 1) == 0
+                    and (kv.k.data_ptr() | kv.v.data_ptr()) % 16 == 0)
+
+    def _split_launch(self, requests: int, kv_heads: int, group: int, max_keys: int) -> tuple[int, int, int, int]:
+        units = requests * kv_heads * -(-group // 16)
+        rings, room = self.split_choices(group)
+        ctas, stages, cluster, min_keys = self.split_plan(units, max_keys, self.sm_count, rings, room,
+                                                          self.split_cta_limit, self.split_max, self.split_tile)
+        if FORCE_SPLIT_PLAN:
+            ctas, stages, cluster = FORCE_SPLIT_PLAN
+        if FORCE_SPLIT_KEYS:
+            min_keys = FORCE_SPLIT_KEYS
+        return ctas, stages, cluster, min_keys
+
+    def run_singles(self, q: Any, out: Any, ctx: Any, kv: Any, requests: int, q_heads: int, kv_heads: int, scale: float,
+                    window: int, distance: Any, sinks: Any = None, softcap: float = 0.0, slopes: Any = None,
+                    gates: Any = None, shares: Any = None, tickets: Any = None) -> None:
+        """One query token for each of the first ``requests`` requests, with the options of ``run_portions`` except kept
+        first keys, on the split decode kernel (``splits_decode``; key and value heads of this build's size); the softmax
+        weights enter the value product as three bfloat16 terms, which hold all their bits.  ``shares`` and ``tickets``:
+        the caller's scratch memory (tickets zero, and left so), used where it is large enough."""
+        ops = self.ops
+        table = ctx.block_tables[kv.group]
+        max_keys = table.shape[1] * kv.page_size
+        if window > 0:
+            max_keys = min(max_keys, window)
+        ctas, stages, cluster, min_keys = self._split_launch(requests, kv_heads, q_heads // kv_heads, max_keys)
+        units = requests * kv_heads * -(-(q_heads // kv_heads) // 16)
+        if (shares is None or tickets is None or tickets.numel() < units
+                or shares.numel() < units * (ctas // cluster) * 16 * (self.head_dim + 4)):
+            shares, tickets = self._split_shares, self._split_tickets
+        pointer = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+        r1, r2 = distance if distance is not None else (None, None)
+        self._decode_split_options(q.data_ptr(), q.shape[1], out.data_ptr(), out.shape[1], kv.k.data_ptr(), kv.v.data_ptr(),
+                                   table.data_ptr(), table.shape[1], kv.num_pages, ctx.context_lens.data_ptr(), requests,
+                                   q_heads, kv_heads, kv.page_size, ctas, min_keys, stages, cluster,
+                                   shares.data_ptr(), tickets.data_ptr(), scale, window, pointer(r1),
+                                   pointer(r2), pointer(sinks), float(softcap), pointer(slopes), pointer(gates),
+                                   0 if gates is None else gates.stride(0), 1, ops.error_word.data_ptr(), ops.stream)
+
     def _run_decode(self, qkv: Any, out: Any, ctx: Any, kv: Any, table: Any, requests: int, q_heads: int,
                     kv_heads: int, scale: float, window: int) -> None:
         """One query token for each of the first ``requests`` requests of the step (their token row
@@ -321,21 +368,12 @@ class TensorAttention:
         max_keys = table.shape[1] * kv.page_size
         if window > 0:
             max_keys = min(max_keys, window)
-        page = kv.page_size
         ops.launches += 1
-        if (self._decode_split is not None and page >= 16 and page & (page - 1) == 0
-                and (kv.k.data_ptr() | kv.v.data_ptr()) % 16 == 0):
-            units = requests * kv_heads * -(-group // 16)
-            rings, room = self.split_choices(group)
-            ctas, stages, cluster, min_keys = self.split_plan(units, max_keys, self.sm_count, rings, room,
-                                                              self.split_cta_limit, self.split_max, self.split_tile)
-            if FORCE_SPLIT_PLAN:
-                ctas, stages, cluster = FORCE_SPLIT_PLAN
-            if FORCE_SPLIT_KEYS:
-                min_keys = FORCE_SPLIT_KEYS
+        if self.splits_decode(kv):
+            ctas, stages, cluster, min_keys = self._split_launch(requests, kv_heads, group, max_keys)
             self._decode_split(qkv.data_ptr(), qkv.shape[1], out.data_ptr(), out.shape[1], kv.k.data_ptr(),
                                kv.v.data_ptr(), table.data_ptr(), table.shape[1], kv.num_pages,
-                               ctx.context_lens.data_ptr(), requests, q_heads, kv_heads, page, ctas,
+                               ctx.context_lens.data_ptr(), requests, q_heads, kv_heads, kv.page_size, ctas,
                                min_keys, stages, cluster, self._split_shares.data_ptr(),
                                self._split_tickets.data_ptr(), scale, window, ops.error_word.data_ptr(),
                                ops.stream)

@@ -1,5 +1,6 @@
-"""The tcgen05 kernel for prompt portions with options (windows, kept keys, penalties, caps, slopes, sinks, gates), against
-plain attention in 64 bits and against the mma.sync kernel, which computes the same for other sizes."""
+"""The kernels for layers with options (windows, kept keys, penalties, caps, slopes, sinks, gates): prompt portions on tcgen05, against
+plain attention in 64 bits and against the mma.sync kernel, which computes the same for other sizes; single tokens on the
+split decode kernel."""
 
 import math
 from types import SimpleNamespace
@@ -127,3 +128,59 @@ def test_portions_with_options(option, dim, kv_heads, group, page):
                 assert float((got - want).abs().max()) <= bound, (r, t)
             row += 1
     assert torch.allclose(results[0], results[1], rtol=2.0 ** -7, atol=2.0 ** -8)
+
+
+@pytest.mark.parametrize("dim,kv_heads,group,page", [(128, 2, 8, 16), (64, 1, 3, 32), (192, 1, 16, 16), (128, 1, 20, 128), (256, 2, 1, 64)])
+@pytest.mark.parametrize("option", [0, 1, 4, 6, 7])
+def test_single_tokens_with_options(option, dim, kv_heads, group, page):
+    """First tokens, contexts at and beside the edges of blocks and ranges, one that many CTAs share; pages in descending
+    order, gone behind a window.  The weights enter whole, the result is rounded once."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+
+    ops = Runtime("cuda:0", "bfloat16").ops
+    ops.require_portion_attention(dim)
+    fast = ops._tensor_attention[dim]
+    asked = (OPTIONS + [dict(window=300, slopes=True, gates=True, penalty=True, cap=3.0)])[option]
+    heads = kv_heads * group
+    contexts = [0, 15, 16, 63, 64, 300, 2100]
+    count, total_keys = len(contexts), max(contexts) + 1
+    scale = (-1 if asked.get("negative") else 1) * dim ** -0.5
+    o = SimpleNamespace(window=asked.get("window", 0), keep=0, cap=asked.get("cap", 0.0), slopes=None, penalty=None,
+                        sinks=rand(heads, seed=3) if asked.get("sink") else None,
+                        gates=rand(count, heads + 1, seed=4) if asked.get("gates") else None)
+    if asked.get("slopes"):
+        o.slopes = torch.tensor([2.0 ** (-8.0 * (h + 1) / heads) for h in range(heads)])
+    if asked.get("penalty"):
+        o.penalty = (rand(heads, seed=1).abs(), rand(heads, seed=2).abs())
+    width = -(-total_keys // page)
+    table = torch.full((count, width), -1, dtype=torch.int32)
+    pools = [torch.full((count * width, kv_heads, page, dim), 100.0).bfloat16() for _ in range(2)]
+    keys, values = [], []
+    for r, context in enumerate(contexts):
+        k, v = rand(context + 1, kv_heads, dim, seed=10 + r, scale=1.5).bfloat16(), rand(context + 1, kv_heads, dim, seed=30 + r).bfloat16()
+        keys.append(k.double()), values.append(v.double())
+        lowest = max(0, context - o.window + 1) if o.window else 0
+        for index in range(lowest // page, -(-(context + 1) // page)):
+            table[r, index] = r * width + width - 1 - index
+            rows = slice(index * page, min((index + 1) * page, context + 1))
+            for pool, source in zip(pools, (k, v)):
+                pool[table[r, index], :, :rows.stop - rows.start] = source[rows].transpose(0, 1)
+    q = rand(count, heads * dim, seed=6, scale=1.5).bfloat16()
+    pools = [pool.cuda() for pool in pools]
+    kv = SimpleNamespace(group=0, k=pools[0], v=pools[1], num_pages=count * width, page_size=page)
+    ctx = SimpleNamespace(block_tables=[table.cuda()], context_lens=torch.tensor(contexts, dtype=torch.int32).cuda())
+    assert fast.splits_decode(kv)
+    device = lambda t: None if t is None else t.cuda()  # noqa: E731
+    gates, sinks, slopes = device(o.gates), device(o.sinks), device(o.slopes)
+    penalty = None if o.penalty is None else tuple(device(t) for t in o.penalty)
+    out = torch.full((count + 1, heads * dim), 7.0, dtype=torch.bfloat16).cuda()
+    fast.run_singles(q.cuda(), out, ctx, kv, count, heads, kv_heads, scale, o.window, penalty, sinks=sinks, softcap=o.cap,
+                     slopes=slopes, gates=None if gates is None else gates[:, 1:])
+    ops.check_errors()
+    assert float((out[count] - 7.0).abs().max()) == 0 and int(fast._split_tickets.abs().sum()) == 0
+    for r, context in enumerate(contexts):
+        want = oracle(q[r].double().view(heads, dim), keys[r], values[r], context, group, scale, o, heads)
+        if o.gates is not None:
+            want = want * torch.sigmoid(o.gates[r, 1:].double()).view(-1, 1)
+        got = out[r].view(heads, dim).double().cpu()
+        assert float((got - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-6, r
