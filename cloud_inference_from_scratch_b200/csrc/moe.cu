@@ -30,59 +30,81 @@ constexpr int kMaxExperts = 1024;
 constexpr int kRowTile = 128;         // rows of a tile of the grouped products
 
 // ---------------------------------------------------------------- route
-// One block of four warps per token: the token's row goes to shared memory as float32, the warps
-// share the experts (a lane strides over the row with 16-byte loads of the router matrix where the
-// row length allows), then the first warp turns logits into scores and chooses.
+// One block of eight warps per kTokens tokens: their rows go to shared memory as float32, the warps share the experts (a
+// lane strides over a router row with 16-byte loads where the row length allows, and meets every token with it), then a warp
+// a token turns logits into scores and chooses.  A token's sums are added in the same order whatever kTokens.  With one
+// token a block every token asks L2 for the whole router matrix (2,048 tokens of 2,048, 16 experts: 262 MB, 35 us); four
+// share it where there are tokens enough for every SM.
 // ids / weights: [tokens][top]; counts[e] += 1 per choice.
 constexpr int kRouteWarps = 8;
-template <typename T>
+__host__ __device__ __forceinline__ int route_scores(int experts) { return (2 * experts + 3) & ~3; }
+__host__ __device__ __forceinline__ int route_row(int hidden, int groups) { return ((hidden > groups ? hidden : groups) + 3) & ~3; }
+template <typename T, int kTokens>
 __global__ void __launch_bounds__(kRouteWarps * 32)
 moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
                  const float* __restrict__ correction, int* __restrict__ ids,
                  float* __restrict__ weights, int* __restrict__ counts, int tokens,
                  int hidden, int experts, int top, int renormalize, const float* __restrict__ logit_bias,
                  int chosen_softmax, int sigmoid, int groups, int keep_groups, float norm_floor) {
-  extern __shared__ __align__(16) float score_s[];      // [2 * experts]: scores, then choice scores; then the row
+  extern __shared__ __align__(16) float route_smem[];      // per token: scores, choice scores; then the rows
   pdl_wait();
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x;
-  float* score = score_s;
-  float* choice = score + experts;
-  float* row_s = score_s + ((2 * experts + 3) & ~3);
-  const T* row = x + (size_t)t * hidden;
-  for (int k = threadIdx.x; k < hidden; k += blockDim.x) row_s[k] = to_float(row[k]);
+  const int t0 = blockIdx.x * kTokens, count = min(kTokens, tokens - t0);
+  const int score_ld = route_scores(experts), row_ld = route_row(hidden, groups);
+  float* rows_s = route_smem + kTokens * score_ld;
+  for (int i = 0; i < count; ++i) {
+    const T* row = x + (size_t)(t0 + i) * hidden;
+    for (int k = threadIdx.x; k < hidden; k += blockDim.x) rows_s[i * row_ld + k] = to_float(row[k]);
+  }
   __syncthreads();
   const bool wide = hidden % 4 == 0;
+  constexpr int kDeep = kTokens > 1 ? 4 : 8;      // router loads in flight
   for (int e = warp; e < experts; e += kRouteWarps) {
     const float* w = router + (size_t)e * hidden;
-    float dot = 0.f;
+    float dot[kTokens] = {};
     if (wide) {
-      // eight 16-byte loads of the router row are asked for before the first is used: the row comes
+      // several 16-byte loads of the router row are asked for before the first is used: the row comes
       // from memory once a step and nothing else hides that trip
-      for (int k0 = 4 * lane; k0 < hidden; k0 += 8 * 128) {
-        float4 wv[8];
+      for (int k0 = 4 * lane; k0 < hidden; k0 += kDeep * 128) {
+        float4 wv[kDeep];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
+        for (int u = 0; u < kDeep; ++u)
           wv[u] = k0 + 128 * u < hidden ? *reinterpret_cast<const float4*>(w + k0 + 128 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < kDeep; ++u) {
           if (k0 + 128 * u >= hidden) break;
-          const float4 xv = *reinterpret_cast<const float4*>(row_s + k0 + 128 * u);
-          dot = fmaf(xv.x, wv[u].x, dot);
-          dot = fmaf(xv.y, wv[u].y, dot);
-          dot = fmaf(xv.z, wv[u].z, dot);
-          dot = fmaf(xv.w, wv[u].w, dot);
+#pragma unroll
+          for (int i = 0; i < kTokens; ++i) {
+            if (i >= count) break;
+            const float4 xv = *reinterpret_cast<const float4*>(rows_s + i * row_ld + k0 + 128 * u);
+            dot[i] = fmaf(xv.x, wv[u].x, dot[i]);
+            dot[i] = fmaf(xv.y, wv[u].y, dot[i]);
+            dot[i] = fmaf(xv.z, wv[u].z, dot[i]);
+            dot[i] = fmaf(xv.w, wv[u].w, dot[i]);
+          }
         }
       }
     } else {
-      for (int k = lane; k < hidden; k += 32) dot = fmaf(row_s[k], w[k], dot);
+      for (int k = lane; k < hidden; k += 32) {
+        const float wk = w[k];
+#pragma unroll
+        for (int i = 0; i < kTokens; ++i)
+          if (i < count) dot[i] = fmaf(rows_s[i * row_ld + k], wk, dot[i]);
+      }
     }
-    dot = warp_sum(dot);
-    if (lane == 0) score[e] = logit_bias ? dot + logit_bias[e] : dot;
+#pragma unroll
+    for (int i = 0; i < kTokens; ++i) {
+      const float total = warp_sum(dot[i]);
+      if (lane == 0) route_smem[i * score_ld + e] = logit_bias ? total + logit_bias[e] : total;
+    }
   }
   __syncthreads();
-  if (warp != 0) return;
+  if (warp >= count) return;
+  const int t = t0 + warp;
+  float* score = route_smem + warp * score_ld;
+  float* choice = score + experts;
+  float* row_s = rows_s + warp * row_ld;
   __syncwarp();
   if (chosen_softmax) {
     // the largest logits win (lowest index on ties); their weights are exp(z - z_first) over the sum of those
@@ -466,6 +488,24 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const float* 
   pdl_wait();
   pdl_trigger();
   const int t = blockIdx.x;
+  if constexpr (sizeof(TOut) == 4) {
+    if (hidden % 4 == 0 && ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
+      for (int i = threadIdx.x * 4; i < hidden; i += blockDim.x * 4) {
+        float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int j = 0; j < top; ++j) {
+          const float w = weights ? weights[(size_t)t * top + j] : 1.f;
+          const float4 v = *reinterpret_cast<const float4*>(rows + ((size_t)t * top + j) * hidden + i);
+          total.x = fmaf(w, v.x, total.x);
+          total.y = fmaf(w, v.y, total.y);
+          total.z = fmaf(w, v.z, total.z);
+          total.w = fmaf(w, v.w, total.w);
+        }
+        *reinterpret_cast<float4*>(y + (size_t)t * hidden + i) = total;
+      }
+      return;
+    }
+  }
   for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
     float total = 0.f;
     for (int j = 0; j < top; ++j)
@@ -498,24 +538,31 @@ extern "C" int cie_moe_route(const void* x, const float* router, const float* co
   cudaStream_t s = (cudaStream_t)stream;
   if (counts && cudaMemsetAsync(counts, 0, sizeof(int) * experts, s) != cudaSuccess) CIE_FAIL("moe_route: memset failed");
   const int warps = kRouteWarps;
-  const size_t smem = (size_t)(((2 * experts + 3) & ~3) + (hidden > groups ? hidden : groups)) * sizeof(float);
-  if (smem > 200 * 1024) CIE_FAIL("moe_route: a row of %d elements does not fit shared memory", hidden);
-  const int blocks = tokens;
+  const size_t one = (size_t)(route_scores(experts) + route_row(hidden, groups)) * sizeof(float);
+  if (one > 200 * 1024) CIE_FAIL("moe_route: a row of %d elements does not fit shared memory", hidden);
+  // four tokens a block from two blocks an SM on, as long as two such blocks fit an SM's shared memory
+  const bool four = tokens >= 4 * 2 * 148 && 4 * one <= 100 * 1024;
+  const size_t smem = four ? 4 * one : one;
+  const int blocks = four ? (tokens + 3) / 4 : tokens;
+#define CIE_MOE_ROUTE(T, N)                                                                                                  \
+  do {                                                                                                                       \
+    if (smem > 48 * 1024 && cudaFuncSetAttribute((moe_route_kernel<T, N>), cudaFuncAttributeMaxDynamicSharedMemorySize,      \
+                                                 (int)smem) != cudaSuccess)                                                  \
+      CIE_FAIL("moe_route: cannot reserve %zu bytes of shared memory", smem);                                                \
+    CIE_LAUNCH("moe_route", (moe_route_kernel<T, N>), dim3(blocks), dim3(warps * 32), smem, s, (const T*)x, router,          \
+               correction, ids, weights, counts, tokens, hidden, experts, top, renormalize, logit_bias, chosen_softmax,      \
+               sigmoid, groups, keep_groups, norm_floor);                                                                    \
+  } while (0)
   if (dtype == kFloat32) {
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(moe_route_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      CIE_FAIL("moe_route: cannot reserve %zu bytes of shared memory", smem);
-    CIE_LAUNCH("moe_route", moe_route_kernel<float>, dim3(blocks), dim3(warps * 32), smem, s, (const float*)x, router,
-               correction, ids, weights, counts, tokens, hidden, experts, top, renormalize, logit_bias, chosen_softmax, sigmoid,
-               groups, keep_groups, norm_floor);
+    if (four) CIE_MOE_ROUTE(float, 4);
+    else CIE_MOE_ROUTE(float, 1);
   } else if (dtype == kBFloat16) {
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      CIE_FAIL("moe_route: cannot reserve %zu bytes of shared memory", smem);
-    CIE_LAUNCH("moe_route", moe_route_kernel<__nv_bfloat16>, dim3(blocks), dim3(warps * 32), smem, s,
-               (const __nv_bfloat16*)x, router, correction, ids, weights, counts, tokens, hidden, experts, top,
-               renormalize, logit_bias, chosen_softmax, sigmoid, groups, keep_groups, norm_floor);
+    if (four) CIE_MOE_ROUTE(__nv_bfloat16, 4);
+    else CIE_MOE_ROUTE(__nv_bfloat16, 1);
   } else {
     CIE_FAIL("moe_route: unknown element type code %d", dtype);
   }
+#undef CIE_MOE_ROUTE
   if (!counts) return 0;
   CIE_LAUNCH("moe_plan", moe_plan_kernel, dim3(1), dim3(1024), 0, s, ids, counts, offsets, cursors, place_to_pair,
              tiles, tile_count, tokens * top, experts);
