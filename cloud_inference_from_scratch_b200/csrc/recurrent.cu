@@ -496,7 +496,6 @@ gated_delta_prepare_kernel(const float* __restrict__ conv, int conv_stride, int 
     float g = 0.f;
     if (tid == 0) g = expf(-expf(a_log[head]) * softplus_f(proj[(size_t)t * proj_stride + a_off + head] + dt_bias[head]));
     if (tid == 1) g = sigmoid_f(proj[(size_t)t * proj_stride + b_off + head]);
-    if (tid == 2) g = -expf(a_log[head]) * softplus_f(proj[(size_t)t * proj_stride + a_off + head] + dt_bias[head]);   // log of the decay
     dst[2 * pad + tid] = g;
   }
   for (int i = tid; i < vpad; i += blockDim.x) dst[2 * pad + kStreamGates + i] = i < vdim ? row[v_off + head * vdim + i] : 0.f;
@@ -1018,140 +1017,240 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
 // token to t, the rule's writes u_t obey  u_t = b_t (v_t - c_t S_0^T k_t - sum_(s<t) (c_t / c_s) (k_s . k_t) u_s),  a
 // triangular system:  (I + A) U = diag(b) (V - diag(c) K S_0),  A_ts = b_t (c_t / c_s) (k_t . k_s) for s < t.  With
 // T = (I + A)^-1:  U = T diag(b) V - (T diag(b c) K) S_0 = U' - W S_0.  So:
-//   1. prepare (above): unit k and q, decay, write strength and log decay of every token
-//   2. per (chunk, head):      A, T by forward substitution (a lane a column of T), U' and W
-//   3. per (request, head, 32 value columns): walks the chunks with its columns of S in registers:
+//   1. per (chunk, head):      unit k and q; A, T by forward substitution (a lane a column of T), U' and W
+//   2. per (request, head, 32 value columns): walks the chunks with its columns of S in registers:
 //                              U = U' - W S_0,  S <- c_C S_0 + sum_s (c_C / c_s) k_s u_s^T; leaves S_0 of every chunk
-//   4. per (chunk, head):      o_t = c_t S_0^T q_t + sum_(s<=t) (c_t / c_s) (q_t . k_s) u_s   (the matrix memory's output
+//   3. per (chunk, head):      o_t = c_t S_0^T q_t + sum_(s<=t) (c_t / c_s) (q_t . k_s) u_s   (the matrix memory's output
 //                              kernel with i = m = 0 and no denominator)
 // Ratios of decays are exponentials of differences of summed logarithms, never quotients.  Float32 on the CUDA cores.
-// Keys up to kMemDim, values a multiple of 4.
+// Keys up to kMemDim, values a multiple of 4.  All three are bounded by the data shared memory returns (a 16-byte load of
+// a warp takes 4 cycles, broadcast or not), which the tiles of a thread are chosen by: four portions of 333 tokens, 16
+// heads of 128 x 128: the layer 388 us with a prepare kernel of its own and tiles of a column a lane, 271 this way (solve and
+// prepare 113 us and walk 139 before).
 constexpr int kWalkColumns = 32;
-constexpr int kWalkWarps = 16;                   // warps of the walk
-constexpr int kWalkRows = kMemDim / kWalkWarps;  // state rows of a warp
+constexpr int kSolveRow = kMemChunk + 4;         // row of the solve's matrices, transposed: [earlier token][token]
 
-// grid (chunks, heads).  packed: the prepared rows [k: P][q: P][gates][v: VP] per head and token.
+__host__ __device__ constexpr int gated_solve_floats(int P, int vdim) {
+  return kMemChunk * (vdim + P + 4) + 3 * kMemChunk * kSolveRow;
+}
+__host__ __device__ constexpr int gated_walk_stage(int P) {
+  return kMemChunk * (2 * P + kWalkColumns + kMemGates);
+}
+__host__ __device__ constexpr int gated_walk_floats(int P) {
+  return 2 * gated_walk_stage(P) + (P / 32 + 1) * kMemChunk * kWalkColumns;
+}
+
+// grid (chunks, heads).  unit: [head][token][k: P][q: P], zeros past dim.
 __global__ void __launch_bounds__(256)
-delta_chunk_solve_kernel(const float* __restrict__ packed, int tokens, int row_floats, int P,
-                         float* __restrict__ gates, float* __restrict__ w_out, float* __restrict__ u_out,
-                         const int* __restrict__ chunk_row, const int* __restrict__ chunk_count, int heads, int vdim) {
-  constexpr int C = kMemChunk;
+gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_off, int k_off, int v_off,
+                         const float* __restrict__ proj, int proj_stride, int b_off, int a_off,
+                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float q_scale,
+                         float* __restrict__ unit, int tokens, int P, float* __restrict__ gates,
+                         float* __restrict__ w_out, float* __restrict__ u_out, const int* __restrict__ chunk_row,
+                         const int* __restrict__ chunk_count, int heads, int kv_heads, int dim, int vdim) {
+  constexpr int C = kMemChunk, TL = kSolveRow;
   extern __shared__ __align__(16) float smem[];
-  const int kd = P + 1;
+  const int kd = P + 4;
   float* v_s = smem;                       // [C][vdim]
-  float* k_s = v_s + C * vdim;             // [C][P + 1]
-  float* a_s = k_s + C * kd;               // [C][C + 1]
-  float* t_s = a_s + C * (C + 1);          // [C][C + 1]
-  __shared__ float beta_s[C], lg_s[C], bc_s[C];
+  float* k_s = v_s + C * vdim;             // [C][P + 4]
+  float* a_s = k_s + C * kd;               // A
+  float* tv_s = a_s + C * TL;              // T diag(b)
+  float* tk_s = tv_s + C * TL;             // T diag(b c)
+  __shared__ float beta_s[C], lg_s[C];
   pdl_wait();
   pdl_trigger();
-  const int chunk = blockIdx.x, head = blockIdx.y, tid = threadIdx.x;
-  const int row0 = chunk_row[chunk], n = chunk_count[chunk];
-  const float* rows = packed + (size_t)head * tokens * row_floats;
-  if (tid < n) {
-    float lg = 0.f;
-    for (int r = 0; r <= tid; ++r) lg += rows[(size_t)(row0 + r) * row_floats + 2 * P + 2];
-    const float beta = rows[(size_t)(row0 + tid) * row_floats + 2 * P + 1];
-    lg_s[tid] = lg;
-    beta_s[tid] = beta;
-    bc_s[tid] = beta * expf(lg);
-    *reinterpret_cast<float4*>(gates + ((size_t)(row0 + tid) * heads + head) * kMemGates) = make_float4(0.f, lg, 0.f, 0.f);
+  const int chunk = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int row0 = chunk_row[chunk], n = chunk_count[chunk], base = (head / (heads / kv_heads)) * dim;
+  if (warp == 0) {
+    float g = 0.f, beta = 0.f, lg = 0.f;
+    if (lane < n) {
+      const float* row = proj + (size_t)(row0 + lane) * proj_stride;
+      g = -expf(a_log[head]) * softplus_f(row[a_off + head] + dt_bias[head]);      // log of the decay
+      beta = sigmoid_f(row[b_off + head]);
+    }
+#pragma unroll
+    for (int r = 0; r < C; ++r) {
+      const float x = __shfl_sync(0xffffffffu, g, r);
+      if (r <= lane) lg += x;
+    }
+    lg_s[lane] = lg;
+    beta_s[lane] = beta;
+    if (lane < n) *reinterpret_cast<float4*>(gates + ((size_t)(row0 + lane) * heads + head) * kMemGates) = make_float4(0.f, lg, 0.f, 0.f);
   }
-  stage_rows(k_s, kd, rows, row_floats, row0, n, 0, P, [](int) { return 1.f; });
-  stage_rows(v_s, vdim, rows, row_floats, row0, n, 2 * P + kStreamGates, vdim, [](int) { return 1.f; });
+#pragma unroll
+  for (int i = 0; i < C / 8; ++i) {        // unit k and q, the squares in the order of the scan
+    const int t = warp + 8 * i;
+    if (t >= n) break;
+    const float* row = conv + (size_t)(row0 + t) * conv_stride + base;
+    float k[kMemDim / 32], q[kMemDim / 32], ksq = 0.f, qsq = 0.f;
+#pragma unroll
+    for (int x = 0; x < kMemDim / 32; ++x) {
+      const bool in = lane + 32 * x < dim;
+      k[x] = in ? row[k_off + lane + 32 * x] : 0.f;
+      q[x] = in ? row[q_off + lane + 32 * x] : 0.f;
+    }
+#pragma unroll
+    for (int x = 0; x < kMemDim / 32; ++x) {
+      ksq = fmaf(k[x], k[x], ksq);
+      qsq = fmaf(q[x], q[x], qsq);
+    }
+    const float k_inv = rsqrtf(warp_sum(ksq) + 1e-6f), q_inv = rsqrtf(warp_sum(qsq) + 1e-6f);
+    float* dst = unit + ((size_t)head * tokens + row0 + t) * (2 * P) + lane;
+#pragma unroll
+    for (int x = 0; x < kMemDim / 32; ++x) {
+      if (32 * x >= P) break;
+      dst[32 * x] = k_s[t * kd + lane + 32 * x] = k[x] * k_inv;
+      dst[P + 32 * x] = q[x] * q_inv * q_scale;
+    }
+  }
+  stage_rows(v_s, vdim, conv, conv_stride, row0, n, v_off + head * vdim, vdim, [](int) { return 1.f; });
   __syncthreads();
   {
-    // a warp takes four tokens that follow each other, a lane an earlier token
-    constexpr int kQ = C / 8;
-    const int t0 = (tid >> 5) * kQ, j = tid & 31;
-    float a[kQ] = {};
-    if (t0 < n && j < t0 + kQ - 1 && j < n) {
-      for (int x = 0; x < P; ++x) {
-        const float kx = k_s[j * kd + x];
+    // A: four lanes share a 4 x 4 tile, each every fourth 16 bytes of the rows
+    const int part = tid & 3, t0 = (tid >> 5) * 4, s0 = ((tid >> 2) & 7) * 4;
+    float dot[4][4] = {};
+    if (s0 <= t0) {
+      for (int x = part * 4; x < P; x += 16) {
+        float4 tv[4];
 #pragma unroll
-        for (int t = 0; t < kQ; ++t) a[t] = fmaf(k_s[(t0 + t) * kd + x], kx, a[t]);
+        for (int i = 0; i < 4; ++i) tv[i] = *reinterpret_cast<const float4*>(k_s + (t0 + i) * kd + x);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 sv = *reinterpret_cast<const float4*>(k_s + (s0 + j) * kd + x);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            dot[i][j] = fmaf(tv[i].x, sv.x, dot[i][j]);
+            dot[i][j] = fmaf(tv[i].y, sv.y, dot[i][j]);
+            dot[i][j] = fmaf(tv[i].z, sv.z, dot[i][j]);
+            dot[i][j] = fmaf(tv[i].w, sv.w, dot[i][j]);
+          }
+        }
       }
     }
 #pragma unroll
-    for (int t = 0; t < kQ; ++t) {
-      const int row = t0 + t;
-      a_s[row * (C + 1) + j] = (j < row && row < n) ? a[t] * beta_s[row] * expf(lg_s[row] - lg_s[j]) : 0.f;
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float total = dot[i][j];
+        total += __shfl_xor_sync(0xffffffffu, total, 1);
+        total += __shfl_xor_sync(0xffffffffu, total, 2);
+        const int t = t0 + i, s = s0 + j;
+        if (part == j) a_s[s * TL + t] = (s < t && t < n) ? total * beta_s[t] * expf(lg_s[t] - lg_s[s]) : 0.f;
+      }
+  }
+  __syncthreads();
+  if (tid < C) {            // column tid of T = (I + A)^-1: once a row is known it leaves all the rows below it
+    float x[C];
+#pragma unroll
+    for (int t = 0; t < C; ++t) x[t] = t == tid ? 1.f : 0.f;
+#pragma unroll
+    for (int s = 0; s < C - 1; ++s) {
+#pragma unroll
+      for (int t4 = (s + 1) / 4 * 4; t4 < C; t4 += 4) {
+        const float4 m = *reinterpret_cast<const float4*>(a_s + s * TL + t4);
+        if (t4 > s) x[t4] = fmaf(-m.x, x[s], x[t4]);
+        if (t4 + 1 > s) x[t4 + 1] = fmaf(-m.y, x[s], x[t4 + 1]);
+        if (t4 + 2 > s) x[t4 + 2] = fmaf(-m.z, x[s], x[t4 + 2]);
+        x[t4 + 3] = fmaf(-m.w, x[s], x[t4 + 3]);
+      }
+    }
+    const float beta = beta_s[tid], bc = beta * expf(lg_s[tid]);
+#pragma unroll
+    for (int t = 0; t < C; t += 4) {
+      *reinterpret_cast<float4*>(tv_s + tid * TL + t) = make_float4(x[t] * beta, x[t + 1] * beta, x[t + 2] * beta, x[t + 3] * beta);
+      *reinterpret_cast<float4*>(tk_s + tid * TL + t) = make_float4(x[t] * bc, x[t + 1] * bc, x[t + 2] * bc, x[t + 3] * bc);
     }
   }
   __syncthreads();
-  if (tid < C) {            // column tid of T = (I + A)^-1: T_tj = [t = j] - sum_(s<t) A_ts T_sj
-    float col[C];
+  // U' and W: a thread 8 tokens and 4 columns of [V, K]; 12 cycles of loads for 32 products of a warp
+  const int pieces = (vdim + P) / 4, groups = (pieces + 31) / 32 * 4;
+  for (int item = warp; item < groups; item += 8) {
+    const int piece = item / 4 * 32 + lane, t0 = (item & 3) * 8;
+    if (piece >= pieces || t0 >= n) continue;
+    const bool value = piece < vdim / 4;
+    const int c = value ? piece * 4 : piece * 4 - vdim, ld = value ? vdim : kd;
+    const float* x = (value ? v_s : k_s) + c;
+    const float* m = (value ? tv_s : tk_s) + t0;
+    float4 acc[8];
 #pragma unroll
-    for (int t = 0; t < C; ++t) {
-      float x = t == tid ? 1.f : 0.f;
+    for (int i = 0; i < 8; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](int j, int from) {        // token j to tokens t0 + from and later
+      const float4 xv = *reinterpret_cast<const float4*>(x + j * ld);
+      const float4 lo = *reinterpret_cast<const float4*>(m + j * TL), hi = *reinterpret_cast<const float4*>(m + j * TL + 4);
+      const float w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-      for (int j = 0; j < t; ++j) x = fmaf(-a_s[t * (C + 1) + j], col[j], x);
-      col[t] = x;
-      t_s[t * (C + 1) + tid] = x;
-    }
-  }
-  __syncthreads();
-  const int wide = vdim + P;
-  for (int e = tid; e < n * wide; e += blockDim.x) {
-    const int t = e / wide, c = e % wide;
-    float acc = 0.f;
-    if (c < vdim) {
-      for (int j = 0; j <= t; ++j) acc = fmaf(t_s[t * (C + 1) + j] * beta_s[j], v_s[j * vdim + c], acc);
-      u_out[((size_t)(row0 + t) * heads + head) * vdim + c] = acc;
-    } else {
-      const int x = c - vdim;
-      for (int j = 0; j <= t; ++j) acc = fmaf(t_s[t * (C + 1) + j] * bc_s[j], k_s[j * kd + x], acc);
-      w_out[((size_t)(row0 + t) * heads + head) * P + x] = acc;
-    }
+      for (int i = 0; i < 8; ++i) {
+        if (i < from) continue;
+        acc[i].x = fmaf(w[i], xv.x, acc[i].x);
+        acc[i].y = fmaf(w[i], xv.y, acc[i].y);
+        acc[i].z = fmaf(w[i], xv.z, acc[i].z);
+        acc[i].w = fmaf(w[i], xv.w, acc[i].w);
+      }
+    };
+#pragma unroll 4
+    for (int j = 0; j < t0; ++j) add(j, 0);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) add(t0 + q, q);
+    float* dst = value ? u_out + c : w_out + c;
+    const int width = value ? vdim : P;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (t0 + i < n) *reinterpret_cast<float4*>(dst + ((size_t)(row0 + t0 + i) * heads + head) * width) = acc[i];
   }
 }
 
-// grid (requests, heads, blocks of kWalkColumns value columns); warp w keeps kWalkRows state rows of the block's
-// columns in registers, a lane a column.  What a chunk brings (W, k, U', the summed log decays) comes
-// through two cp.async stages, a chunk ahead.
-__global__ void __launch_bounds__(kWalkWarps * 32)
-delta_chunk_walk_kernel(const float* __restrict__ packed, int tokens, int row_floats, int P,
-                        const float* __restrict__ gates, const float* __restrict__ w_in, float* __restrict__ u_io,
-                        float* __restrict__ before, float* __restrict__ state, long long state_stride,
+// grid (requests, heads, blocks of kWalkColumns value columns), P threads; a thread keeps 8 rows of 4 columns of S in
+// registers (a warp 32 rows, eight lanes a row): 8 cycles of loads for 32 products of a warp against W, 12 against k.  (A
+// lane a column of 8 rows, as this kernel first was, takes 8 cycles for 8 products and a partial sum of every warp.)  What
+// a chunk brings (W, k, U', the summed log decays) comes through two cp.async stages, a chunk ahead.
+__global__ void __launch_bounds__(kMemDim)
+gated_delta_walk_kernel(const float* __restrict__ unit, int tokens, int P, const float* __restrict__ gates,
+                        const float* __restrict__ w_in, float* __restrict__ u_io, float* __restrict__ before,
+                        float* __restrict__ state, long long state_stride,
                         const int* __restrict__ request_chunk_start, const int* __restrict__ chunk_row,
                         const int* __restrict__ chunk_count, const int* __restrict__ slots,
                         const int* __restrict__ request_active, int heads, int dim, int vdim, int max_slots, int* err) {
-  constexpr int C = kMemChunk, kRows = kWalkRows, kCols = kWalkColumns;
+  constexpr int C = kMemChunk, kCols = kWalkColumns;
   extern __shared__ __align__(16) float smem[];
-  const int stage_floats = 2 * C * P + C * kCols + C * kMemGates;
+  const int stage_floats = gated_walk_stage(P);
   float* part_s = smem + 2 * stage_floats;        // [warps][C][kCols]
-  float* u_s = part_s + kWalkWarps * C * kCols;   // [C][kCols]
-  __shared__ float weight_s[C];
+  float* u_s = part_s + P / 32 * C * kCols;       // [C][kCols]: u_t c_C / c_t
   pdl_wait();
   pdl_trigger();
   const int request = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * kCols, tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31, column = col0 + lane, r0 = warp * kRows;
+  const int warp = tid >> 5, lane = tid & 31, warps = P / 32, rg = lane >> 3;
+  const int c = (lane & 7) * 4, column = col0 + c, r0 = warp * 32 + rg * 8;
   const int slot = slots[request];
   if (slot < 0 || slot >= max_slots) {
     if (tid == 0) atomicOr(err, kErrBadRequest);
     return;
   }
-  const bool live = column < vdim;
-  const int warps = P / kRows;                     // warps that hold rows
-  float* s_base = state + (size_t)slot * state_stride + (size_t)head * dim * vdim;
-  float s[kRows];
+  const bool live = column < vdim;                // whole pieces of four, as vdim is
+  float* s_base = state + (size_t)slot * state_stride + (size_t)head * dim * vdim + column;
+  float4 s[8];
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) s[r] = (live && r0 + r < dim) ? s_base[(size_t)(r0 + r) * vdim + column] : 0.f;
+  for (int r = 0; r < 8; ++r) {
+    s[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live && r0 + r < dim) {
+      const float* src = s_base + (size_t)(r0 + r) * vdim;
+      s[r] = make_float4(src[0], src[1], src[2], src[3]);
+    }
+  }
   const int first = request_chunk_start[request], last = request_chunk_start[request + 1];
-  const float* rows = packed + (size_t)head * tokens * row_floats;
+  const float* rows = unit + (size_t)head * tokens * 2 * P;
   const int columns = min(kCols, vdim - col0);     // a multiple of 4, as vdim is
   auto issue = [&](int chunk) {
     if (chunk < last) {
       float* dst = smem + (size_t)((chunk - first) & 1) * stage_floats;
       const int row0 = chunk_row[chunk], n = chunk_count[chunk];
       const int pw = P / 4, pu = columns / 4;
-      for (int c = tid; c < n * pw; c += blockDim.x) {
-        const int t = c / pw, piece = c % pw;
+      for (int e = tid; e < n * pw; e += blockDim.x) {
+        const int t = e / pw, piece = e % pw;
         stream_cp_async16(dst + t * P + 4 * piece, w_in + ((size_t)(row0 + t) * heads + head) * P + 4 * piece);
-        stream_cp_async16(dst + C * P + t * P + 4 * piece, rows + (size_t)(row0 + t) * row_floats + 4 * piece);
+        stream_cp_async16(dst + C * P + t * P + 4 * piece, rows + (size_t)(row0 + t) * 2 * P + 4 * piece);
       }
-      for (int c = tid; c < n * pu; c += blockDim.x) {
-        const int t = c / pu, piece = c % pu;
+      for (int e = tid; e < n * pu; e += blockDim.x) {
+        const int t = e / pu, piece = e % pu;
         stream_cp_async16(dst + 2 * C * P + t * kCols + 4 * piece,
                           u_io + ((size_t)(row0 + t) * heads + head) * vdim + col0 + 4 * piece);
       }
@@ -1170,48 +1269,72 @@ delta_chunk_walk_kernel(const float* __restrict__ packed, int tokens, int row_fl
     issue(chunk + 1);
     asm volatile("cp.async.wait_group 1;\n" ::);
     __syncthreads();
-    if (warp < warps) {
-      float* dst = before + ((size_t)chunk * heads + head) * dim * vdim;
+    if (live) {
+      float* dst = before + ((size_t)chunk * heads + head) * dim * vdim + column;
 #pragma unroll
-      for (int r = 0; r < kRows; ++r)
-        if (live && r0 + r < dim) dst[(size_t)(r0 + r) * vdim + column] = s[r];
-      for (int t = 0; t < n; ++t) {
-        float acc = 0.f;
+      for (int r = 0; r < 8; ++r)
+        if (r0 + r < dim) *reinterpret_cast<float4*>(dst + (size_t)(r0 + r) * vdim) = s[r];
+    }
+    // W S: four tokens at a time (rows past n hold anything: their sums are not read); the four lanes that share the
+    // columns leave a token each
+    for (int t0 = 0; t0 < n; t0 += 4) {
+      float4 acc[4];
 #pragma unroll
-        for (int r = 0; r < kRows; r += 4) {
-          const float4 w4 = *reinterpret_cast<const float4*>(w_s + t * P + r0 + r);
-          acc = fmaf(w4.x, s[r], acc);
-          acc = fmaf(w4.y, s[r + 1], acc);
-          acc = fmaf(w4.z, s[r + 2], acc);
-          acc = fmaf(w4.w, s[r + 3], acc);
+      for (int i = 0; i < 4; ++i) {
+        const float4 lo = *reinterpret_cast<const float4*>(w_s + (t0 + i) * P + r0), hi = *reinterpret_cast<const float4*>(w_s + (t0 + i) * P + r0 + 4);
+        const float w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          acc[i].x = fmaf(w[r], s[r].x, acc[i].x);
+          acc[i].y = fmaf(w[r], s[r].y, acc[i].y);
+          acc[i].z = fmaf(w[r], s[r].z, acc[i].z);
+          acc[i].w = fmaf(w[r], s[r].w, acc[i].w);
         }
-        part_s[(warp * C + t) * kCols + lane] = acc;
       }
+      auto merge = [&](float4& keep, const float4& give, int lanes) {
+        keep.x += __shfl_xor_sync(0xffffffffu, give.x, lanes);
+        keep.y += __shfl_xor_sync(0xffffffffu, give.y, lanes);
+        keep.z += __shfl_xor_sync(0xffffffffu, give.z, lanes);
+        keep.w += __shfl_xor_sync(0xffffffffu, give.w, lanes);
+      };
+      const bool odd = rg & 1, upper = rg & 2;
+      float4 even_keep = odd ? acc[1] : acc[0], high_keep = odd ? acc[3] : acc[2];
+      merge(even_keep, odd ? acc[0] : acc[1], 8);
+      merge(high_keep, odd ? acc[2] : acc[3], 8);
+      float4 keep = upper ? high_keep : even_keep;
+      merge(keep, upper ? even_keep : high_keep, 16);
+      *reinterpret_cast<float4*>(part_s + (warp * C + t0 + rg) * kCols + c) = keep;
     }
     __syncthreads();
-    if (tid < n) weight_s[tid] = expf(g_s[(n - 1) * kMemGates + 1] - g_s[tid * kMemGates + 1]);
-    for (int t = warp; t < n; t += kWalkWarps) {
-      float u = ut_s[t * kCols + lane];
-      for (int w = 0; w < warps; ++w) u -= part_s[(w * C + t) * kCols + lane];
-      u_s[t * kCols + lane] = u;
-      if (live) u_io[((size_t)(row0 + t) * heads + head) * vdim + column] = u;
+    const float lg_last = g_s[(n - 1) * kMemGates + 1];
+    for (int t = tid >> 3; t < n; t += P / 8) {
+      float4 u = *reinterpret_cast<const float4*>(ut_s + t * kCols + c);
+      for (int w = 0; w < warps; ++w) {
+        const float4 x = *reinterpret_cast<const float4*>(part_s + (w * C + t) * kCols + c);
+        u.x -= x.x; u.y -= x.y; u.z -= x.z; u.w -= x.w;
+      }
+      if (live) *reinterpret_cast<float4*>(u_io + ((size_t)(row0 + t) * heads + head) * vdim + column) = u;
+      const float weight = expf(lg_last - g_s[t * kMemGates + 1]);
+      *reinterpret_cast<float4*>(u_s + t * kCols + c) = make_float4(u.x * weight, u.y * weight, u.z * weight, u.w * weight);
     }
     __syncthreads();
-    if (warp < warps) {
-      const float lg_last = g_s[(n - 1) * kMemGates + 1];
-      const float keep = expf(lg_last);
+    const float keep = expf(lg_last);
 #pragma unroll
-      for (int r = 0; r < kRows; ++r) s[r] *= keep;
-      for (int t = 0; t < n; ++t) {
-        const float u = u_s[t * kCols + lane] * weight_s[t];
+    for (int r = 0; r < 8; ++r) {
+      s[r].x *= keep; s[r].y *= keep; s[r].z *= keep; s[r].w *= keep;
+    }
+#pragma unroll 4
+    for (int t = 0; t < n; ++t) {
+      const float4 u = *reinterpret_cast<const float4*>(u_s + t * kCols + c);
+      const float4 lo = *reinterpret_cast<const float4*>(k_s + t * P + r0), hi = *reinterpret_cast<const float4*>(k_s + t * P + r0 + 4);
+      const float k[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-        for (int r = 0; r < kRows; r += 4) {
-          const float4 k4 = *reinterpret_cast<const float4*>(k_s + t * P + r0 + r);
-          s[r] = fmaf(k4.x, u, s[r]);
-          s[r + 1] = fmaf(k4.y, u, s[r + 1]);
-          s[r + 2] = fmaf(k4.z, u, s[r + 2]);
-          s[r + 3] = fmaf(k4.w, u, s[r + 3]);
-        }
+      for (int r = 0; r < 8; ++r) {
+        s[r].x = fmaf(k[r], u.x, s[r].x);
+        s[r].y = fmaf(k[r], u.y, s[r].y);
+        s[r].z = fmaf(k[r], u.z, s[r].z);
+        s[r].w = fmaf(k[r], u.w, s[r].w);
       }
     }
     __syncthreads();        // everybody is done with this chunk's stage and with u_s before they are filled again
@@ -1219,37 +1342,13 @@ delta_chunk_walk_kernel(const float* __restrict__ packed, int tokens, int row_fl
   asm volatile("cp.async.wait_group 0;\n" ::);
   if (!request_active[request] || !live) return;
 #pragma unroll
-  for (int r = 0; r < kRows; ++r)
-    if (r0 + r < dim) s_base[(size_t)(r0 + r) * vdim + column] = s[r];
+  for (int r = 0; r < 8; ++r)
+    if (r0 + r < dim) {
+      float* dst = s_base + (size_t)(r0 + r) * vdim;
+      dst[0] = s[r].x; dst[1] = s[r].y; dst[2] = s[r].z; dst[3] = s[r].w;
+    }
 }
 
-// ---------------------------------------------------------------- per-head norm x gain x gate
-// out[t][g*size + i] = gain * o / rms(o over the head) * act(gate); gain index i (shared) or g*size + i.  With
-// `denominators` [tokens][heads], o is first divided by its token's and head's number.
-// act 0: sigmoid(z), 1: z * sigmoid(z).  A warp per (token, head).
-template <typename T>
-__global__ void __launch_bounds__(32)
-head_norm_gate_kernel(const float* __restrict__ o, int o_stride, const float* __restrict__ denominators,
-                      const float* __restrict__ gate, int gate_stride, const float* __restrict__ gain, int gain_shared,
-                      int act, T* __restrict__ out, int out_stride, int size, float eps) {
-  pdl_wait();
-  pdl_trigger();
-  const int t = blockIdx.x, g = blockIdx.y, lane = threadIdx.x;
-  const float* row = o + (size_t)t * o_stride + (size_t)g * size;
-  const float below = denominators ? denominators[(size_t)t * gridDim.y + g] : 1.f;
-  float sq = 0.f;
-  for (int i = lane; i < size; i += 32) {
-    const float x = row[i] / below;
-    sq = fmaf(x, x, sq);
-  }
-  const float inv = rsqrtf(warp_sum(sq) / (float)size + eps);
-  for (int i = lane; i < size; i += 32) {
-    const int c = g * size + i;
-    const float z = gate[(size_t)t * gate_stride + c];
-    const float a = act ? z * sigmoid_f(z) : sigmoid_f(z);
-    out[(size_t)t * out_stride + c] = from_float<T>(gain[gain_shared ? i : c] * ((row[i] / below) * inv) * a);
-  }
-}
 
 }  // namespace cie
 
@@ -1355,8 +1454,7 @@ extern "C" int cie_mlstm_chunked(const float* proj, int proj_stride, int q_off, 
 // Floats of scratch memory the gated delta rule in chunks wants: the prepared rows, every token's summed log decays,
 // W and U per token, and the state before every chunk.
 extern "C" long long cie_gated_delta_chunk_floats(int tokens, int chunks, int heads, int dim, int vdim) {
-  const long long row = 2 * stream_pad(dim) + kStreamGates + stream_value_pad(dim, vdim, false);
-  return (long long)tokens * heads * (row + kMemGates + stream_pad(dim) + vdim) + (long long)chunks * heads * dim * vdim;
+  return (long long)tokens * heads * (3 * stream_pad(dim) + kMemGates + vdim) + (long long)chunks * heads * dim * vdim;
 }
 
 // The gated delta rule over a step with prompt portions, in chunks of cie_mlstm_chunk_tokens() tokens (work lists as
@@ -1375,34 +1473,29 @@ extern "C" int cie_gated_delta_chunked(const float* conv, int conv_stride, int q
   if (heads < 1 || heads > 65535 || kv_heads < 1 || heads % kv_heads)
     CIE_FAIL("gated_delta_chunked: %d heads do not divide over %d q/k heads", heads, kv_heads);
   cudaStream_t s = (cudaStream_t)stream;
-  const int P = stream_pad(dim), row_floats = 2 * P + kStreamGates + stream_value_pad(dim, vdim, false);
-  float* packed = scratch;
-  float* gates = packed + (size_t)tokens * heads * row_floats;
+  const int P = stream_pad(dim);
+  float* unit = scratch;
+  float* gates = unit + (size_t)tokens * heads * 2 * P;
   float* w = gates + (size_t)tokens * heads * kMemGates;
   float* u = w + (size_t)tokens * heads * P;
   float* before = u + (size_t)tokens * heads * vdim;
-  const size_t smem2 = (size_t)(kMemChunk * (vdim + P + 1) + 2 * kMemChunk * (kMemChunk + 1)) * sizeof(float);
-  const size_t smem3 = (size_t)(2 * (2 * kMemChunk * P + kMemChunk * kWalkColumns + kMemChunk * kMemGates) +
-                                (kWalkWarps + 1) * kMemChunk * kWalkColumns) * sizeof(float);
-  const size_t smem4 = chunk_output_smem(dim, vdim);
-  if (cudaFuncSetAttribute(delta_chunk_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess ||
-      cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) != cudaSuccess ||
-      cudaFuncSetAttribute(chunk_output_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4) != cudaSuccess)
-    CIE_FAIL("gated_delta_chunked: cannot reserve %zu / %zu / %zu bytes of shared memory", smem2, smem3, smem4);
-  CIE_LAUNCH("gated_delta_prepare", gated_delta_prepare_kernel, dim3(tokens, heads), dim3(128), 0, s, conv, conv_stride,
-             q_off, k_off, v_off, proj, proj_stride, b_off, a_off, a_log, dt_bias, q_scale, packed, tokens, heads, kv_heads,
-             dim, vdim);
+  const size_t smem1 = gated_solve_floats(P, vdim) * sizeof(float), smem2 = gated_walk_floats(P) * sizeof(float);
+  const size_t smem3 = chunk_output_smem(dim, vdim);
+  if (cudaFuncSetAttribute(gated_delta_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess ||
+      cudaFuncSetAttribute(gated_delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess ||
+      cudaFuncSetAttribute(chunk_output_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) != cudaSuccess)
+    CIE_FAIL("gated_delta_chunked: cannot reserve %zu / %zu / %zu bytes of shared memory", smem1, smem2, smem3);
   const dim3 grid(chunks, heads);
-  CIE_LAUNCH("delta_chunk_solve", delta_chunk_solve_kernel, grid, dim3(256), smem2, s, (const float*)packed, tokens,
-             row_floats, P, gates, w, u, chunk_row, chunk_count, heads, vdim);
-  CIE_LAUNCH("delta_chunk_walk", delta_chunk_walk_kernel, dim3(requests, heads, (vdim + kWalkColumns - 1) / kWalkColumns),
-             dim3(kWalkWarps * 32), smem3, s, (const float*)packed, tokens, row_floats, P, (const float*)gates, (const float*)w, u,
-             before, state, state_stride, request_chunk_start, chunk_row, chunk_count, slots, request_active, heads, dim,
-             vdim, max_slots, err);
-  const RowsOf q_rows{packed, (long long)tokens * row_floats, row_floats, P, 0};
-  const RowsOf k_rows{packed, (long long)tokens * row_floats, row_floats, 0, 0};
+  CIE_LAUNCH("gated_delta_solve", gated_delta_solve_kernel, grid, dim3(256), smem1, s, conv, conv_stride, q_off, k_off, v_off,
+             proj, proj_stride, b_off, a_off, a_log, dt_bias, q_scale, unit, tokens, P, gates, w, u, chunk_row, chunk_count,
+             heads, kv_heads, dim, vdim);
+  CIE_LAUNCH("gated_delta_walk", gated_delta_walk_kernel, dim3(requests, heads, (vdim + kWalkColumns - 1) / kWalkColumns),
+             dim3(P), smem2, s, (const float*)unit, tokens, P, (const float*)gates, (const float*)w, u, before, state,
+             state_stride, request_chunk_start, chunk_row, chunk_count, slots, request_active, heads, dim, vdim, max_slots, err);
+  const RowsOf q_rows{unit, (long long)tokens * 2 * P, 2 * P, P, 0};
+  const RowsOf k_rows{unit, (long long)tokens * 2 * P, 2 * P, 0, 0};
   const RowsOf v_rows{u, 0, heads * vdim, 0, vdim};
-  CIE_LAUNCH("delta_chunk_output", chunk_output_kernel<false>, grid, dim3(kMemWarps * 32), smem4, s, q_rows, k_rows, v_rows,
+  CIE_LAUNCH("delta_chunk_output", chunk_output_kernel<false>, grid, dim3(kMemWarps * 32), smem3, s, q_rows, k_rows, v_rows,
              1.f, (const float*)gates, (const float*)before, out, out_stride, chunk_row, chunk_count, heads, dim, vdim);
   return 0;
 }
