@@ -1017,6 +1017,7 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
 // token to t, the rule's writes u_t obey  u_t = b_t (v_t - c_t S_0^T k_t - sum_(s<t) (c_t / c_s) (k_s . k_t) u_s),  a
 // triangular system:  (I + A) U = diag(b) (V - diag(c) K S_0),  A_ts = b_t (c_t / c_s) (k_t . k_s) for s < t.  With
 // T = (I + A)^-1:  U = T diag(b) V - (T diag(b c) K) S_0 = U' - W S_0.  So:
+//   0. per (chunk, head):      the summed logarithms of the decays, the write strengths
 //   1. per (chunk, head):      unit k and q; A, T by forward substitution (a lane a column of T), U' and W
 //   2. per (request, head, 32 value columns): walks the chunks with its columns of S in registers:
 //                              U = U' - W S_0,  S <- c_C S_0 + sum_s (c_C / c_s) k_s u_s^T; leaves S_0 of every chunk
@@ -1040,13 +1041,36 @@ __host__ __device__ constexpr int gated_walk_floats(int P) {
   return 2 * gated_walk_stage(P) + (P / 32 + 1) * kMemChunk * kWalkColumns;
 }
 
+// grid (chunks, blocks of 8 heads): a warp a head, a lane a token.  gates: as the outputs read them (i = m = 0).
+__global__ void __launch_bounds__(256)
+gated_delta_gates_kernel(const float* __restrict__ proj, int proj_stride, int b_off, int a_off,
+                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ gates,
+                         float* __restrict__ strength, const int* __restrict__ chunk_row,
+                         const int* __restrict__ chunk_count, int heads) {
+  pdl_wait();
+  pdl_trigger();
+  const int head = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (head >= heads) return;
+  const int row = chunk_row[blockIdx.x] + lane;
+  const bool in = lane < chunk_count[blockIdx.x];
+  const float* z = proj + (size_t)row * proj_stride;
+  const float g = in ? -expf(a_log[head]) * softplus_f(z[a_off + head] + dt_bias[head]) : 0.f;
+  float sum = 0.f;
+#pragma unroll
+  for (int r = 0; r < kMemChunk; ++r) {
+    const float x = __shfl_sync(0xffffffffu, g, r);
+    if (r <= lane) sum += x;
+  }
+  if (!in) return;
+  *reinterpret_cast<float4*>(gates + ((size_t)row * heads + head) * kMemGates) = make_float4(0.f, sum, 0.f, 0.f);
+  strength[(size_t)row * heads + head] = sigmoid_f(z[b_off + head]);
+}
+
 // grid (chunks, heads).  unit: [head][token][k: P][q: P], zeros past dim.
 __global__ void __launch_bounds__(256)
-gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_off, int k_off, int v_off,
-                         const float* __restrict__ proj, int proj_stride, int b_off, int a_off,
-                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float q_scale,
-                         float* __restrict__ unit, int tokens, int P, float* __restrict__ gates,
-                         float* __restrict__ w_out, float* __restrict__ u_out, const int* __restrict__ chunk_row,
+gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_off, int k_off, int v_off, float q_scale,
+                         float* __restrict__ unit, int tokens, int P, const float* __restrict__ gates,
+                         const float* __restrict__ strength, float* __restrict__ w_out, float* __restrict__ u_out, const int* __restrict__ chunk_row,
                          const int* __restrict__ chunk_count, int heads, int kv_heads, int dim, int vdim) {
   constexpr int C = kMemChunk, TL = kSolveRow;
   extern __shared__ __align__(16) float smem[];
@@ -1061,21 +1085,9 @@ gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_
   pdl_trigger();
   const int chunk = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row0 = chunk_row[chunk], n = chunk_count[chunk], base = (head / (heads / kv_heads)) * dim;
-  if (warp == 0) {
-    float g = 0.f, beta = 0.f, lg = 0.f;
-    if (lane < n) {
-      const float* row = proj + (size_t)(row0 + lane) * proj_stride;
-      g = -expf(a_log[head]) * softplus_f(row[a_off + head] + dt_bias[head]);      // log of the decay
-      beta = sigmoid_f(row[b_off + head]);
-    }
-#pragma unroll
-    for (int r = 0; r < C; ++r) {
-      const float x = __shfl_sync(0xffffffffu, g, r);
-      if (r <= lane) lg += x;
-    }
-    lg_s[lane] = lg;
-    beta_s[lane] = beta;
-    if (lane < n) *reinterpret_cast<float4*>(gates + ((size_t)(row0 + lane) * heads + head) * kMemGates) = make_float4(0.f, lg, 0.f, 0.f);
+  if (tid < C) {
+    lg_s[tid] = tid < n ? gates[((size_t)(row0 + tid) * heads + head) * kMemGates + 1] : 0.f;
+    beta_s[tid] = tid < n ? strength[(size_t)(row0 + tid) * heads + head] : 0.f;
   }
 #pragma unroll
   for (int i = 0; i < C / 8; ++i) {        // unit k and q, the squares in the order of the scan
@@ -1454,7 +1466,7 @@ extern "C" int cie_mlstm_chunked(const float* proj, int proj_stride, int q_off, 
 // Floats of scratch memory the gated delta rule in chunks wants: the prepared rows, every token's summed log decays,
 // W and U per token, and the state before every chunk.
 extern "C" long long cie_gated_delta_chunk_floats(int tokens, int chunks, int heads, int dim, int vdim) {
-  return (long long)tokens * heads * (3 * stream_pad(dim) + kMemGates + vdim) + (long long)chunks * heads * dim * vdim;
+  return (long long)tokens * heads * (3 * stream_pad(dim) + kMemGates + 1 + vdim) + (long long)chunks * heads * dim * vdim;
 }
 
 // The gated delta rule over a step with prompt portions, in chunks of cie_mlstm_chunk_tokens() tokens (work lists as
@@ -1479,6 +1491,7 @@ extern "C" int cie_gated_delta_chunked(const float* conv, int conv_stride, int q
   float* w = gates + (size_t)tokens * heads * kMemGates;
   float* u = w + (size_t)tokens * heads * P;
   float* before = u + (size_t)tokens * heads * vdim;
+  float* strength = before + (size_t)chunks * heads * dim * vdim;
   const size_t smem1 = gated_solve_floats(P, vdim) * sizeof(float), smem2 = gated_walk_floats(P) * sizeof(float);
   const size_t smem3 = chunk_output_smem(dim, vdim);
   if (cudaFuncSetAttribute(gated_delta_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess ||
@@ -1486,9 +1499,11 @@ extern "C" int cie_gated_delta_chunked(const float* conv, int conv_stride, int q
       cudaFuncSetAttribute(chunk_output_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) != cudaSuccess)
     CIE_FAIL("gated_delta_chunked: cannot reserve %zu / %zu / %zu bytes of shared memory", smem1, smem2, smem3);
   const dim3 grid(chunks, heads);
+  CIE_LAUNCH("gated_delta_gates", gated_delta_gates_kernel, dim3(chunks, (heads + 7) / 8), dim3(256), 0, s, proj, proj_stride,
+             b_off, a_off, a_log, dt_bias, gates, strength, chunk_row, chunk_count, heads);
   CIE_LAUNCH("gated_delta_solve", gated_delta_solve_kernel, grid, dim3(256), smem1, s, conv, conv_stride, q_off, k_off, v_off,
-             proj, proj_stride, b_off, a_off, a_log, dt_bias, q_scale, unit, tokens, P, gates, w, u, chunk_row, chunk_count,
-             heads, kv_heads, dim, vdim);
+             q_scale, unit, tokens, P, (const float*)gates, (const float*)strength, w, u, chunk_row, chunk_count, heads, kv_heads,
+             dim, vdim);
   CIE_LAUNCH("gated_delta_walk", gated_delta_walk_kernel, dim3(requests, heads, (vdim + kWalkColumns - 1) / kWalkColumns),
              dim3(P), smem2, s, (const float*)unit, tokens, P, (const float*)gates, (const float*)w, u, before, state,
              state_stride, request_chunk_start, chunk_row, chunk_count, slots, request_active, heads, dim, vdim, max_slots, err);

@@ -585,7 +585,7 @@ class Ops:
             reserve = int(self._gated_delta_chunk_floats(rows, -(-rows // self.mlstm_chunk_tokens) + ctx.num_requests,
                                                          heads, dim, vdim))
             scratch = self.scratch(f"recurrent.delta_chunks.{heads}x{dim}x{vdim}", floats, reserve=max(floats, reserve))
-            self.launches += 3
+            self.launches += 4
             self._gated_delta_chunked(_ptr(conv), conv.stride(0), q_off, k_off, v_off, _ptr(proj), proj.stride(0),
                                       b_off, a_off, _ptr(a_log), _ptr(dt_bias), float(q_scale), _ptr(scratch), _ptr(out),
                                       out.stride(0), _ptr(state), state.stride(0), _ptr(ctx.slots),
