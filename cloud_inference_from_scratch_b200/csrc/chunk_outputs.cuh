@@ -6,10 +6,10 @@
 // by a block of 256 threads (dim and vdim up to 128).  What bounds it is the data shared memory returns (128 bytes a cycle,
 // broadcast or not), so a thread takes 8 tokens and 4 columns: 12 cycles of loads for 32 products of a warp.  The warps form
 // two halves that take every second 16 rows of S (and every second token s) and add their sums up at the end.  S comes
-// once, 32 rows at a time, through two cp.async stages that are on their way while the weights are made; a warp that read
-// all of S for four tokens (as these kernels first did) asks L2 for the state eight times over.  Gated linear attention's
-// outputs of 2,048 tokens, 16 heads of 128 x 128, with their scores: 207 us that way, 116 us this way; the gated delta
-// rule's of 1,330 tokens 71 us.
+// once, 32 rows at a time, through two cp.async stages, which the callers lay over rows that they need no more: three blocks
+// fit an SM, and their waits overlap.  A warp that read all of S for four tokens (as these kernels first did) asks L2 for the
+// state eight times over.  Gated linear attention's outputs of 2,048 tokens, 16 heads of 128 x 128, with their scores: 207 us
+// that way, 116 with stages of their own (two blocks an SM), 99 this way; the gated delta rule's of 1,330 tokens 71 and 57.
 #pragma once
 
 #include "common.cuh"
@@ -20,15 +20,15 @@ constexpr int kOutTokens = 32, kOutThreads = 256, kOutRows = 32;      // tokens 
 constexpr int kOutWeights = kOutTokens + 4;                           // row of the weights: a_s[s * kOutWeights + t]
 
 __host__ __device__ __forceinline__ int pad4(int x) { return (x + 3) & ~3; }
-__host__ __device__ constexpr int out_ring_floats(int vdim) { return 2 * kOutRows * ((vdim + 3) & ~3); }
 
 // The stages of S: rows [dim][vdim] from global memory, vdim padded to whole 16-byte pieces, rows past dim zeros.
 struct StateRing {
-  float* ring;            // out_ring_floats(vdim)
+  float* first;           // the stages, kOutRows rows each
+  float* second;
   const float* state;
   int dim, vdim;
   __device__ __forceinline__ int blocks() const { return (dim + kOutRows - 1) / kOutRows; }
-  __device__ __forceinline__ float* stage(int block) const { return ring + (block & 1) * kOutRows * pad4(vdim); }
+  __device__ __forceinline__ float* stage(int block) const { return block & 1 ? second : first; }
   __device__ __forceinline__ void issue(int block) const {
     if (block < blocks()) {
       const int ld = pad4(vdim), first = block * kOutRows;
@@ -108,13 +108,13 @@ __device__ __forceinline__ void chunk_outputs(const StateRing& s, const float* q
   __syncthreads();            // the ring is free: the second half's sums go through it
   if (half == 1 && live) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(s.ring + (t0 + i) * ld + c) = acc[i];
+    for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(s.first + (t0 + i) * ld + c) = acc[i];
   }
   __syncthreads();
   if (half == 0 && live) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float4 other = *reinterpret_cast<const float4*>(s.ring + (t0 + i) * ld + c);
+      const float4 other = *reinterpret_cast<const float4*>(s.first + (t0 + i) * ld + c);
       write(t0 + i, c, make_float4(acc[i].x + other.x, acc[i].y + other.y, acc[i].z + other.z, acc[i].w + other.w));
     }
   }

@@ -292,7 +292,7 @@ __global__ void gla_chunk_prefix_kernel(float* __restrict__ chunk_state, const f
 }
 
 // (3) outputs of a chunk from the state before it and the chunk's own tokens
-__global__ void __launch_bounds__(kOutThreads)
+__global__ void __launch_bounds__(kOutThreads, 3)
 gla_chunk_output_kernel(GlaRows in, float* __restrict__ out, int out_stride, const float* __restrict__ chunk_state,
                         const int* __restrict__ chunk_row, const int* __restrict__ chunk_count, int heads, int dim,
                         int vdim) {
@@ -300,16 +300,15 @@ gla_chunk_output_kernel(GlaRows in, float* __restrict__ out, int out_stride, con
   extern __shared__ __align__(16) float smem[];
   const int ld = pad4(dim), vld = pad4(vdim);
   float* q_s = smem;                              // [kChunk][ld]
-  float* k_s = q_s + kChunk * ld;
-  float* b_s = k_s + kChunk * ld;
-  float* v_s = b_s + kChunk * ld;                 // [kChunk][vld]
+  float* v_s = q_s + kChunk * ld;                 // [kChunk][vld]
   float* a_s = v_s + kChunk * vld;                // [kChunk][kOutWeights]
+  float* k_s = a_s + kChunk * kOutWeights;        // [kChunk][ld], then stages of the state: three blocks fit an SM
+  float* b_s = k_s + kChunk * max(ld, vld);       // the same
   pdl_wait();
   pdl_trigger();
   const int chunk = blockIdx.x, head = blockIdx.y;
   const int row0 = chunk_row[chunk], n = chunk_count[chunk];
-  const StateRing ring{a_s + kChunk * kOutWeights, chunk_state + ((size_t)chunk * heads + head) * dim * vdim, dim, vdim};
-  ring.issue(0);
+  const StateRing ring{k_s, b_s, chunk_state + ((size_t)chunk * heads + head) * dim * vdim, dim, vdim};
   stage_rows(q_s, ld, in.proj, in.proj_stride, row0, n, in.q_off + head * dim, dim, in.q_scale);
   stage_rows(k_s, ld, in.proj, in.proj_stride, row0, n, in.k_off + head * dim, dim, 1.f);
   stage_rows(v_s, vld, in.proj, in.proj_stride, row0, n, in.v_off + head * vdim, vdim, 1.f);
@@ -359,6 +358,7 @@ gla_chunk_output_kernel(GlaRows in, float* __restrict__ out, int out_stride, con
       }
   }
   __syncthreads();
+  ring.issue(0);
   // what the carried state is read with: q_i * exp(b_i)
   for (int e = threadIdx.x; e < n * ld; e += kOutThreads) q_s[e] *= exp2f(b_s[e]);
   // (chunk_outputs meets before it reads)
@@ -417,7 +417,7 @@ extern "C" int cie_gla_chunked(const float* proj, int proj_stride, int q_off, in
     CIE_FAIL("gla_chunked: key / value sizes %d / %d are above %d", dim, vdim, kChunkDim);
   cudaStream_t s = (cudaStream_t)stream;
   const size_t smem1 = (size_t)kChunk * (dim + vdim) * sizeof(float);
-  const size_t smem3 = ((size_t)kChunk * (3 * pad4(dim) + pad4(vdim) + kOutWeights) + out_ring_floats(vdim)) * sizeof(float);
+  const size_t smem3 = (size_t)kChunk * (pad4(dim) + pad4(vdim) + kOutWeights + 2 * max(pad4(dim), pad4(vdim))) * sizeof(float);
   static bool raised = false;
   if (!raised) {
     if (cudaFuncSetAttribute(gla_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||

@@ -907,11 +907,11 @@ struct RowsOf {
 // Rows of q and k are `key_row(dim)` floats long: the rows that a load of eight lanes meets then lie in different banks.
 __host__ __device__ __forceinline__ int key_row(int dim) { return pad4(dim) % 8 == 0 ? pad4(dim) + 4 : pad4(dim); }
 static size_t chunk_output_smem(int dim, int vdim) {
-  return ((size_t)kMemChunk * (2 * key_row(dim) + pad4(vdim) + kOutWeights) + out_ring_floats(vdim)) * sizeof(float);
+  return (size_t)kMemChunk * (key_row(dim) + 2 * pad4(vdim) + kOutWeights + max(key_row(dim), pad4(vdim))) * sizeof(float);
 }
 
 template <bool kMemory>
-__global__ void __launch_bounds__(kOutThreads)
+__global__ void __launch_bounds__(kOutThreads, 3)
 chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
                     const float* __restrict__ gates, const float* __restrict__ chunk_sums,
                     float* __restrict__ out, int out_stride, const int* __restrict__ chunk_row,
@@ -920,9 +920,10 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
   extern __shared__ __align__(16) float smem[];
   const int ld = key_row(dim), padded = pad4(dim), vld = pad4(vdim);
   float* q_s = smem;                              // [kMemChunk][ld]
-  float* k_s = q_s + kMemChunk * ld;
-  float* v_s = k_s + kMemChunk * ld;              // [kMemChunk][vld]
+  float* v_s = q_s + kMemChunk * ld;              // [kMemChunk][vld]
   float* a_s = v_s + kMemChunk * vld;             // [kMemChunk][kOutWeights]
+  float* first_s = a_s + kMemChunk * kOutWeights; // [kOutRows][vld]
+  float* k_s = first_s + kOutRows * vld;          // [kMemChunk][ld], then the second stage of the state: three blocks fit an SM
   __shared__ float gi_s[kMemChunk], gb_s[kMemChunk], gm_s[kMemChunk], below_s[kMemChunk];
   __shared__ float m_before;
   pdl_wait();
@@ -931,7 +932,7 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
   const int row0 = chunk_row[chunk], n = chunk_count[chunk];
   const size_t cells = (size_t)dim * vdim + (kMemory ? dim : 0);
   const float* before = chunk_sums + ((size_t)chunk * heads + head) * cells;
-  const StateRing ring{a_s + kMemChunk * kOutWeights, before, dim, vdim};
+  const StateRing ring{first_s, k_s, before, dim, vdim};
   ring.issue(0);
   if (threadIdx.x < n) {
     const float4 g = *reinterpret_cast<const float4*>(gates + ((size_t)(row0 + threadIdx.x) * heads + head) * kMemGates);
