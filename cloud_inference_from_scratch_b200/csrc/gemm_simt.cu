@@ -1,7 +1,7 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) on the CUDA cores, float32 accumulation, any M, N, K.
 //
-// This is the whole-model 32-bit path's matrix product (no tensor cores, no TF32) and the
-// fallback of the bfloat16 path for shapes the tensor-core kernel refuses.  Each output element
+// This is the 32-bit path's matrix product for rows that the tensor-core form (gemm_f32_tcgen05.cu: whole aligned pieces, 512
+// columns and more) does not take, and the fallback of the bfloat16 path for shapes the tensor-core kernel refuses.  Each output element
 // is the sum over k in ascending order with one fused multiply-add per k, so a row's result does
 // not depend on how many other rows the call has or where the row sits in it, nor on the kernel and tile it is worked out in.
 // The reference runs these products through cuBLAS (src/cloud_engine/model.py:100,134-136,217,227).

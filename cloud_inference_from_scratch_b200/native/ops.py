@@ -118,6 +118,12 @@ class Ops:
         self._scaled_sum = ew.function("cie_scaled_sum", [v, v, f, f, ll, v])
         gs = _Lib(load_library("gemm_simt.cu"))
         self._gemm_simt = gs.function("cie_gemm_simt", [v, v, v, v, i, i, i, i, i, i, v])
+        self._gemm_f32 = None
+        if self.code == F32:
+            gf = _Lib(load_library("gemm_f32_tcgen05.cu"))
+            self._gemm_f32 = gf.function("cie_gemm_f32_tc", [v, v, v, v, i, i, i, i, v, v])
+            self._gemm_f32_takes = gf.handle.cie_gemm_f32_tc_takes
+            self._gemm_f32_takes.argtypes = [v, v, i]
         ag = _Lib(load_library("attention_generic.cu"))
         self._attention_generic_sink = ag.function(
             "cie_attention_generic_sink",
@@ -1678,6 +1684,10 @@ class Ops:
             self._cublas_linear(x, weight, bias, out)
             return out
         self.launches += 1
+        if (self._gemm_f32 is not None and x.dtype == weight.dtype == out.dtype == self.torch.float32
+                and self._gemm_f32_takes(_ptr(x), _ptr(weight), k)):
+            self._gemm_f32(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), m, n, k, 0, self.error_word.data_ptr(), self.stream)
+            return out
         self._gemm_simt(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), m, n, k, self._code_of(x),
                         self._code_of(out), 0 if self.code == F32 else 1, self.stream)
         return out
