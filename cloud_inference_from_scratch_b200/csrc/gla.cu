@@ -320,42 +320,71 @@ gla_chunk_output_kernel(GlaRows in, float* __restrict__ out, int out_stride, con
       q_s[at] = k_s[at] = b_s[at] = 0.f;
     }
   __syncthreads();
-  // a[i][j] = sum_d q_i[d] k_j[d] exp(b_i[d] - b_j[d]) for j <= i: eight lanes share two rows i and two rows j, a lane the
-  // 16-byte pieces lane, lane + 8, ..; one load from shared memory for two products and one exponential
-  const int lane8 = threadIdx.x & 7, blocks = (n + 1) / 2;
-  for (int p = threadIdx.x >> 3; p < blocks * (blocks + 1) / 2; p += kOutThreads / 8) {
+  // a[i][j] = sum_d q_i[d] k_j[d] exp(b_i[d] - b_j[d]) for j <= i, in tiles of 4 x 4 that a warp takes together, a lane the
+  // 16-byte pieces lane, lane + 32, ..  Below the diagonal the exponential is exp(b_i - b_r) exp(b_r - b_j) with r the last
+  // token of the columns' four: both exponents are at most zero, and a factor vanishes only where the product does; 8
+  // exponentials for 16 products instead of 16.  On the diagonal every pair has its own.
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, blocks = (n + 3) / 4;
+  for (int p = warp; p < blocks * (blocks + 1) / 2; p += kOutThreads / 32) {
     int bi = (int)((sqrtf(8.f * (float)p + 1.f) - 1.f) * 0.5f);
     while (bi * (bi + 1) / 2 > p) --bi;
     while ((bi + 1) * (bi + 2) / 2 <= p) ++bi;
-    const int i = 2 * bi, j = 2 * (p - bi * (bi + 1) / 2);
-    float dot[2][2] = {};
-    for (int x = lane8 * 4; x < ld; x += 32) {
-      float q[2][4], bq[2][4], k[2][4], bk[2][4];
+    const int bj = p - bi * (bi + 1) / 2, i0 = 4 * bi, j0 = 4 * bj;
+    float dot[16] = {};      // [i][j]
+    for (int x = lane * 4; x < ld; x += 128) {
+      float q[4][4], k[4][4];
+      if (bi != bj) {
+        float last[4];
+        *reinterpret_cast<float4*>(last) = *reinterpret_cast<const float4*>(b_s + (j0 + 3) * ld + x);
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        *reinterpret_cast<float4*>(q[r]) = *reinterpret_cast<const float4*>(q_s + (i + r) * ld + x);
-        *reinterpret_cast<float4*>(bq[r]) = *reinterpret_cast<const float4*>(b_s + (i + r) * ld + x);
-        *reinterpret_cast<float4*>(k[r]) = *reinterpret_cast<const float4*>(k_s + (j + r) * ld + x);
-        *reinterpret_cast<float4*>(bk[r]) = *reinterpret_cast<const float4*>(b_s + (j + r) * ld + x);
+        for (int r = 0; r < 4; ++r) {
+          float b[4];
+          *reinterpret_cast<float4*>(q[r]) = *reinterpret_cast<const float4*>(q_s + (i0 + r) * ld + x);
+          *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(b_s + (i0 + r) * ld + x);
+#pragma unroll
+          for (int y = 0; y < 4; ++y) q[r][y] *= exp2f(b[y] - last[y]);
+          *reinterpret_cast<float4*>(k[r]) = *reinterpret_cast<const float4*>(k_s + (j0 + r) * ld + x);
+          if (r == 3) continue;
+          *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(b_s + (j0 + r) * ld + x);
+#pragma unroll
+          for (int y = 0; y < 4; ++y) k[r][y] *= exp2f(last[y] - b[y]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) dot[4 * i + j] = fmaf(q[i][y], k[j][y], dot[4 * i + j]);
+      } else {
+        float b[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          *reinterpret_cast<float4*>(q[r]) = *reinterpret_cast<const float4*>(q_s + (i0 + r) * ld + x);
+          *reinterpret_cast<float4*>(k[r]) = *reinterpret_cast<const float4*>(k_s + (i0 + r) * ld + x);
+          *reinterpret_cast<float4*>(b[r]) = *reinterpret_cast<const float4*>(b_s + (i0 + r) * ld + x);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j <= i; ++j)
+#pragma unroll
+            for (int y = 0; y < 4; ++y)
+              dot[4 * i + j] = fmaf(q[i][y] * k[j][y], i == j ? 1.f : exp2f(b[i][y] - b[j][y]), dot[4 * i + j]);
       }
-#pragma unroll
-      for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int y = 0; y < 4; ++y) dot[r][c] = fmaf(q[r][y] * k[c][y], exp2f(bq[r][y] - bk[c][y]), dot[r][c]);
     }
-    const unsigned mine = 0xffu << (threadIdx.x & 24);      // the eight lanes: others of the warp may have no block left
+    // the lanes' sums: every step a lane gives half of its cells away
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int half = 8; half >= 1; half >>= 1) {
+      const bool upper = lane & (2 * half);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        float total = dot[r][c];
-        total += __shfl_xor_sync(mine, total, 1);
-        total += __shfl_xor_sync(mine, total, 2);
-        total += __shfl_xor_sync(mine, total, 4);
-        if (lane8 == 0 && j + c <= i + r) a_s[(j + c) * kOutWeights + i + r] = total;
+      for (int e = 0; e < half; ++e) {
+        const float mine = upper ? dot[e + half] : dot[e], other = upper ? dot[e] : dot[e + half];
+        dot[e] = mine + __shfl_xor_sync(0xffffffffu, other, 2 * half);
       }
+    }
+    const float total = dot[0] + __shfl_xor_sync(0xffffffffu, dot[0], 1);
+    const int i = i0 + (lane >> 3), j = j0 + (lane >> 1 & 3);      // the cell that the steps left here
+    if (!(lane & 1) && j <= i) a_s[j * kOutWeights + i] = total;
   }
   __syncthreads();
   ring.issue(0);
