@@ -9,7 +9,7 @@
 // once, 32 rows at a time, through two cp.async stages, which the callers lay over rows that they need no more: three blocks
 // fit an SM, and their waits overlap.  A warp that read all of S for four tokens (as these kernels first did) asks L2 for the
 // state eight times over.  Gated linear attention's outputs of 2,048 tokens, 16 heads of 128 x 128, with their scores: 207 us
-// that way, 116 with stages of their own (two blocks an SM), 99 this way; the gated delta rule's of 1,330 tokens 71 and 57.
+// that way, 116 with stages of their own (two blocks an SM), 79 this way; the gated delta rule's of 1,330 tokens 71 and 52.
 #pragma once
 
 #include "common.cuh"
@@ -20,6 +20,33 @@ constexpr int kOutTokens = 32, kOutThreads = 256, kOutRows = 32;      // tokens 
 constexpr int kOutWeights = kOutTokens + 4;                           // row of the weights: a_s[s * kOutWeights + t]
 
 __host__ __device__ __forceinline__ int pad4(int x) { return (x + 3) & ~3; }
+
+// Calls load(row, piece) and then store(row, piece, value) for the 16-byte pieces of n rows, four loads a thread in flight;
+// places by addition: a division a piece costs as much as the rest of the copy.
+template <typename Load, typename Store>
+__device__ __forceinline__ void each_piece(int n, int pieces, Load load, Store store) {
+  int r = threadIdx.x / pieces, c = threadIdx.x - r * pieces;
+  const int dr = blockDim.x / pieces, dc = blockDim.x - dr * pieces;
+  while (r < n) {
+    float4 v[4];
+    int row[4], piece[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      row[u] = r;
+      piece[u] = c;
+      if (r < n) v[u] = load(r, c);
+      r += dr;
+      c += dc;
+      if (c >= pieces) {
+        c -= pieces;
+        ++r;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (row[u] < n) store(row[u], piece[u], v[u]);
+  }
+}
 
 // The stages of S: rows [dim][vdim] from global memory, vdim padded to whole 16-byte pieces, rows past dim zeros.
 struct StateRing {
@@ -34,9 +61,13 @@ struct StateRing {
       const int ld = pad4(vdim), first = block * kOutRows;
       float* dst = stage(block);
       if (vdim % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0) {
-        const int pieces = vdim / 4;
-        for (int e = threadIdx.x; e < kOutRows * pieces; e += kOutThreads) {
-          const int r = e / pieces, c = (e - r * pieces) * 4;
+        const int pieces = vdim / 4, dr = kOutThreads / pieces, dc = (kOutThreads - dr * pieces) * 4;
+        int r = threadIdx.x / pieces, c = (threadIdx.x - r * pieces) * 4;
+        for (; r < kOutRows; r += dr, c += dc) {
+          if (c >= vdim) {
+            c -= vdim;
+            if (++r >= kOutRows) break;
+          }
           const bool in = first + r < dim;
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * ld + c)),
                        "l"(state + (in ? (size_t)(first + r) * vdim + c : 0)), "r"(in ? 16 : 0));

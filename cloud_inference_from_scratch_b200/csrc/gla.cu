@@ -126,13 +126,13 @@ constexpr int kChunkCols = kChunkDim / 32;              // value columns of a la
 __device__ __forceinline__ void stage_rows(float* __restrict__ dst, int ld, const float* __restrict__ src, int stride,
                                            int row0, int n, int col0, int width, float factor) {
   if (width % 4 == 0 && col0 % 4 == 0 && stride % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    const int pieces = width / 4;
-    for (int e = threadIdx.x; e < n * pieces; e += blockDim.x) {
-      const int j = e / pieces, i = (e % pieces) * 4;
-      float4 v = *reinterpret_cast<const float4*>(src + (size_t)(row0 + j) * stride + col0 + i);
-      v.x *= factor; v.y *= factor; v.z *= factor; v.w *= factor;
-      *reinterpret_cast<float4*>(dst + j * ld + i) = v;
-    }
+    const float* from = src + (size_t)row0 * stride + col0;
+    each_piece(
+        n, width / 4, [&](int j, int i) { return *reinterpret_cast<const float4*>(from + (size_t)j * stride + 4 * i); },
+        [&](int j, int i, float4 v) {
+          v.x *= factor; v.y *= factor; v.z *= factor; v.w *= factor;
+          *reinterpret_cast<float4*>(dst + j * ld + 4 * i) = v;
+        });
     return;
   }
   for (int e = threadIdx.x; e < n * width; e += blockDim.x) {

@@ -755,14 +755,14 @@ template <typename Factor>
 __device__ __forceinline__ void stage_rows(float* __restrict__ dst, int ld, const float* __restrict__ proj, int proj_stride,
                                            int row0, int n, int col0, int width, Factor factor) {
   if (width % 4 == 0 && col0 % 4 == 0 && proj_stride % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(proj) & 15) == 0) {
-    const int pieces = width / 4;
-    for (int e = threadIdx.x; e < n * pieces; e += blockDim.x) {
-      const int j = e / pieces, i = (e % pieces) * 4;
-      float4 x = *reinterpret_cast<const float4*>(proj + (size_t)(row0 + j) * proj_stride + col0 + i);
-      const float f = factor(j);
-      x.x *= f; x.y *= f; x.z *= f; x.w *= f;
-      *reinterpret_cast<float4*>(dst + j * ld + i) = x;
-    }
+    const float* from = proj + (size_t)row0 * proj_stride + col0;
+    each_piece(
+        n, width / 4, [&](int j, int i) { return *reinterpret_cast<const float4*>(from + (size_t)j * proj_stride + 4 * i); },
+        [&](int j, int i, float4 x) {
+          const float f = factor(j);
+          x.x *= f; x.y *= f; x.z *= f; x.w *= f;
+          *reinterpret_cast<float4*>(dst + j * ld + 4 * i) = x;
+        });
     return;
   }
   for (int e = threadIdx.x; e < n * width; e += blockDim.x) {
@@ -1027,7 +1027,7 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
 // Ratios of decays are exponentials of differences of summed logarithms, never quotients.  Float32 on the CUDA cores.
 // Keys up to kMemDim, values a multiple of 4.  All three are bounded by the data shared memory returns (a 16-byte load of
 // a warp takes 4 cycles, broadcast or not), which the tiles of a thread are chosen by: four portions of 333 tokens, 16
-// heads of 128 x 128: the layer 388 us with a prepare kernel of its own and tiles of a column a lane, 271 this way (solve and
+// heads of 128 x 128: the layer 388 us with a prepare kernel of its own and tiles of a column a lane, 271 so (252 with the outputs of today; solve and
 // prepare 113 us and walk 139 before).
 constexpr int kWalkColumns = 32;
 constexpr int kSolveRow = kMemChunk + 4;         // row of the solve's matrices, transposed: [earlier token][token]
@@ -1256,17 +1256,16 @@ gated_delta_walk_kernel(const float* __restrict__ unit, int tokens, int P, const
     if (chunk < last) {
       float* dst = smem + (size_t)((chunk - first) & 1) * stage_floats;
       const int row0 = chunk_row[chunk], n = chunk_count[chunk];
-      const int pw = P / 4, pu = columns / 4;
-      for (int e = tid; e < n * pw; e += blockDim.x) {
-        const int t = e / pw, piece = e % pw;
+      const int pu = columns / 4;
+      for (int t = tid / (P / 4); t < n; t += 4) {      // P threads: four rows at a time
+        const int piece = tid % (P / 4);
         stream_cp_async16(dst + t * P + 4 * piece, w_in + ((size_t)(row0 + t) * heads + head) * P + 4 * piece);
         stream_cp_async16(dst + C * P + t * P + 4 * piece, rows + (size_t)(row0 + t) * 2 * P + 4 * piece);
       }
-      for (int e = tid; e < n * pu; e += blockDim.x) {
-        const int t = e / pu, piece = e % pu;
-        stream_cp_async16(dst + 2 * C * P + t * kCols + 4 * piece,
-                          u_io + ((size_t)(row0 + t) * heads + head) * vdim + col0 + 4 * piece);
-      }
+      if (const int piece = tid & 7; piece < pu)
+        for (int t = tid >> 3; t < n; t += P / 8)
+          stream_cp_async16(dst + 2 * C * P + t * kCols + 4 * piece,
+                            u_io + ((size_t)(row0 + t) * heads + head) * vdim + col0 + 4 * piece);
       for (int t = tid; t < n; t += blockDim.x)
         stream_cp_async16(dst + 2 * C * P + C * kCols + t * kMemGates, gates + ((size_t)(row0 + t) * heads + head) * kMemGates);
     }
