@@ -1027,8 +1027,8 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
 // Ratios of decays are exponentials of differences of summed logarithms, never quotients.  Float32 on the CUDA cores.
 // Keys up to kMemDim, values a multiple of 4.  All three are bounded by the data shared memory returns (a 16-byte load of
 // a warp takes 4 cycles, broadcast or not), which the tiles of a thread are chosen by: four portions of 333 tokens, 16
-// heads of 128 x 128: the layer 388 us with a prepare kernel of its own and tiles of a column a lane, 271 so (252 with the outputs of today; solve and
-// prepare 113 us and walk 139 before).
+// heads of 128 x 128: solve 38 and walk 92 us, where solve and a prepare kernel of its own took 113 and the walk 139 with
+// tiles of a column a lane; the layer 388 -> 271.
 constexpr int kWalkColumns = 32;
 constexpr int kSolveRow = kMemChunk + 4;         // row of the solve's matrices, transposed: [earlier token][token]
 
