@@ -119,7 +119,8 @@ gla_scan_kernel(GlaRows in, float* __restrict__ out, int out_stride, float* __re
 // ---------------------------------------------------------------- prompt portions in chunks
 constexpr int kChunk = 32;
 constexpr int kChunkDim = 128;                          // largest key and value size of the chunked kernels
-constexpr int kChunkRows = kChunkDim / kScanWarps;      // state rows of a warp
+constexpr int kChunkRows = 8;                           // state rows of a warp of the chunk sums
+constexpr int kStateRows = kChunkRows * kScanWarps;     // and of a block
 constexpr int kChunkCols = kChunkDim / 32;              // value columns of a lane
 
 // dst[j * ld + i] = src[row0 + j][col0 + i] * factor for j < n, i < width
@@ -170,46 +171,51 @@ __global__ void gla_decay_sums_kernel(float* __restrict__ z, int z_stride, const
 }
 
 // (1) chunk_state[chunk][head] = sum_j (k_j * exp(b_n - b_j)) v_j^T; chunk_decay[chunk][head][d] = exp(b_n[d]).
-__global__ void __launch_bounds__(kScanWarps * 32)
+// grid (chunks, heads, blocks of kStateRows state rows): with all 128 rows in a block (16 a warp, two blocks an SM) it took
+// 59 us for 2,048 tokens of 16 heads of 128 x 128, 54 this way; it waits for its rows more than it computes.
+__global__ void __launch_bounds__(kScanWarps * 32, 4)
 gla_chunk_state_kernel(GlaRows in, float* __restrict__ chunk_state, float* __restrict__ chunk_decay,
                        const int* __restrict__ chunk_row, const int* __restrict__ chunk_count, int heads, int dim,
                        int vdim) {
   extern __shared__ __align__(16) float smem[];
-  float* k_s = smem;                          // [kChunk][dim], times exp(b_n - b_j)
-  float* v_s = k_s + kChunk * dim;            // [kChunk][vdim]
+  float* k_s = smem;                          // [kChunk][kStateRows], times exp(b_n - b_j)
+  float* v_s = k_s + kChunk * kStateRows;     // [kChunk][vdim]
   pdl_wait();
   pdl_trigger();
-  const int chunk = blockIdx.x, head = blockIdx.y;
+  const int chunk = blockIdx.x, head = blockIdx.y, d0 = blockIdx.z * kStateRows, rows = min(kStateRows, dim - d0);
   const int row0 = chunk_row[chunk], n = chunk_count[chunk];
   stage_rows(v_s, vdim, in.proj, in.proj_stride, row0, n, in.v_off + head * vdim, vdim, 1.f);
-  const float* b_last = in.z + (size_t)(row0 + n - 1) * in.z_stride + head * dim;
-  const int k_col = in.k_off + head * dim;
+  const float* b_first = in.z + (size_t)row0 * in.z_stride + head * dim + d0;
+  const float* b_last = b_first + (size_t)(n - 1) * in.z_stride;
+  const int k_col = in.k_off + head * dim + d0;
+  const float* k_first = in.proj + (size_t)row0 * in.proj_stride + k_col;
   if (dim % 4 == 0 && k_col % 4 == 0 && in.proj_stride % 4 == 0 && in.z_stride % 4 == 0 &&
       ((reinterpret_cast<uintptr_t>(in.proj) | reinterpret_cast<uintptr_t>(in.z)) & 15) == 0) {
-    // 16-byte pieces of the key rows and of the sums (one index division a piece)
-    const int pieces = dim / 4;
-    for (int e = threadIdx.x; e < n * pieces; e += blockDim.x) {
-      const int j = e / pieces, d = (e % pieces) * 4;
-      const float4 b = *reinterpret_cast<const float4*>(in.z + (size_t)(row0 + j) * in.z_stride + head * dim + d);
-      const float4 last = *reinterpret_cast<const float4*>(b_last + d);
-      float4 k = *reinterpret_cast<const float4*>(in.proj + (size_t)(row0 + j) * in.proj_stride + k_col + d);
-      k.x *= expf(last.x - b.x); k.y *= expf(last.y - b.y); k.z *= expf(last.z - b.z); k.w *= expf(last.w - b.w);
-      *reinterpret_cast<float4*>(k_s + j * dim + d) = k;
-    }
+    // 16-byte pieces of the key rows and of the sums
+    each_piece(
+        n, rows / 4,
+        [&](int j, int i) {
+          const float4 b = *reinterpret_cast<const float4*>(b_first + (size_t)j * in.z_stride + 4 * i);
+          const float4 last = *reinterpret_cast<const float4*>(b_last + 4 * i);
+          float4 k = *reinterpret_cast<const float4*>(k_first + (size_t)j * in.proj_stride + 4 * i);
+          k.x *= expf(last.x - b.x); k.y *= expf(last.y - b.y); k.z *= expf(last.z - b.z); k.w *= expf(last.w - b.w);
+          return k;
+        },
+        [&](int j, int i, const float4& k) { *reinterpret_cast<float4*>(k_s + j * kStateRows + 4 * i) = k; });
   } else {
-    for (int e = threadIdx.x; e < n * dim; e += blockDim.x) {
-      const int j = e / dim, d = e % dim;
-      const float b = in.z[(size_t)(row0 + j) * in.z_stride + head * dim + d];
-      k_s[e] = in.proj[(size_t)(row0 + j) * in.proj_stride + k_col + d] * expf(b_last[d] - b);
+    for (int e = threadIdx.x; e < n * rows; e += blockDim.x) {
+      const int j = e / rows, d = e % rows;
+      const float b = b_first[(size_t)j * in.z_stride + d];
+      k_s[j * kStateRows + d] = k_first[(size_t)j * in.proj_stride + d] * expf(b_last[d] - b);
     }
   }
-  for (int d = threadIdx.x; d < dim; d += blockDim.x)
-    chunk_decay[((size_t)chunk * heads + head) * dim + d] = expf(b_last[d]);
+  for (int d = threadIdx.x; d < rows; d += blockDim.x)
+    chunk_decay[((size_t)chunk * heads + head) * dim + d0 + d] = expf(b_last[d]);
   __syncthreads();
   // a warp owns kChunkRows state rows that follow each other, a lane the value columns lane, lane + 32, ...
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i0 = warp * kChunkRows;
-  const bool whole = dim % 4 == 0 && i0 + kChunkRows <= dim;
+  const bool whole = i0 + kChunkRows <= rows;
   float u[kChunkRows][kChunkCols] = {};
   for (int j = 0; j < n; ++j) {
     float vv[kChunkCols], kv[kChunkRows];
@@ -218,23 +224,23 @@ gla_chunk_state_kernel(GlaRows in, float* __restrict__ chunk_state, float* __res
     if (whole) {
 #pragma unroll
       for (int r = 0; r < kChunkRows; r += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(k_s + j * dim + i0 + r);
+        const float4 k4 = *reinterpret_cast<const float4*>(k_s + j * kStateRows + i0 + r);
         kv[r] = k4.x; kv[r + 1] = k4.y; kv[r + 2] = k4.z; kv[r + 3] = k4.w;
       }
     } else {
 #pragma unroll
-      for (int r = 0; r < kChunkRows; ++r) kv[r] = i0 + r < dim ? k_s[j * dim + i0 + r] : 0.f;
+      for (int r = 0; r < kChunkRows; ++r) kv[r] = i0 + r < rows ? k_s[j * kStateRows + i0 + r] : 0.f;
     }
 #pragma unroll
     for (int r = 0; r < kChunkRows; ++r)
 #pragma unroll
       for (int c = 0; c < kChunkCols; ++c) u[r][c] = fmaf(kv[r], vv[c], u[r][c]);
   }
-  float* dst = chunk_state + ((size_t)chunk * heads + head) * dim * vdim;
+  float* dst = chunk_state + (((size_t)chunk * heads + head) * dim + d0) * vdim;
 #pragma unroll
   for (int r = 0; r < kChunkRows; ++r) {
     const int i = i0 + r;
-    if (i >= dim) continue;
+    if (i >= rows) continue;
 #pragma unroll
     for (int c = 0; c < kChunkCols; ++c)
       if (lane + 32 * c < vdim) dst[(size_t)i * vdim + lane + 32 * c] = u[r][c];
@@ -445,7 +451,7 @@ extern "C" int cie_gla_chunked(const float* proj, int proj_stride, int q_off, in
   if (dim > kChunkDim || vdim > kChunkDim)
     CIE_FAIL("gla_chunked: key / value sizes %d / %d are above %d", dim, vdim, kChunkDim);
   cudaStream_t s = (cudaStream_t)stream;
-  const size_t smem1 = (size_t)kChunk * (dim + vdim) * sizeof(float);
+  const size_t smem1 = (size_t)kChunk * (kStateRows + vdim) * sizeof(float);
   const size_t smem3 = (size_t)kChunk * (pad4(dim) + pad4(vdim) + kOutWeights + 2 * max(pad4(dim), pad4(vdim))) * sizeof(float);
   static bool raised = false;
   if (!raised) {
@@ -463,7 +469,8 @@ extern "C" int cie_gla_chunked(const float* proj, int proj_stride, int q_off, in
   while (sum_threads < dim) sum_threads <<= 1;
   CIE_LAUNCH("gla_decay_sums", gla_decay_sums_kernel, grid, dim3(sum_threads), 0, s, z, z_stride, z_bias, inv_tau,
              chunk_row, chunk_count, dim);
-  CIE_LAUNCH("gla_chunk_state", gla_chunk_state_kernel, grid, block, smem1, s, in, chunk_state, chunk_decay, chunk_row,
+  const dim3 grid1(chunks, heads, (dim + kStateRows - 1) / kStateRows);
+  CIE_LAUNCH("gla_chunk_state", gla_chunk_state_kernel, grid1, block, smem1, s, in, chunk_state, chunk_decay, chunk_row,
              chunk_count, heads, dim, vdim);
   if (pieces)
     CIE_LAUNCH("gla_chunk_prefix", gla_chunk_prefix_kernel<4>, grid2, dim3(128), 0, s, chunk_state,
