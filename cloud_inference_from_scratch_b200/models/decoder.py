@@ -268,6 +268,6 @@ class DecoderModel:
         x = self.final_norm.forward(residual, pending, ctx, rows=ctx.logit_rows)
         logits = rt.workspace.get("logits", ctx.num_logit_rows, spec.vocab_size, torch.float32,
                                   per_request=True)
-        rt.ops.linear(x, self.head, None, logits)
+        rt.ops.linear(x, self.head, None, logits, few_rows=True)
         rt.ops.shape_logits(logits, spec.logit_scale, spec.logit_softcap)
         return logits

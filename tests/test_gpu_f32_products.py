@@ -65,5 +65,8 @@ def test_the_runtime_sends_long_aligned_rows_there(ops):
     for k, there in ((512, True), (508, False), (514, False)):
         x, w = rand(5, k, seed=1).cuda(), rand(9, k, seed=2).cuda()
         out = ops.linear(x, w, None, torch.empty(5, 9).cuda())
+        few = ops.linear(x, w, None, torch.empty(5, 9).cuda(), few_rows=True)
+        assert torch.equal(few[:1], ops.linear(x[:1].contiguous(), w, None, torch.empty(1, 9).cuda(), few_rows=True))
+        assert torch.equal(out, few) != there
         assert torch.equal(out, product(ops, x, w, None)) if there else not ops._gemm_f32_takes(x.data_ptr(), w.data_ptr(), k)
         assert float((out.double() - x.double() @ w.double().T).abs().max()) <= 1e-4
