@@ -1046,7 +1046,18 @@ decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
     const int k0 = begin + it * SPLIT_TILE + warp * DN;      // this warp's 16 keys of the stage
     if (landed && k0 < end) {
       const bf16* k_tile = ring + stage * SPLIT_STAGE + warp * SPLIT_BLOCK;
-      const bf16* v_tile = k_tile + SPLIT_WARPS * SPLIT_BLOCK;
+      bf16* v_tile = ring + stage * SPLIT_STAGE + (SPLIT_WARPS + warp) * SPLIT_BLOCK;
+      if (k0 < first || k0 + DN > end) {
+        // a block that is not whole: values that the request does not see are cleared, since a weight of zero times what the
+        // page's former owner left there need not be zero
+        for (int e = lane; e < DN * CHUNKS; e += 32) {
+          const int r = e / CHUNKS;
+          if (k0 + r < first || k0 + r >= end)
+            *reinterpret_cast<uint4*>(const_cast<bf16*>(tile_ptr<true>(v_tile, r, e % CHUNKS * 8))) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        if (it + stages < tiles) bw::fence_async_smem();      // ordinary stores, before a later copy into the stage
+        __syncwarp();
+      }
       float s[DN / 8][4];
       scores<DN / 16, true>(q_frag, k_tile, s, lane);
       if constexpr (kOptions) {

@@ -27,6 +27,14 @@ def rand(*shape, seed, scale=1.0):
     return torch.randn(*shape, generator=generator) * scale
 
 
+def nobodys_pages(*shape):
+    """What pages hold that no request has, and the rows of a page behind a request's last key: whatever a former owner left,
+    overflows among it."""
+    pool = torch.full(shape, math.nan)
+    pool[1::3], pool[2::3] = math.inf, 100.0
+    return pool.bfloat16()
+
+
 def oracle(q, k, v, position, group, scale, o, heads):
     """One token's rows [heads, dim] over keys [.., kv, dim] of positions 0 .. position."""
     out = torch.empty(heads, v.shape[2], dtype=torch.float64)
@@ -154,7 +162,7 @@ def test_single_tokens_with_options(option, dim, kv_heads, group, page):
         o.penalty = (rand(heads, seed=1).abs(), rand(heads, seed=2).abs())
     width = -(-total_keys // page)
     table = torch.full((count, width), -1, dtype=torch.int32)
-    pools = [torch.full((count * width, kv_heads, page, dim), 100.0).bfloat16() for _ in range(2)]
+    pools = [nobodys_pages(count * width, kv_heads, page, dim) for _ in range(2)]
     keys, values = [], []
     for r, context in enumerate(contexts):
         k, v = rand(context + 1, kv_heads, dim, seed=10 + r, scale=1.5).bfloat16(), rand(context + 1, kv_heads, dim, seed=30 + r).bfloat16()
