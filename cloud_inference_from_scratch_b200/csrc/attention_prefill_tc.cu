@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const __grid_con
   unsigned char* v_s = k_s + STAGES * TILE_BYTES;    // [STAGES][TILE_BYTES]
   unsigned char* p_s = v_s + STAGES * TILE_BYTES;
   __shared__ __align__(8) uint64_t k_full[STAGES], k_empty[STAGES], v_full[STAGES], v_empty[STAGES], s_full[2], s_free[2], p_full, pv_done[2];
+  __shared__ __align__(8) uint64_t v_edge;      // values that rows have to be cleared of before they are full
   __shared__ uint32_t tmem_slot;
   __shared__ int pages_s[TABLE_SLOTS];   // the block-table entries this CTA's keys need
   __shared__ int last_s;                 // key ranges: did this CTA draw the tile's last ticket?
@@ -174,12 +175,10 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const __grid_con
     mbar_init(&s_full[0], 1); mbar_init(&s_full[1], 1);
     mbar_init(&s_free[0], 128); mbar_init(&s_free[1], 128);
     mbar_init(&p_full, 128);
+    mbar_init(&v_edge, 1);
     mbar_init(&pv_done[0], 1); mbar_init(&pv_done[1], 1);
     mbar_init_fence();
   }
-  // Value stages start as zeros: rows that no copy fills must not hold NaN or Inf bits.
-  for (int idx = tid; idx < STAGES * TILE_BYTES / 16; idx += THREADS)
-    reinterpret_cast<uint4*>(v_s)[idx] = make_uint4(0u, 0u, 0u, 0u);
   {
     const int needed = min((valid_hi + a.page_size - 1) / a.page_size, min(a.table_width, TABLE_SLOTS));
     for (int idx = tid; idx < needed; idx += THREADS) pages_s[idx] = table_row[idx];
@@ -258,33 +257,57 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_tc_kernel(const __grid_con
       if (run) {
         if (part == 0 && lane == 0) {
           // the whole box counts, also where it reaches past the keys in use or past the pool's end
-          mbar_expect_tx(&full[s], TILE_BYTES);
+          mbar_expect_tx(full, TILE_BYTES);
           const int group = kvh * (a.page_size / 8) + (k0 % a.page_size) / 8;
-          if constexpr (HALVES == 2) tma_load_5d(ring + s * TILE_BYTES, run_map, &full[s], 0, 0, 0, group, first_page);
-          else tma_load_4d(ring + s * TILE_BYTES, run_map, &full[s], 0, 0, group, first_page);
+          if constexpr (HALVES == 2) tma_load_5d(ring + s * TILE_BYTES, run_map, full, 0, 0, 0, group, first_page);
+          else tma_load_4d(ring + s * TILE_BYTES, run_map, full, 0, 0, group, first_page);
         }
         __syncwarp();
         return true;
       }
       // the first warp of the ring announces the bytes of the whole tile (a copy of another warp
       // may complete before that: the phase still waits for this arrival)
-      if (part == 0 && lane == 0) mbar_expect_tx(&full[s], (uint32_t)blocks * 16u * D * 2u);
+      if (part == 0 && lane == 0) mbar_expect_tx(full, (uint32_t)blocks * 16u * D * 2u);
       __syncwarp();
       if (mine) {   // one copy per block of 16 keys (they lie in one page)
-        if constexpr (HALVES == 2) tma_load_4d(ring + s * TILE_BYTES + block * BLOCK_BYTES, map, &full[s], 0, 0, 0, row / 8);
-        else tma_load_3d(ring + s * TILE_BYTES + block * BLOCK_BYTES, map, &full[s], 0, 0, row / 8);
+        if constexpr (HALVES == 2) tma_load_4d(ring + s * TILE_BYTES + block * BLOCK_BYTES, map, full, 0, 0, 0, row / 8);
+        else tma_load_3d(ring + s * TILE_BYTES + block * BLOCK_BYTES, map, full, 0, 0, row / 8);
       }
       __syncwarp();
       return true;
     };
+    // Values behind the last key are cleared once they have landed (the first warp of their ring, which has asked for the
+    // tile after by then): a weight of zero times what a page's former owner, or the owner of the page behind, left there
+    // need not be zero.
+    auto clear = [&](int j) -> bool {
+      if (!__all_sync(0xffffffffu, mbar_wait(&v_edge, 0, a.err))) return false;
+      const int s = j % STAGES, k0 = tile_of(j) * BN;
+      clear_rows<D>(v_s + s * TILE_BYTES, valid_hi - k0, BN, lane);
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&v_full[s]);
+      return true;
+    };
     bool alive = true, waited = false;
+    int edge = -1;                 // the tile that waits to be cleared
     for (int j = 0; j < tiles && alive; ++j) {
       if (!waited && tile_of(j) * BN + BN > context) {   // a tile with keys of this step: the kernel before writes them
         pdl_wait();
         waited = true;
       }
-      alive = for_keys ? load(j, k_s, &k_map, &k_run_map, k_full, k_empty) : load(j, v_s, &v_map, &v_run_map, v_full, v_empty);
+      if (for_keys) {
+        alive = load(j, k_s, &k_map, &k_run_map, &k_full[j % STAGES], k_empty);
+        continue;
+      }
+      const bool at_edge = tile_of(j) * BN + BN > valid_hi;
+      alive = load(j, v_s, &v_map, &v_run_map, at_edge ? &v_edge : &v_full[j % STAGES], v_empty);
+      if (alive && edge >= 0) {
+        alive = clear(edge);
+        edge = -1;
+      }
+      if (at_edge && part == 0) edge = j;
     }
+    if (alive && edge >= 0) clear(edge);
     if (!waited) pdl_wait();
   } else if (warp == MMA_WARP) {
     if (lane == 0) {

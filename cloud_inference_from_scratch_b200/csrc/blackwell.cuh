@@ -72,6 +72,22 @@ __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, u
 // bytes by TMA or the tensor cores.
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// Rows [first, end) of a tile of keys or values of D elements become zeros: 8 rows of 128 bytes (64 columns) follow each other,
+// then the same rows' next 64 columns (the swizzle moves pieces within a row only).  A whole warp, lanes side by side.
+template <int D>
+__device__ __forceinline__ void clear_rows(unsigned char* tile, int first, int end, int lane) {
+  for (int g = first >> 3; g * 8 < end; ++g) {
+    const int r = g * 8 + (lane >> 3);
+    const bool low = r >= first && r < end, high = r + 4 >= first && r + 4 < end;
+    uint4* at = reinterpret_cast<uint4*>(tile + g * (D / 64) * 1024) + lane;
+#pragma unroll
+    for (int half = 0; half < D / 64; ++half) {
+      if (low) at[half * 64] = make_uint4(0u, 0u, 0u, 0u);
+      if (high) at[half * 64 + 32] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+}
+
 // ---- tensor memory
 template <int COLS>
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot) {   // whole warp

@@ -774,16 +774,29 @@ __device__ __noinline__ void attention_phase(const Phase& p, Consumer& shared_st
         if (live_rows <= 8) softmax_update<2, 1>(s, mx, l, o);
         else softmax_update<2, 2>(s, mx, l, o);
       }
-      const bf16* v_tile;
+      bf16* v_tile;
       if constexpr (PG_KEY_STAGES == 2) {
         c.release(k_slot);
         c.ring.advance();
         c.wait_full();
-        v_tile = reinterpret_cast<const bf16*>(c.ring.base + (size_t)c.ring.slot * PG_STAGE_BYTES + box_index * PG_BLOCK_BYTES);
+        v_tile = reinterpret_cast<bf16*>(c.ring.base + (size_t)c.ring.slot * PG_STAGE_BYTES + box_index * PG_BLOCK_BYTES);
       } else {
-        v_tile = k_tile + 4 * PG_BLOCK_BYTES / 2;
+        v_tile = reinterpret_cast<bf16*>(c.ring.base + (size_t)k_slot * PG_STAGE_BYTES + (4 + box_index) * PG_BLOCK_BYTES);
       }
-      if (mine && c.alive) accumulate<1, true>(s, v_tile, o, lane);
+      if (mine && c.alive) {
+        if (k0 < k.first || k0 + 16 > k.end) {
+          // a block that is not whole: values that the request does not see are cleared, since a weight of zero times what
+          // the page's former owner left there need not be zero
+          for (int e = lane; e < 16 * CHUNKS; e += 32) {
+            const int r = e / CHUNKS;
+            if (k0 + r < k.first || k0 + r >= k.end)
+              *reinterpret_cast<uint4*>(const_cast<bf16*>(tile_ptr<true>(v_tile, r, e % CHUNKS * 8))) = make_uint4(0u, 0u, 0u, 0u);
+          }
+          bw::fence_async_smem();      // ordinary stores, before a later copy into the stage
+          __syncwarp();
+        }
+        accumulate<1, true>(s, v_tile, o, lane);
+      }
       c.release(c.ring.slot);
       c.ring.advance();
     }

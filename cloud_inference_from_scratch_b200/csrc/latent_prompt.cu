@@ -187,6 +187,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
   unsigned char* k_s = q_s + k_bytes;                  // [STAGES][k_bytes]
   unsigned char* v_s = k_s + STAGES * k_bytes;         // [STAGES][v_bytes]
   __shared__ __align__(8) uint64_t k_full[STAGES], k_empty[STAGES], v_full[STAGES], v_empty[STAGES];
+  __shared__ __align__(8) uint64_t v_edge[STAGES];      // values that rows have to be cleared of before they are full
   __shared__ __align__(8) uint64_t q_full, s_full[2], p_full[2], pv_done[2];
   __shared__ uint32_t tmem_slot;
   __shared__ float m_s[2][BM], l_s[2][BM];
@@ -197,6 +198,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1);
       mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
+      mbar_init(&v_edge[s], 1);
     }
     mbar_init(&q_full, 1);
     for (int g = 0; g < 2; ++g) { mbar_init(&s_full[g], 1); mbar_init(&p_full[g], BM); mbar_init(&pv_done[g], 1); }
@@ -222,8 +224,8 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
 
   bool alive = true;
   if (warp == TMA_WARP) {
+    const int column = blockIdx.x * (a.dim + a.vdim);
     if (lane == 0) {
-      const int column = blockIdx.x * (a.dim + a.vdim);
       // the queries: plain part and rotated part begin at pieces of their own; what a piece holds beyond a part's padded
       // columns takes part in no product
       const int q_column = head * (padded16(a.dim) + padded16(a.rot)), q_row = first_token - a.token0;
@@ -231,21 +233,53 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       for (int p = 0; p < k_pieces; ++p)
         tma_load_2d(q_s + p * PIECE_BYTES, &q_map, &q_full,
                     q_column + (p < k_plain ? p * PIECE : padded16(a.dim) + (p - k_plain) * PIECE), q_row);
-      for (int j = 0; j < tiles; ++j) {
-        const int s = j % STAGES, row = row0 + (tile0 + j) * BN;
-        const uint32_t before = ((j / STAGES) - 1) & 1;
-        if (j >= STAGES && !mbar_wait(&k_empty[s], before, a.err)) { alive = false; break; }
+    }
+    // Values of rows that no query sees (of the portion behind, or in front of the window) are cleared once they have
+    // landed, by the whole warp and before it needs the stage again: a weight of zero times another request's infinity
+    // would not be zero.
+    uint32_t edges = 0, phases = 0;          // bit s: stage s holds a tile to be cleared; the parity to wait for on v_edge[s]
+    auto cleared = [&](int j) -> bool {
+      const int s = j % STAGES, k0 = (tile0 + j) * BN;
+      if (!(edges >> s & 1)) return true;
+      edges &= ~(1u << s);
+      if (!__all_sync(0xffffffffu, mbar_wait(&v_edge[s], phases >> s & 1, a.err))) return false;
+      phases ^= 1u << s;
+      for (int p = 0; p < v_pieces; ++p) {
+        unsigned char* piece = v_s + s * v_bytes + p * PIECE_BYTES;
+        clear_rows<PIECE>(piece, 0, min(lowest - k0, BN), lane);
+        clear_rows<PIECE>(piece, valid_hi - k0, BN, lane);
+      }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&v_full[s]);
+      return true;
+    };
+    for (int j = 0; j < tiles && alive; ++j) {
+      const int s = j % STAGES, k0 = (tile0 + j) * BN, row = row0 + k0;
+      const uint32_t before = ((j / STAGES) - 1) & 1;
+      if (j >= STAGES) alive = __all_sync(0xffffffffu, mbar_wait(&k_empty[s], before, a.err));
+      if (!alive) break;
+      if (lane == 0) {
         mbar_expect_tx(&k_full[s], (uint32_t)k_bytes);       // a whole box counts, also where it reaches past the matrix
         for (int p = 0; p < k_plain; ++p)
           tma_load_2d(k_s + s * k_bytes + p * PIECE_BYTES, &kv_map, &k_full[s], column + p * PIECE, row);
         for (int p = k_plain; p < k_pieces; ++p)
           tma_load_2d(k_s + s * k_bytes + p * PIECE_BYTES, &r_map, &k_full[s], (p - k_plain) * PIECE, row);
-        if (j >= STAGES && !mbar_wait(&v_empty[s], before, a.err)) { alive = false; break; }
-        mbar_expect_tx(&v_full[s], (uint32_t)v_bytes);
-        for (int p = 0; p < v_pieces; ++p)
-          tma_load_2d(v_s + s * v_bytes + p * PIECE_BYTES, &kv_map, &v_full[s], column + a.dim + p * PIECE, row);
       }
+      __syncwarp();
+      if (j >= STAGES) alive = cleared(j - STAGES) && __all_sync(0xffffffffu, mbar_wait(&v_empty[s], before, a.err));
+      if (!alive) break;
+      const bool edge = k0 + BN > valid_hi || k0 < lowest;
+      if (edge) edges |= 1u << s;
+      if (lane == 0) {
+        uint64_t* full = edge ? &v_edge[s] : &v_full[s];
+        mbar_expect_tx(full, (uint32_t)v_bytes);
+        for (int p = 0; p < v_pieces; ++p)
+          tma_load_2d(v_s + s * v_bytes + p * PIECE_BYTES, &kv_map, full, column + a.dim + p * PIECE, row);
+      }
+      __syncwarp();
     }
+    for (int j = max(tiles - STAGES, 0); j < tiles && alive; ++j) alive = cleared(j);
     __syncwarp();
   } else if (warp == MMA_WARP) {
     if (lane == 0) {
