@@ -161,8 +161,6 @@ prompt_options_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
     for (int g = 0; g < 2; ++g) { mbar_init(&s_full[g], 1); mbar_init(&p_full[g], BM); mbar_init(&pv_done[g], 1); }
     mbar_init_fence();
   }
-  // Value stages start as zeros: rows that no copy fills must not hold NaN or Inf bits.
-  for (int idx = tid; idx < STAGES * TILE_BYTES / 16; idx += THREADS) reinterpret_cast<uint4*>(v_s)[idx] = make_uint4(0u, 0u, 0u, 0u);
   {
     const int needed = min((valid_hi + a.page_size - 1) / a.page_size, min(a.table_width, TABLE_SLOTS));
     for (int idx = tid; idx < needed; idx += THREADS) pages_s[idx] = table_row[idx];
@@ -309,9 +307,24 @@ prompt_options_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_co
     const float scale = kScores != kPlain ? 1.f : a.scale_log2;      // of what the weights are made from
     float m_used = -INFINITY, l = 0.f;
     for (int j = g; j < tiles; j += 2) {
+      const int k0 = tile_k0(j);
+      if (k0 + BN > valid_hi || (k0 < valid_lo && k0 + BN > a.keep_first)) {
+        // Values of keys that no row sees are cleared (a thread a key, its pieces in turn so that eight lanes meet all banks): a
+        // weight of zero times what a page's former owner, or the owner of the page behind, left there need not be zero, nor
+        // what lies in a stage where no copy went.  While the scores are worked out it costs little; by the TMA warp, beside
+        // the softmax, the layer of 2,048 tokens took 2 us longer.
+        if (!mbar_wait(&v_full[j % STAGES], (j / STAGES) & 1, a.err)) { alive = false; break; }
+        const int key = k0 + r;
+        if (key >= valid_hi || (key < valid_lo && key >= a.keep_first)) {
+          unsigned char* row_v = v_s + (j % STAGES) * TILE_BYTES + (r >> 3) * GROUP_BYTES + (r & 7) * 128;
+#pragma unroll
+          for (int c = 0; c < HALVES * 8; ++c)
+            *reinterpret_cast<uint4*>(row_v + (c >> 3) * 1024 + (((c + r) & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        fence_async_smem();      // before the products, which this thread's arrival on p_full lets go, and later copies
+      }
       if (!mbar_wait(&s_full[g], (j >> 1) & 1, a.err)) { alive = false; break; }
       tc_fence_after();
-      const int k0 = tile_k0(j);
       // columns lo .. hi of this tile are visible, and those below `first`
       const int hi = pos - k0, lo = a.window > 0 ? hi - a.window + 1 : 0, first = a.window > 0 ? a.keep_first - k0 : 0;
       const bool masked = k0 + BN - 1 > pos_lo || (a.window > 0 && k0 < valid_hi - a.window);      // the same for the CTA

@@ -88,7 +88,7 @@ def test_portions_with_options(option, dim, kv_heads, group, page):
         o.gates = rand(tokens, heads + 1, seed=4)
     width = -(-max(c + n for c, n in zip(contexts, lengths)) // page)
     table = torch.full((count, width), -1, dtype=torch.int32)
-    pools = [torch.full((count * width, kv_heads, page, dim), 100.0).bfloat16() for _ in range(2)]      # nobody's pages
+    pools = [nobodys_pages(count * width, kv_heads, page, dim) for _ in range(2)]
     keys, values = [], []
     for r in range(count):
         total = contexts[r] + lengths[r]
