@@ -14,8 +14,11 @@
 // A second kernel divides every head of o by its own root mean square, multiplies by a gain vector and
 // by sigmoid(gate), and rounds once.
 //
-// A request's result depends on its own tokens and state only: the batch, the cut of a prompt into
-// portions and the slot do not change the order of a single addition.
+// A request's result is worked out from its own tokens and state alone, whatever the batch and the slot.  The scan and the
+// stream make the same additions in the same order.  The chunks group them (a chunk begins with its portion), and a step is
+// run in chunks or not by what all of its requests together cost: so the cut of a prompt into portions and the requests
+// beside it may change the order of a request's additions, as they may in other float32 sums of this framework, and with it
+// the last bits; the difference stays within 1e-5 of the largest value.
 #include "common.cuh"
 #include "head_gate.cuh"
 
@@ -310,7 +313,7 @@ delta_stream_kernel(const float* __restrict__ packed, float* __restrict__ out, i
 // Float32 on the CUDA cores.  A token's results read rows of tokens up to its own alone (no weight of zero times a later
 // row).  Against the stream below, whose chain of one token is 450 instructions long and which a prompt of one request
 // and 32 heads runs on 32 SMs: 2,048 tokens, 32 heads of 64: 246 us in chunks, 1,790 as a stream (heads of 128, 16 of them:
-// 515 and 3,945); a whole layer at width 2,048 403 instead of 1,965.  What bounds delta_chunk is the data that shared memory
+// 515 and 3,945).  What bounds delta_chunk is the data that shared memory
 // can return (128 bytes a cycle: a 16-byte load of a warp is four cycles), hence tiles of 4 x 4 and more a thread; [M; Q]
 // instead of the low-rank form keeps the walk at one product and one barrier a chunk.
 constexpr int kDeltaChunkTokens = 32;

@@ -1364,7 +1364,8 @@ class Ops:
 
     def plan_delta(self, host: Any, heads: int, dim: int) -> dict[str, Any]:
         """Work lists of the generalized delta rule's chunked form (see ``plan_lightning``), for steps that it
-        serves faster than a walk token by token."""
+        serves faster than a walk token by token.  The step decides as a whole: a request's additions are ordered one way
+        or the other by what it shares the step with."""
         self._load_delta()
         if host.num_single == host.num_requests or dim > self.delta_stream_max_dim:
             return {}
@@ -1389,7 +1390,7 @@ class Ops:
         request or more on average) first works out, for all tokens at once, what the recurrence reads
         and then streams it through a ring of copies: the same additions in the same order.  With ``plan``
         (``plan_delta``, on the device) the step runs in chunks: what a chunk does to any state in parallel, then a
-        walk over each request's chunks."""
+        walk over each request's chunks, with the additions in another order."""
         self._flush()
         self._load_delta()
         r_off, k_off, v_off, a_off = offsets

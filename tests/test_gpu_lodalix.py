@@ -550,6 +550,39 @@ def test_delta_rule_in_chunks(dim, lengths):
         assert float((state[count - r].double().cpu() - held).abs().max()) <= 1e-5 * float(after.abs().max())
 
 
+@pytest.mark.parametrize("short", [2, 9])          # scanned, and streamed: eight tokens a request and more
+def test_delta_rule_of_a_request_alone_and_beside_many(short):
+    """What a step runs (chunks or a walk) is decided by all of its requests: the same portion alone, in chunks, and beside
+    300 short ones, token by token.  Both are within 1e-5 of the largest value of the rule in 64 bits (above), so within
+    twice that of each other."""
+    rt = runtime("float32")
+    heads, dim, own = 3, 64, 96
+    width = heads * dim
+    lengths = [own] + [short] * 300
+    tokens = sum(lengths)
+    proj, decay = rand(tokens, 5 * width, seed=1).cuda(), rand(tokens, width, seed=2, scale=6.0).cuda()
+    w0, a0 = rand(width, seed=3, scale=3.0).cuda(), rand(width, seed=4).cuda()
+    before = rand(len(lengths), heads, dim, dim, seed=5, scale=0.3)
+    results = []
+    for count in (1, len(lengths)):
+        lens = np.asarray(lengths[:count], dtype=np.int32)
+        starts = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+        host = SimpleNamespace(query_start=starts, query_lens=lens, num_single=0, num_requests=count)
+        plan = rt.ops.plan_delta(host, heads, dim)
+        assert bool(plan) == (count == 1)
+        ctx = SimpleNamespace(query_start=torch.from_numpy(starts).cuda(), num_requests=count,
+                              slots=torch.arange(count, dtype=torch.int32).cuda(),
+                              request_active=torch.ones(count, dtype=torch.int32).cuda())
+        state = before.clone().cuda()
+        out = torch.empty(int(starts[-1]), width).cuda()
+        rt.ops.delta_scan(proj[:starts[-1]], (0, width, 2 * width, 3 * width), decay[:starts[-1]], w0, a0, out, state, ctx, heads,
+                          dim, plan={key: torch.from_numpy(value).cuda() for key, value in plan.items()} or None)
+        rt.ops.check_errors()
+        results.append((out[:own], state[0]))
+    for alone, beside in zip(*results):
+        assert float((alone - beside).abs().max()) <= 2e-5 * float(alone.abs().max())
+
+
 def test_delta_rule_unlearns_along_its_key():
     """With removal rate 1 and no decay, writing a key a second time REPLACES what it held: the
     first value is gone and the read gives the second."""
