@@ -108,11 +108,11 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
   __syncwarp();
   if (chosen_softmax) {
     // the largest logits win (lowest index on ties); their weights are exp(z - z_first) over the sum of those
-    for (int e = lane; e < experts; e += 32) choice[e] = score[e];
+    for (int e = lane; e < experts; e += 32) choice[e] = fmaxf(score[e], -FLT_MAX);
     __syncwarp();
     float first = 0.f, total = 0.f, mine = 0.f;
     for (int j = 0; j < top; ++j) {
-      float best = -FLT_MAX;
+      float best = -INFINITY;
       int best_e = experts;
       for (int e = lane; e < experts; e += 32)
         if (choice[e] > best) { best = choice[e]; best_e = e; }
@@ -121,13 +121,14 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
         const int other_e = __shfl_xor_sync(0xffffffffu, best_e, offset);
         if (other > best || (other == best && other_e < best_e)) { best = other; best_e = other_e; }
       }
-      if (j == 0) first = best;
-      const float w = expf(best - first);
+      const float z = score[best_e];
+      if (j == 0) first = z;
+      const float w = expf(z - first);
       total += w;
       if (lane == j) mine = w;
       if (lane == 0) {
         ids[(size_t)t * top + j] = best_e;
-        choice[best_e] = -FLT_MAX;
+        choice[best_e] = -INFINITY;
         if (counts) atomicAdd(counts + best_e, 1);
       }
       __syncwarp();
@@ -148,7 +149,7 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
     const float z = score[e], s = sigmoid ? 1.f / (1.f + expf(-z)) : expf(z - m) / sum;
     score[e] = s;
     // sigmoids that nothing is added to lie in the order of their logits, which stay apart where the sigmoids round to 1
-    choice[e] = sigmoid && !correction && keep_groups == groups ? z : s + (correction ? correction[e] : 0.f);
+    choice[e] = fmaxf(sigmoid && !correction && keep_groups == groups ? z : s + (correction ? correction[e] : 0.f), -FLT_MAX);
   }
   __syncwarp();
   if (keep_groups < groups) {
@@ -170,13 +171,13 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
       int better = 0;
       for (int o = 0; o < groups; ++o) better += strength[o] > strength[g] || (strength[o] == strength[g] && o < g);
       if (better >= keep_groups)
-        for (int e = g * size; e < (g + 1) * size; ++e) choice[e] = -FLT_MAX;
+        for (int e = g * size; e < (g + 1) * size; ++e) choice[e] = -INFINITY;
     }
     __syncwarp();
   }
   float chosen_sum = 0.f;
   for (int j = 0; j < top; ++j) {
-    float best = -FLT_MAX;
+    float best = -INFINITY;
     int best_e = experts;
     for (int e = lane; e < experts; e += 32)
       if (choice[e] > best) { best = choice[e]; best_e = e; }
@@ -189,7 +190,7 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
     if (lane == 0) {
       ids[(size_t)t * top + j] = best_e;
       weights[(size_t)t * top + j] = score[best_e];
-      choice[best_e] = -FLT_MAX;
+      choice[best_e] = -INFINITY;
       if (counts) atomicAdd(counts + best_e, 1);
     }
     chosen_sum += score[best_e];

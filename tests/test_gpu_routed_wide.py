@@ -50,3 +50,36 @@ def test_many_pairs(monkeypatch, tokens, hidden, ff, weight_inputs, columns):
         want[token] += y if weight_inputs else weight * y
     assert float((out[:tokens].double().cpu() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
     assert float((out[tokens] - 7.0).abs().max()) == 0
+
+
+@pytest.mark.parametrize("tokens", [37, 1185])          # a token a block, and four
+@pytest.mark.parametrize("kind", ["softmax", "scores", "sigmoid", "grouped"])
+def test_tokens_whose_logits_are_nan_or_infinite(kind, tokens):
+    """They get experts that there are, each once, and nobody beside them notices."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+
+    rt = Runtime("cuda:0", "bfloat16")
+    rt.ops._load_moe()
+    hidden, experts, top = 64, 12, 3
+    x = rand(tokens, hidden, seed=1).bfloat16()
+    router, correction = rand(experts, hidden, seed=2).cuda(), rand(experts, seed=4).cuda()
+    results = []
+    for broken in (False, True):
+        rows = x.clone()
+        if broken:
+            rows[1::8, 5], rows[2::8], rows[7::8, 0] = float("nan"), float("inf"), -float("inf")
+        rows = rows.cuda()
+        ids = torch.empty(tokens, top, dtype=torch.int32).cuda()
+        weights = torch.empty(tokens, top).cuda()
+        rt.ops._moe_route(rows.data_ptr(), router.data_ptr(), correction.data_ptr() if kind == "grouped" else None,
+                          ids.data_ptr(), weights.data_ptr(), None, None, None, None, None, None, tokens, hidden, experts, top, 1,
+                          None, int(kind == "softmax"), int(kind in ("sigmoid", "grouped")), 3 if kind == "grouped" else 1,
+                          2 if kind == "grouped" else 1, 1e-20, rt.ops._code_of(rows), rt.ops.stream)
+        results.append((ids.cpu(), weights.cpu()))
+    whole = [t for t in range(tokens) if t % 8 not in (1, 2, 7)]
+    for plain, beside in zip(*results):
+        assert torch.equal(plain[whole], beside[whole])
+    ids = results[1][0].long()
+    assert int(ids.min()) >= 0 and int(ids.max()) < experts
+    assert all(len(set(row)) == top for row in ids.tolist())
+    assert bool(results[1][1][1::8].isnan().all())
