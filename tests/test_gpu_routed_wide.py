@@ -52,6 +52,56 @@ def test_many_pairs(monkeypatch, tokens, hidden, ff, weight_inputs, columns):
     assert float((out[tokens] - 7.0).abs().max()) == 0
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("hidden", [70, 72, 1032])          # single elements, pieces of four, several loads a lane
+@pytest.mark.parametrize("kind", ["softmax", "sigmoid", "grouped"])
+def test_a_router_block_of_four_tokens_adds_like_one_of_a_single_token(kind, hidden, dtype):
+    """1,185 tokens at once (four a block, one alone in the last) and 500 at a time (one a block): the same choices and the
+    same bits of their weights."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+
+    rt = Runtime("cuda:0", dtype)
+    rt.ops._load_moe()
+    tokens, experts, top = 1185, 12, 3
+    x = rand(tokens, hidden, seed=1).to(rt.dtype).cuda()
+    router, bias, correction = rand(experts, hidden, seed=2).cuda(), rand(experts, seed=3).cuda(), rand(experts, seed=4).cuda()
+    pointer = lambda t, wanted=True: t.data_ptr() if wanted else None  # noqa: E731
+
+    def route(rows):
+        ids = torch.empty(rows.shape[0], top, dtype=torch.int32).cuda()
+        weights = torch.empty(rows.shape[0], top).cuda()
+        rt.ops._moe_route(rows.data_ptr(), router.data_ptr(), pointer(correction, kind != "softmax"), ids.data_ptr(),
+                          weights.data_ptr(), None, None, None, None, None, None, rows.shape[0], hidden, experts, top, 1,
+                          pointer(bias, kind == "softmax"), int(kind == "softmax"), int(kind == "sigmoid"),
+                          3 if kind == "grouped" else 1, 2 if kind == "grouped" else 1, 1e-20, rt.ops._code_of(x), rt.ops.stream)
+        return ids, weights
+
+    together = route(x)
+    apart = [route(x[first:first + 500]) for first in range(0, tokens, 500)]
+    for whole, pieces in zip(together, zip(*apart)):
+        assert torch.equal(whole, torch.cat(pieces))
+
+
+@pytest.mark.parametrize("hidden,weighted", [(72, True), (72, False), (4096, True)])
+def test_the_sum_of_the_experts_rows_in_pieces_and_element_by_element(hidden, weighted):
+    """Rows that begin on 16 bytes and rows that do not: the same additions in the same order."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+
+    ops = Runtime("cuda:0", "bfloat16").ops
+    ops._load_moe()
+    tokens, top = 37, 5
+    values, weights = rand(tokens * top * hidden, seed=1).cuda(), rand(tokens, top, seed=2).cuda()
+    results = []
+    for shift in (0, 1):
+        rows = torch.zeros(values.numel() + 4).cuda()
+        rows[shift:shift + values.numel()] = values
+        out = torch.full((tokens + 1, hidden), 7.0).cuda()
+        ops._moe_combine(rows[shift:].data_ptr(), weights.data_ptr() if weighted else None, out.data_ptr(), tokens, hidden, top,
+                         ops._code_of(out), ops.stream)
+        results.append(out)
+    assert torch.equal(*results) and float((results[0][tokens] - 7.0).abs().max()) == 0
+
+
 @pytest.mark.parametrize("tokens", [37, 1185])          # a token a block, and four
 @pytest.mark.parametrize("kind", ["softmax", "scores", "sigmoid", "grouped"])
 def test_tokens_whose_logits_are_nan_or_infinite(kind, tokens):
