@@ -19,6 +19,17 @@ constexpr int kErrBadPage = 1;      // a block-table entry needed by a token was
 constexpr int kErrBadToken = 2;     // a token id outside the vocabulary
 constexpr int kErrBadRequest = 4;   // a request index outside the batch
 
+// Multiprocessors of the device that the first call finds current (a process works on one kind of device).
+inline int device_sms() {
+  static const int count = [] {
+    int device = 0, found = 0;
+    const bool known = cudaGetDevice(&device) == cudaSuccess &&
+                       cudaDeviceGetAttribute(&found, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && found > 0;
+    return known ? found : 148;
+  }();
+  return count;
+}
+
 template <typename T>
 __device__ __forceinline__ float to_float(T v);
 template <>

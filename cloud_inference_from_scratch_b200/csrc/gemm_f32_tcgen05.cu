@@ -257,12 +257,7 @@ cudaError_t launch_tiles(const float* a, const float* w, const float* bias, floa
   constexpr int smem = kStages * stage_bytes(BN) + 1024;
   static const cudaError_t raised = cudaFuncSetAttribute(gemm_f32_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (raised != cudaSuccess) return raised;
-  static const int sms = [] {
-    int device = 0, count = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-      count = 148;
-    return count;
-  }();
+  const int sms = device_sms();
   const long long tiles = (long long)((m + kRows - 1) / kRows) * ((n + BN - 1) / BN);
   return launch(gemm_f32_tc_kernel<BN>, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(kThreads), smem, stream, a, w, bias, c,
                 m, n, k, err);
@@ -285,7 +280,7 @@ extern "C" int cie_gemm_f32_tc(const float* a, const float* w, const float* bias
   // narrow tiles while they do not make a second round: 64 x 2,048 results of 2,048 32 us against 37 with wide ones, 300 x
   // 2,048 (192 narrow tiles, 96 wide ones) 67 against 48
   const long long narrow = (long long)((m + kRows - 1) / kRows) * ((n + 31) / 32);
-  if (columns != 32 && columns != 64) columns = narrow <= 148 ? 32 : 64;
+  if (columns != 32 && columns != 64) columns = narrow <= device_sms() ? 32 : 64;
   const cudaError_t status = columns == 32 ? launch_tiles<32>(a, w, bias, c, m, n, k, err, (cudaStream_t)stream)
                                            : launch_tiles<64>(a, w, bias, c, m, n, k, err, (cudaStream_t)stream);
   if (status != cudaSuccess) CIE_FAIL("gemm_f32_tc: launch failed: %s", cudaGetErrorString(status));

@@ -161,12 +161,7 @@ constexpr F32Tile kF32Tiles[] = {{8, 128, 46.f, 33.f}, {16, 128, 54.f, 39.f}, {3
 constexpr int kF32TileCount = sizeof(kF32Tiles) / sizeof(kF32Tiles[0]);
 
 int f32_tile(int m, int n) {
-  static const int sms = [] {
-    int device = 0, count = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
-      count = 148;
-    return count;
-  }();
+  const int sms = device_sms();
   int best = 0;
   float least = 0.f;
   for (int i = 0; i < kF32TileCount; ++i) {

@@ -542,7 +542,7 @@ extern "C" int cie_moe_route(const void* x, const float* router, const float* co
   const size_t one = (size_t)(route_scores(experts) + route_row(hidden, groups)) * sizeof(float);
   if (one > 200 * 1024) CIE_FAIL("moe_route: a row of %d elements does not fit shared memory", hidden);
   // four tokens a block from two blocks an SM on, as long as two such blocks fit an SM's shared memory
-  const bool four = tokens >= 4 * 2 * 148 && 4 * one <= 100 * 1024;
+  const bool four = tokens >= 4 * 2 * device_sms() && 4 * one <= 100 * 1024;
   const size_t smem = four ? 4 * one : one;
   const int blocks = four ? (tokens + 3) / 4 : tokens;
 #define CIE_MOE_ROUTE(T, N)                                                                                                  \

@@ -314,16 +314,10 @@ moe_grouped_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 
 template <bool kGateUp>
 static int launch_wide(const CUtensorMap& map_a, const CUtensorMap& map_b, const GroupedArgs& a, cudaStream_t stream) {
-  static int sms = 0;
-  if (!sms) {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        cudaFuncSetAttribute(moe_grouped_wide_kernel<kGateUp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WIDE_SMEM) != cudaSuccess) {
-      sms = 0;
-      CIE_FAIL("moe_tcgen05: cannot set the wide kernel up");
-    }
-  }
-  CIE_LAUNCH("moe_tcgen05", moe_grouped_wide_kernel<kGateUp>, dim3(sms), dim3(WIDE_THREADS), WIDE_SMEM, stream, map_a, map_b, a);
+  static const cudaError_t raised =
+      cudaFuncSetAttribute(moe_grouped_wide_kernel<kGateUp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WIDE_SMEM);
+  if (raised != cudaSuccess) CIE_FAIL("moe_tcgen05: cannot set the wide kernel up: %s", cudaGetErrorString(raised));
+  CIE_LAUNCH("moe_tcgen05", moe_grouped_wide_kernel<kGateUp>, dim3(device_sms()), dim3(WIDE_THREADS), WIDE_SMEM, stream, map_a, map_b, a);
   return 0;
 }
 
@@ -351,7 +345,7 @@ static int tile_columns(int pairs, int experts, int columns) {
   const int forced = asked ? atoi(asked) : 0;
   if (forced == 128 || forced == 256) return forced;
   const long long rows = pairs < experts ? pairs : (long long)experts * ((pairs + experts * BM - 1) / (experts * BM));
-  return rows * ((columns + WIDE - 1) / WIDE) >= 3 * 148 ? 256 : 128;
+  return rows * ((columns + WIDE - 1) / WIDE) >= 3ll * device_sms() ? 256 : 128;
 }
 
 }  // namespace cie
@@ -376,7 +370,7 @@ extern "C" int cie_moe_gate_up_tcgen05(const void* x, void* sorted, const void* 
   const int pairs = tokens * top;
   const long long pieces = (long long)pairs * (hidden / 8);
   int blocks = (int)((pieces + 255) / 256);
-  if (blocks > 148 * 8) blocks = 148 * 8;
+  if (blocks > device_sms() * 8) blocks = device_sms() * 8;
   CIE_LAUNCH("moe_gather_rows", moe_gather_rows_kernel, dim3(blocks), dim3(256), 0, s, (const bf16*)x, (bf16*)sorted,
              place_to_pair, pairs, top, hidden);
   const int bn = tile_columns(pairs, experts, 2 * ff);
