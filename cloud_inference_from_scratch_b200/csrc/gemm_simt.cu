@@ -151,13 +151,16 @@ gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w, const 
 
 // The tiles, and what they cost for 2,048 columns of K (B200, us): one CTA an SM, and every further CTA of the SM.  A CTA
 // alone waits for shared memory and its own products; several together are bound by what shared memory returns (128 bytes a
-// cycle), which is why larger tiles win once there are enough of them.
+// cycle), which is why larger tiles win once there are enough of them.  Who comes here has few rows (logits) or short ones:
+// logits of 151,936 x 2,048 take 313 us with 1 to 8 rows (8 x 128), 372 with 16 (16 x 128; 576 with 8 x 128), 665 with 17
+// (32 x 32; 705 with 16 x 128) and 1,045 with 64 (64 x 128; 1,338 with 32 x 32); 300 rows of 2,048 x 508 33 (32 x 32; 36 with
+// 16 x 128), 1,000 rows 59 (128 x 128; 73 with 32 x 32); 300 of 2,048 x 64 6, 1,000 10.
 struct F32Tile {
   int rows, columns;
   float alone, further;
 };
 constexpr F32Tile kF32Tiles[] = {{8, 128, 46.f, 33.f}, {16, 128, 54.f, 39.f}, {32, 32, 52.f, 19.f},
-                                 {64, 64, 94.f, 62.f}, {64, 128, 183.f, 101.f}, {128, 128, 220.f, 221.f}};
+                                 {64, 128, 183.f, 101.f}, {128, 128, 220.f, 221.f}};
 constexpr int kF32TileCount = sizeof(kF32Tiles) / sizeof(kF32Tiles[0]);
 
 int f32_tile(int m, int n) {
@@ -191,8 +194,7 @@ cudaError_t launch_f32(int tile, const float* a, const float* w, const float* bi
     case 0: CIE_F32_TILE(8, 128, 2, 4)
     case 1: CIE_F32_TILE(16, 128, 4, 4)
     case 2: CIE_F32_TILE(32, 32, 4, 4)
-    case 3: CIE_F32_TILE(64, 64, 4, 4)
-    case 4: CIE_F32_TILE(64, 128, 8, 8)
+    case 3: CIE_F32_TILE(64, 128, 8, 8)
     default: CIE_F32_TILE(128, 128, 8, 8)
   }
 #undef CIE_F32_TILE

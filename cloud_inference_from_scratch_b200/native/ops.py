@@ -1628,7 +1628,9 @@ class Ops:
 
         ``few_rows``: this product gets a row a request and never a whole prompt (the logits).  In 32-bit it then stays on
         the CUDA cores, whatever the number of rows, so that a row's bits do not depend on it: one row of 151,936 x 2,048
-        takes 310 us there and 580 on the tensor cores, which work on 128 rows at a time; they are ahead from about 32.
+        takes 313 us there and 580 on the tensor cores, which work on 128 rows at a time and are ahead from 17 rows on (582
+        against 665).  The layers' products go to the tensor cores at every number of rows, for the same reason; one row of
+        22,016 x 2,048 costs 108 us there (73 on the CUDA cores), of 2,048 x 11,008 139 (239), of 2,048 x 2,048 28 (46).
 
         Returns ``out``; or, when ``allow_partials`` and the product was cut along K, a
         ``Partials`` that a consuming kernel adds up (then ``out`` was not written); or, when the
