@@ -171,8 +171,8 @@ __global__ void gla_decay_sums_kernel(float* __restrict__ z, int z_stride, const
 }
 
 // (1) chunk_state[chunk][head] = sum_j (k_j * exp(b_n - b_j)) v_j^T; chunk_decay[chunk][head][d] = exp(b_n[d]).
-// grid (chunks, heads, blocks of kStateRows state rows): with all 128 rows in a block (16 a warp, two blocks an SM) it took
-// 59 us for 2,048 tokens of 16 heads of 128 x 128, 54 this way; it waits for its rows more than it computes.
+// grid (chunks, heads, blocks of kStateRows state rows): 2,048 tokens of 16 heads of 128 x 128 take 54 us, 59 with all 128 rows
+// in a block (16 a warp, two blocks an SM): it waits for its rows more than it computes.
 __global__ void __launch_bounds__(kScanWarps * 32, 4)
 gla_chunk_state_kernel(GlaRows in, float* __restrict__ chunk_state, float* __restrict__ chunk_decay,
                        const int* __restrict__ chunk_row, const int* __restrict__ chunk_count, int heads, int dim,

@@ -55,7 +55,7 @@ __device__ __forceinline__ void head_gate_store(__nv_bfloat16* dst, const float 
 }
 
 // Rows of whole, aligned 16-byte pieces and heads of up to 8 L elements: L lanes a head, both pieces a lane may have and
-// the gate's asked for together.  What bounds it is memory; a block of one warp a head, as this was, is bound by how fast
+// the gate's asked for together.  What bounds it is memory; a block of one warp a head is bound by how fast
 // blocks start (2,048 tokens: 32 heads of 64 69 us, 16 heads of 128 39 us; their bytes take 6.3).
 template <typename T, int L>
 __global__ void __launch_bounds__(256) head_gate_kernel(HeadGate a, T* __restrict__ out, int rows) {

@@ -1214,7 +1214,7 @@ gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_
 
 // grid (requests, heads, blocks of kWalkColumns value columns), P threads; a thread keeps 8 rows of 4 columns of S in
 // registers (a warp 32 rows, eight lanes a row): 8 cycles of loads for 32 products of a warp against W, 12 against k.  (A
-// lane a column of 8 rows, as this kernel first was, takes 8 cycles for 8 products and a partial sum of every warp.)  What
+// lane a column of 8 rows would take 8 cycles for 8 products and a partial sum of every warp.)  What
 // a chunk brings (W, k, U', the summed log decays) comes through two cp.async stages, a chunk ahead.
 __global__ void __launch_bounds__(kMemDim)
 gated_delta_walk_kernel(const float* __restrict__ unit, int tokens, int P, const float* __restrict__ gates,

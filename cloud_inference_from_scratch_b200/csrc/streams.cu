@@ -158,7 +158,7 @@ __device__ __forceinline__ void store_four(__nv_bfloat16* p, const float4& v) {
 
 // The row goes by in pieces of four elements where every part is whole, aligned ones, and the angles of a token are worked
 // out once, not once a head (a sine and a cosine each: 2,048 tokens of 16 + 2 heads of 128, half of every head rotated:
-// 26 us before, 19 now; its bytes take 5).
+// 19 us, 26 where a thread takes single elements and works out their angles itself; its bytes take 5).
 constexpr int kMaxAngles = 128;      // pairs whose angles are kept (more are worked out where they are used)
 template <typename TI, typename T>
 __global__ void norm_kv_write_kernel(const TI* __restrict__ src, const float* __restrict__ bias,

@@ -49,7 +49,6 @@ LATENT_PROMPT_KEYS = 1 << 17
 LATENT_PROMPT_BYTES = 1 << 28
 
 
-
 class _Lib:
     """A loaded library whose entry points return 0 or set ``cie_last_error``."""
 
