@@ -106,6 +106,8 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
   float* choice = score + experts;
   float* row_s = rows_s + warp * row_ld;
   __syncwarp();
+  // Choice scores are the lowest float at least, those of experts that are taken or out of the running -inf: `top` experts of
+  // the token are found whatever its logits hold (NaN counts as the lowest score, and stays in the weights).
   if (chosen_softmax) {
     // the largest logits win (lowest index on ties); their weights are exp(z - z_first) over the sum of those
     for (int e = lane; e < experts; e += 32) choice[e] = fmaxf(score[e], -FLT_MAX);
