@@ -1941,6 +1941,12 @@ class Ops:
         table = ctx.block_tables[kv.group]
         self.launches += 1
         tokens = qkv.shape[0]
+        # the split decode kernel is ahead at every size: 8 requests of 2,048 keys, 16 heads of 128 on 2 kv heads 11 us
+        # against 30 with a sink, 9 against 24 with a window and a penalty; one of 16 keys 4 against 13
+        by_split = (few_tokens and split is not None and head_dim == (value_dim or head_dim) == split.head_dim
+                    and not (window and keep_first) and split.splits_decode(kv) and qkv.shape[1] % 8 == 0
+                    and out.shape[1] % 4 == 0 and (qkv.data_ptr() | out.data_ptr()) % 16 == 0
+                    and os.environ.get("CIE_PENALISED_TC", "1") != "0")
         splits, shares, tickets = 1, None, None
         if few_tokens:
             units = tokens * kv_heads * -(-(q_heads // kv_heads) // 8)
@@ -1949,20 +1955,18 @@ class Ops:
                 keys = min(keys, window + keep_first)
             # a range keeps at least 128 keys; no more CTAs than one an SM
             splits = max(1, min(keys // 128, self.sm_count // max(units, 1), 16))
-            if splits > 1:
+            # (the group kernel's memory is made at the first decode step, whichever kernel takes it, and never replaced for
+            # a step that the split kernel takes: that would drop every captured step graph for nothing)
+            if splits > 1 and not (by_split and self._group_tickets is not None):
                 shares = self.scratch("attention.shares", units * splits * self._group_share_floats)
                 if self._group_tickets is None or self._group_tickets.numel() < units:
                     self._group_tickets = self.torch.zeros(max(units, 1024), dtype=self.torch.int32, device=self.device)
                     self.scratch_generation += 1
                 tickets = self._group_tickets
-            # the split decode kernel is ahead at every size: 8 requests of 2,048 keys, 16 heads of 128 on 2 kv heads 11 us
-            # against 30 with a sink, 9 against 24 with a window and a penalty; one of 16 keys 4 against 13
-            if (split is not None and head_dim == (value_dim or head_dim) == split.head_dim and not (window and keep_first)
-                    and split.splits_decode(kv) and qkv.shape[1] % 8 == 0 and out.shape[1] % 4 == 0
-                    and (qkv.data_ptr() | out.data_ptr()) % 16 == 0 and os.environ.get("CIE_PENALISED_TC", "1") != "0"):
-                split.run_singles(qkv, out, ctx, kv, tokens, q_heads, kv_heads, scale, window, distance, sinks=sinks,
-                                  softcap=softcap, slopes=slopes, gates=gates, shares=shares, tickets=tickets)
-                return
+        if by_split:
+            split.run_singles(qkv, out, ctx, kv, tokens, q_heads, kv_heads, scale, window, distance, sinks=sinks,
+                              softcap=softcap, slopes=slopes, gates=gates)
+            return
         r1, r2 = distance if distance is not None else (None, None)
         self._attention_generic_sink(
             _ptr(qkv), qkv.shape[1], _ptr(out), out.shape[1], _ptr(kv.k), _ptr(kv.v), _ptr(ctx.positions),

@@ -335,27 +335,22 @@ class TensorAttention:
 
     def run_singles(self, q: Any, out: Any, ctx: Any, kv: Any, requests: int, q_heads: int, kv_heads: int, scale: float,
                     window: int, distance: Any, sinks: Any = None, softcap: float = 0.0, slopes: Any = None,
-                    gates: Any = None, shares: Any = None, tickets: Any = None) -> None:
+                    gates: Any = None) -> None:
         """One query token for each of the first ``requests`` requests, with the options of ``run_portions`` except kept
         first keys, on the split decode kernel (``splits_decode``; key and value heads of this build's size); the softmax
-        weights enter the value product as three bfloat16 terms, which hold all their bits.  ``shares`` and ``tickets``:
-        the caller's scratch memory (tickets zero, and left so), used where it is large enough."""
+        weights enter the value product as three bfloat16 terms, which hold all their bits."""
         ops = self.ops
         table = ctx.block_tables[kv.group]
         max_keys = table.shape[1] * kv.page_size
         if window > 0:
             max_keys = min(max_keys, window)
         ctas, stages, cluster, min_keys = self._split_launch(requests, kv_heads, q_heads // kv_heads, max_keys)
-        units = requests * kv_heads * -(-(q_heads // kv_heads) // 16)
-        if (shares is None or tickets is None or tickets.numel() < units
-                or shares.numel() < units * (ctas // cluster) * 16 * (self.head_dim + 4)):
-            shares, tickets = self._split_shares, self._split_tickets
         pointer = lambda t: None if t is None else t.data_ptr()  # noqa: E731
         r1, r2 = distance if distance is not None else (None, None)
         self._decode_split_options(q.data_ptr(), q.shape[1], out.data_ptr(), out.shape[1], kv.k.data_ptr(), kv.v.data_ptr(),
                                    table.data_ptr(), table.shape[1], kv.num_pages, ctx.context_lens.data_ptr(), requests,
                                    q_heads, kv_heads, kv.page_size, ctas, min_keys, stages, cluster,
-                                   shares.data_ptr(), tickets.data_ptr(), scale, window, pointer(r1),
+                                   self._split_shares.data_ptr(), self._split_tickets.data_ptr(), scale, window, pointer(r1),
                                    pointer(r2), pointer(sinks), float(softcap), pointer(slopes), pointer(gates),
                                    0 if gates is None else gates.stride(0), 1, ops.error_word.data_ptr(), ops.stream)
 
