@@ -26,6 +26,7 @@
 #include <cuda.h>
 
 #include <cfloat>
+#include <mutex>
 
 #ifndef HEAD_DIM
 #define HEAD_DIM 128
@@ -1444,36 +1445,49 @@ extern "C" int cie_attention_decode(const void* q, int q_stride, void* out, int 
 // How many CTAs of the split decode kernel with a ring of `stages` stages, clusters of `cluster`
 // CTAs and `rows` head rows a unit fit one SM (its shared memory decides); 0 if the head size is not its kind or the sizes are
 // out of range, -1 on failure.
-template <bool kCluster>
+// The most shared memory that launches of a build may ask for: raised, never lowered, since other objects and plans rely on
+// what they have been granted.
+template <bool kCluster, bool kOptions>
+static cudaError_t split_reserve(size_t smem) {
+  static std::mutex guard;
+  static size_t granted = 0;
+  const std::lock_guard<std::mutex> lock(guard);
+  if (smem <= granted) return cudaSuccess;
+  const cudaError_t status = cudaFuncSetAttribute((decode_split_kernel<kCluster, kOptions>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (status == cudaSuccess) granted = smem;
+  return status;
+}
+
+template <bool kCluster, bool kOptions>
 static int split_ctas_per_sm(int stages, int cluster, int rows) {
   const size_t smem = split_smem(stages, cluster, rows);
-  if (cudaFuncSetAttribute((decode_split_kernel<kCluster, false>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  if (split_reserve<kCluster, kOptions>(smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
   int ctas = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, (decode_split_kernel<kCluster, false>), SPLIT_WARPS * 32, smem) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, (decode_split_kernel<kCluster, kOptions>), SPLIT_WARPS * 32, smem) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
   return ctas;
 }
 
-// rows: head rows of a unit (query heads per kv head, at most 16)
-extern "C" int cie_attention_decode_split_ctas_per_sm(int stages, int cluster, int rows) {
+// rows: head rows of a unit (query heads per kv head, at most 16); options: of the build with options
+extern "C" int cie_attention_decode_split_ctas_per_sm(int stages, int cluster, int rows, int options) {
   if (D % 64 || stages < SPLIT_MIN_STAGES || stages > SPLIT_MAX_STAGES || cluster < 1 || cluster > 16 || rows < 1 || rows > 16) return 0;
-  return cluster > 1 ? split_ctas_per_sm<true>(stages, cluster, rows) : split_ctas_per_sm<false>(stages, 1, rows);
+  if (options) return cluster > 1 ? split_ctas_per_sm<true, true>(stages, cluster, rows) : split_ctas_per_sm<false, true>(stages, 1, rows);
+  return cluster > 1 ? split_ctas_per_sm<true, false>(stages, cluster, rows) : split_ctas_per_sm<false, false>(stages, 1, rows);
 }
 
 // How many clusters of `cluster` CTAs of the split decode kernel the device runs at one time with a
 // ring of `stages` stages and `rows` head rows a unit (a cluster stays inside one GPC); -1 if the
 // query fails, 0 if the sizes are not the kernel's.
-extern "C" int cie_attention_decode_split_clusters(int stages, int cluster, int rows) {
-  if (D % 64 || stages < SPLIT_MIN_STAGES || stages > SPLIT_MAX_STAGES || rows < 1 || rows > 16) return 0;
-  if (cluster != 2 && cluster != 4 && cluster != 8 && cluster != 16) return 0;
+template <bool kOptions>
+static int split_clusters(int stages, int cluster, int rows) {
   const size_t smem = split_smem(stages, cluster, rows);
-  if (cudaFuncSetAttribute((decode_split_kernel<true, false>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      (cluster > 8 && cudaFuncSetAttribute((decode_split_kernel<true, false>), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
+  if (split_reserve<true, kOptions>(smem) != cudaSuccess ||
+      (cluster > 8 && cudaFuncSetAttribute((decode_split_kernel<true, kOptions>), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
     cudaGetLastError();
     return -1;
   }
@@ -1489,7 +1503,7 @@ extern "C" int cie_attention_decode_split_clusters(int stages, int cluster, int 
   config.attrs = &attribute;
   config.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, (decode_split_kernel<true, false>), &config) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, (decode_split_kernel<true, kOptions>), &config) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
@@ -1497,6 +1511,11 @@ extern "C" int cie_attention_decode_split_clusters(int stages, int cluster, int 
 }
 
 extern "C" int cie_attention_decode_split_max() { return SPLIT_MAX; }
+extern "C" int cie_attention_decode_split_clusters(int stages, int cluster, int rows, int options) {
+  if (D % 64 || stages < SPLIT_MIN_STAGES || stages > SPLIT_MAX_STAGES || rows < 1 || rows > 16) return 0;
+  if (cluster != 2 && cluster != 4 && cluster != 8 && cluster != 16) return 0;
+  return options ? split_clusters<true>(stages, cluster, rows) : split_clusters<false>(stages, cluster, rows);
+}
 extern "C" int cie_attention_decode_split_tile() { return SPLIT_TILE; }
 
 #ifdef SPLIT_TRACE
@@ -1518,15 +1537,8 @@ template <bool kOptions>
 static int launch_split(const CUtensorMap& k_map, const CUtensorMap& v_map, const SplitArgs& a, int requests, cudaStream_t stream) {
   const int cluster = a.cluster;
   const size_t smem = split_smem(a.stages, cluster, a.group < 16 ? a.group : 16);
-  static size_t configured[2] = {0, 0};
-  const int variant = cluster > 1 ? 1 : 0;
-  if (smem > configured[variant]) {
-    cudaError_t status = variant
-        ? cudaFuncSetAttribute((decode_split_kernel<true, kOptions>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-        : cudaFuncSetAttribute((decode_split_kernel<false, kOptions>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (status != cudaSuccess) CIE_FAIL("attention_decode_split: shared memory %zu: %s", smem, cudaGetErrorString(status));
-    configured[variant] = smem;
-  }
+  const cudaError_t granted = cluster > 1 ? split_reserve<true, kOptions>(smem) : split_reserve<false, kOptions>(smem);
+  if (granted != cudaSuccess) CIE_FAIL("attention_decode_split: shared memory %zu: %s", smem, cudaGetErrorString(granted));
   if (cluster > 8) {
     // clusters of more than 8 CTAs need the kernel's consent
     static bool allowed = false;

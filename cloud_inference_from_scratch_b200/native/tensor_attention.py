@@ -123,16 +123,16 @@ class TensorAttention:
             self.split_max = int(lib.handle.cie_attention_decode_split_max())
             self.split_tile = int(lib.handle.cie_attention_decode_split_tile())
             per_sm = lib.handle.cie_attention_decode_split_ctas_per_sm
-            per_sm.argtypes = [i, i, i]
+            per_sm.argtypes = [i, i, i, i]
             per_sm.restype = c_int
             self._split_per_sm = per_sm
             at_once = lib.handle.cie_attention_decode_split_clusters
-            at_once.argtypes = [i, i, i]
+            at_once.argtypes = [i, i, i, i]
             at_once.restype = c_int
             self._split_at_once = at_once
             self.split_cluster_max = int(os.environ.get("CIE_DECODE_SPLIT_CLUSTER", "16"))
-            self._split_rings: dict[tuple[int, int], dict[int, int]] = {}
-            self._split_plans: dict[int, tuple[dict[int, dict[int, int]], dict[int, int]]] = {}
+            self._split_rings: dict[tuple[int, int, bool], dict[int, int]] = {}
+            self._split_plans: dict[tuple[int, bool], tuple[dict[int, dict[int, int]], dict[int, int]]] = {}
             if not self.split_rings(1, 1):
                 raise RuntimeError(f"the split decode kernel does not fit this device at head size {head_dim}")
             # shares that meet in global memory (several clusters, or CTAs without a cluster, on one
@@ -193,34 +193,34 @@ class TensorAttention:
             self._cluster_room[splits] = room
         return room
 
-    def split_rings(self, cluster: int, rows: int) -> dict[int, int]:
-        """Ring depths the split decode kernel can be launched with for clusters of ``cluster`` CTAs
-        and ``rows`` head rows a unit, and how many CTAs an SM then holds (a CTA of a cluster keeps
+    def split_rings(self, cluster: int, rows: int, options: bool = False) -> dict[int, int]:
+        """Ring depths the split decode kernel (its build with or without options) can be launched with for clusters of
+        ``cluster`` CTAs and ``rows`` head rows a unit, and how many CTAs an SM then holds (a CTA of a cluster keeps
         room for its peers' shares of the rows it owns); asked of the device once."""
-        key = (cluster, min(16, rows))
+        key = (cluster, min(16, rows), options)
         if key not in self._split_rings:
-            rings = {stages: int(self._split_per_sm(stages, key[0], key[1])) for stages in range(1, 9)}
+            rings = {stages: int(self._split_per_sm(stages, *key)) for stages in range(1, 9)}
             self._split_rings[key] = {stages: ctas for stages, ctas in rings.items() if ctas >= 1}
         return self._split_rings[key]
 
-    def split_choices(self, rows: int) -> tuple[dict[int, dict[int, int]], dict[int, int]]:
+    def split_choices(self, rows: int, options: bool = False) -> tuple[dict[int, dict[int, int]], dict[int, int]]:
         """What the split decode kernel can be launched with for ``rows`` head rows a unit, asked of
         the device once: cluster size -> (ring depth -> CTAs an SM holds), and cluster size -> how
         many such clusters run at one time with the deepest ring with which an SM still holds two CTAs."""
         rows = min(16, rows)
-        if rows not in self._split_plans:
-            rings = {1: self.split_rings(1, rows)}
+        if (rows, options) not in self._split_plans:
+            rings = {1: self.split_rings(1, rows, options)}
             room: dict[int, int] = {}
             for cluster in (2, 4, 8, 16):
                 if cluster > self.split_cluster_max:
                     continue
-                paired = [depth for depth, ctas in self.split_rings(cluster, rows).items() if ctas >= 2]
-                at_once = int(self._split_at_once(max(paired), cluster, rows)) if paired else 0
+                paired = [depth for depth, ctas in self.split_rings(cluster, rows, options).items() if ctas >= 2]
+                at_once = int(self._split_at_once(max(paired), cluster, rows, options)) if paired else 0
                 if at_once >= 1:
-                    rings[cluster] = self.split_rings(cluster, rows)
+                    rings[cluster] = self.split_rings(cluster, rows, options)
                     room[cluster] = at_once
-            self._split_plans[rows] = (rings, room)
-        return self._split_plans[rows]
+            self._split_plans[rows, options] = (rings, room)
+        return self._split_plans[rows, options]
 
     @staticmethod
     def split_plan(units: int, max_keys: int, sm_count: int, rings: dict[int, dict[int, int]], room: dict[int, int],
@@ -322,9 +322,10 @@ class TensorAttention:
         return bool(self._decode_split is not None and page >= 16 and page & (page - 1) == 0
                     and (kv.k.data_ptr() | kv.v.data_ptr()) % 16 == 0)
 
-    def _split_launch(self, requests: int, kv_heads: int, group: int, max_keys: int) -> tuple[int, int, int, int]:
+    def _split_launch(self, requests: int, kv_heads: int, group: int, max_keys: int,
+                      options: bool = False) -> tuple[int, int, int, int]:
         units = requests * kv_heads * -(-group // 16)
-        rings, room = self.split_choices(group)
+        rings, room = self.split_choices(group, options)
         ctas, stages, cluster, min_keys = self.split_plan(units, max_keys, self.sm_count, rings, room,
                                                           self.split_cta_limit, self.split_max, self.split_tile)
         if FORCE_SPLIT_PLAN:
@@ -344,7 +345,7 @@ class TensorAttention:
         max_keys = table.shape[1] * kv.page_size
         if window > 0:
             max_keys = min(max_keys, window)
-        ctas, stages, cluster, min_keys = self._split_launch(requests, kv_heads, q_heads // kv_heads, max_keys)
+        ctas, stages, cluster, min_keys = self._split_launch(requests, kv_heads, q_heads // kv_heads, max_keys, True)
         pointer = lambda t: None if t is None else t.data_ptr()  # noqa: E731
         r1, r2 = distance if distance is not None else (None, None)
         self._decode_split_options(q.data_ptr(), q.shape[1], out.data_ptr(), out.shape[1], kv.k.data_ptr(), kv.v.data_ptr(),

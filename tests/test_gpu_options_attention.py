@@ -192,3 +192,25 @@ def test_single_tokens_with_options(option, dim, kv_heads, group, page):
             want = want * torch.sigmoid(o.gates[r, 1:].double()).view(-1, 1)
         got = out[r].view(heads, dim).double().cpu()
         assert float((got - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-6, r
+
+
+@pytest.mark.parametrize("options", [False, True])
+def test_what_one_object_asks_the_device_takes_nothing_from_another(options):
+    """The shared memory that launches may ask for belongs to the kernel: an object with fewer head rows on a kv head, which
+    asks what rings fit, must not lower it."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+    from test_gpu_kernels import tensor_case
+
+    one = {torch.bfloat16: Runtime("cuda:0", "bfloat16").ops}
+
+    def decode():
+        if options:
+            test_single_tokens_with_options(1, 128, 1, 20, 128)
+        else:
+            tensor_case(one, 128, [3000, 77], [1, 1], 16, 1, 128, 16, seed=1)
+
+    decode()
+    other = Runtime("cuda:0", "bfloat16").ops
+    other.require_portion_attention(128)
+    other._tensor_attention[128].split_choices(1, options)
+    decode()
