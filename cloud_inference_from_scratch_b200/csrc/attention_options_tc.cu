@@ -507,8 +507,10 @@ extern "C" int cie_attention_prompt_options(const void* q, int q_stride, void* o
   CUtensorMap k_run = k_map, v_run = v_map;
   a.run_pages = 0;
   int run_pages = 0, groups = 0;
-  if (page_size <= BN && BN % page_size == 0) { run_pages = BN / page_size; groups = page_size / 8; }
-  else if (page_size > BN && page_size % BN == 0) { run_pages = 1; groups = BN / 8; }
+  // (two tiles of keys are few copies either way, and a map costs the host a quarter of a microsecond to encode)
+  const bool many = (long long)table_width * page_size > 2 * BN;
+  if (many && page_size <= BN && BN % page_size == 0) { run_pages = BN / page_size; groups = page_size / 8; }
+  else if (many && page_size > BN && page_size % BN == 0) { run_pages = 1; groups = BN / 8; }
   if (run_pages > 0 && tensor_map_bf16_page_runs(k_pool, num_pages, kv_heads, page_size, D, groups, run_pages, &k_run) &&
       tensor_map_bf16_page_runs(v_pool, num_pages, kv_heads, page_size, D, groups, run_pages, &v_run))
     a.run_pages = run_pages;

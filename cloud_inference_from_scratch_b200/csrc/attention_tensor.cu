@@ -3,7 +3,7 @@
 //  * prefill_kernel: ragged causal attention of prompt portions (cached prefix + the portion
 //    itself) on mma.sync, for what the tcgen05 kernels (attention_prefill_tc.cu, and with options
 //    attention_options_tc.cu) do not take: head sizes other than 64 and 128, pages that are no
-//    multiple of 16 tokens, options over tables of at most 64 keys.  One CTA
+//    multiple of 16 tokens.  One CTA
 //    takes a tile of 128 query rows of ONE request and ONE kv head; a row is a (token, query head
 //    of the group) pair, so the heads of a group share every K/V load.  K/V tiles of 64 keys are
 //    gathered row by row from the pages with bulk asynchronous copies (any page size), double

@@ -403,23 +403,23 @@ class TensorAttention:
         ops._flush()
         ops.launches += 1
         r1, r2 = distance if distance is not None else (None, None)
-        # tables of up to 64 keys hold one tile of the mma.sync kernel, which is set up in less (64 tokens, 16 heads of 128:
-        # 14.7 us against 17.7; from 100 keys on the tcgen05 kernel is ahead)
+        # the tcgen05 kernel is ahead at every size: a portion of 16 tokens and nothing before it, 16 heads of 128 on 2 kv heads,
+        # 9.5 us against 11.7, of 64 9.2 and 11.4, of 100 9.5 and 18.4
         if (self._prompt_options is not None and split_weights and kv.page_size % 16 == 0
-                and table.shape[1] * kv.page_size > 64
-                and (key_dim or self.head_dim) == (value_dim or self.head_dim) == self.head_dim
-                and qkv.shape[1] % 8 == 0 and out.shape[1] % 8 == 0
-                and (qkv.data_ptr() | out.data_ptr() | kv.k.data_ptr() | kv.v.data_ptr()) % 16 == 0):
-            pointer = lambda t: None if t is None else t.data_ptr()  # noqa: E731
-            self._prompt_options(qkv.data_ptr(), qkv.shape[1], out.data_ptr(), out.shape[1], kv.k.data_ptr(),
-                                 kv.v.data_ptr(), table.data_ptr(), table.shape[1], kv.num_pages,
-                                 plan["tile_request"].data_ptr(), plan["tile_q0"].data_ptr(),
-                                 plan["tile_request"].shape[0], ctx.context_lens.data_ptr(), ctx.query_lens.data_ptr(),
-                                 ctx.query_start.data_ptr(), q_heads, kv_heads, kv.page_size, heads_per_tile(group),
-                                 scale, window, pointer(r1), pointer(r2), int(keep_first), pointer(sinks), float(softcap),
-                                 pointer(slopes), pointer(gates), 0 if gates is None else gates.stride(0),
-                                 ops.error_word.data_ptr(), ops.stream)
-            return
+                and (key_dim or self.head_dim) == (value_dim or self.head_dim) == self.head_dim):
+            q_at, out_at, k_at, v_at = qkv.data_ptr(), out.data_ptr(), kv.k.data_ptr(), kv.v.data_ptr()
+            q_stride, out_stride = qkv.shape[1], out.shape[1]
+            if (q_at | out_at | k_at | v_at) % 16 == 0 and (q_stride | out_stride) % 8 == 0:
+                tiles = plan["tile_request"]
+                self._prompt_options(q_at, q_stride, out_at, out_stride, k_at, v_at, table.data_ptr(), table.shape[1],
+                                     kv.num_pages, tiles.data_ptr(), plan["tile_q0"].data_ptr(), tiles.shape[0],
+                                     ctx.context_lens.data_ptr(), ctx.query_lens.data_ptr(), ctx.query_start.data_ptr(),
+                                     q_heads, kv_heads, kv.page_size, heads_per_tile(group), scale, window,
+                                     None if r1 is None else r1.data_ptr(), None if r2 is None else r2.data_ptr(), keep_first,
+                                     None if sinks is None else sinks.data_ptr(), softcap,
+                                     None if slopes is None else slopes.data_ptr(), None if gates is None else gates.data_ptr(),
+                                     0 if gates is None else gates.stride(0), ops.error_word.data_ptr(), ops.stream)
+                return
         self._prefill_ex(qkv.data_ptr(), qkv.shape[1], out.data_ptr(), out.shape[1], kv.k.data_ptr(),
                          kv.v.data_ptr(), table.data_ptr(), table.shape[1], kv.num_pages,
                          plan["tile_request"].data_ptr(), plan["tile_q0"].data_ptr(),
