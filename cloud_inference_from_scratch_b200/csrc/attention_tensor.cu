@@ -1051,10 +1051,12 @@ decode_split_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
       if (k0 < first || k0 + DN > end) {
         // a block that is not whole: values that the request does not see are cleared, since a weight of zero times what the
         // page's former owner left there need not be zero
-        for (int e = lane; e < DN * CHUNKS; e += 32) {
-          const int r = e / CHUNKS;
-          if (k0 + r < first || k0 + r >= end)
-            *reinterpret_cast<uint4*>(const_cast<bf16*>(tile_ptr<true>(v_tile, r, e % CHUNKS * 8))) = make_uint4(0u, 0u, 0u, 0u);
+        constexpr int kColumns = kBlockCopies ? D : 64;      // else 16 rows of 64 columns follow each other
+#pragma unroll
+        for (int part = 0; part < D / kColumns; ++part) {
+          unsigned char* rows = reinterpret_cast<unsigned char*>(v_tile + part * DN * kColumns);
+          if (k0 < first) bw::clear_rows<kColumns>(rows, 0, min(first - k0, DN), lane);
+          if (k0 + DN > end) bw::clear_rows<kColumns>(rows, end - k0, DN, lane);
         }
         if (it + stages < tiles) bw::fence_async_smem();      // ordinary stores, before a later copy into the stage
         __syncwarp();
@@ -1509,13 +1511,13 @@ static int split_clusters(int stages, int cluster, int rows) {
   }
   return clusters;
 }
-
-extern "C" int cie_attention_decode_split_max() { return SPLIT_MAX; }
 extern "C" int cie_attention_decode_split_clusters(int stages, int cluster, int rows, int options) {
   if (D % 64 || stages < SPLIT_MIN_STAGES || stages > SPLIT_MAX_STAGES || rows < 1 || rows > 16) return 0;
   if (cluster != 2 && cluster != 4 && cluster != 8 && cluster != 16) return 0;
   return options ? split_clusters<true>(stages, cluster, rows) : split_clusters<false>(stages, cluster, rows);
 }
+
+extern "C" int cie_attention_decode_split_max() { return SPLIT_MAX; }
 extern "C" int cie_attention_decode_split_tile() { return SPLIT_TILE; }
 
 #ifdef SPLIT_TRACE

@@ -787,11 +787,8 @@ __device__ __noinline__ void attention_phase(const Phase& p, Consumer& shared_st
         if (k0 < k.first || k0 + 16 > k.end) {
           // a block that is not whole: values that the request does not see are cleared, since a weight of zero times what
           // the page's former owner left there need not be zero
-          for (int e = lane; e < 16 * CHUNKS; e += 32) {
-            const int r = e / CHUNKS;
-            if (k0 + r < k.first || k0 + r >= k.end)
-              *reinterpret_cast<uint4*>(const_cast<bf16*>(tile_ptr<true>(v_tile, r, e % CHUNKS * 8))) = make_uint4(0u, 0u, 0u, 0u);
-          }
+          if (k0 < k.first) bw::clear_rows<D>(reinterpret_cast<unsigned char*>(v_tile), 0, min(k.first - k0, 16), lane);
+          if (k0 + 16 > k.end) bw::clear_rows<D>(reinterpret_cast<unsigned char*>(v_tile), k.end - k0, 16, lane);
           bw::fence_async_smem();      // ordinary stores, before a later copy into the stage
           __syncwarp();
         }
