@@ -194,6 +194,62 @@ def test_single_tokens_with_options(option, dim, kv_heads, group, page):
         assert float((got - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-6, r
 
 
+@pytest.mark.parametrize("option", [2, 1, 4])
+def test_a_short_portion_whatever_the_width_of_the_table(option):
+    """A table as wide as the longest request of the step, or of the model where graphs are enabled, changes no bit."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+    from cloud_inference_from_scratch_b200.native.tensor_attention import plan_tiles
+
+    ops = Runtime("cuda:0", "bfloat16").ops
+    ops.require_portion_attention(128)
+    asked, heads, kv_heads, page, length = OPTIONS[option], 16, 2, 16, 33
+    pools = [rand(64, kv_heads, page, 128, seed=s).bfloat16().cuda() for s in (1, 2)]
+    kv = SimpleNamespace(group=0, k=pools[0], v=pools[1], num_pages=64, page_size=page)
+    q = rand(length, heads * 128, seed=3).bfloat16().cuda()
+    penalty = tuple(rand(heads, seed=s).abs().cuda() for s in (4, 5)) if asked.get("penalty") else None
+    sinks = rand(heads, seed=6).cuda() if asked.get("sink") else None
+    lens = np.asarray([length], dtype=np.int32)
+    plan = {name: torch.from_numpy(array).cuda() for name, array in plan_tiles(lens, heads // kv_heads).items()}
+    as_int = lambda numbers: torch.tensor(numbers, dtype=torch.int32).cuda()  # noqa: E731
+    results = []
+    for width in (3, 4, 5, 17, 40):
+        ctx = SimpleNamespace(block_tables=[torch.arange(7, 7 + width, dtype=torch.int32).view(1, -1).cuda()], context_lens=as_int([0]),
+                              query_lens=as_int([length]), query_start=as_int([0, length]), num_single=0, num_requests=1)
+        out = torch.empty_like(q)
+        ops._tensor_attention[128].run_portions(q, out, ctx, kv, heads, kv_heads, 128 ** -0.5, asked.get("window", 0), plan, penalty,
+                                                True, keep_first=asked.get("keep", 0), sinks=sinks, softcap=asked.get("cap", 0.0))
+        results.append(out)
+    ops.check_errors()
+    assert all(torch.equal(results[0], other) for other in results[1:])
+
+
+def test_a_larger_step_of_single_tokens_makes_no_memory():
+    """The split decode kernel has its own, sized once; a batch and a table that grow behind a captured graph must not ask for
+    the group kernel's."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+
+    ops = Runtime("cuda:0", "bfloat16").ops
+    ops.require_portion_attention(128)
+    page, heads, kv_heads = 16, 16, 2
+    pools = [rand(600, kv_heads, page, 128, seed=s).bfloat16().cuda() for s in (1, 2)]
+    kv = SimpleNamespace(group=0, k=pools[0], v=pools[1], num_pages=600, page_size=page)
+    sinks = rand(heads, seed=3).cuda()
+    for requests, width in ((2, 17), (4, 130)):
+        q = rand(requests, heads * 128, seed=4).bfloat16().cuda()
+        out = torch.empty_like(q)
+        as_int = lambda numbers: torch.tensor(numbers, dtype=torch.int32).cuda()  # noqa: E731
+        contexts = [page * width - 1 - r for r in range(requests)]
+        table = torch.arange(requests * width, dtype=torch.int32).view(requests, width).cuda()
+        ctx = SimpleNamespace(block_tables=[table], context_lens=as_int(contexts), positions=as_int(contexts),
+                              request_of_token=as_int(list(range(requests))), num_single=requests, num_requests=requests)
+        ops.attention_penalised(q, out, ctx, kv, heads, kv_heads, 128, 128, 128 ** -0.5, 0, None, sinks=sinks)
+        ops.check_errors()
+        if width == 17:
+            generation = ops.scratch_generation
+            ops.freeze_scratch()
+    assert ops.scratch_generation == generation
+
+
 @pytest.mark.parametrize("options", [False, True])
 def test_what_one_object_asks_the_device_takes_nothing_from_another(options):
     """The shared memory that launches may ask for belongs to the kernel: an object with fewer head rows on a kv head, which
