@@ -1041,7 +1041,9 @@ class Ops:
                 "cie_gla_scan", [v, i, i, i, i, v, i, v, f, f, v, i, v, v, v, v, i, i, i, i, i, v, v])
             self._gla_chunked = lib.function(
                 "cie_gla_chunked",
-                [v, i, i, i, i, v, i, v, f, f, v, i, v, v, v, v, v, v, v, v, i, i, i, i, i, i, v, v])
+                [v, i, i, i, i, v, i, v, f, f, v, i, v, v, v, v, v, v, v, i, i, i, i, i, i, v, v])
+            lib.handle.cie_gla_chunk_floats.restype = ctypes.c_longlong
+            self._gla_chunk_floats = lib.handle.cie_gla_chunk_floats
             self.gla_scan_max_dim = int(lib.handle.cie_gla_scan_max_dim())
             self.gla_chunk_tokens = int(lib.handle.cie_gla_chunk_tokens())
             self.gla_chunk_max_dim = int(lib.handle.cie_gla_chunk_max_dim())
@@ -1066,7 +1068,7 @@ class Ops:
         """Gated linear attention over every request's new tokens from the state in its slot (``state``: float32
         [slots, heads, dim, vdim]): ``S <- diag(alpha) S + k v^T``, ``o = S^T (q * q_scale)`` with
         ``alpha = sigmoid(z + z_bias)^(1 / tau)`` per head and key channel.  ``proj`` is float32 [T, *] with q, k
-        and v at the columns ``offsets``; ``z`` float32 [T, heads * dim] (the chunked form overwrites it);
+        and v at the columns ``offsets``; ``z`` float32 [T, heads * dim];
         ``out`` float32 [T, heads * vdim].  With
         ``plan`` (chunk lists of a step with prompt portions) and sizes the chunked kernels take, the recurrence
         runs in chunks; else token by token."""
@@ -1083,11 +1085,10 @@ class Ops:
             # room for the chunks of the largest step the runtime knows of (and a partial chunk for many requests),
             # so that a long prompt after captured steps does not have to grow the buffers
             most = max(chunks, self.max_rows // self.gla_chunk_tokens + 64)
-            sums = self.scratch(f"gla.chunks.{heads}x{dim}x{vdim}", chunks * heads * dim * vdim,
-                                reserve=most * heads * dim * vdim)
-            decays = self.scratch(f"gla.decays.{heads}x{dim}", chunks * heads * dim, reserve=most * heads * dim)
-            self.launches += 4
-            self._gla_chunked(*head, _ptr(sums), _ptr(decays), _ptr(plan["chunk_row"]), _ptr(plan["chunk_count"]),
+            cells = self.scratch(f"gla.chunks.{heads}x{dim}", int(self._gla_chunk_floats(chunks, heads, dim)),
+                                 reserve=int(self._gla_chunk_floats(most, heads, dim)))
+            self.launches += 2
+            self._gla_chunked(*head, _ptr(cells), _ptr(plan["chunk_row"]), _ptr(plan["chunk_count"]),
                               _ptr(plan["request_chunk_start"]), _ptr(ctx.slots), _ptr(ctx.request_active), chunks,
                               ctx.num_requests, heads, dim, vdim, state.shape[0], _ptr(self.error_word), self.stream)
             return

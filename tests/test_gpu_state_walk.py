@@ -1,0 +1,98 @@
+"""Recurrences in chunks whose states are walked on the tensor cores (``state_walk.cuh``): chunk and block edges, key and
+value sizes that are no whole blocks, and values that are not finite."""
+
+import pytest
+import torch
+
+from test_gpu_bilipel import F, close, fake_step, rand, runtime
+
+pytestmark = pytest.mark.gpu
+
+
+def plan_of(rt, ctx):
+    return {name: torch.from_numpy(a).cuda() for name, a in rt.ops.plan_gla(ctx.host).items()}
+
+
+def gla_case(lengths, heads, dim, vdim, shift=0, seed=3):
+    """Inputs of a step, and the plain recurrence's outputs and states in 64 bits."""
+    tokens = sum(lengths)
+    proj = rand(tokens, shift + 2 * heads * dim + heads * vdim, seed=seed)
+    z, bias = rand(tokens, heads * dim, scale=2.0, seed=seed + 1), rand(heads * dim, scale=2.0, seed=seed + 2)
+    return proj, z, bias, rand(len(lengths), heads, dim, vdim, scale=0.5, seed=seed + 3)
+
+
+def gla_plain(proj, z, bias, start, lengths, heads, dim, vdim, shift, tau):
+    tokens = sum(lengths)
+    q = proj[:, shift:shift + heads * dim].to(F).view(tokens, heads, dim) * dim ** -0.5
+    k = proj[:, shift + heads * dim:shift + 2 * heads * dim].to(F).view(tokens, heads, dim)
+    v = proj[:, shift + 2 * heads * dim:].to(F).view(tokens, heads, vdim)
+    alpha = torch.sigmoid(z.to(F) + bias.to(F)).pow(1.0 / tau).view(tokens, heads, dim)
+    out, state, t = [], start.to(F).clone(), 0
+    for r, count in enumerate(lengths):
+        for _ in range(count):
+            state[r] = alpha[t].unsqueeze(-1) * state[r] + k[t].unsqueeze(-1) * v[t].unsqueeze(-2)
+            out.append(torch.einsum("hdv,hd->hv", state[r], q[t]))
+            t += 1
+    return torch.stack(out), state
+
+
+def gla_run(proj, z, bias, start, lengths, heads, dim, vdim, shift, tau):
+    rt = runtime("float32")
+    rt.ops.require_gla()
+    ctx, _ = fake_step(lengths, [0] * len(lengths), 16, torch.float32, 1, 8, 8)
+    ctx.slots = torch.arange(len(lengths), dtype=torch.int32).cuda()
+    ctx.request_active = torch.ones(len(lengths), dtype=torch.int32).cuda()
+    state = start.clone().cuda()
+    out = torch.empty(sum(lengths), heads * vdim, dtype=torch.float32).cuda()
+    offsets = (shift, shift + heads * dim, shift + 2 * heads * dim)
+    rt.ops.gla(proj.cuda(), offsets, z.cuda(), bias.cuda(), tau, dim ** -0.5, out, state, ctx, heads, dim, vdim,
+               plan=plan_of(rt, ctx))
+    rt.ops.check_errors()
+    return out.view(-1, heads, vdim).cpu(), state.cpu()
+
+
+# blocks of 16 columns (few heads) and of 32 (many), with and without a multiprocessor of their own, warps of 32 keys that
+# are partly or wholly there, tiles of 8 tokens, rows that allow 16-byte copies and rows that do not
+@pytest.mark.parametrize("lengths,heads,dim,vdim,shift", [
+    ([1, 7, 8, 9, 16, 17, 31, 32, 33, 65], 2, 128, 128, 8), ([40, 3], 80, 64, 33, 0), ([64, 2, 97], 50, 32, 64, 3),
+    ([70], 3, 33, 17, 0), ([25, 1, 1], 90, 96, 16, 4), ([2, 34], 1, 1, 1, 0), ([100], 20, 100, 128, 0)])
+def test_gated_linear_attention_at_the_edges_of_chunks_and_blocks(lengths, heads, dim, vdim, shift):
+    inputs = gla_case(lengths, heads, dim, vdim, shift)
+    want, final = gla_plain(*inputs, lengths, heads, dim, vdim, shift, 4.0)
+    got, state = gla_run(*inputs, lengths, heads, dim, vdim, shift, 4.0)
+    # sums of at most 128 products and a few dozen tokens' states: some 1e-6 of the spread
+    close(got, want, "float32", tight=2e-5)
+    close(state, final, "float32", tight=2e-5)
+
+
+@pytest.mark.parametrize("what", ["nan value", "infinite value", "huge key", "infinite state"])
+@pytest.mark.parametrize("heads", [1, 80])
+def test_values_that_are_not_finite_reach_the_tokens_behind_them_only(what, heads):
+    """As the recurrence has them: earlier tokens of the same chunk, other requests and other heads see nothing of them."""
+    lengths, dim, vdim, at = [50, 40], 64, 64, 20
+    proj, z, bias, start = gla_case(lengths, heads, dim, vdim)
+    if what == "nan value":
+        proj[at, 2 * heads * dim + 5] = float("nan")
+    elif what == "infinite value":
+        proj[at, 2 * heads * dim + 5] = float("inf")
+    elif what == "huge key":
+        proj[at, heads * dim + 7] = 3.4025e38      # finite, and infinite once rounded to the 11 bits of a tensor core's operand
+        proj[at, 2 * heads * dim:2 * heads * dim + vdim] *= 1e-3
+    else:
+        start[0, 0, 3, 5] = float("inf")
+    want, final = gla_plain(proj, z, bias, start, lengths, heads, dim, vdim, 0, 4.0)
+    got, state = gla_run(proj, z, bias, start, lengths, heads, dim, vdim, 0, 4.0)
+    first = 0 if what == "infinite state" else at
+    calm = torch.ones(want.shape, dtype=torch.bool)
+    columns = slice(None) if what == "huge key" else slice(5, 6)
+    calm[first:lengths[0], 0, columns] = False
+    close(got[calm], want[calm], "float32", tight=2e-5)
+    close(state[1], final[1], "float32", tight=2e-5)
+    if heads > 1:
+        close(state[0, 1:], final[0, 1:], "float32", tight=2e-5)
+    spoilt = got[first:lengths[0], 0, columns].double()
+    if what == "huge key":
+        exact = want[first:lengths[0], 0, columns]
+        assert torch.isfinite(spoilt).all() and float((spoilt - exact).abs().max() / exact.abs().max()) < 2e-5
+    else:
+        assert not torch.isfinite(spoilt).any()
