@@ -28,6 +28,7 @@
 // (one number per column, or a vector of a head's size shared by the heads) and by sigmoid or SiLU of a
 // gate, and rounds once.
 #include "chunk_outputs.cuh"
+#include "state_walk.cuh"
 #include "common.cuh"
 #include "head_gate.cuh"
 
@@ -895,8 +896,6 @@ mlstm_chunk_prefix_kernel(float* __restrict__ chunk_sums, float* __restrict__ st
 }
 
 // grid (chunks, heads).  chunk_sums holds, after the walk, the state before each chunk.
-// kMemory: the matrix memory (a denominator from the normaliser); else the gated delta rule in chunks (below), whose
-// rows come with i_t = m_t = 0, b_t = the log decays summed from the chunk's first token, and v = the chunk's writes.
 // q, k, v: where a head's rows are (see RowsOf).
 struct RowsOf {
   const float* base;      // row t of head h starts at base + h * head_base + t * stride + col0 + h * head_col
@@ -910,9 +909,8 @@ static size_t chunk_output_smem(int dim, int vdim) {
   return (size_t)kMemChunk * (key_row(dim) + 2 * pad4(vdim) + kOutWeights + max(key_row(dim), pad4(vdim))) * sizeof(float);
 }
 
-template <bool kMemory>
 __global__ void __launch_bounds__(kOutThreads, 3)
-chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
+mlstm_chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
                     const float* __restrict__ gates, const float* __restrict__ chunk_sums,
                     float* __restrict__ out, int out_stride, const int* __restrict__ chunk_row,
                     const int* __restrict__ chunk_count, int heads, int dim, int vdim) {
@@ -930,7 +928,7 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
   pdl_trigger();
   const int chunk = blockIdx.x, head = blockIdx.y;
   const int row0 = chunk_row[chunk], n = chunk_count[chunk];
-  const size_t cells = (size_t)dim * vdim + (kMemory ? dim : 0);
+  const size_t cells = (size_t)dim * vdim + dim;
   const float* before = chunk_sums + ((size_t)chunk * heads + head) * cells;
   const StateRing ring{first_s, k_s, before, dim, vdim};
   ring.issue(0);
@@ -992,12 +990,10 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
   // what the carried state is read with; the matrix memory's denominators
   for (int t = warp; t < n; t += kMemWarps) {
     const float carried = expf(gb_s[t] + m_before - gm_s[t]);
-    if (kMemory) {
-      float nq = 0.f;
-      for (int x = lane; x < dim; x += 32) nq = fmaf(before[(size_t)dim * vdim + x], q_s[t * ld + x], nq);
-      nq = warp_sum(nq) * carried + warp_sum(lane <= t ? a_s[lane * kOutWeights + t] : 0.f);
-      if (lane == 0) below_s[t] = fmaxf(fabsf(nq), expf(-gm_s[t])) + 1e-6f;
-    }
+    float nq = 0.f;
+    for (int x = lane; x < dim; x += 32) nq = fmaf(before[(size_t)dim * vdim + x], q_s[t * ld + x], nq);
+    nq = warp_sum(nq) * carried + warp_sum(lane <= t ? a_s[lane * kOutWeights + t] : 0.f);
+    if (lane == 0) below_s[t] = fmaxf(fabsf(nq), expf(-gm_s[t])) + 1e-6f;
     for (int x = lane; x < padded; x += 32) q_s[t * ld + x] *= carried;
   }
   // (chunk_outputs meets before it reads)
@@ -1005,10 +1001,8 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
   const bool wide = vdim % 4 == 0 && out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
   chunk_outputs(ring, q_s, ld, a_s, v_s, [&](int t, int c, float4 o) {
     if (t >= n) return;
-    if (kMemory) {
-      const float below = below_s[t];
-      o = make_float4(o.x / below, o.y / below, o.z / below, o.w / below);
-    }
+    const float below = below_s[t];
+    o = make_float4(o.x / below, o.y / below, o.z / below, o.w / below);
     store4(dst + (size_t)t * out_stride, c, vdim, o, wide);
   });
 }
@@ -1019,27 +1013,20 @@ chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_scale,
 // triangular system:  (I + A) U = diag(b) (V - diag(c) K S_0),  A_ts = b_t (c_t / c_s) (k_t . k_s) for s < t.  With
 // T = (I + A)^-1:  U = T diag(b) V - (T diag(b c) K) S_0 = U' - W S_0.  So:
 //   0. per (chunk, head):      the summed logarithms of the decays, the write strengths
-//   1. per (chunk, head):      unit k and q; A, T by forward substitution (a lane a column of T), U' and W
-//   2. per (request, head, 32 value columns): walks the chunks with its columns of S in registers:
-//                              U = U' - W S_0,  S <- c_C S_0 + sum_s (c_C / c_s) k_s u_s^T; leaves S_0 of every chunk
-//   3. per (chunk, head):      o_t = c_t S_0^T q_t + sum_(s<=t) (c_t / c_s) (q_t . k_s) u_s   (the matrix memory's output
-//                              kernel with i = m = 0 and no denominator)
-// Ratios of decays are exponentials of differences of summed logarithms, never quotients.  Float32 on the CUDA cores.
-// Keys up to kMemDim, values a multiple of 4.  All three are bounded by the data shared memory returns (a 16-byte load of
-// a warp takes 4 cycles, broadcast or not), which the tiles of a thread are chosen by: four portions of 333 tokens, 16
-// heads of 128 x 128: solve 38 and walk 92 us, where solve and a prepare kernel of its own took 113 and the walk 139 with
-// tiles of a column a lane; the layer 388 -> 271.
-constexpr int kWalkColumns = 32;
+//   1. per (chunk, q/k head):  the products k_t . k_s and q_t . k_s of unit rows, which all its heads share
+//   2. per (chunk, head):      A, T by forward substitution (a lane a column of T), U' and W, the scaled rows of q and k
+//   3. per (request, head, block of value columns): walks the chunks with its columns of S in registers (state_walk.cuh):
+//                              U = U' - W S_0,  o_t = c_t S_0^T q_t + sum_(s<=t) (c_t / c_s) (q_t . k_s) u_s,
+//                              S <- c_C S_0 + sum_s (c_C / c_s) k_s u_s^T
+// Ratios of decays are exponentials of differences of summed logarithms, never quotients.  1 and 2 work in float32 on the
+// CUDA cores, 3 as accurately on the tensor cores.  Keys up to kMemDim, values a multiple of 4.  Four portions of 333 tokens,
+// 16 heads of 128 x 128: 13 and 32 and 71 us, 120 in all; with the states of all chunks through memory and the walk and the
+// outputs on the CUDA cores 164; a prompt of 2,048 tokens 232 against 514.
 constexpr int kSolveRow = kMemChunk + 4;         // row of the solve's matrices, transposed: [earlier token][token]
+constexpr int kScores = kMemChunk * kMemChunk;   // floats of k_t . k_s of a chunk, and of q_t . k_s: row t, column s
 
 __host__ __device__ constexpr int gated_solve_floats(int P, int vdim) {
   return kMemChunk * (vdim + P + 4) + 3 * kMemChunk * kSolveRow;
-}
-__host__ __device__ constexpr int gated_walk_stage(int P) {
-  return kMemChunk * (2 * P + kWalkColumns + kMemGates);
-}
-__host__ __device__ constexpr int gated_walk_floats(int P) {
-  return 2 * gated_walk_stage(P) + (P / 32 + 1) * kMemChunk * kWalkColumns;
 }
 
 // grid (chunks, blocks of 8 heads): a warp a head, a lane a token.  gates: as the outputs read them (i = m = 0).
@@ -1067,13 +1054,110 @@ gated_delta_gates_kernel(const float* __restrict__ proj, int proj_stride, int b_
   strength[(size_t)row * heads + head] = sigmoid_f(z[b_off + head]);
 }
 
-// grid (chunks, heads).  unit: [head][token][k: P][q: P], zeros past dim.
+// grid (chunks, q/k heads).  scores: [chunks][kv_heads][k . k, q . k]; inverse: [token][kv_heads] one over the lengths of k
+// and q (q's times q_scale).
 __global__ void __launch_bounds__(256)
-gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_off, int k_off, int v_off, float q_scale,
-                         float* __restrict__ unit, int tokens, int P, const float* __restrict__ gates,
-                         const float* __restrict__ strength, float* __restrict__ w_out, float* __restrict__ u_out, const int* __restrict__ chunk_row,
+gated_delta_scores_kernel(const float* __restrict__ conv, int conv_stride, int q_off, int k_off, float q_scale,
+                          float* __restrict__ scores, float2* __restrict__ inverse, const int* __restrict__ chunk_row,
+                          const int* __restrict__ chunk_count, int kv_heads, int dim, int P) {
+  constexpr int C = kMemChunk;
+  extern __shared__ __align__(16) float smem[];
+  const int kd = P + 4;
+  float* k_s = smem;                       // [C][P + 4]
+  float* q_s = k_s + C * kd;               // [C][P + 4]
+  pdl_wait();
+  pdl_trigger();
+  const int chunk = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int row0 = chunk_row[chunk], n = chunk_count[chunk], base = group * dim;
+  float k[C / 8][kMemDim / 32], q[C / 8][kMemDim / 32];      // four tokens a warp, all asked for together
+#pragma unroll
+  for (int i = 0; i < C / 8; ++i) {
+    const int t = warp + 8 * i;
+    const float* row = conv + (size_t)(row0 + t) * conv_stride + base;
+#pragma unroll
+    for (int x = 0; x < kMemDim / 32; ++x) {
+      const bool in = t < n && lane + 32 * x < dim;
+      k[i][x] = in ? row[k_off + lane + 32 * x] : 0.f;
+      q[i][x] = in ? row[q_off + lane + 32 * x] : 0.f;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < C / 8; ++i) {        // unit k and q, the squares in the order of the scan
+    const int t = warp + 8 * i;
+    float ksq = 0.f, qsq = 0.f;
+#pragma unroll
+    for (int x = 0; x < kMemDim / 32; ++x) {
+      ksq = fmaf(k[i][x], k[i][x], ksq);
+      qsq = fmaf(q[i][x], q[i][x], qsq);
+    }
+    const float k_inv = rsqrtf(warp_sum(ksq) + 1e-6f), q_inv = rsqrtf(warp_sum(qsq) + 1e-6f) * q_scale;
+    if (lane == 0 && t < n) inverse[(size_t)(row0 + t) * kv_heads + group] = make_float2(k_inv, q_inv);
+#pragma unroll
+    for (int x = 0; x < kMemDim / 32; ++x) {
+      if (32 * x >= P) break;
+      k_s[t * kd + lane + 32 * x] = k[i][x] * k_inv;
+      q_s[t * kd + lane + 32 * x] = q[i][x] * q_inv;
+    }
+  }
+  __syncthreads();
+  // four lanes share a 4 x 4 tile, each every fourth 16 bytes of the rows
+  const int part = tid & 3, t0 = (tid >> 5) * 4, s0 = ((tid >> 2) & 7) * 4;
+  float kk[4][4] = {}, qk[4][4] = {};
+  if (s0 <= t0) {
+    for (int x = part * 4; x < P; x += 16) {
+      float4 tk[4], tq[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        tk[i] = *reinterpret_cast<const float4*>(k_s + (t0 + i) * kd + x);
+        tq[i] = *reinterpret_cast<const float4*>(q_s + (t0 + i) * kd + x);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float4 sv = *reinterpret_cast<const float4*>(k_s + (s0 + j) * kd + x);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          kk[i][j] = fmaf(tk[i].x, sv.x, kk[i][j]);
+          kk[i][j] = fmaf(tk[i].y, sv.y, kk[i][j]);
+          kk[i][j] = fmaf(tk[i].z, sv.z, kk[i][j]);
+          kk[i][j] = fmaf(tk[i].w, sv.w, kk[i][j]);
+          qk[i][j] = fmaf(tq[i].x, sv.x, qk[i][j]);
+          qk[i][j] = fmaf(tq[i].y, sv.y, qk[i][j]);
+          qk[i][j] = fmaf(tq[i].z, sv.z, qk[i][j]);
+          qk[i][j] = fmaf(tq[i].w, sv.w, qk[i][j]);
+        }
+      }
+    }
+  }
+  float* to = scores + ((size_t)chunk * kv_heads + group) * (2 * kScores);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float own_k = 0.f, own_q = 0.f;        // the lane's column of the four
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float a = kk[i][j], b = qk[i][j];
+      a += __shfl_xor_sync(0xffffffffu, a, 1);
+      b += __shfl_xor_sync(0xffffffffu, b, 1);
+      a += __shfl_xor_sync(0xffffffffu, a, 2);
+      b += __shfl_xor_sync(0xffffffffu, b, 2);
+      if (part == j) {
+        own_k = a;
+        own_q = b;
+      }
+    }
+    to[(t0 + i) * C + s0 + part] = own_k;
+    to[kScores + (t0 + i) * C + s0 + part] = own_q;
+  }
+}
+
+// grid (chunks, heads): the cell of a chunk and head (state_walk.cuh), and the rows U'.
+__global__ void __launch_bounds__(256)
+gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_off, int k_off, int v_off,
+                         const float* __restrict__ scores, const float2* __restrict__ inverse, int P,
+                         const float* __restrict__ gates, const float* __restrict__ strength, float* __restrict__ cells,
+                         float* __restrict__ u_out, const int* __restrict__ chunk_row,
                          const int* __restrict__ chunk_count, int heads, int kv_heads, int dim, int vdim) {
   constexpr int C = kMemChunk, TL = kSolveRow;
+  static_assert(kMemChunk == kChunkTokens, "chunks of the walk's size");
   extern __shared__ __align__(16) float smem[];
   const int kd = P + 4;
   float* v_s = smem;                       // [C][vdim]
@@ -1082,75 +1166,57 @@ gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_
   float* tv_s = a_s + C * TL;              // T diag(b)
   float* tk_s = tv_s + C * TL;             // T diag(b c)
   __shared__ float beta_s[C], lg_s[C];
+  __shared__ int unsafe_s;
   pdl_wait();
   pdl_trigger();
   const int chunk = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row0 = chunk_row[chunk], n = chunk_count[chunk], base = (head / (heads / kv_heads)) * dim;
+  const int row0 = chunk_row[chunk], n = chunk_count[chunk], group = head / (heads / kv_heads), base = group * dim;
+  float* cell = cells + ((size_t)chunk * heads + head) * walk_cell_floats(P, true);
   if (tid < C) {
     lg_s[tid] = tid < n ? gates[((size_t)(row0 + tid) * heads + head) * kMemGates + 1] : 0.f;
     beta_s[tid] = tid < n ? strength[(size_t)(row0 + tid) * heads + head] : 0.f;
   }
+  if (tid == 0) unsafe_s = 0;
+  const float* from = scores + ((size_t)chunk * kv_heads + group) * (2 * kScores) + tid * 4;
+  const float4 kk = *reinterpret_cast<const float4*>(from), qk = *reinterpret_cast<const float4*>(from + kScores);
+  stage_rows(v_s, vdim, conv, conv_stride, row0, n, v_off + head * vdim, vdim, [](int) { return 1.f; });
+  __syncthreads();
+  bool unsafe = false;
+  {
+    // A, and what the chunk's tokens read of each other
+    const int t = tid >> 3, s0 = (tid & 7) * 4;
+    const float kv[4] = {kk.x, kk.y, kk.z, kk.w}, qv[4] = {qk.x, qk.y, qk.z, qk.w};
+    float seen[4];
 #pragma unroll
-  for (int i = 0; i < C / 8; ++i) {        // unit k and q, the squares in the order of the scan
+    for (int j = 0; j < 4; ++j) {
+      const int s = s0 + j;
+      const float ratio = s <= t && t < n ? expf(lg_s[t] - lg_s[s]) : 0.f;
+      a_s[s * TL + t] = s < t && t < n ? kv[j] * beta_s[t] * ratio : 0.f;
+      seen[j] = s <= t && t < n ? qv[j] * ratio : 0.f;
+      unsafe |= tf32_unsafe(seen[j]);
+    }
+    *reinterpret_cast<float4*>(cell + walk_cell_a(P, true) + t * kWalkA + s0) = make_float4(seen[0], seen[1], seen[2], seen[3]);
+  }
+  const float lg_last = lg_s[n - 1];
+#pragma unroll
+  for (int i = 0; i < C / 8; ++i) {        // the rows of k and q as the state is written and read with; zeros past the last one
     const int t = warp + 8 * i;
-    if (t >= n) break;
     const float* row = conv + (size_t)(row0 + t) * conv_stride + base;
-    float k[kMemDim / 32], q[kMemDim / 32], ksq = 0.f, qsq = 0.f;
-#pragma unroll
-    for (int x = 0; x < kMemDim / 32; ++x) {
-      const bool in = lane + 32 * x < dim;
-      k[x] = in ? row[k_off + lane + 32 * x] : 0.f;
-      q[x] = in ? row[q_off + lane + 32 * x] : 0.f;
-    }
-#pragma unroll
-    for (int x = 0; x < kMemDim / 32; ++x) {
-      ksq = fmaf(k[x], k[x], ksq);
-      qsq = fmaf(q[x], q[x], qsq);
-    }
-    const float k_inv = rsqrtf(warp_sum(ksq) + 1e-6f), q_inv = rsqrtf(warp_sum(qsq) + 1e-6f);
-    float* dst = unit + ((size_t)head * tokens + row0 + t) * (2 * P) + lane;
+    const float2 inv = t < n ? inverse[(size_t)(row0 + t) * kv_heads + group] : make_float2(0.f, 0.f);
+    const float read = t < n ? expf(lg_s[t]) : 0.f, write = t < n ? expf(lg_last - lg_s[t]) : 0.f;
 #pragma unroll
     for (int x = 0; x < kMemDim / 32; ++x) {
       if (32 * x >= P) break;
-      dst[32 * x] = k_s[t * kd + lane + 32 * x] = k[x] * k_inv;
-      dst[P + 32 * x] = q[x] * q_inv * q_scale;
+      const int c = lane + 32 * x;
+      const bool in = t < n && c < dim;
+      const float k = in ? row[k_off + c] * inv.x : 0.f, q = in ? row[q_off + c] * inv.y * read : 0.f;
+      k_s[t * kd + c] = k;
+      cell[t * walk_q_row(P) + c] = q;
+      cell[walk_cell_k(P, true) + t * walk_k_row(P) + c] = k * write;
+      unsafe |= tf32_unsafe(q) || tf32_unsafe(k);
     }
   }
-  stage_rows(v_s, vdim, conv, conv_stride, row0, n, v_off + head * vdim, vdim, [](int) { return 1.f; });
-  __syncthreads();
-  {
-    // A: four lanes share a 4 x 4 tile, each every fourth 16 bytes of the rows
-    const int part = tid & 3, t0 = (tid >> 5) * 4, s0 = ((tid >> 2) & 7) * 4;
-    float dot[4][4] = {};
-    if (s0 <= t0) {
-      for (int x = part * 4; x < P; x += 16) {
-        float4 tv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) tv[i] = *reinterpret_cast<const float4*>(k_s + (t0 + i) * kd + x);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 sv = *reinterpret_cast<const float4*>(k_s + (s0 + j) * kd + x);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            dot[i][j] = fmaf(tv[i].x, sv.x, dot[i][j]);
-            dot[i][j] = fmaf(tv[i].y, sv.y, dot[i][j]);
-            dot[i][j] = fmaf(tv[i].z, sv.z, dot[i][j]);
-            dot[i][j] = fmaf(tv[i].w, sv.w, dot[i][j]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float total = dot[i][j];
-        total += __shfl_xor_sync(0xffffffffu, total, 1);
-        total += __shfl_xor_sync(0xffffffffu, total, 2);
-        const int t = t0 + i, s = s0 + j;
-        if (part == j) a_s[s * TL + t] = (s < t && t < n) ? total * beta_s[t] * expf(lg_s[t] - lg_s[s]) : 0.f;
-      }
-  }
+  for (int d = tid; d < P; d += 256) cell[walk_cell_decay(P, true) + d] = expf(lg_last);
   __syncthreads();
   if (tid < C) {            // column tid of T = (I + A)^-1: once a row is known it leaves all the rows below it
     float x[C];
@@ -1179,7 +1245,7 @@ gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_
   const int pieces = (vdim + P) / 4, groups = (pieces + 31) / 32 * 4;
   for (int item = warp; item < groups; item += 8) {
     const int piece = item / 4 * 32 + lane, t0 = (item & 3) * 8;
-    if (piece >= pieces || t0 >= n) continue;
+    if (piece >= pieces) continue;
     const bool value = piece < vdim / 4;
     const int c = value ? piece * 4 : piece * 4 - vdim, ld = value ? vdim : kd;
     const float* x = (value ? v_s : k_s) + c;
@@ -1200,167 +1266,28 @@ gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_
         acc[i].w = fmaf(w[i], xv.w, acc[i].w);
       }
     };
+    if (t0 < n) {
 #pragma unroll 4
-    for (int j = 0; j < t0; ++j) add(j, 0);
+      for (int j = 0; j < t0; ++j) add(j, 0);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) add(t0 + q, q);
-    float* dst = value ? u_out + c : w_out + c;
-    const int width = value ? vdim : P;
+      for (int q = 0; q < 8; ++q) add(t0 + q, q);
+    }
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (t0 + i < n) *reinterpret_cast<float4*>(dst + ((size_t)(row0 + t0 + i) * heads + head) * width) = acc[i];
+    for (int i = 0; i < 8; ++i) {
+      if (value) {
+        if (t0 + i < n) *reinterpret_cast<float4*>(u_out + c + ((size_t)(row0 + t0 + i) * heads + head) * vdim) = acc[i];
+      } else {
+        if (t0 + i >= n) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        unsafe |= tf32_unsafe(acc[i].x) || tf32_unsafe(acc[i].y) || tf32_unsafe(acc[i].z) || tf32_unsafe(acc[i].w);
+        *reinterpret_cast<float4*>(cell + walk_cell_w(P) + (t0 + i) * walk_q_row(P) + c) = acc[i];
+      }
+    }
   }
+  if (unsafe) unsafe_s = 1;
+  __syncthreads();
+  if (tid == 0)
+    *reinterpret_cast<float2*>(cell + walk_cell_decay(P, true) + P) = make_float2((float)unsafe_s, __int_as_float(n));
 }
-
-// grid (requests, heads, blocks of kWalkColumns value columns), P threads; a thread keeps 8 rows of 4 columns of S in
-// registers (a warp 32 rows, eight lanes a row): 8 cycles of loads for 32 products of a warp against W, 12 against k.  (A
-// lane a column of 8 rows would take 8 cycles for 8 products and a partial sum of every warp.)  What
-// a chunk brings (W, k, U', the summed log decays) comes through two cp.async stages, a chunk ahead.
-__global__ void __launch_bounds__(kMemDim)
-gated_delta_walk_kernel(const float* __restrict__ unit, int tokens, int P, const float* __restrict__ gates,
-                        const float* __restrict__ w_in, float* __restrict__ u_io, float* __restrict__ before,
-                        float* __restrict__ state, long long state_stride,
-                        const int* __restrict__ request_chunk_start, const int* __restrict__ chunk_row,
-                        const int* __restrict__ chunk_count, const int* __restrict__ slots,
-                        const int* __restrict__ request_active, int heads, int dim, int vdim, int max_slots, int* err) {
-  constexpr int C = kMemChunk, kCols = kWalkColumns;
-  extern __shared__ __align__(16) float smem[];
-  const int stage_floats = gated_walk_stage(P);
-  float* part_s = smem + 2 * stage_floats;        // [warps][C][kCols]
-  float* u_s = part_s + P / 32 * C * kCols;       // [C][kCols]: u_t c_C / c_t
-  pdl_wait();
-  pdl_trigger();
-  const int request = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * kCols, tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31, warps = P / 32, rg = lane >> 3;
-  const int c = (lane & 7) * 4, column = col0 + c, r0 = warp * 32 + rg * 8;
-  const int slot = slots[request];
-  if (slot < 0 || slot >= max_slots) {
-    if (tid == 0) atomicOr(err, kErrBadRequest);
-    return;
-  }
-  const bool live = column < vdim;                // whole pieces of four, as vdim is
-  float* s_base = state + (size_t)slot * state_stride + (size_t)head * dim * vdim + column;
-  float4 s[8];
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    s[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live && r0 + r < dim) {
-      const float* src = s_base + (size_t)(r0 + r) * vdim;
-      s[r] = make_float4(src[0], src[1], src[2], src[3]);
-    }
-  }
-  const int first = request_chunk_start[request], last = request_chunk_start[request + 1];
-  const float* rows = unit + (size_t)head * tokens * 2 * P;
-  const int columns = min(kCols, vdim - col0);     // a multiple of 4, as vdim is
-  auto issue = [&](int chunk) {
-    if (chunk < last) {
-      float* dst = smem + (size_t)((chunk - first) & 1) * stage_floats;
-      const int row0 = chunk_row[chunk], n = chunk_count[chunk];
-      const int pu = columns / 4;
-      for (int t = tid / (P / 4); t < n; t += 4) {      // P threads: four rows at a time
-        const int piece = tid % (P / 4);
-        stream_cp_async16(dst + t * P + 4 * piece, w_in + ((size_t)(row0 + t) * heads + head) * P + 4 * piece);
-        stream_cp_async16(dst + C * P + t * P + 4 * piece, rows + (size_t)(row0 + t) * 2 * P + 4 * piece);
-      }
-      if (const int piece = tid & 7; piece < pu)
-        for (int t = tid >> 3; t < n; t += P / 8)
-          stream_cp_async16(dst + 2 * C * P + t * kCols + 4 * piece,
-                            u_io + ((size_t)(row0 + t) * heads + head) * vdim + col0 + 4 * piece);
-      for (int t = tid; t < n; t += blockDim.x)
-        stream_cp_async16(dst + 2 * C * P + C * kCols + t * kMemGates, gates + ((size_t)(row0 + t) * heads + head) * kMemGates);
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  };
-  issue(first);
-  for (int chunk = first; chunk < last; ++chunk) {
-    const float* w_s = smem + (size_t)((chunk - first) & 1) * stage_floats;
-    const float* k_s = w_s + C * P;
-    const float* ut_s = k_s + C * P;
-    const float* g_s = ut_s + C * kCols;
-    const int row0 = chunk_row[chunk], n = chunk_count[chunk];
-    issue(chunk + 1);
-    asm volatile("cp.async.wait_group 1;\n" ::);
-    __syncthreads();
-    if (live) {
-      float* dst = before + ((size_t)chunk * heads + head) * dim * vdim + column;
-#pragma unroll
-      for (int r = 0; r < 8; ++r)
-        if (r0 + r < dim) *reinterpret_cast<float4*>(dst + (size_t)(r0 + r) * vdim) = s[r];
-    }
-    // W S: four tokens at a time (rows past n hold anything: their sums are not read); the four lanes that share the
-    // columns leave a token each
-    for (int t0 = 0; t0 < n; t0 += 4) {
-      float4 acc[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 lo = *reinterpret_cast<const float4*>(w_s + (t0 + i) * P + r0), hi = *reinterpret_cast<const float4*>(w_s + (t0 + i) * P + r0 + 4);
-        const float w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-        acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          acc[i].x = fmaf(w[r], s[r].x, acc[i].x);
-          acc[i].y = fmaf(w[r], s[r].y, acc[i].y);
-          acc[i].z = fmaf(w[r], s[r].z, acc[i].z);
-          acc[i].w = fmaf(w[r], s[r].w, acc[i].w);
-        }
-      }
-      auto merge = [&](float4& keep, const float4& give, int lanes) {
-        keep.x += __shfl_xor_sync(0xffffffffu, give.x, lanes);
-        keep.y += __shfl_xor_sync(0xffffffffu, give.y, lanes);
-        keep.z += __shfl_xor_sync(0xffffffffu, give.z, lanes);
-        keep.w += __shfl_xor_sync(0xffffffffu, give.w, lanes);
-      };
-      const bool odd = rg & 1, upper = rg & 2;
-      float4 even_keep = odd ? acc[1] : acc[0], high_keep = odd ? acc[3] : acc[2];
-      merge(even_keep, odd ? acc[0] : acc[1], 8);
-      merge(high_keep, odd ? acc[2] : acc[3], 8);
-      float4 keep = upper ? high_keep : even_keep;
-      merge(keep, upper ? even_keep : high_keep, 16);
-      *reinterpret_cast<float4*>(part_s + (warp * C + t0 + rg) * kCols + c) = keep;
-    }
-    __syncthreads();
-    const float lg_last = g_s[(n - 1) * kMemGates + 1];
-    for (int t = tid >> 3; t < n; t += P / 8) {
-      float4 u = *reinterpret_cast<const float4*>(ut_s + t * kCols + c);
-      for (int w = 0; w < warps; ++w) {
-        const float4 x = *reinterpret_cast<const float4*>(part_s + (w * C + t) * kCols + c);
-        u.x -= x.x; u.y -= x.y; u.z -= x.z; u.w -= x.w;
-      }
-      if (live) *reinterpret_cast<float4*>(u_io + ((size_t)(row0 + t) * heads + head) * vdim + column) = u;
-      const float weight = expf(lg_last - g_s[t * kMemGates + 1]);
-      *reinterpret_cast<float4*>(u_s + t * kCols + c) = make_float4(u.x * weight, u.y * weight, u.z * weight, u.w * weight);
-    }
-    __syncthreads();
-    const float keep = expf(lg_last);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      s[r].x *= keep; s[r].y *= keep; s[r].z *= keep; s[r].w *= keep;
-    }
-#pragma unroll 4
-    for (int t = 0; t < n; ++t) {
-      const float4 u = *reinterpret_cast<const float4*>(u_s + t * kCols + c);
-      const float4 lo = *reinterpret_cast<const float4*>(k_s + t * P + r0), hi = *reinterpret_cast<const float4*>(k_s + t * P + r0 + 4);
-      const float k[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        s[r].x = fmaf(k[r], u.x, s[r].x);
-        s[r].y = fmaf(k[r], u.y, s[r].y);
-        s[r].z = fmaf(k[r], u.z, s[r].z);
-        s[r].w = fmaf(k[r], u.w, s[r].w);
-      }
-    }
-    __syncthreads();        // everybody is done with this chunk's stage and with u_s before they are filled again
-  }
-  asm volatile("cp.async.wait_group 0;\n" ::);
-  if (!request_active[request] || !live) return;
-#pragma unroll
-  for (int r = 0; r < 8; ++r)
-    if (r0 + r < dim) {
-      float* dst = s_base + (size_t)(r0 + r) * vdim;
-      dst[0] = s[r].x; dst[1] = s[r].y; dst[2] = s[r].z; dst[3] = s[r].w;
-    }
-}
-
 
 }  // namespace cie
 
@@ -1444,7 +1371,7 @@ extern "C" int cie_mlstm_chunked(const float* proj, int proj_stride, int q_off, 
   float* sums = scratch + (size_t)tokens * heads * kMemGates;
   const size_t smem2 = (size_t)kMemChunk * (dim + vdim) * sizeof(float);
   const size_t smem4 = chunk_output_smem(dim, vdim);
-  if (smem4 > 48 * 1024 && cudaFuncSetAttribute(chunk_output_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (smem4 > 48 * 1024 && cudaFuncSetAttribute(mlstm_chunk_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 (int)smem4) != cudaSuccess)
     CIE_FAIL("mlstm_chunked: cannot reserve %zu bytes of shared memory", smem4);
   const dim3 grid(chunks, heads), block(kMemWarps * 32);
@@ -1458,15 +1385,16 @@ extern "C" int cie_mlstm_chunked(const float* proj, int proj_stride, int q_off, 
              dim3(256), 0, s, sums, state, state_stride, (const float*)gates, request_chunk_start, chunk_row, chunk_count,
              slots, request_active, heads, dim, vdim, max_slots, err);
   const RowsOf q_rows{proj, 0, proj_stride, q_off, dim}, k_rows{proj, 0, proj_stride, k_off, dim}, v_rows{proj, 0, proj_stride, v_off, vdim};
-  CIE_LAUNCH("mlstm_chunk_output", chunk_output_kernel<true>, grid, block, smem4, s, q_rows, k_rows, v_rows, q_scale,
+  CIE_LAUNCH("mlstm_chunk_output", mlstm_chunk_output_kernel, grid, block, smem4, s, q_rows, k_rows, v_rows, q_scale,
              (const float*)gates, (const float*)sums, out, out_stride, chunk_row, chunk_count, heads, dim, vdim);
   return 0;
 }
 
-// Floats of scratch memory the gated delta rule in chunks wants: the prepared rows, every token's summed log decays,
-// W and U per token, and the state before every chunk.
-extern "C" long long cie_gated_delta_chunk_floats(int tokens, int chunks, int heads, int dim, int vdim) {
-  return (long long)tokens * heads * (3 * stream_pad(dim) + kMemGates + 1 + vdim) + (long long)chunks * heads * dim * vdim;
+// Floats of scratch memory the gated delta rule in chunks wants: the cells, the products of unit rows, U' and the summed
+// log decays and strengths per token, and the rows' lengths.
+extern "C" long long cie_gated_delta_chunk_floats(int tokens, int chunks, int heads, int kv_heads, int dim, int vdim) {
+  return (long long)chunks * (heads * (long long)walk_cell_floats(walk_pad(dim), true) + kv_heads * 2ll * kScores) +
+         (long long)tokens * (heads * (long long)(kMemGates + 1 + vdim) + 2ll * kv_heads);
 }
 
 // The gated delta rule over a step with prompt portions, in chunks of cie_mlstm_chunk_tokens() tokens (work lists as
@@ -1485,33 +1413,27 @@ extern "C" int cie_gated_delta_chunked(const float* conv, int conv_stride, int q
   if (heads < 1 || heads > 65535 || kv_heads < 1 || heads % kv_heads)
     CIE_FAIL("gated_delta_chunked: %d heads do not divide over %d q/k heads", heads, kv_heads);
   cudaStream_t s = (cudaStream_t)stream;
-  const int P = stream_pad(dim);
-  float* unit = scratch;
-  float* gates = unit + (size_t)tokens * heads * 2 * P;
-  float* w = gates + (size_t)tokens * heads * kMemGates;
-  float* u = w + (size_t)tokens * heads * P;
-  float* before = u + (size_t)tokens * heads * vdim;
-  float* strength = before + (size_t)chunks * heads * dim * vdim;
-  const size_t smem1 = gated_solve_floats(P, vdim) * sizeof(float), smem2 = gated_walk_floats(P) * sizeof(float);
-  const size_t smem3 = chunk_output_smem(dim, vdim);
-  if (cudaFuncSetAttribute(gated_delta_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1) != cudaSuccess ||
-      cudaFuncSetAttribute(gated_delta_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess ||
-      cudaFuncSetAttribute(chunk_output_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) != cudaSuccess)
-    CIE_FAIL("gated_delta_chunked: cannot reserve %zu / %zu / %zu bytes of shared memory", smem1, smem2, smem3);
-  const dim3 grid(chunks, heads);
+  const int P = walk_pad(dim);
+  float* cells = scratch;
+  float* scores = cells + (size_t)chunks * heads * walk_cell_floats(P, true);
+  float* gates = scores + (size_t)chunks * kv_heads * 2 * kScores;
+  float* u = gates + (size_t)tokens * heads * kMemGates;
+  float2* inverse = reinterpret_cast<float2*>(u + (size_t)tokens * heads * vdim);
+  float* strength = reinterpret_cast<float*>(inverse + (size_t)tokens * kv_heads);
+  const size_t smem1 = (size_t)2 * kMemChunk * (P + 4) * sizeof(float), smem2 = gated_solve_floats(P, vdim) * sizeof(float);
+  if (cudaFuncSetAttribute(gated_delta_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess)
+    CIE_FAIL("gated_delta_chunked: cannot reserve %zu bytes of shared memory", smem2);
   CIE_LAUNCH("gated_delta_gates", gated_delta_gates_kernel, dim3(chunks, (heads + 7) / 8), dim3(256), 0, s, proj, proj_stride,
              b_off, a_off, a_log, dt_bias, gates, strength, chunk_row, chunk_count, heads);
-  CIE_LAUNCH("gated_delta_solve", gated_delta_solve_kernel, grid, dim3(256), smem1, s, conv, conv_stride, q_off, k_off, v_off,
-             q_scale, unit, tokens, P, (const float*)gates, (const float*)strength, w, u, chunk_row, chunk_count, heads, kv_heads,
-             dim, vdim);
-  CIE_LAUNCH("gated_delta_walk", gated_delta_walk_kernel, dim3(requests, heads, (vdim + kWalkColumns - 1) / kWalkColumns),
-             dim3(P), smem2, s, (const float*)unit, tokens, P, (const float*)gates, (const float*)w, u, before, state,
-             state_stride, request_chunk_start, chunk_row, chunk_count, slots, request_active, heads, dim, vdim, max_slots, err);
-  const RowsOf q_rows{unit, (long long)tokens * 2 * P, 2 * P, P, 0};
-  const RowsOf k_rows{unit, (long long)tokens * 2 * P, 2 * P, 0, 0};
-  const RowsOf v_rows{u, 0, heads * vdim, 0, vdim};
-  CIE_LAUNCH("delta_chunk_output", chunk_output_kernel<false>, grid, dim3(kMemWarps * 32), smem3, s, q_rows, k_rows, v_rows,
-             1.f, (const float*)gates, (const float*)before, out, out_stride, chunk_row, chunk_count, heads, dim, vdim);
+  CIE_LAUNCH("gated_delta_scores", gated_delta_scores_kernel, dim3(chunks, kv_heads), dim3(256), smem1, s, conv, conv_stride, q_off,
+             k_off, q_scale, scores, inverse, chunk_row, chunk_count, kv_heads, dim, P);
+  CIE_LAUNCH("gated_delta_solve", gated_delta_solve_kernel, dim3(chunks, heads), dim3(256), smem2, s, conv, conv_stride, q_off, k_off,
+             v_off, (const float*)scores, (const float2*)inverse, P, (const float*)gates, (const float*)strength, cells, u, chunk_row,
+             chunk_count, heads, kv_heads, dim, vdim);
+  const WalkArgs walk{cells, u, (long long)heads * vdim, vdim, out, out_stride, state, state_stride, chunk_row, chunk_count,
+                      request_chunk_start, slots, request_active, heads, dim, vdim, max_slots, err};
+  const cudaError_t walked = launch_state_walk<true>(walk, P, requests, s);
+  if (walked != cudaSuccess) CIE_FAIL("gated_delta_walk: launch failed: %s", cudaGetErrorString(walked));
   return 0;
 }
 

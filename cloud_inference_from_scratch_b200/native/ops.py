@@ -575,7 +575,7 @@ class Ops:
         ``proj`` float32 rows hold the write-strength and decay projections (heads each) from ``gate_offsets``;
         ``out`` float32 [T, heads * vdim].  Single tokens: one kernel.  Prompt portions with ``plan``
         (``plan_memory_chunks``, on the device), keys and values up to ``mlstm_chunk_max_dim`` and values a multiple
-        of 4: in chunks (a triangular system per chunk, a walk over each request's chunks, outputs in parallel);
+        of 4: in chunks (a triangular system per chunk, a walk over each request's chunks that works the outputs out);
         other prompt portions: prepare + stream."""
         self._flush()
         self._load_recurrent()
@@ -585,10 +585,10 @@ class Ops:
         if (plan and tokens >= 8 * ctx.num_requests and max(dim, vdim) <= self.mlstm_chunk_max_dim and vdim % 4 == 0
                 and os.environ.get("CIE_RECURRENT_CHUNKS", "1") != "0"):
             chunks = plan["chunk_row"].shape[0]
-            floats = int(self._gated_delta_chunk_floats(tokens, chunks, heads, dim, vdim))
+            floats = int(self._gated_delta_chunk_floats(tokens, chunks, heads, kv_heads, dim, vdim))
             rows = max(tokens, self.max_rows)
             reserve = int(self._gated_delta_chunk_floats(rows, -(-rows // self.mlstm_chunk_tokens) + ctx.num_requests,
-                                                         heads, dim, vdim))
+                                                         heads, kv_heads, dim, vdim))
             scratch = self.scratch(f"recurrent.delta_chunks.{heads}x{dim}x{vdim}", floats, reserve=max(floats, reserve))
             self.launches += 4
             self._gated_delta_chunked(_ptr(conv), conv.stride(0), q_off, k_off, v_off, _ptr(proj), proj.stride(0),

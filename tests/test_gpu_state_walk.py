@@ -96,3 +96,69 @@ def test_values_that_are_not_finite_reach_the_tokens_behind_them_only(what, head
         assert torch.isfinite(spoilt).all() and float((spoilt - exact).abs().max() / exact.abs().max()) < 2e-5
     else:
         assert not torch.isfinite(spoilt).any()
+
+
+def delta_case(lengths, heads, groups, dim, vdim, seed=5):
+    tokens = sum(lengths)
+    conv = rand(tokens, 2 * groups * dim + heads * vdim, seed=seed)
+    return conv, rand(tokens, 2 * heads, seed=seed + 1), rand(heads, scale=0.7, seed=seed + 2), rand(heads, seed=seed + 3), \
+        rand(len(lengths), heads * dim * vdim, scale=0.5, seed=seed + 4)
+
+
+def delta_plain(conv, gates, a_log, dt, start, lengths, heads, groups, dim, vdim):
+    qk = groups * dim
+    rows = conv.to(F)
+    q, k = rows[:, :qk].view(-1, groups, dim), rows[:, qk:2 * qk].view(-1, groups, dim)
+    q, k = ((x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(heads // groups, 1) for x in (q, k))
+    v = rows[:, 2 * qk:].view(-1, heads, vdim)
+    write = torch.sigmoid(gates[:, :heads].to(F))
+    decay = torch.exp(-torch.exp(a_log.to(F)) * torch.nn.functional.softplus(gates[:, heads:].to(F) + dt.to(F)))
+    out, state, t = [], start.to(F).view(-1, heads, dim, vdim).clone(), 0
+    for r, count in enumerate(lengths):
+        for _ in range(count):
+            kept = decay[t].view(-1, 1, 1) * state[r]
+            u = write[t].unsqueeze(-1) * (v[t] - torch.einsum("hdv,hd->hv", kept, k[t]))
+            state[r] = kept + k[t].unsqueeze(-1) * u.unsqueeze(-2)
+            out.append(torch.einsum("hdv,hd->hv", state[r], q[t]) * dim ** -0.5)
+            t += 1
+    return torch.stack(out), state
+
+
+def delta_run(conv, gates, a_log, dt, start, lengths, heads, groups, dim, vdim):
+    rt = runtime("float32")
+    ctx, _ = fake_step(lengths, [0] * len(lengths), 16, torch.float32, 1, 8, 8)
+    ctx.slots = torch.arange(len(lengths), dtype=torch.int32).cuda()
+    ctx.request_active = torch.ones(len(lengths), dtype=torch.int32).cuda()
+    plan = {name: torch.from_numpy(a).cuda() for name, a in rt.ops.plan_memory_chunks(ctx.host).items()}
+    state, qk = start.clone().cuda(), groups * dim
+    out = torch.empty(sum(lengths), heads * vdim, dtype=torch.float32).cuda()
+    rt.ops.gated_delta_scan(conv.cuda(), (0, qk, 2 * qk), gates.cuda(), (0, heads), a_log.cuda(), dt.cuda(), dim ** -0.5, out,
+                            state, ctx, heads, groups, dim, vdim, plan=plan)
+    rt.ops.check_errors()
+    return out.view(-1, heads, vdim).cpu(), state.view(-1, heads, dim, vdim).cpu()
+
+
+@pytest.mark.parametrize("lengths,heads,groups,dim,vdim", [
+    ([31, 32, 33, 65, 8], 2, 1, 128, 128), ([40, 24], 80, 40, 64, 36), ([64, 2, 97], 51, 17, 33, 64), ([70], 3, 3, 96, 16),
+    ([100], 20, 10, 1, 4)])
+def test_gated_delta_rule_at_the_edges_of_chunks_and_blocks(lengths, heads, groups, dim, vdim):
+    inputs = delta_case(lengths, heads, groups, dim, vdim)
+    want, final = delta_plain(*inputs, lengths, heads, groups, dim, vdim)
+    got, state = delta_run(*inputs, lengths, heads, groups, dim, vdim)
+    close(got, want, "float32", tight=2e-5)
+    close(state, final, "float32", tight=2e-5)
+
+
+@pytest.mark.parametrize("heads", [1, 80])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_writes_that_are_not_finite_reach_the_tokens_behind_them_only(bad, heads):
+    lengths, dim, at = [50, 40], 64, 20
+    conv, gates, a_log, dt, start = delta_case(lengths, heads, heads, dim, dim)
+    conv[at, 2 * heads * dim + 5] = bad
+    want, final = delta_plain(conv, gates, a_log, dt, start, lengths, heads, heads, dim, dim)
+    got, state = delta_run(conv, gates, a_log, dt, start, lengths, heads, heads, dim, dim)
+    calm = torch.ones(want.shape, dtype=torch.bool)
+    calm[at:lengths[0], 0, 5] = False
+    close(got[calm], want[calm], "float32", tight=2e-5)
+    close(state[1], final[1], "float32", tight=2e-5)
+    assert not torch.isfinite(got[at:lengths[0], 0, 5]).any() and not torch.isfinite(state[0, 0, :, 5]).any()
