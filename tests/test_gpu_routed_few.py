@@ -1,0 +1,54 @@
+"""Routed experts of few pairs: the products that stream the chosen experts' weights."""
+
+import pytest
+import torch
+
+from test_gpu_routed_wide import rand
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hidden,ff", [(72, 16), (264, 144), (1032, 272), (2080, 48)])
+@pytest.mark.parametrize("tokens", [1, 8, 9, 20, 21])
+@pytest.mark.parametrize("weight_inputs", [False, True])
+def test_few_pairs(tokens, hidden, ff, weight_inputs):
+    """An expert that every token chooses (units of eight pairs, one more, two and a half), one that none does; k that ends
+    inside a block of 32, with fewer blocks than warps and with several steps a warp; weight rows that end inside a unit.  A
+    token alone gives the same bits.  The activation is rounded to bfloat16 once, the sums are float32: 2^-7 of the largest."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+
+    rt = Runtime("cuda:0", "bfloat16")
+    rt.ops._load_moe()
+    experts, top = 6, 3
+    x = rand(tokens, hidden, seed=1).bfloat16()
+    router, bias = rand(experts, hidden, seed=2, scale=0.3), torch.tensor([0.0, 90.0, -90.0, 0.5, 0.0, -1.0])
+    gate, up = (rand(experts, ff, hidden, seed=s, scale=hidden ** -0.5).bfloat16() for s in (3, 4))
+    down = rand(experts, hidden, ff, seed=5, scale=ff ** -0.5).bfloat16()
+    assert rt.ops.moe_interleaves(hidden, ff) and tokens * top <= rt.ops.moe_few_pairs
+    both = rt.ops.interleave_gate_up(gate.cuda(), up.cuda())
+
+    def run(rows):
+        out = torch.full((rows.shape[0] + 1, hidden), 7.0).cuda()
+        rt.ops.routed_experts(rows.cuda(), router.cuda(), None, both, None, down.cuda(), top, False, out[:-1], rt.workspace,
+                              router_bias=bias.cuda(), chosen_softmax=True, weight_inputs=weight_inputs)
+        rt.ops.check_errors()
+        assert float((out[-1] - 7.0).abs().max()) == 0
+        return out[:-1].cpu()
+
+    out = run(x)
+    logits = x.double() @ router.double().T + bias.double()
+    best, chosen = torch.topk(logits, top, dim=1)
+    assert bool((chosen == 1).any(1).all()) and not bool((chosen == 2).any())
+    share = torch.softmax(best, dim=1)
+    want = torch.zeros(tokens, hidden, dtype=torch.float64)
+    for e in range(experts):
+        token, place = torch.nonzero(chosen == e, as_tuple=True)
+        rows, weight = x[token].double(), share[token, place].unsqueeze(1)
+        if weight_inputs:
+            rows = rows * weight
+        g = rows @ gate[e].double().T
+        y = (g * torch.sigmoid(g) * (rows @ up[e].double().T)) @ down[e].double().T
+        want[token] += y if weight_inputs else weight * y
+    assert float((out.double() - want).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
+    for t in range(tokens):
+        assert torch.equal(run(x[t:t + 1])[0], out[t])
