@@ -30,12 +30,13 @@ constexpr int kMaxExperts = 1024;
 constexpr int kRowTile = 128;         // rows of a tile of the grouped products
 
 // ---------------------------------------------------------------- route
-// One block of eight warps per kTokens tokens: their rows go to shared memory as float32, the warps share the experts (a
-// lane strides over a router row with 16-byte loads where the row length allows, and meets every token with it), then a warp
-// a token turns logits into scores and chooses.  A token's sums are added in the same order whatever kTokens.  With one
-// token a block every token asks L2 for the whole router matrix (2,048 tokens of 2,048, 16 experts: 262 MB, 35 us); four
-// share it where there are tokens enough for every SM.
-// ids / weights: [tokens][top]; counts[e] += 1 per choice.
+// One block of eight warps per kTokens tokens: their rows go to shared memory as float32, the warps share the experts, two at
+// a time (a lane strides over the router rows with 16-byte loads where the row length allows, and meets every token with
+// them), then a warp a token turns logits into scores and chooses.  A token's sums are added in the same order whatever
+// kTokens.  With one token a block every token asks L2 for the whole router matrix (2,048 tokens of 2,048, 16 experts: 262
+// MB, 35 us); four share it where there are tokens enough for every SM: 33 us with rows staged an element at a time and one
+// expert after the other, 15 with pieces of 16 bytes, four of a thread under way, and two experts.
+// ids / weights: [tokens][top].
 constexpr int kRouteWarps = 8;
 __host__ __device__ __forceinline__ int route_scores(int experts) { return (2 * experts + 3) & ~3; }
 __host__ __device__ __forceinline__ int route_row(int hidden, int groups) { return ((hidden > groups ? hidden : groups) + 3) & ~3; }
@@ -43,7 +44,7 @@ template <typename T, int kTokens>
 __global__ void __launch_bounds__(kRouteWarps * 32)
 moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
                  const float* __restrict__ correction, int* __restrict__ ids,
-                 float* __restrict__ weights, int* __restrict__ counts, int tokens,
+                 float* __restrict__ weights, int tokens,
                  int hidden, int experts, int top, int renormalize, const float* __restrict__ logit_bias,
                  int chosen_softmax, int sigmoid, int groups, int keep_groups, float norm_floor) {
   extern __shared__ __align__(16) float route_smem[];      // per token: scores, choice scores; then the rows
@@ -53,24 +54,53 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
   const int t0 = blockIdx.x * kTokens, count = min(kTokens, tokens - t0);
   const int score_ld = route_scores(experts), row_ld = route_row(hidden, groups);
   float* rows_s = route_smem + kTokens * score_ld;
-  for (int i = 0; i < count; ++i) {
-    const T* row = x + (size_t)(t0 + i) * hidden;
-    for (int k = threadIdx.x; k < hidden; k += blockDim.x) rows_s[i * row_ld + k] = to_float(row[k]);
+  constexpr int kPiece = 16 / sizeof(T);
+  if (hidden % kPiece == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    // 16-byte pieces of all tokens, four of a thread asked for together
+    const int pieces = hidden / kPiece, total = count * pieces;
+    const uint4* rows = reinterpret_cast<const uint4*>(x + (size_t)t0 * hidden);
+    for (int p0 = threadIdx.x; p0 < total; p0 += 4 * kRouteWarps * 32) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (p0 + u * kRouteWarps * 32 < total) v[u] = rows[p0 + u * kRouteWarps * 32];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int p = p0 + u * kRouteWarps * 32;
+        if (p >= total) break;
+        const int i = p / pieces;
+        const T* from = reinterpret_cast<const T*>(&v[u]);
+        float* to = rows_s + i * row_ld + (p - i * pieces) * kPiece;
+#pragma unroll
+        for (int e = 0; e < kPiece; e += 4)
+          *reinterpret_cast<float4*>(to + e) = make_float4(to_float(from[e]), to_float(from[e + 1]), to_float(from[e + 2]), to_float(from[e + 3]));
+      }
+    }
+  } else {
+    for (int i = 0; i < count; ++i) {
+      const T* row = x + (size_t)(t0 + i) * hidden;
+      for (int k = threadIdx.x; k < hidden; k += blockDim.x) rows_s[i * row_ld + k] = to_float(row[k]);
+    }
   }
   __syncthreads();
   const bool wide = hidden % 4 == 0;
-  constexpr int kDeep = kTokens > 1 ? 4 : 8;      // router loads in flight
-  for (int e = warp; e < experts; e += kRouteWarps) {
+  constexpr int kDeep = kTokens > 1 ? 4 : 8;      // router loads in flight, of two experts each
+  for (int e = warp; e < experts; e += 2 * kRouteWarps) {
+    const bool both = e + kRouteWarps < experts;
     const float* w = router + (size_t)e * hidden;
-    float dot[kTokens] = {};
+    const float* w2 = router + (size_t)(both ? e + kRouteWarps : e) * hidden;
+    float dot[2][kTokens] = {};
     if (wide) {
-      // several 16-byte loads of the router row are asked for before the first is used: the row comes
-      // from memory once a step and nothing else hides that trip
+      // several 16-byte loads of the router rows are asked for before the first is used: the rows come
+      // from memory once a step and nothing else hides that trip; two experts share what is read of the tokens
       for (int k0 = 4 * lane; k0 < hidden; k0 += kDeep * 128) {
-        float4 wv[kDeep];
+        float4 wv[2][kDeep];
 #pragma unroll
-        for (int u = 0; u < kDeep; ++u)
-          wv[u] = k0 + 128 * u < hidden ? *reinterpret_cast<const float4*>(w + k0 + 128 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int u = 0; u < kDeep; ++u) {
+          const bool in = k0 + 128 * u < hidden;
+          wv[0][u] = in ? *reinterpret_cast<const float4*>(w + k0 + 128 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+          wv[1][u] = in && both ? *reinterpret_cast<const float4*>(w2 + k0 + 128 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
 #pragma unroll
         for (int u = 0; u < kDeep; ++u) {
           if (k0 + 128 * u >= hidden) break;
@@ -78,25 +108,36 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
           for (int i = 0; i < kTokens; ++i) {
             if (i >= count) break;
             const float4 xv = *reinterpret_cast<const float4*>(rows_s + i * row_ld + k0 + 128 * u);
-            dot[i] = fmaf(xv.x, wv[u].x, dot[i]);
-            dot[i] = fmaf(xv.y, wv[u].y, dot[i]);
-            dot[i] = fmaf(xv.z, wv[u].z, dot[i]);
-            dot[i] = fmaf(xv.w, wv[u].w, dot[i]);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              dot[x][i] = fmaf(xv.x, wv[x][u].x, dot[x][i]);
+              dot[x][i] = fmaf(xv.y, wv[x][u].y, dot[x][i]);
+              dot[x][i] = fmaf(xv.z, wv[x][u].z, dot[x][i]);
+              dot[x][i] = fmaf(xv.w, wv[x][u].w, dot[x][i]);
+            }
           }
         }
       }
     } else {
       for (int k = lane; k < hidden; k += 32) {
-        const float wk = w[k];
+        const float wk = w[k], wk2 = w2[k];
 #pragma unroll
         for (int i = 0; i < kTokens; ++i)
-          if (i < count) dot[i] = fmaf(rows_s[i * row_ld + k], wk, dot[i]);
+          if (i < count) {
+            dot[0][i] = fmaf(rows_s[i * row_ld + k], wk, dot[0][i]);
+            dot[1][i] = fmaf(rows_s[i * row_ld + k], wk2, dot[1][i]);
+          }
       }
     }
 #pragma unroll
-    for (int i = 0; i < kTokens; ++i) {
-      const float total = warp_sum(dot[i]);
-      if (lane == 0) route_smem[i * score_ld + e] = logit_bias ? total + logit_bias[e] : total;
+    for (int x = 0; x < 2; ++x) {
+      if (x && !both) break;
+      const int at = e + x * kRouteWarps;
+#pragma unroll
+      for (int i = 0; i < kTokens; ++i) {
+        const float total = warp_sum(dot[x][i]);
+        if (lane == 0) route_smem[i * score_ld + at] = logit_bias ? total + logit_bias[at] : total;
+      }
     }
   }
   __syncthreads();
@@ -131,7 +172,6 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
       if (lane == 0) {
         ids[(size_t)t * top + j] = best_e;
         choice[best_e] = -INFINITY;
-        if (counts) atomicAdd(counts + best_e, 1);
       }
       __syncwarp();
     }
@@ -193,7 +233,6 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
       ids[(size_t)t * top + j] = best_e;
       weights[(size_t)t * top + j] = score[best_e];
       choice[best_e] = -INFINITY;
-      if (counts) atomicAdd(counts + best_e, 1);
     }
     chosen_sum += score[best_e];
     __syncwarp();
@@ -202,45 +241,83 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
 }
 
 // ---------------------------------------------------------------- plan
-// One block.  offsets[e] = first place of expert e (offsets[experts] = pairs); place_to_pair[p] =
-// the (token, choice) pair at place p; tiles: (expert, first place, rows) per tile, tile_count[0].
-__global__ void moe_plan_kernel(const int* __restrict__ ids, const int* __restrict__ counts,
-                                int* __restrict__ offsets, int* __restrict__ cursors,
-                                int* __restrict__ place_to_pair, int* __restrict__ tiles,
-                                int* __restrict__ tile_count, int pairs, int experts) {
-  __shared__ int off_s[kMaxExperts + 1];
-  __shared__ int tile_s[kMaxExperts + 1];
+// One block.  counts[e]: pairs of expert e; offsets[e] = its first place (offsets[experts] = pairs); place_to_pair[p] =
+// the (token, choice) pair at place p; tiles: (expert, first place, rows) per tile, tile_count[0].  Pairs of an expert that
+// a warp meets together are counted by one of its lanes, in shared memory.  8,192 pairs of 16 experts: 12 us (cold), whose
+// choices a thread at a time, one expert after the other in the sums and with counters in global memory, took as long; it also
+// spares the router its counters and a memset.
+__global__ void __launch_bounds__(1024)
+moe_plan_kernel(const int* __restrict__ ids, int* __restrict__ counts, int* __restrict__ offsets,
+                int* __restrict__ place_to_pair, int* __restrict__ tiles, int* __restrict__ tile_count, int pairs,
+                int experts) {
+  __shared__ int count_s[kMaxExperts], off_s[kMaxExperts], tile_s[kMaxExperts];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) count_s[e] = 0;
+  __syncthreads();
   pdl_wait();
   pdl_trigger();
-  if (threadIdx.x == 0) {
+  // a number of the expert's counter for this lane's pair
+  auto draw = [&](int* counter, int e) {
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    const int leader = __ffs(same) - 1;
+    int base = 0;
+    if (lane == leader && e >= 0) base = atomicAdd(counter + e, __popc(same));
+    return __shfl_sync(0xffffffffu, base, leader) + __popc(same & ((1u << lane) - 1u));
+  };
+  constexpr int kDeep = 8;                   // choices of a lane asked for together
+  int id[kDeep];
+  auto fetch = [&](int p0) {
+#pragma unroll
+    for (int u = 0; u < kDeep; ++u) id[u] = p0 + u * 1024 + lane < pairs ? ids[p0 + u * 1024 + lane] : -1;
+  };
+  for (int p0 = warp * 32; p0 < pairs; p0 += kDeep * 1024) {
+    fetch(p0);
+#pragma unroll
+    for (int u = 0; u < kDeep; ++u)
+      if (p0 + u * 1024 < pairs) draw(count_s, id[u]);
+  }
+  __syncthreads();
+  if (warp == 0) {
     int total = 0, tile_total = 0;
-    for (int e = 0; e < experts; ++e) {
-      off_s[e] = total;
-      tile_s[e] = tile_total;
-      total += counts[e];
-      tile_total += (counts[e] + kRowTile - 1) / kRowTile;
-    }
-    off_s[experts] = total;
-    tile_s[experts] = tile_total;
-    tile_count[0] = tile_total;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e <= experts; e += blockDim.x) {
-    offsets[e] = off_s[e];
-    if (e < experts) {
-      cursors[e] = 0;
-      const int n = off_s[e + 1] - off_s[e];
-      for (int j = 0, tile = tile_s[e]; j < n; j += kRowTile, ++tile) {
-        tiles[3 * tile] = e;
-        tiles[3 * tile + 1] = off_s[e] + j;
-        tiles[3 * tile + 2] = min(kRowTile, n - j);
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int n = e0 + lane < experts ? count_s[e0 + lane] : 0, n_tiles = (n + kRowTile - 1) / kRowTile;
+      int upto = n, tiles_upto = n_tiles;
+      for (int offset = 1; offset < 32; offset <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, upto, offset), b = __shfl_up_sync(0xffffffffu, tiles_upto, offset);
+        if (lane >= offset) { upto += a; tiles_upto += b; }
       }
+      if (e0 + lane < experts) {
+        off_s[e0 + lane] = total + upto - n;
+        tile_s[e0 + lane] = tile_total + tiles_upto - n_tiles;
+      }
+      total += __shfl_sync(0xffffffffu, upto, 31);
+      tile_total += __shfl_sync(0xffffffffu, tiles_upto, 31);
+    }
+    if (lane == 0) {
+      offsets[experts] = total;
+      tile_count[0] = tile_total;
     }
   }
   __syncthreads();
-  for (int pair = threadIdx.x; pair < pairs; pair += blockDim.x) {
-    const int e = ids[pair];
-    place_to_pair[off_s[e] + atomicAdd(cursors + e, 1)] = pair;
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+    const int n = count_s[e];
+    counts[e] = n;
+    offsets[e] = off_s[e];
+    for (int j = 0, tile = tile_s[e]; j < n; j += kRowTile, ++tile) {
+      tiles[3 * tile] = e;
+      tiles[3 * tile + 1] = off_s[e] + j;
+      tiles[3 * tile + 2] = min(kRowTile, n - j);
+    }
+  }
+  __syncthreads();
+  for (int p0 = warp * 32; p0 < pairs; p0 += kDeep * 1024) {
+    if (pairs > kDeep * 1024) fetch(p0);
+#pragma unroll
+    for (int u = 0; u < kDeep; ++u) {
+      if (p0 + u * 1024 >= pairs) break;
+      const int place = draw(off_s, id[u]);
+      if (id[u] >= 0) place_to_pair[place] = p0 + u * 1024 + lane;
+    }
   }
 }
 
@@ -523,7 +600,7 @@ using namespace cie;
 
 extern "C" int cie_moe_row_tile() { return kRowTile; }
 
-// counts, offsets (experts + 1), cursors, tile_count (1) and tiles (3 * (pairs / 64 + experts)) are
+// counts, offsets (experts + 1), cursors (not used), tile_count (1) and tiles (3 * (pairs / 64 + experts)) are
 // int32 scratch of the caller; counts is zeroed here.  counts null: only the choices and their weights are wanted.
 extern "C" int cie_moe_route(const void* x, const float* router, const float* correction, int* ids,
                              float* weights, int* counts, int* offsets, int* cursors, int* place_to_pair,
@@ -539,7 +616,6 @@ extern "C" int cie_moe_route(const void* x, const float* router, const float* co
   if (experts < 1 || experts > kMaxExperts) CIE_FAIL("moe_route: 1..%d experts, got %d", kMaxExperts, experts);
   if (top < 1 || top > experts || top > 32) CIE_FAIL("moe_route: top %d of %d experts (at most 32)", top, experts);
   cudaStream_t s = (cudaStream_t)stream;
-  if (counts && cudaMemsetAsync(counts, 0, sizeof(int) * experts, s) != cudaSuccess) CIE_FAIL("moe_route: memset failed");
   const int warps = kRouteWarps;
   const size_t one = (size_t)(route_scores(experts) + route_row(hidden, groups)) * sizeof(float);
   if (one > 200 * 1024) CIE_FAIL("moe_route: a row of %d elements does not fit shared memory", hidden);
@@ -553,7 +629,7 @@ extern "C" int cie_moe_route(const void* x, const float* router, const float* co
                                                  (int)smem) != cudaSuccess)                                                  \
       CIE_FAIL("moe_route: cannot reserve %zu bytes of shared memory", smem);                                                \
     CIE_LAUNCH("moe_route", (moe_route_kernel<T, N>), dim3(blocks), dim3(warps * 32), smem, s, (const T*)x, router,          \
-               correction, ids, weights, counts, tokens, hidden, experts, top, renormalize, logit_bias, chosen_softmax,      \
+               correction, ids, weights, tokens, hidden, experts, top, renormalize, logit_bias, chosen_softmax,              \
                sigmoid, groups, keep_groups, norm_floor);                                                                    \
   } while (0)
   if (dtype == kFloat32) {
@@ -567,8 +643,8 @@ extern "C" int cie_moe_route(const void* x, const float* router, const float* co
   }
 #undef CIE_MOE_ROUTE
   if (!counts) return 0;
-  CIE_LAUNCH("moe_plan", moe_plan_kernel, dim3(1), dim3(1024), 0, s, ids, counts, offsets, cursors, place_to_pair,
-             tiles, tile_count, tokens * top, experts);
+  CIE_LAUNCH("moe_plan", moe_plan_kernel, dim3(1), dim3(1024), 0, s, (const int*)ids, counts, offsets, place_to_pair, tiles,
+             tile_count, tokens * top, experts);
   return 0;
 }
 

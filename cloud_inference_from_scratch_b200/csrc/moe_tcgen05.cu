@@ -45,16 +45,25 @@ __device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 
 // sorted[p] = x[place_to_pair[p] / top], 16 bytes a thread.
-__global__ void moe_gather_rows_kernel(const bf16* __restrict__ x, bf16* __restrict__ sorted,
-                                       const int* __restrict__ place_to_pair, int pairs, int top, int hidden) {
+// A warp a row, eight of its pieces asked for together: 8,192 rows of 2,048: 9 us cold, 11 with a division and a
+// dependent load a piece (its bytes take 6)
+__global__ void __launch_bounds__(256)
+moe_gather_rows_kernel(const bf16* __restrict__ x, bf16* __restrict__ sorted, const int* __restrict__ place_to_pair, int pairs,
+                       int top, int hidden) {
   pdl_wait();
   pdl_trigger();
-  const int pieces = hidden / 8;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)pairs * pieces;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int p = (int)(i / pieces), c = (int)(i % pieces);
-    const int token = place_to_pair[p] / top;
-    reinterpret_cast<uint4*>(sorted + (size_t)p * hidden)[c] = reinterpret_cast<const uint4*>(x + (size_t)token * hidden)[c];
+  const int pieces = hidden / 8, lane = threadIdx.x & 31, p = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (p >= pairs) return;
+  const uint4* from = reinterpret_cast<const uint4*>(x + (size_t)(place_to_pair[p] / top) * hidden);
+  uint4* to = reinterpret_cast<uint4*>(sorted + (size_t)p * hidden);
+  for (int c = lane; c < pieces; c += 256) {
+    uint4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (c + 32 * u < pieces) v[u] = from[c + 32 * u];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (c + 32 * u < pieces) to[c + 32 * u] = v[u];
   }
 }
 
@@ -368,10 +377,7 @@ extern "C" int cie_moe_gate_up_tcgen05(const void* x, void* sorted, const void* 
     CIE_FAIL("moe_gate_up_tcgen05: operands must be 16-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
   const int pairs = tokens * top;
-  const long long pieces = (long long)pairs * (hidden / 8);
-  int blocks = (int)((pieces + 255) / 256);
-  if (blocks > device_sms() * 8) blocks = device_sms() * 8;
-  CIE_LAUNCH("moe_gather_rows", moe_gather_rows_kernel, dim3(blocks), dim3(256), 0, s, (const bf16*)x, (bf16*)sorted,
+  CIE_LAUNCH("moe_gather_rows", moe_gather_rows_kernel, dim3((pairs + 7) / 8), dim3(256), 0, s, (const bf16*)x, (bf16*)sorted,
              place_to_pair, pairs, top, hidden);
   const int bn = tile_columns(pairs, experts, 2 * ff);
   CUtensorMap map_a, map_b;
