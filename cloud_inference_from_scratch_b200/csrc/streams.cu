@@ -156,9 +156,7 @@ __device__ __forceinline__ void store_four(__nv_bfloat16* p, const float4& v) {
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
-// The row goes by in pieces of four elements where every part is whole, aligned ones, and the angles of a token are worked
-// out once, not once a head (a sine and a cosine each: 2,048 tokens of 16 + 2 heads of 128, half of every head rotated:
-// 19 us, 26 where a thread takes single elements and works out their angles itself; its bytes take 5).
+// Rows of any kind, an element or four at a time; the angles of a token are worked out once, not once a head.
 constexpr int kMaxAngles = 128;      // pairs whose angles are kept (more are worked out where they are used)
 template <typename TI, typename T>
 __global__ void norm_kv_write_kernel(const TI* __restrict__ src, const float* __restrict__ bias,
@@ -340,6 +338,140 @@ __global__ void norm_kv_write_kernel(const TI* __restrict__ src, const float* __
   }
 }
 
+// The same for rows whose parts are whole, aligned pieces of four elements, norms of whole projections or none, rotations of
+// halves that are whole pieces, and values that are not mixed: a thread keeps its pieces in registers, and the block meets
+// twice (the sums; the scaled row, whose other half the rotation reads).  What bounds it is how long a token's chain is and how
+// many tokens run at one time: angles, page and gains, which no kernel of the step writes, are there before the wait.  2,048
+// tokens of 16 + 2 heads of 128, half of every head rotated: 17 us cold (its bytes 5), 22 on
+// the kernel above; the attention layer of 2,048 tokens 101.5 -> 97, of eight single tokens 34.5 -> 32.
+constexpr int kRowPieces = 3;      // pieces of a thread at most: six blocks of 256 threads an SM
+template <typename TI, typename T, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads > 256 ? 2 : 6)
+norm_kv_pieces_kernel(const TI* __restrict__ src, const float* __restrict__ bias, T* __restrict__ q_out, int q_stride,
+                      const int* __restrict__ positions, const int* __restrict__ request_of_token,
+                      const int* __restrict__ table, int table_width, int num_pages, T* __restrict__ k_pool,
+                      T* __restrict__ v_pool, const float* __restrict__ q_gain, const float* __restrict__ k_gain, int q_heads,
+                      int kv_heads, int dim, int vdim, int page_size, int qk_norm, int v_norm, float eps, int write_cache,
+                      int src_stride, const float* __restrict__ inv_freq, int rot_dims, float magnitude, int interleaved,
+                      const QkvExtra extra, int* err) {
+  extern __shared__ __align__(16) float row_s[];
+  __shared__ float2 sums_s[kThreads / 32];
+  __shared__ __align__(16) float sin_s[kMaxAngles], cos_s[kMaxAngles];
+  const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int q_width = q_heads * dim, k_width = kv_heads * dim, width = q_width + k_width + kv_heads * vdim;
+  const int pos = positions[t], pairs = inv_freq ? rot_dims / 2 : 0;
+  for (int i = tid; i < pairs; i += kThreads) {
+    float sn, cs;
+    sincosf((float)pos * inv_freq[i], &sn, &cs);
+    sin_s[i] = sn * magnitude;
+    cos_s[i] = cs * magnitude;
+  }
+  const int request = request_of_token[t], index = pos / page_size;
+  const int page = index < table_width ? table[(size_t)request * table_width + index] : -1;
+  const bool kept = write_cache && !(extra.active && !extra.active[request]), bad = kept && (page < 0 || page >= num_pages);
+  const size_t slot = (size_t)page * kv_heads * page_size + (size_t)(pos % page_size);   // + head * page_size
+  pdl_wait();
+  pdl_trigger();
+  if (bad && tid == 0) atomicOr(err, kErrBadPage);
+  const TI* row = src + (size_t)t * src_stride;
+  float4 v[kRowPieces];
+#pragma unroll
+  for (int u = 0; u < kRowPieces; ++u) {
+    const int i = (u * kThreads + tid) * 4;
+    if (i < width) v[u] = load_four(row + i);
+  }
+  float sq_q = 0.f, sq_k = 0.f;
+#pragma unroll
+  for (int u = 0; u < kRowPieces; ++u) {
+    const int i = (u * kThreads + tid) * 4;
+    if (i >= width) break;
+    if (bias) {
+      const float4 b = load_four(bias + i);
+      v[u].x += b.x; v[u].y += b.y; v[u].z += b.z; v[u].w += b.w;
+    }
+    const float sq = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, v[u].w * v[u].w)));
+    if (i < q_width) sq_q += sq;
+    else if (i < q_width + k_width) sq_k += sq;
+  }
+  float inv_q = 1.f, inv_k = 1.f;
+  if (qk_norm) {
+    sq_q = warp_sum(sq_q);
+    sq_k = warp_sum(sq_k);
+    if (lane == 0) sums_s[warp] = make_float2(sq_q, sq_k);
+    __syncthreads();
+    float2 total = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+      total.x += sums_s[w].x;
+      total.y += sums_s[w].y;
+    }
+    inv_q = rsqrtf(total.x / (float)q_width + eps);
+    inv_k = rsqrtf(total.y / (float)k_width + eps);
+  }
+#pragma unroll
+  for (int u = 0; u < kRowPieces; ++u) {
+    const int i = (u * kThreads + tid) * 4;
+    if (i >= width) break;
+    if (qk_norm && i < q_width + k_width) {
+      const float4 gain = i < q_width ? load_four(q_gain + i) : load_four(k_gain + i - q_width);
+      const float inv = i < q_width ? inv_q : inv_k;
+      v[u].x = gain.x * (v[u].x * inv); v[u].y = gain.y * (v[u].y * inv);
+      v[u].z = gain.z * (v[u].z * inv); v[u].w = gain.w * (v[u].w * inv);
+    }
+    *reinterpret_cast<float4*>(row_s + i) = v[u];
+  }
+  __syncthreads();
+  const float warmth = extra.heat_every > 0 ? 1.f + extra.heat * logf((float)((pos + 1) / extra.heat_every) + 1.f) : 1.f;
+  T* q_row = q_out + (size_t)t * q_stride;
+#pragma unroll
+  for (int u = 0; u < kRowPieces; ++u) {
+    const int i = (u * kThreads + tid) * 4;
+    if (i >= q_width + k_width) break;
+    const int h = i / dim, d = i - h * dim;
+    if (d < 2 * pairs) {
+      if (interleaved) {
+        const float2 sn = *reinterpret_cast<const float2*>(sin_s + d / 2), cs = *reinterpret_cast<const float2*>(cos_s + d / 2);
+        v[u] = make_float4(v[u].x * cs.x - v[u].y * sn.x, v[u].y * cs.x + v[u].x * sn.x,
+                           v[u].z * cs.y - v[u].w * sn.y, v[u].w * cs.y + v[u].z * sn.y);
+      } else {
+        const bool second = d >= pairs;
+        const int at = second ? d - pairs : d;
+        const float4 sn = *reinterpret_cast<const float4*>(sin_s + at), cs = *reinterpret_cast<const float4*>(cos_s + at);
+        const float4 o = *reinterpret_cast<const float4*>(row_s + (second ? i - pairs : i + pairs));
+        // the first of a pair is u cos - v sin, the second v cos + u sin
+        if (second) v[u] = make_float4(v[u].x * cs.x + o.x * sn.x, v[u].y * cs.y + o.y * sn.y, v[u].z * cs.z + o.z * sn.z, v[u].w * cs.w + o.w * sn.w);
+        else v[u] = make_float4(v[u].x * cs.x - o.x * sn.x, v[u].y * cs.y - o.y * sn.y, v[u].z * cs.z - o.z * sn.z, v[u].w * cs.w - o.w * sn.w);
+      }
+    }
+    if (i < q_width) {
+      if (extra.heat_every > 0) { v[u].x *= warmth; v[u].y *= warmth; v[u].z *= warmth; v[u].w *= warmth; }
+      if (extra.q_factor) {
+        const float f = extra.q_factor[h];
+        v[u].x *= f; v[u].y *= f; v[u].z *= f; v[u].w *= f;
+      }
+      store_four(q_row + i, v[u]);
+    } else if (kept && !bad) {
+      store_four(k_pool + (slot + (size_t)(h - q_heads) * page_size) * dim + d, v[u]);
+    }
+  }
+  if (!kept || bad) return;
+  // value heads: a warp per head at a time
+  for (int h = warp; h < kv_heads; h += kThreads / 32) {
+    const float* head = row_s + q_width + k_width + h * vdim;
+    float inv = 1.f;
+    if (v_norm) {
+      float sq = 0.f;
+      for (int d = lane; d < vdim; d += 32) sq = fmaf(head[d], head[d], sq);
+      inv = rsqrtf(warp_sum(sq) / (float)vdim + eps);
+    }
+    for (int d = lane * 4; d < vdim; d += 128) {
+      float4 x = *reinterpret_cast<const float4*>(head + d);
+      x.x *= inv; x.y *= inv; x.z *= inv; x.w *= inv;
+      store_four(v_pool + (slot + (size_t)h * page_size) * vdim + d, x);
+    }
+  }
+}
+
 }  // namespace cie
 
 using namespace cie;
@@ -436,8 +568,21 @@ extern "C" int cie_norm_kv_write(const void* src, const float* bias, void* q_out
   if (src_stride == 0) src_stride = width;
   if (src_stride < width) CIE_FAIL("norm_kv_write: source rows of %d elements are shorter than q, k and v (%d)", src_stride, width);
   const size_t smem = (size_t)width * sizeof(float);
+  const auto aligned = [](auto... p) { return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) == 0; };
+  const bool in_pieces = (dim | vdim | src_stride | q_stride) % 4 == 0 && aligned(src, q_out, bias, q_gain, k_gain, k_pool, v_pool) &&
+                         qk_norm <= 1 && !v_mix && (!inv_freq || (rot_dims / 2 <= kMaxAngles && (interleaved ? rot_dims % 4 == 0 : rot_dims % 8 == 0)));
+#define CIE_NORM_PIECES(TI, T, N)                                                                               \
+  CIE_LAUNCH("norm_kv_write", (norm_kv_pieces_kernel<TI, T, N>), dim3(tokens), dim3(N), smem, (cudaStream_t)stream, \
+             (const TI*)src, bias, (T*)q_out, q_stride, positions, request_of_token, table, table_width,         \
+             num_pages, (T*)k_pool, (T*)v_pool, q_gain, k_gain, q_heads, kv_heads, dim, vdim, page_size,         \
+             qk_norm, v_norm, eps, write_cache, src_stride, inv_freq, rot_dims, magnitude, interleaved, extra, err)
 #define CIE_NORM_KV(TI, T)                                                                                      \
   do {                                                                                                           \
+    if (in_pieces && smem <= 40 * 1024 && width <= 4 * kRowPieces * 512) {                                       \
+      if (width <= 4 * kRowPieces * 256) CIE_NORM_PIECES(TI, T, 256);                                            \
+      else CIE_NORM_PIECES(TI, T, 512);                                                                          \
+      return 0;                                                                                                  \
+    }                                                                                                           \
     if (allow_shared(norm_kv_write_kernel<TI, T>, smem, "norm_kv_write")) return 1;                              \
     CIE_LAUNCH("norm_kv_write", (norm_kv_write_kernel<TI, T>), dim3(tokens), dim3(256), smem, (cudaStream_t)stream, \
                (const TI*)src, bias, (T*)q_out, q_stride, positions, request_of_token, table, table_width,       \
@@ -450,5 +595,6 @@ extern "C" int cie_norm_kv_write(const void* src, const float* bias, void* q_out
     else CIE_NORM_KV(T, T);
   })
 #undef CIE_NORM_KV
+#undef CIE_NORM_PIECES
   return 0;
 }

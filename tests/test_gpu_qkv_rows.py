@@ -1,0 +1,71 @@
+"""Norm, rotation and cache write of rows whose parts are whole pieces of four elements: the block sizes by row width and
+number of tokens, against the same in 64 bits."""
+
+import pytest
+import torch
+
+from test_gpu_routed_wide import rand
+
+pytestmark = pytest.mark.gpu
+
+
+def rotated(x, positions, inv_freq, dims, magnitude, interleaved):
+    angle = positions.double().view(-1, 1, 1) * inv_freq.double()
+    cos, sin = torch.cos(angle) * magnitude, torch.sin(angle) * magnitude
+    first, second = (slice(0, dims, 2), slice(1, dims, 2)) if interleaved else (slice(0, dims // 2), slice(dims // 2, dims))
+    out = x.clone()
+    out[..., first] = x[..., first] * cos - x[..., second] * sin
+    out[..., second] = x[..., second] * cos + x[..., first] * sin
+    return out
+
+
+@pytest.mark.parametrize("tokens,heads,kv_heads,dim,vdim", [
+    (3, 2, 1, 4, 8), (400, 4, 2, 64, 64), (5, 16, 2, 128, 128), (300, 33, 1, 128, 60), (400, 60, 4, 128, 64)])
+@pytest.mark.parametrize("norm,v_norm,bias,interleaved,rot", [
+    (1, 0, False, False, 1), (0, 1, True, True, 1), (1, 1, True, False, 0), (0, 0, False, False, 1)])
+def test_rows_in_pieces(tokens, heads, kv_heads, dim, vdim, norm, v_norm, bias, interleaved, rot):
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+
+    ops = Runtime("cuda:0", "float32").ops
+    ops._load_streams()
+    page_size, eps, magnitude = 16, 1e-6, 1.25
+    rot_dims = max(dim // 2 // 8 * 8, 4 if interleaved else 0) * rot
+    q_width, k_width, v_width = heads * dim, kv_heads * dim, kv_heads * vdim
+    width = q_width + k_width + v_width
+    src = rand(tokens, width + 4, seed=1)
+    gains = [1 + rand(n, seed=s, scale=0.2) for n, s in ((q_width, 2), (k_width, 3))]
+    shift = rand(width, seed=4)
+    positions = (torch.arange(tokens) * 7 % (tokens + 40)).int()
+    pages = -(-(tokens + 40) // page_size)
+    table = torch.randperm(pages, generator=torch.Generator().manual_seed(5)).int().view(1, -1)
+    freq = 10000.0 ** (-torch.arange(rot_dims // 2) / max(rot_dims // 2, 1)) if rot_dims else None
+    k_pool = torch.full((pages, kv_heads, page_size, dim), 7.0).cuda()
+    v_pool = torch.full((pages, kv_heads, page_size, vdim), 7.0).cuda()
+    out = torch.full((tokens + 1, q_width + 4), 7.0).cuda()
+    on = [t.cuda() if t is not None else None for t in (src, shift if bias else None, positions, table, *gains, freq)]
+    pointer = lambda t: t.data_ptr() if t is not None else None  # noqa: E731
+    requests = torch.zeros(tokens, dtype=torch.int32).cuda()
+    ops._norm_kv_write(pointer(on[0]), pointer(on[1]), out.data_ptr(), q_width + 4, pointer(on[2]), requests.data_ptr(),
+                       pointer(on[3]), pages, pages, k_pool.data_ptr(), v_pool.data_ptr(), pointer(on[4]), pointer(on[5]),
+                       tokens, heads, kv_heads, dim, vdim, page_size, norm, v_norm, eps, 1, width + 4, 0, pointer(on[6]),
+                       rot_dims, magnitude, int(interleaved), None, 0.0, 0, None, 0, None, None, 0, ops.error_word.data_ptr(),
+                       ops.stream)
+    ops.check_errors()
+    x = src[:, :width].double() + (shift.double() if bias else 0)
+    q, k, v = x[:, :q_width], x[:, q_width:q_width + k_width], x[:, q_width + k_width:].view(tokens, kv_heads, vdim)
+    if norm:
+        q, k = (t / torch.sqrt((t * t).mean(1, keepdim=True) + eps) * g.double() for t, g in ((q, gains[0]), (k, gains[1])))
+    q, k = q.view(tokens, heads, dim), k.view(tokens, kv_heads, dim)
+    if rot_dims:
+        q, k = (rotated(t, positions, freq, rot_dims, magnitude, interleaved) for t in (q, k))
+    if v_norm:
+        v = v / torch.sqrt((v * v).mean(2, keepdim=True) + eps)
+    page, place = table[0][positions.long() // page_size].long(), positions.long() % page_size
+    got = out.cpu().double()
+    # products and sums of float32; an angle of up to 440 is off by half a unit of its last place, 1.5e-5
+    assert float((got[:tokens, :q_width] - q.reshape(tokens, -1)).abs().max()) < 2e-4
+    assert float((got[tokens:] - 7).abs().max()) == 0 and float((got[:, q_width:] - 7).abs().max()) == 0
+    last = {int(p): t for t, p in enumerate(positions)}      # a position that comes twice: either row may win
+    single = torch.tensor([t for p, t in last.items() if int((positions == p).sum()) == 1])
+    assert float((k_pool.cpu()[page, :, place].double() - k)[single].abs().max()) < 2e-4
+    assert float((v_pool.cpu()[page, :, place].double() - v)[single].abs().max()) < 2e-5
