@@ -28,6 +28,7 @@ namespace cie {
 
 constexpr int kMaxExperts = 1024;
 constexpr int kRowTile = 128;         // rows of a tile of the grouped products
+constexpr int kTokenTile = 256;       // rows of a tile of the products in moe_tcgen05.cu at most
 
 // ---------------------------------------------------------------- route
 // One block of eight warps per kTokens tokens: their rows go to shared memory as float32, the warps share the experts, two at
@@ -242,15 +243,18 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
 
 // ---------------------------------------------------------------- plan
 // One block.  counts[e]: pairs of expert e; offsets[e] = its first place (offsets[experts] = pairs); place_to_pair[p] =
-// the (token, choice) pair at place p; tiles: (expert, first place, rows) per tile, tile_count[0].  Pairs of an expert that
+// the (token, choice) pair at place p; tiles: (expert, first place, rows) per tile, tile_count[0]; behind room for the most of
+// those there can be (`token_list`: the buffer has that room), how many tiles of up to kTokenTile rows there are and the same of them, the rows of an expert divided
+// evenly among them (in sixteens).  Pairs of an expert that
 // a warp meets together are counted by one of its lanes, in shared memory.  8,192 pairs of 16 experts: 12 us (cold), whose
 // choices a thread at a time, one expert after the other in the sums and with counters in global memory, took as long; it also
 // spares the router its counters and a memset.
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ ids, int* __restrict__ counts, int* __restrict__ offsets,
                 int* __restrict__ place_to_pair, int* __restrict__ tiles, int* __restrict__ tile_count, int pairs,
-                int experts) {
-  __shared__ int count_s[kMaxExperts], off_s[kMaxExperts], tile_s[kMaxExperts];
+                int experts, bool token_list) {
+  __shared__ int count_s[kMaxExperts], off_s[kMaxExperts], tile_s[kMaxExperts], token_tile_s[kMaxExperts];
+  int* token_tiles = tiles + 3 * ((pairs + kRowTile - 1) / kRowTile + experts);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int e = threadIdx.x; e < experts; e += blockDim.x) count_s[e] = 0;
   __syncthreads();
@@ -278,24 +282,29 @@ moe_plan_kernel(const int* __restrict__ ids, int* __restrict__ counts, int* __re
   }
   __syncthreads();
   if (warp == 0) {
-    int total = 0, tile_total = 0;
+    int total = 0, tile_total = 0, token_total = 0;
     for (int e0 = 0; e0 < experts; e0 += 32) {
       const int n = e0 + lane < experts ? count_s[e0 + lane] : 0, n_tiles = (n + kRowTile - 1) / kRowTile;
-      int upto = n, tiles_upto = n_tiles;
+      const int n_token = (n + kTokenTile - 1) / kTokenTile;
+      int upto = n, tiles_upto = n_tiles, token_upto = n_token;
       for (int offset = 1; offset < 32; offset <<= 1) {
         const int a = __shfl_up_sync(0xffffffffu, upto, offset), b = __shfl_up_sync(0xffffffffu, tiles_upto, offset);
-        if (lane >= offset) { upto += a; tiles_upto += b; }
+        const int c = __shfl_up_sync(0xffffffffu, token_upto, offset);
+        if (lane >= offset) { upto += a; tiles_upto += b; token_upto += c; }
       }
       if (e0 + lane < experts) {
         off_s[e0 + lane] = total + upto - n;
         tile_s[e0 + lane] = tile_total + tiles_upto - n_tiles;
+        token_tile_s[e0 + lane] = token_total + token_upto - n_token;
       }
       total += __shfl_sync(0xffffffffu, upto, 31);
       tile_total += __shfl_sync(0xffffffffu, tiles_upto, 31);
+      token_total += __shfl_sync(0xffffffffu, token_upto, 31);
     }
     if (lane == 0) {
       offsets[experts] = total;
       tile_count[0] = tile_total;
+      if (token_list) token_tiles[0] = token_total;
     }
   }
   __syncthreads();
@@ -307,6 +316,15 @@ moe_plan_kernel(const int* __restrict__ ids, int* __restrict__ counts, int* __re
       tiles[3 * tile] = e;
       tiles[3 * tile + 1] = off_s[e] + j;
       tiles[3 * tile + 2] = min(kRowTile, n - j);
+    }
+    if (token_list && n > 0) {
+      const int parts = (n + kTokenTile - 1) / kTokenTile, rows = ((n + parts - 1) / parts + 15) & ~15;
+      int* to = token_tiles + 1 + 3 * token_tile_s[e];
+      for (int i = 0; i < parts; ++i, to += 3) {
+        to[0] = e;
+        to[1] = off_s[e] + i * rows;
+        to[2] = min(rows, n - i * rows);
+      }
     }
   }
   __syncthreads();
@@ -600,7 +618,8 @@ using namespace cie;
 
 extern "C" int cie_moe_row_tile() { return kRowTile; }
 
-// counts, offsets (experts + 1), cursors (not used), tile_count (1) and tiles (3 * (pairs / 64 + experts)) are
+// counts, offsets (experts + 1), cursors (not used), tile_count (1) and tiles (3 * (pairs / 128 + experts) and 3 * (pairs / 256
+// + experts) + 1 more with two tokens and more, both rounded up) are
 // int32 scratch of the caller; counts is zeroed here.  counts null: only the choices and their weights are wanted.
 extern "C" int cie_moe_route(const void* x, const float* router, const float* correction, int* ids,
                              float* weights, int* counts, int* offsets, int* cursors, int* place_to_pair,
@@ -644,7 +663,7 @@ extern "C" int cie_moe_route(const void* x, const float* router, const float* co
 #undef CIE_MOE_ROUTE
   if (!counts) return 0;
   CIE_LAUNCH("moe_plan", moe_plan_kernel, dim3(1), dim3(1024), 0, s, (const int*)ids, counts, offsets, place_to_pair, tiles,
-             tile_count, tokens * top, experts);
+             tile_count, tokens * top, experts, tokens > 1);
   return 0;
 }
 

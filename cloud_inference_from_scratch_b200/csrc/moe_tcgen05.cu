@@ -1,23 +1,27 @@
 // The grouped products of routed experts on the 5th-generation tensor cores.
 //
-// The (token, expert) pairs of a step are grouped by expert on the device (moe.cu: places, tiles of
-// up to 128 rows of one expert).  Here a CTA takes one such tile and 128 output columns: the tile's
-// rows and the expert's weight rows come by TMA (128-byte swizzle) into a three-stage ring, one
-// thread issues tcgen05.mma into a float32 accumulator in tensor memory, and the four warps read
-// it back with tcgen05.ld for the epilogue.  Rows must lie one after another for TMA, so the
+// The (token, expert) pairs of a step are grouped by expert on the device (moe.cu: places, and tiles of up to 256 of them that
+// belong to one expert and divide its rows evenly).  Weights are the left operand: a CTA an SM walks over tiles of 128
+// weight rows and the tile's tokens, rounded up to 16, so that nothing is multiplied for tokens that an expert does
+// not have.  Both come by TMA (128-byte swizzle) into a ring, one thread issues tcgen05.mma into float32 accumulators in
+// tensor memory, and eight warps read a tile back with tcgen05.ld while the next one's products run; a lane holds a weight row, so that 32
+// lanes write neighbouring columns of a token.  Rows must lie one after another for TMA, so the
 // gate/up product first gathers the tokens' rows by place (one memory-bound kernel); the down
 // product reads the activations, which the gate/up product wrote by place.
 //
 //   gate_up  W = [experts][2F][H], gate and up rows of an expert interleaved in blocks of 16 (16 gate
-//            rows, their 16 up rows, ...): a thread holds both halves of SiLU(gate) * up and writes
-//            act[place][channel] (bfloat16)
+//            rows, their 16 up rows, ...): lanes exchange them, every lane works one SiLU(gate) * up out of
+//            two tokens, act[place][channel] (bfloat16)
 //   down     W = [experts][H][F]; the result goes, float32, to the row of the tile row's pair
 //
-// A tile's rows beyond the expert's last (they belong to the next expert, or lie outside the buffer
-// and read as zero) and columns beyond the expert's last are computed and never stored.  Two CTAs
-// share an SM (97 KB of shared memory and 128 tensor-memory columns each), so one CTA's epilogue
-// runs beside the other's products.  Steps of many pairs run on one CTA an SM that walks tiles of 256 columns
-// (moe_grouped_wide_kernel).  Every wait on an mbarrier is bounded.
+// A tile's rows beyond the expert's last (they belong to the next expert, or lie outside the buffer and read as zero) are
+// computed and never stored.  Every wait on an mbarrier is bounded.
+// What bounds a large product: a stage's way through copy, products and back, 2 us of which four stages of 48 KB cover less
+// than the products would use up (85 us of the 98 below without the epilogue, 70 without loads), and the epilogue's
+// instructions.  2,048 tokens, 4 of 16 experts of 1,376 channels, 2,048 wide: 98 and 58 us, with token rows as the
+// left operand in tiles of 128 by 256 119 and 66.  Tiles of 256 weight rows take up all of tensor memory, so that nothing hides
+// their epilogue: 100 and 61.  Asking L2 for later weights: 3 us more.  The layer of 17 tokens 94 -> 88, 512 tokens 123 -> 103,
+// 2,048 tokens of 32 experts of 2,048 channels, 4,096 wide, 689 -> 589.
 #include "blackwell.cuh"
 #include "common.cuh"
 #include "glu.cuh"
@@ -29,22 +33,12 @@ namespace cie {
 using namespace bw;
 using bf16 = __nv_bfloat16;
 
-constexpr int BM = 128, BK = 64, UMMA_K = 16, STAGES = 3;
-constexpr int A_STAGE_BYTES = BM * BK * 2;
-// BN, the output columns of a tile: 128 here, 256 in the kernel further down
-template <int BN> constexpr int stage_bytes() { return A_STAGE_BYTES + BN * BK * 2; }
-template <int BN> constexpr size_t smem_bytes() { return (size_t)STAGES * stage_bytes<BN>() + 1024; }
+constexpr int BM = 128, BK = 64, UMMA_K = 16;
+constexpr int TOKENS = 256, TOKEN_BOX = 64;      // tokens of a tile at most; of one copy
+constexpr int WEIGHT_BYTES = BM * BK * 2, BOX_BYTES = TOKEN_BOX * BK * 2;
+constexpr int STAGES = 4, STAGE_BYTES = WEIGHT_BYTES + TOKENS * BK * 2;
+constexpr size_t GROUPED_SMEM = (size_t)STAGES * STAGE_BYTES + 1024;
 
-__device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// sorted[p] = x[place_to_pair[p] / top], 16 bytes a thread.
 // A warp a row, eight of its pieces asked for together: 8,192 rows of 2,048: 9 us cold, 11 with a division and a
 // dependent load a piece (its bytes take 6)
 __global__ void __launch_bounds__(256)
@@ -70,8 +64,7 @@ moe_gather_rows_kernel(const bf16* __restrict__ x, bf16* __restrict__ sorted, co
 struct GroupedArgs {
   void* out;
   const int* place_to_pair;
-  const int* tiles;        // (expert, first place, rows) per tile
-  const int* tile_count;
+  const int* tiles;        // how many, then (expert, first place, rows) of each
   int rows_per_expert;     // weight rows of one expert (2F or H)
   int n;                   // output columns of a row (F or H)
   int k;
@@ -79,283 +72,177 @@ struct GroupedArgs {
   GluAct glu_act;          // gate_up
 };
 
-// One row of a tile (tensor-memory lane `r` of a warp's quarter, whose first column is `lane_base`) to where it goes; whole
-// warps.
-template <bool kGateUp, int BN>
-__device__ __forceinline__ void write_tile(const GroupedArgs& a, uint32_t lane_base, int r, int place0, int rows, int col0_tile) {
-  const bool live = r < rows;
-  if constexpr (kGateUp) {
-    bf16* dst_row = reinterpret_cast<bf16*>(a.out) + (size_t)(place0 + r) * a.n;
-    const float weight = live && a.glu_act.weights ? a.glu_act.weights[a.place_to_pair[place0 + r]] : 1.f;
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 32) {
-      uint32_t gate[16], up[16];
-      tmem_load16(lane_base + c0, gate);          // every lane of the warp takes part in the load
-      tmem_load16(lane_base + c0 + 16, up);
-      const int channel0 = (col0_tile + c0) / 2;  // 32 interleaved rows hold 16 channels
-      if (!live || channel0 >= a.n) continue;
-      if (channel0 + 16 <= a.n) {
-        uint32_t packed[8];
+// The results of 128 weight rows (a warp the 32 lanes whose first column is `from`) and every second 32 of a tile's tokens
+// (from `first` on) to where they go.  pairs: those of the lane's tokens, which are read before the results are waited for.
+constexpr int kTurns = TOKENS / 64;
+template <bool kGateUp>
+__device__ __forceinline__ void write_tile(const GroupedArgs& a, uint32_t from, int row0, int place0, int rows, int first,
+                                           const int (&pairs)[kTurns]) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float v0 = glu(a.glu_act, __uint_as_float(gate[2 * j]), __uint_as_float(up[2 * j]), weight);
-          const float v1 = glu(a.glu_act, __uint_as_float(gate[2 * j + 1]), __uint_as_float(up[2 * j + 1]), weight);
-          __nv_bfloat162 pair = __floats2bfloat162_rn(v0, v1);
-          packed[j] = *reinterpret_cast<uint32_t*>(&pair);
-        }
-        reinterpret_cast<uint4*>(dst_row + channel0)[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        reinterpret_cast<uint4*>(dst_row + channel0)[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-      } else {
+  for (int turn = 0; turn < kTurns; ++turn) {
+    const int c0 = first + 64 * turn;
+    if (c0 >= rows) break;
+    uint32_t raw[32];
+    tmem_ld32(from + c0, raw);                     // every lane of the warp takes part in the load
+    const int pair = pairs[turn];
+    const float weight = kGateUp && a.glu_act.weights ? a.glu_act.weights[pair] : 1.f;
+    tc_wait_ld();
+    if constexpr (kGateUp) {
+      // lanes 0 .. 15 hold 16 gate rows, 16 .. 31 their up rows: the lower lanes take the even tokens, the upper the odd ones
+      const bool upper = lane >= 16;
+      const int channel = row0 / 2 + (lane & 15);
+      bf16* dst = reinterpret_cast<bf16*>(a.out) + (size_t)(place0 + c0 + upper) * a.n + channel;
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (channel0 + j < a.n) dst_row[channel0 + j] = __float2bfloat16_rn(glu(a.glu_act, __uint_as_float(gate[j]), __uint_as_float(up[j]), weight));
+      for (int c = 0; c < 32; c += 2) {
+        const float mine = __uint_as_float(upper ? raw[c + 1] : raw[c]);
+        const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(upper ? raw[c] : raw[c + 1]), 16);
+        const float w = __shfl_sync(0xffffffffu, weight, c + upper);
+        if (c0 + c + upper < rows && channel < a.n)
+          dst[(size_t)c * a.n] = __float2bfloat16_rn(glu_rounded(a.glu_act, upper ? other : mine, upper ? mine : other, w));
       }
-    }
-  } else {
-    const int pair = live ? a.place_to_pair[place0 + r] : 0;
-    float* dst_row = reinterpret_cast<float*>(a.out) + (size_t)pair * a.n;
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 16) {
-      uint32_t raw[16];
-      tmem_load16(lane_base + c0, raw);
-      const int col0 = col0_tile + c0;
-      if (!live || col0 >= a.n) continue;
-      if (col0 + 16 <= a.n) {
+    } else {
+      float* dst = reinterpret_cast<float*>(a.out) + row0 + lane;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          reinterpret_cast<float4*>(dst_row + col0)[j] =
-              make_float4(__uint_as_float(raw[4 * j]), __uint_as_float(raw[4 * j + 1]),
-                          __uint_as_float(raw[4 * j + 2]), __uint_as_float(raw[4 * j + 3]));
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (col0 + j < a.n) dst_row[col0 + j] = __uint_as_float(raw[j]);
+      for (int c = 0; c < 32; ++c) {
+        const int to = __shfl_sync(0xffffffffu, pair, c);
+        if (c0 + c < rows && row0 + lane < a.n) dst[(size_t)to * a.n] = __uint_as_float(raw[c]);
       }
     }
   }
 }
 
-template <bool kGateUp, int BN>
-__global__ void __launch_bounds__(128) moe_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
-                                                                   const __grid_constant__ CUtensorMap map_b,
-                                                                   const GroupedArgs a) {
-  constexpr int STAGE_BYTES = stage_bytes<BN>();
+// map_w: weight rows of all experts in boxes of 128, map_x: token rows in boxes of TOKEN_BOX.  Warps: copies, products, two
+// groups of eight that write every second tile out.
+constexpr int GROUPED_THREADS = 64 + 16 * 32;
+template <bool kGateUp>
+__global__ void __launch_bounds__(GROUPED_THREADS, 1)
+moe_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GroupedArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* stage_base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full_bar[STAGES];
-  __shared__ __align__(8) uint64_t empty_bar[STAGES];
-  __shared__ __align__(8) uint64_t acc_bar;
+  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
-
-  pdl_wait();
-  pdl_trigger();
-  if ((int)blockIdx.y >= a.tile_count[0]) return;       // the grid holds the most tiles a step can have
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int expert = a.tiles[3 * blockIdx.y], place0 = a.tiles[3 * blockIdx.y + 1], rows = a.tiles[3 * blockIdx.y + 2];
-  const int col0_tile = blockIdx.x * BN;                 // first weight row of the tile inside the expert
-  const int b_row0 = expert * a.rows_per_expert + col0_tile;
-  const int k_tiles = (a.k + BK - 1) / BK;
-
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
-    mbar_init(&acc_bar, 1);
-    mbar_init_fence();
-  }
-  if (warp == 0) {
-    __syncwarp();
-    tmem_alloc<BN>(&tmem_base_s);
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = tmem_base_s;
-
-  if (warp == 0) {
-    if (lane == 0) {     // copies
-      for (int kt = 0; kt < k_tiles; ++kt) {
-        const int s = kt % STAGES;
-        const uint32_t phase = (kt / STAGES) & 1;
-        if (!mbar_wait(&empty_bar[s], phase ^ 1, a.err)) break;
-        mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-        unsigned char* dst = stage_base + (size_t)s * STAGE_BYTES;
-        tma_load_2d(dst, &map_a, &full_bar[s], kt * BK, place0);
-        tma_load_2d(dst + A_STAGE_BYTES, &map_b, &full_bar[s], kt * BK, b_row0);
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0) {     // products
-      constexpr uint32_t idesc = idesc_bf16(BM, BN);
-      for (int kt = 0; kt < k_tiles; ++kt) {
-        const int s = kt % STAGES;
-        const uint32_t phase = (kt / STAGES) & 1;
-        if (!mbar_wait(&full_bar[s], phase, a.err)) break;
-        tc_fence_after();
-        const uint32_t a_addr = smem_u32(stage_base + (size_t)s * STAGE_BYTES);
-        const uint64_t a_desc = smem_desc_sw128(a_addr), b_desc = smem_desc_sw128(a_addr + A_STAGE_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < BK / UMMA_K; ++kk)
-          umma_bf16(tmem_base, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (kt > 0 || kk > 0) ? 1u : 0u);
-        tc_commit(&empty_bar[s]);
-      }
-      tc_commit(&acc_bar);
-    }
-    __syncwarp();
-  }
-
-  // ---- epilogue: warp w reads tensor-memory lanes 32w .. 32w + 31 (rows of the tile)
-  const bool ready = mbar_wait(&acc_bar, 0, a.err);
-  tc_fence_after();
-  if (ready) {
-    write_tile<kGateUp, BN>(a, tmem_base + ((uint32_t)(warp * 32) << 16), warp * 32 + lane, place0, rows, col0_tile);
-  } else {
-    // a wait ran out: give copies that may still be in flight time to land before leaving
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_free<BN>(tmem_base);
-}
-
-// Many tiles: one CTA an SM walks 128 x 256 tiles (row tile by row tile, all columns of one after another, so that the CTAs
-// of a moment share their rows and the weights of a few experts).  Four stages of 48 KB; two accumulators of 256 columns in
-// tensor memory, so that four warps write a tile out while the next one's products run.  With 256 columns the operands of a
-// product are 96 bytes of shared memory a cycle; 128 columns (above, two CTAs an SM) ask for all 128 it has.
-constexpr int WIDE = 256, WIDE_STAGES = 4, WIDE_THREADS = 192;      // warps: copies, products, four that write out
-constexpr size_t WIDE_SMEM = (size_t)WIDE_STAGES * stage_bytes<WIDE>() + 1024;
-
-template <bool kGateUp>
-__global__ void __launch_bounds__(WIDE_THREADS, 1)
-moe_grouped_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GroupedArgs a) {
-  constexpr int STAGE_BYTES = stage_bytes<WIDE>();
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* stage_base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full_bar[WIDE_STAGES], empty_bar[WIDE_STAGES], acc_full[2], acc_empty[2];
-  __shared__ uint32_t tmem_base_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    for (int s = 0; s < WIDE_STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
-    }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_empty[i], 4);
+      mbar_init(&acc_empty[i], 8);
     }
     mbar_init_fence();
   }
   pdl_wait();
   pdl_trigger();
-  if (warp == 1) tmem_alloc<2 * WIDE>(&tmem_base_s);
+  if (warp == 1) tmem_alloc<2 * TOKENS>(&tmem_base_s);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_s;
-  const int column_tiles = (a.rows_per_expert + WIDE - 1) / WIDE, total = a.tile_count[0] * column_tiles;
+  const int row_tiles = (a.rows_per_expert + BM - 1) / BM, total = a.tiles[0] * row_tiles;
   const int k_tiles = (a.k + BK - 1) / BK;
   bool alive = true;
+  // tile t: all weight rows of one tile of tokens after another, so that the CTAs of a moment share tokens and a few experts
+  struct Tile { int expert, place0, rows, row0; };
+  auto tile_at = [&](int t) {
+    const int of_tokens = t / row_tiles;
+    const int* at = a.tiles + 1 + 3 * of_tokens;
+    return Tile{at[0], at[1], at[2], (t - of_tokens * row_tiles) * BM};
+  };
 
   if (warp == 0) {
     if (lane == 0) {     // copies
-      int it = 0;        // stages filled so far
+      int s = 0;
+      uint32_t phase = 1;
       for (int t = blockIdx.x; t < total && alive; t += gridDim.x) {
-        const int row_tile = t / column_tiles, col0 = (t - row_tile * column_tiles) * WIDE;
-        const int place0 = a.tiles[3 * row_tile + 1], b_row0 = a.tiles[3 * row_tile] * a.rows_per_expert + col0;
-        for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-          const int s = it % WIDE_STAGES;
-          if (!mbar_wait(&empty_bar[s], ((it / WIDE_STAGES) & 1) ^ 1, a.err)) { alive = false; break; }
-          mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-          unsigned char* dst = stage_base + (size_t)s * STAGE_BYTES;
-          tma_load_2d(dst, &map_a, &full_bar[s], kt * BK, place0);
-          tma_load_2d(dst + A_STAGE_BYTES, &map_b, &full_bar[s], kt * BK, b_row0);
+        const Tile tile = tile_at(t);
+        const int boxes = (tile.rows + TOKEN_BOX - 1) / TOKEN_BOX, w_row = tile.expert * a.rows_per_expert + tile.row0;
+        for (int kt = 0; kt < k_tiles; ++kt) {
+          if (!mbar_wait(&empty_bar[s], phase, a.err)) { alive = false; break; }
+          mbar_expect_tx(&full_bar[s], WEIGHT_BYTES + boxes * BOX_BYTES);
+          unsigned char* dst = ring + (size_t)s * STAGE_BYTES;
+          tma_load_2d(dst, &map_w, &full_bar[s], kt * BK, w_row);
+          for (int b = 0; b < boxes; ++b)
+            tma_load_2d(dst + WEIGHT_BYTES + b * BOX_BYTES, &map_x, &full_bar[s], kt * BK, tile.place0 + b * TOKEN_BOX);
+          if (++s == STAGES) { s = 0; phase ^= 1; }
         }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     if (lane == 0) {     // products
-      constexpr uint32_t idesc = idesc_bf16(BM, WIDE);
-      int it = 0, n = 0;
+      int s = 0, n = 0;
+      uint32_t phase = 0;
       for (int t = blockIdx.x; t < total && alive; t += gridDim.x, ++n) {
-        const int acc = n & 1;
-        // the accumulator's last tile has been written out
-        if (!mbar_wait(&acc_empty[acc], ((n >> 1) & 1) ^ 1, a.err)) { alive = false; break; }
+        const Tile tile = tile_at(t);
+        const uint32_t idesc = idesc_bf16(BM, (tile.rows + 15) & ~15);
+        // the accumulator's last results have been written out
+        if (!mbar_wait(&acc_empty[n & 1], ((n >> 1) & 1) ^ 1, a.err)) { alive = false; break; }
         tc_fence_after();
-        for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-          const int s = it % WIDE_STAGES;
-          if (!mbar_wait(&full_bar[s], (it / WIDE_STAGES) & 1, a.err)) { alive = false; break; }
+        const uint32_t acc = tmem_base + (n & 1) * TOKENS;
+        for (int kt = 0; kt < k_tiles; ++kt) {
+          if (!mbar_wait(&full_bar[s], phase, a.err)) { alive = false; break; }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(stage_base + (size_t)s * STAGE_BYTES);
-          const uint64_t a_desc = smem_desc_sw128(a_addr), b_desc = smem_desc_sw128(a_addr + A_STAGE_BYTES);
+          const uint32_t at = smem_u32(ring + (size_t)s * STAGE_BYTES);
+          const uint64_t w_desc = smem_desc_sw128(at), x_desc = smem_desc_sw128(at + WEIGHT_BYTES);
 #pragma unroll
           for (int kk = 0; kk < BK / UMMA_K; ++kk)
-            umma_bf16(tmem_base + acc * WIDE, a_desc + 2 * kk, b_desc + 2 * kk, idesc, (kt > 0 || kk > 0) ? 1u : 0u);
+            umma_bf16(acc, w_desc + 2 * kk, x_desc + 2 * kk, idesc, (kt > 0 || kk > 0) ? 1u : 0u);
           tc_commit(&empty_bar[s]);
+          if (++s == STAGES) { s = 0; phase ^= 1; }
         }
-        if (alive) tc_commit(&acc_full[acc]);
+        if (!alive) break;
+        tc_commit(&acc_full[n & 1]);
       }
     }
     __syncwarp();
   } else {
-    const int quarter = warp & 3;      // the tensor-memory lanes a warp may read
+    const int quarter = warp & 3, group = (warp - 2) >> 3;      // the tensor-memory lanes a warp may read
+    const int first = ((warp - 2) >> 2 & 1) * 32;
     int n = 0;
     for (int t = blockIdx.x; t < total && alive; t += gridDim.x, ++n) {
-      const int row_tile = t / column_tiles, col0 = (t - row_tile * column_tiles) * WIDE, acc = n & 1;
-      const int place0 = a.tiles[3 * row_tile + 1], rows = a.tiles[3 * row_tile + 2];
-      alive = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (n >> 1) & 1, a.err));
+      if ((n & 1) != group) continue;
+      const Tile tile = tile_at(t);
+      int pairs[kTurns];
+#pragma unroll
+      for (int turn = 0; turn < kTurns; ++turn) {
+        const int c = first + 64 * turn + lane;
+        pairs[turn] = (!kGateUp || a.glu_act.weights) && c < tile.rows ? a.place_to_pair[tile.place0 + c] : 0;
+      }
+      alive = __all_sync(0xffffffffu, mbar_wait(&acc_full[group], (n >> 1) & 1, a.err));
       if (!alive) break;
       tc_fence_after();
-      write_tile<kGateUp, WIDE>(a, tmem_base + acc * WIDE + ((uint32_t)(quarter * 32) << 16), quarter * 32 + lane, place0, rows, col0);
+      const int row0 = tile.row0 + quarter * 32;
+      if (row0 < a.rows_per_expert)
+        write_tile<kGateUp>(a, tmem_base + group * TOKENS + ((uint32_t)(quarter * 32) << 16), row0, tile.place0, tile.rows,
+                            first, pairs);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[acc]);
+      if (lane == 0) mbar_arrive(&acc_empty[group]);
     }
   }
   if (!alive)      // a wait ran out: give copies and products that may still be in flight time to end before leaving
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_free<2 * WIDE>(tmem_base);
+  if (warp == 1) tmem_free<2 * TOKENS>(tmem_base);
 }
 
 template <bool kGateUp>
-static int launch_wide(const CUtensorMap& map_a, const CUtensorMap& map_b, const GroupedArgs& a, cudaStream_t stream) {
-  static const cudaError_t raised =
-      cudaFuncSetAttribute(moe_grouped_wide_kernel<kGateUp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WIDE_SMEM);
-  if (raised != cudaSuccess) CIE_FAIL("moe_tcgen05: cannot set the wide kernel up: %s", cudaGetErrorString(raised));
-  CIE_LAUNCH("moe_tcgen05", moe_grouped_wide_kernel<kGateUp>, dim3(device_sms()), dim3(WIDE_THREADS), WIDE_SMEM, stream, map_a, map_b, a);
+static int launch_grouped(const char* name, const void* x, const void* w, int pairs, int experts, const GroupedArgs& a, cudaStream_t stream) {
+  CUtensorMap map_w, map_x;
+  if (!tensor_map_bf16(x, pairs, a.k, TOKEN_BOX, &map_x) || !tensor_map_bf16(w, (long long)experts * a.rows_per_expert, a.k, BM, &map_w))
+    CIE_FAIL("%s: cuTensorMapEncodeTiled failed", name);
+  static const cudaError_t raised = cudaFuncSetAttribute(moe_grouped_kernel<kGateUp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GROUPED_SMEM);
+  if (raised != cudaSuccess) CIE_FAIL("%s: cannot set the kernel up: %s", name, cudaGetErrorString(raised));
+  CIE_LAUNCH(name, moe_grouped_kernel<kGateUp>, dim3(device_sms()), dim3(GROUPED_THREADS), GROUPED_SMEM, stream, map_w, map_x, a);
   return 0;
 }
 
-template <bool kGateUp, int BN>
-static int launch_grouped(const CUtensorMap& map_a, const CUtensorMap& map_b, const GroupedArgs& a, dim3 grid,
-                          cudaStream_t stream) {
-  constexpr size_t smem = smem_bytes<BN>();
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t status = cudaFuncSetAttribute(moe_grouped_tcgen05_kernel<kGateUp, BN>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (status != cudaSuccess) CIE_FAIL("moe_tcgen05: shared memory %zu: %s", smem, cudaGetErrorString(status));
-    configured = true;
-  }
-  CIE_LAUNCH("moe_tcgen05", (moe_grouped_tcgen05_kernel<kGateUp, BN>), grid, dim3(128), smem, stream, map_a, map_b, a);
-  return 0;
-}
-
-// Tiles of 256 columns on one CTA an SM from three rounds of them on (below that, tiles of 128 on two CTAs an SM fill the
-// last round better), counting the row tiles of evenly filled experts.  16 experts of 2,048 and 1,376: 512 tokens (176
-// tiles) 133 us against 120, 2,048 tokens (704) 230 against 274; 32 of 4,096 and 2,048: 128 tokens (512) 304 against 320,
-// 2,048 (1,024) 670 against 768.  CIE_MOE_TILE_COLUMNS=128|256 forces one of them.
-static int tile_columns(int pairs, int experts, int columns) {
-  const char* asked = getenv("CIE_MOE_TILE_COLUMNS");
-  const int forced = asked ? atoi(asked) : 0;
-  if (forced == 128 || forced == 256) return forced;
-  const long long rows = pairs < experts ? pairs : (long long)experts * ((pairs + experts * BM - 1) / (experts * BM));
-  return rows * ((columns + WIDE - 1) / WIDE) >= 3ll * device_sms() ? 256 : 128;
-}
+// The list of tiles of up to TOKENS tokens, which moe.cu leaves behind the one of tiles of BM.
+static const int* token_tiles(const int* tiles, int pairs, int experts) { return tiles + 3 * ((pairs + BM - 1) / BM + experts); }
 
 }  // namespace cie
 
@@ -379,16 +266,9 @@ extern "C" int cie_moe_gate_up_tcgen05(const void* x, void* sorted, const void* 
   const int pairs = tokens * top;
   CIE_LAUNCH("moe_gather_rows", moe_gather_rows_kernel, dim3((pairs + 7) / 8), dim3(256), 0, s, (const bf16*)x, (bf16*)sorted,
              place_to_pair, pairs, top, hidden);
-  const int bn = tile_columns(pairs, experts, 2 * ff);
-  CUtensorMap map_a, map_b;
-  if (!tensor_map_bf16(sorted, pairs, hidden, BM, &map_a) ||
-      !tensor_map_bf16(w_gate_up, (long long)experts * 2 * ff, hidden, bn, &map_b))
-    CIE_FAIL("moe_gate_up_tcgen05: cuTensorMapEncodeTiled failed");
-  GroupedArgs a = {act, place_to_pair, tiles, tile_count, 2 * ff, ff, hidden, err,
-                   {clamped, limit, slope, shift, input_weights}};
-  const int max_tiles = (pairs + BM - 1) / BM + experts;
-  const dim3 grid((2 * ff + bn - 1) / bn, max_tiles);
-  return bn == 256 ? launch_wide<true>(map_a, map_b, a, s) : launch_grouped<true, 128>(map_a, map_b, a, grid, s);
+  const GroupedArgs a = {act, place_to_pair, token_tiles(tiles, pairs, experts), 2 * ff, ff, hidden, err,
+                         {clamped, limit, slope, shift, input_weights}};
+  return launch_grouped<true>("moe_gate_up_tcgen05", sorted, w_gate_up, pairs, experts, a, s);
 }
 
 // act: [tokens * top][ff] by place; w_down: [experts][hidden][ff]; rows: float32 [tokens * top][hidden],
@@ -402,14 +282,6 @@ extern "C" int cie_moe_down_tcgen05(const void* act, const void* w_down, float* 
   if ((reinterpret_cast<uintptr_t>(act) | reinterpret_cast<uintptr_t>(w_down) | reinterpret_cast<uintptr_t>(rows)) & 15)
     CIE_FAIL("moe_down_tcgen05: operands must be 16-byte aligned");
   const int pairs = tokens * top;
-  const int bn = tile_columns(pairs, experts, hidden);
-  CUtensorMap map_a, map_b;
-  if (!tensor_map_bf16(act, pairs, ff, BM, &map_a) ||
-      !tensor_map_bf16(w_down, (long long)experts * hidden, ff, bn, &map_b))
-    CIE_FAIL("moe_down_tcgen05: cuTensorMapEncodeTiled failed");
-  GroupedArgs a = {rows, place_to_pair, tiles, tile_count, hidden, hidden, ff, err, {}};
-  const int max_tiles = (pairs + BM - 1) / BM + experts;
-  const dim3 grid((hidden + bn - 1) / bn, max_tiles);
-  cudaStream_t s = (cudaStream_t)stream;
-  return bn == 256 ? launch_wide<false>(map_a, map_b, a, s) : launch_grouped<false, 128>(map_a, map_b, a, grid, s);
+  const GroupedArgs a = {rows, place_to_pair, token_tiles(tiles, pairs, experts), hidden, hidden, ff, err, {}};
+  return launch_grouped<false>("moe_down_tcgen05", act, w_down, pairs, experts, a, (cudaStream_t)stream);
 }

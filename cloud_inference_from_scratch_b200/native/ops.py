@@ -1519,12 +1519,14 @@ class Ops:
         plan = workspace.get("moe.plan", tokens, 6 * experts + 8 + (3 * top + 63) // 64, torch.int32).view(-1)
         counts, offsets, cursors = plan[:experts], plan[experts:2 * experts + 1], plan[2 * experts + 1:3 * experts + 1]
         tile_count, tiles = plan[3 * experts + 1:3 * experts + 2], plan[3 * experts + 2:]
-        assert tiles.numel() >= 3 * (-(-pairs // self.moe_row_tile) + experts)
+        # (tiles of 128 rows and, behind them, tiles of up to 256)
+        listed = 3 * (-(-pairs // self.moe_row_tile) + experts) + 1 + 3 * (-(-pairs // 256) + experts)
+        assert tiles.numel() >= listed or tokens == 1
         act = workspace.get("moe.act", tokens, top * ff, self.dtype)
         rows = workspace.get("moe.rows", tokens, top * hidden, torch.float32)
         code = self._code_of(x)
         # few pairs (a decode step) stream the chosen experts' weights and need no plan
-        few = w_up is None and pairs <= self.moe_few_pairs and max(hidden, ff) <= 12288
+        few = w_up is None and pairs <= self.moe_few_pairs
         self.launches += 4 if few else 5
         self._moe_route(_ptr(x), _ptr(router), _ptr(correction), _ptr(ids), _ptr(weights), None if few else _ptr(counts),
                         _ptr(offsets), _ptr(cursors), _ptr(place_to_pair), _ptr(tiles), _ptr(tile_count), tokens,
