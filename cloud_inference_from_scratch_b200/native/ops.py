@@ -36,6 +36,8 @@ def _ptr(tensor: Any) -> int | None:
 # tensor path (the gate/up product of 64 tokens took 30 us against the library's 17) and its
 # epilogues, which finish a token row per warp, by the number of rows.
 STREAM_MAX_ROWS = 16
+# rows of a float32 product whose terms lie in scratch memory at one time
+F32_BLOCK = 2048
 # Up to this many rows a projection adds itself into the residual stream, or rotates and stores
 # q/k/v (cluster epilogues of the streaming kernel): every row count that kernel takes.
 FUSED_RESIDUAL_MAX_ROWS = STREAM_MAX_ROWS
@@ -120,7 +122,10 @@ class Ops:
         self._gemm_f32 = None
         if self.code == F32:
             gf = _Lib(load_library("gemm_f32_tcgen05.cu"))
-            self._gemm_f32 = gf.function("cie_gemm_f32_tc", [v, v, v, v, i, i, i, i, v, v])
+            self._gemm_f32_tc = gf.function("cie_gemm_f32_tc", [v, v, v, v, i, i, i, i, v, v, v])
+            gf.handle.cie_gemm_f32_tc_floats.restype = ctypes.c_longlong
+            self._gemm_f32_floats = gf.handle.cie_gemm_f32_tc_floats
+            self._gemm_f32 = self._f32_product
             self._gemm_f32_takes = gf.handle.cie_gemm_f32_tc_takes
             self._gemm_f32_takes.argtypes = [v, v, i]
         ag = _Lib(load_library("attention_generic.cu"))
@@ -1693,6 +1698,7 @@ class Ops:
             self._cublas_linear(x, weight, bias, out)
             return out
         self.launches += 1
+        # (the tensor cores' form: and one that splits the rows of x)
         if (self._gemm_f32 is not None and not few_rows and x.dtype == weight.dtype == out.dtype == self.torch.float32
                 and self._gemm_f32_takes(_ptr(x), _ptr(weight), k)):
             self._gemm_f32(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), m, n, k, 0, self.error_word.data_ptr(), self.stream)
@@ -1700,6 +1706,25 @@ class Ops:
         self._gemm_simt(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), m, n, k, self._code_of(x),
                         self._code_of(out), 0 if self.code == F32 else 1, self.stream)
         return out
+
+    def _f32_product(self, x: int, weight: int, bias: int | None, out: int, m: int, n: int, k: int, columns: int, err: int,
+                     stream: int) -> None:
+        """The float32 product on the tensor cores, all operands by address.  The terms of x's rows go through scratch
+        memory that holds F32_BLOCK rows at most (or what there is of it under captured graphs): more rows come in
+        blocks, which changes no bit of a row."""
+        floats = self._gemm_f32_floats
+        held = self._partial_buffers.get("gemm_f32.terms")
+        rows = min(m, F32_BLOCK)
+        need = int(floats(rows, k))
+        if held is None or held.numel() < need:
+            if held is not None and self.scratch_frozen:
+                rows = max(1, min(rows, held.numel() // int(floats(1, k) + 4)))
+                need = int(floats(rows, k))
+            held = self.scratch("gemm_f32.terms", need, reserve=max(int(floats(min(max(m, self.max_rows), F32_BLOCK), k)), 1 << 19))
+        for first in range(0, m, rows):
+            self.launches += 1
+            self._gemm_f32_tc(x + 4 * first * k, weight, bias, out + 4 * first * n, min(rows, m - first), n, k, columns,
+                              held.data_ptr(), err, stream)
 
     def _skinny_gemm(self) -> Any:
         if self._skinny is None:
