@@ -21,6 +21,7 @@
 // the last bits; the difference stays within 1e-5 of the largest value.
 #include "common.cuh"
 #include "head_gate.cuh"
+#include "state_walk.cuh"
 
 CIE_DEFINE_LAST_ERROR()
 
@@ -302,32 +303,29 @@ delta_stream_kernel(const float* __restrict__ packed, float* __restrict__ out, i
 //     A_ts = (u_t b_(t-1)) . (a_s u_s / b_s)      B_ts = (u_t b_(t-1)) . (k_s / b_s)
 //
 // so Y = Y' + W S_0 with the same elimination on both right-hand sides, and with C_ts, D_ts (s <= t) the same products of
-// r_t b_t:
+// r_t b_t, and U = -Y:
 //
-//     O   = (diag-scaled r - C W) S_0 + (D V - C Y')                       = Q S_0 + O'
-//     S_C = b_C ((I - sum_s (a_s u_s / b_s) W_s) S_0 + sum_s (k_s / b_s) v_s - (a_s u_s / b_s) y'_s)   = M S_0 + N
+//     U   = -Y' - W S_0
+//     O   = diag-scaled r S_0 + D V + C U
+//     S_C = b_C S_0 + sum_s (b_C k_s / b_s) v_s + (b_C a_s u_s / b_s) u'_s            (u'_s: row s of U)
 //
-//   1. delta_chunk (per chunk and head): M, Q, N and O'
-//   2. delta_walk  (per request, head, 16 value columns): [S; O] <- [M; Q] S + [N; O'], chunk after chunk
+//   1. delta_chunk (per chunk and head): A, B, C, D, W, Y' and the scaled rows
+//   2. the walk of state_walk.cuh (per request, head and block of value columns)
 //
-// Float32 on the CUDA cores.  A token's results read rows of tokens up to its own alone (no weight of zero times a later
-// row).  Against the stream below, whose chain of one token is 450 instructions long and which a prompt of one request
-// and 32 heads runs on 32 SMs: 2,048 tokens, 32 heads of 64: 246 us in chunks, 1,790 as a stream (heads of 128, 16 of them:
-// 515 and 3,945).  What bounds delta_chunk is the data that shared memory
-// can return (128 bytes a cycle: a 16-byte load of a warp is four cycles), hence tiles of 4 x 4 and more a thread; [M; Q]
-// instead of the low-rank form keeps the walk at one product and one barrier a chunk.
+// Float32: 1 on the CUDA cores, 2 as accurately on the tensor cores.  A token's results read rows of tokens up to its own
+// alone (no weight of zero times a later row).  Against the stream below, whose chain of one token is 450 instructions long and
+// which a prompt of one request and 32 heads runs on 32 SMs: 2,048 tokens, 32 heads of 64: 207 us in chunks, 1,790 as a stream (16
+// heads of 128: 356 and 3,945).  What bounds delta_chunk is the data that shared memory
+// can return (128 bytes a cycle: a 16-byte load of a warp is four cycles), hence tiles of 4 x 4 and more a thread.  With what a
+// chunk does to any state as one matrix, [S; O] <- [M; Q] S + [N; O'], its products on the CUDA cores, the two kernels took
+// 246 us (heads of 128: 515; eight portions of 287 tokens, 32 heads of 128: 1,143, now 635).
 constexpr int kDeltaChunkTokens = 32;
-constexpr int kDeltaWalkColumns = 16;
 constexpr int kDeltaMat = 2 * kDeltaChunkTokens + 4;      // row of the matrices [A C; B D], transposed
 
 template <int P>
 constexpr int delta_chunk_smem() {
   return (6 * kDeltaChunkTokens * (P + 4) + 2 * kDeltaChunkTokens * kDeltaMat + P + kDeltaChunkTokens + 256) * (int)sizeof(float);
 }
-
-// Floats of one chunk and head: [M; Q] and [N; O'], (P + C) rows of P each.
-template <int P>
-constexpr int delta_chunk_cell() { return 2 * (P + kDeltaChunkTokens) * P; }
 
 // grid (chunks, heads), 256 threads
 template <int P>
@@ -435,32 +433,27 @@ delta_chunk_kernel(const float* __restrict__ proj, int proj_stride, int r_off, i
       }
   }
   __syncthreads();
-  // acc[i] += sign * sum_(s <= t) mat_row[s][t] x[s][d] for the thread's TG tokens (`diagonal`: s = t too)
-  auto triangle = [&](const float* mat_row, const float* x, float (&acc)[TG], float sign, bool diagonal) {
+  {
+    // B V, a thread a column of its TG tokens
+    float bv[TG] = {};
+    const float* mat_row = mat + C * ML + g * TG;
     for (int s = 0; s < g * TG; ++s) {
-      const float xv = sign * x[s * LD + d];
+      const float xv = vs[s * LD + d];
 #pragma unroll
       for (int i = 0; i < TG; i += 4) {
-        const float4 m = *reinterpret_cast<const float4*>(mat_row + s * ML + g * TG + i);
-        acc[i] = fmaf(m.x, xv, acc[i]);
-        acc[i + 1] = fmaf(m.y, xv, acc[i + 1]);
-        acc[i + 2] = fmaf(m.z, xv, acc[i + 2]);
-        acc[i + 3] = fmaf(m.w, xv, acc[i + 3]);
+        const float4 m = *reinterpret_cast<const float4*>(mat_row + s * ML + i);
+        bv[i] = fmaf(m.x, xv, bv[i]);
+        bv[i + 1] = fmaf(m.y, xv, bv[i + 1]);
+        bv[i + 2] = fmaf(m.z, xv, bv[i + 2]);
+        bv[i + 3] = fmaf(m.w, xv, bv[i + 3]);
       }
     }
 #pragma unroll
     for (int q = 0; q < TG; ++q) {
-      const float xv = sign * x[(g * TG + q) * LD + d];
+      const float xv = vs[(g * TG + q) * LD + d];
 #pragma unroll
-      for (int i = 0; i < TG; ++i)
-        if (i > q || (i == q && diagonal)) acc[i] = fmaf(mat_row[(g * TG + q) * ML + g * TG + i], xv, acc[i]);
+      for (int i = q + 1; i < TG; ++i) bv[i] = fmaf(mat_row[(g * TG + q) * ML + i], xv, bv[i]);
     }
-  };
-  float dv[TG] = {};
-  {
-    float bv[TG] = {};
-    triangle(mat + C * ML, vs, bv, 1.f, false);
-    triangle(mat + C * ML + C, vs, dv, 1.f, true);
 #pragma unroll
     for (int i = 0; i < TG; ++i) ys[(g * TG + i) * LD + d] = bv[i];
   }
@@ -485,147 +478,32 @@ delta_chunk_kernel(const float* __restrict__ proj, int proj_stride, int r_off, i
     for (int t = 0; t < C; ++t) column[t * LD] = x[t];
   }
   __syncthreads();
-  float* mq = cells + ((size_t)chunk * heads + head) * delta_chunk_cell<P>();
-  float* no = mq + (P + C) * P;
-  {
-    float q[TG];
+  // the cell (tokens past the last one have rows of zeros)
+  float* cell = cells + ((size_t)chunk * heads + head) * walk_cell_floats(P, 2);
+  bool unsafe = false;
+  const float kept = bn[d];
 #pragma unroll
-    for (int i = 0; i < TG; ++i) q[i] = rb[(g * TG + i) * LD + d];
-    triangle(mat + C, ub, q, -1.f, true);
-    triangle(mat + C, ys, dv, -1.f, true);
-#pragma unroll
-    for (int i = 0; i < TG; ++i) {
-      mq[(P + g * TG + i) * P + d] = q[i];
-      no[(P + g * TG + i) * P + d] = dv[i];
-    }
+  for (int i = 0; i < TG; ++i) {
+    const int t = g * TG + i;
+    const float r = rb[t * LD + d], w = ub[t * LD + d], k = kept * ki[t * LD + d], removed = kept * ai[t * LD + d];
+    unsafe |= tf32_unsafe(r) || tf32_unsafe(w) || tf32_unsafe(k) || tf32_unsafe(removed);
+    cell[t * walk_q_row(P) + d] = r;
+    cell[walk_cell_w(P) + t * walk_q_row(P) + d] = w;
+    cell[walk_cell_k(P, 2) + t * walk_k_row(P) + d] = k;
+    cell[walk_cell_k2(P) + t * walk_k_row(P) + d] = removed;
+    cell[walk_cell_v2(P) + t * P + d] = -ys[t * LD + d];
   }
-  // M and N: a thread takes 4 x 4 cells
-  for (int tile = warp; tile < (P / 16) * (P / 32); tile += 8) {
-    const int d0 = tile % (P / 16) * 16 + (lane >> 3) * 4, c0 = tile / (P / 16) * 32 + (lane & 7) * 4;
-    float m[4][4] = {}, z[4][4] = {};
-#pragma unroll 2
-    for (int s = 0; s < n; ++s) {
-      const float4 av = *reinterpret_cast<const float4*>(ai + s * LD + d0), kv = *reinterpret_cast<const float4*>(ki + s * LD + d0);
-      const float4 wv = *reinterpret_cast<const float4*>(ub + s * LD + c0), yv = *reinterpret_cast<const float4*>(ys + s * LD + c0);
-      const float4 xv = *reinterpret_cast<const float4*>(vs + s * LD + c0);
-      const float a4[4] = {av.x, av.y, av.z, av.w}, k4[4] = {kv.x, kv.y, kv.z, kv.w}, w4[4] = {wv.x, wv.y, wv.z, wv.w};
-      const float y4[4] = {yv.x, yv.y, yv.z, yv.w}, v4[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          m[i][j] = fmaf(-a4[i], w4[j], m[i][j]);
-          z[i][j] = fmaf(k4[i], v4[j], fmaf(-a4[i], y4[j], z[i][j]));
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float b = bn[d0 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) m[i][j] = b * ((d0 + i == c0 + j ? 1.f : 0.f) + m[i][j]);
-      *reinterpret_cast<float4*>(mq + (d0 + i) * P + c0) = make_float4(m[i][0], m[i][1], m[i][2], m[i][3]);
-      *reinterpret_cast<float4*>(no + (d0 + i) * P + c0) = make_float4(b * z[i][0], b * z[i][1], b * z[i][2], b * z[i][3]);
-    }
+  if (g == 0) cell[walk_cell_decay(P, 2) + d] = kept;
+  for (int e = tid; e < C * C; e += 256) {
+    const int t = e / C, s = e % C;
+    const float c = mat[s * ML + C + t], dv = mat[(C + s) * ML + C + t];
+    unsafe |= tf32_unsafe(c) || tf32_unsafe(dv);
+    cell[walk_cell_a(P, 2) + t * kWalkA + s] = dv;
+    cell[walk_cell_a2(P) + t * kWalkA + s] = c;
   }
-}
-
-template <int P>
-constexpr int delta_walk_stages() { return P > 64 ? 2 : 3; }
-template <int P>
-constexpr int delta_walk_smem() {
-  return (delta_walk_stages<P>() * (P + kDeltaChunkTokens) * (P + 4) + 2 * P * kDeltaWalkColumns) * (int)sizeof(float);
-}
-
-// grid (requests, heads, P / kDeltaWalkColumns), a warp 16 rows of [M; Q].  S lies in shared memory, [M; Q] of the next
-// chunks comes through a ring of cp.async stages, a thread's part of [N; O'] one chunk ahead in registers; the CTA meets
-// once a chunk.
-template <int P>
-__global__ void __launch_bounds__((P + kDeltaChunkTokens) * 2)
-delta_walk_kernel(const float* __restrict__ cells, float* __restrict__ out, int out_stride, float* __restrict__ state,
-                  const int* __restrict__ chunk_row, const int* __restrict__ chunk_count,
-                  const int* __restrict__ request_chunk_start, const int* __restrict__ slots,
-                  const int* __restrict__ request_active, int heads, int dim, int max_slots, int* err) {
-  constexpr int C = kDeltaChunkTokens, ROWS = P + C, LD = P + 4, VC = kDeltaWalkColumns, STAGES = delta_walk_stages<P>();
-  constexpr int THREADS = ROWS * 2;
-  extern __shared__ __align__(16) float delta_smem[];
-  float* ring = delta_smem;                      // [STAGES][ROWS][LD]
-  float* s_s = ring + STAGES * ROWS * LD;        // [2][P][VC]
-  pdl_wait();
-  pdl_trigger();
-  const int request = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * VC, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int slot = slots[request];
-  if (slot < 0 || slot >= max_slots) {
-    if (tid == 0) atomicOr(err, kErrBadRequest);
-    return;
-  }
-  const int first = request_chunk_start[request], last = request_chunk_start[request + 1];
-  float* s_base = state + ((size_t)slot * heads + head) * dim * dim;
-  for (int e = tid; e < P * VC; e += THREADS) {
-    const int row = e / VC, v = v0 + e % VC;
-    s_s[e] = row < dim && v < dim ? s_base[(size_t)row * dim + v] : 0.f;
-  }
-  auto cell = [&](int chunk) { return cells + ((size_t)chunk * heads + head) * delta_chunk_cell<P>(); };
-  auto issue = [&](int chunk) {
-    if (chunk < last) {
-      const float* src = cell(chunk);
-      float* dst = ring + (chunk - first) % STAGES * ROWS * LD;
-      for (int e = tid; e < ROWS * (P / 4); e += THREADS) delta_cp_async16(dst + e / (P / 4) * LD + e % (P / 4) * 4, src + 4 * e);
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-  };
-  for (int i = 0; i < STAGES - 1; ++i) issue(first + i);
-  const int r0 = warp * 16 + (lane >> 3), c = (lane & 7) * 2;      // rows r0, r0 + 4, ..; two columns
-  float2 next[4];
-  auto fetch = [&](int chunk) {
-    const float* src = cell(chunk) + ROWS * P + r0 * P + v0 + c;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) next[i] = *reinterpret_cast<const float2*>(src + 4 * i * P);
-  };
-  if (first < last) fetch(first);
-  for (int chunk = first; chunk < last; ++chunk) {
-    const int buf = (chunk - first) & 1, row0 = chunk_row[chunk], n = chunk_count[chunk];
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
-    __syncthreads();          // the stage has landed, S is whole, and everybody is done with the stage before
-    issue(chunk + STAGES - 1);
-    float2 acc[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i] = next[i];
-    if (chunk + 1 < last) fetch(chunk + 1);
-    const float* mq = ring + (chunk - first) % STAGES * ROWS * LD + r0 * LD;
-    const float* s = s_s + buf * P * VC + c;
-#pragma unroll 4
-    for (int x = 0; x < P; x += 4) {
-      float2 sv[4];
-#pragma unroll
-      for (int y = 0; y < 4; ++y) sv[y] = *reinterpret_cast<const float2*>(s + (x + y) * VC);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 m = *reinterpret_cast<const float4*>(mq + 4 * i * LD + x);
-        acc[i].x = fmaf(m.x, sv[0].x, acc[i].x); acc[i].y = fmaf(m.x, sv[0].y, acc[i].y);
-        acc[i].x = fmaf(m.y, sv[1].x, acc[i].x); acc[i].y = fmaf(m.y, sv[1].y, acc[i].y);
-        acc[i].x = fmaf(m.z, sv[2].x, acc[i].x); acc[i].y = fmaf(m.z, sv[2].y, acc[i].y);
-        acc[i].x = fmaf(m.w, sv[3].x, acc[i].x); acc[i].y = fmaf(m.w, sv[3].y, acc[i].y);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = r0 + 4 * i;
-      if (row < P) {
-        *reinterpret_cast<float2*>(s_s + (buf ^ 1) * P * VC + row * VC + c) = acc[i];
-      } else if (row - P < n) {
-        float* dst = out + (size_t)(row0 + row - P) * out_stride + head * dim + v0 + c;
-        if (v0 + c < dim) dst[0] = acc[i].x;
-        if (v0 + c + 1 < dim) dst[1] = acc[i].y;
-      }
-    }
-  }
-  asm volatile("cp.async.wait_group 0;\n" ::);
-  __syncthreads();
-  if (request_active[request] && first < last)
-    for (int e = tid; e < P * VC; e += THREADS) {
-      const int row = e / VC, v = v0 + e % VC;
-      if (row < dim && v < dim) s_base[(size_t)row * dim + v] = s_s[((last - first) & 1) * P * VC + e];
-    }
+  const bool any = __syncthreads_or(unsafe);
+  if (tid == 0)
+    *reinterpret_cast<float2*>(cell + walk_cell_decay(P, 2) + P) = make_float2(any ? 1.f : 0.f, __int_as_float(n));
 }
 
 }  // namespace cie
@@ -708,8 +586,7 @@ static int delta_pad(int dim) { return dim <= 32 ? 32 : dim <= 64 ? 64 : 128; }
 
 // Floats of scratch memory the chunked form wants.
 extern "C" long long cie_delta_chunk_floats(int chunks, int heads, int dim) {
-  const int pad = delta_pad(dim);
-  return (long long)chunks * heads * (pad == 32 ? cie::delta_chunk_cell<32>() : pad == 64 ? cie::delta_chunk_cell<64>() : cie::delta_chunk_cell<128>());
+  return (long long)chunks * heads * cie::walk_cell_floats(delta_pad(dim), 2);
 }
 
 // Portions in chunks of cie_delta_chunk_tokens() tokens: first token row and token count of every chunk, and where every
@@ -725,29 +602,22 @@ extern "C" int cie_delta_chunked(const float* proj, int proj_stride, int r_off, 
   if (dim < 1 || dim > kDeltaStreamMaxDim) CIE_FAIL("delta_chunked: head size %d is outside 1..%d", dim, kDeltaStreamMaxDim);
   if (heads > 65535) CIE_FAIL("delta_chunked: too many heads");
   if (reinterpret_cast<uintptr_t>(cells) & 15) CIE_FAIL("delta_chunked: scratch memory must be 16-byte aligned");
-#define CIE_DELTA_CHUNKED(P)                                                                                               \
-  {                                                                                                                        \
-    static const cudaError_t raised = [] {                                                                                 \
-      const cudaError_t one =                                                                                              \
-          cudaFuncSetAttribute(delta_chunk_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, delta_chunk_smem<P>()); \
-      return one != cudaSuccess ? one                                                                                      \
-                                : cudaFuncSetAttribute(delta_walk_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                                       delta_walk_smem<P>());                                              \
-    }();                                                                                                                   \
-    if (raised != cudaSuccess) CIE_FAIL("delta_chunked: %s", cudaGetErrorString(raised));                                  \
-    CIE_LAUNCH("delta_chunk", delta_chunk_kernel<P>, dim3(chunks, heads), dim3(256), delta_chunk_smem<P>(),                \
-               (cudaStream_t)stream, proj, proj_stride, r_off, k_off, v_off, a_off, decay, decay_stride, decay_bias,       \
-               removal_bias, cells, chunk_row, chunk_count, heads, dim);                                                   \
-    CIE_LAUNCH("delta_walk", delta_walk_kernel<P>, dim3(requests, heads, P / kDeltaWalkColumns),                           \
-               dim3((P + kDeltaChunkTokens) * 2), delta_walk_smem<P>(), (cudaStream_t)stream, cells, out, out_stride,      \
-               state, chunk_row, chunk_count, request_chunk_start, slots, request_active, heads, dim, max_slots, err);     \
-  }
-  switch (delta_pad(dim)) {
-    case 32: CIE_DELTA_CHUNKED(32) break;
-    case 64: CIE_DELTA_CHUNKED(64) break;
-    default: CIE_DELTA_CHUNKED(128)
-  }
-#undef CIE_DELTA_CHUNKED
+  const cudaStream_t s = (cudaStream_t)stream;
+  const int pad = delta_pad(dim);
+  auto go = [&](auto kernel, int smem) {
+    const cudaError_t raised = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return raised != cudaSuccess ? raised
+                                 : launch(kernel, dim3(chunks, heads), dim3(256), (size_t)smem, s, proj, proj_stride, r_off, k_off, v_off,
+                                          a_off, decay, decay_stride, decay_bias, removal_bias, cells, chunk_row, chunk_count, heads, dim);
+  };
+  const cudaError_t status = pad == 32   ? go(delta_chunk_kernel<32>, delta_chunk_smem<32>())
+                             : pad == 64 ? go(delta_chunk_kernel<64>, delta_chunk_smem<64>())
+                                         : go(delta_chunk_kernel<128>, delta_chunk_smem<128>());
+  if (status != cudaSuccess) CIE_FAIL("delta_chunk: launch failed: %s", cudaGetErrorString(status));
+  const WalkArgs walk{cells, proj + v_off, proj_stride, dim, out, out_stride, state, (long long)heads * dim * dim, chunk_row, chunk_count,
+                      request_chunk_start, slots, request_active, heads, dim, dim, max_slots, err};
+  const cudaError_t walked = launch_state_walk<2>(walk, pad, requests, s);
+  if (walked != cudaSuccess) CIE_FAIL("delta_walk: launch failed: %s", cudaGetErrorString(walked));
   return 0;
 }
 

@@ -139,7 +139,7 @@ gla_chunk_kernel(GlaRows in, float* __restrict__ cells, const int* __restrict__ 
   pdl_trigger();
   const int chunk = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row0 = chunk_row[chunk], n = chunk_count[chunk];
-  float* cell = cells + ((size_t)chunk * heads + head) * walk_cell_floats(P, false);
+  float* cell = cells + ((size_t)chunk * heads + head) * walk_cell_floats(P, 0);
   const int d = tid % P, group = tid / P, t0 = group * TG;
   if (group < G) {
     const bool live = d < dim;
@@ -182,9 +182,9 @@ gla_chunk_kernel(GlaRows in, float* __restrict__ cells, const int* __restrict__ 
       const float from = q[i] * expf(at), left = k[i] * expf((sum - b[i]) + after);
       unsafe |= tf32_unsafe(from) || tf32_unsafe(left);
       cell[t * walk_q_row(P) + d] = from;
-      cell[walk_cell_k(P, false) + t * walk_k_row(P) + d] = left;
+      cell[walk_cell_k(P, 0) + t * walk_k_row(P) + d] = left;
     }
-    if (group == 0) cell[walk_cell_decay(P, false) + d] = expf(sum + after);
+    if (group == 0) cell[walk_cell_decay(P, 0) + d] = expf(sum + after);
     if (unsafe) unsafe_s = 1;
   } else {
     __syncthreads();
@@ -194,7 +194,7 @@ gla_chunk_kernel(GlaRows in, float* __restrict__ cells, const int* __restrict__ 
   // the exponential is exp(b_i - b_r) exp(b_r - b_j) with r the last token of the columns' four: both exponents are at
   // most zero, and a factor vanishes only where the product does; 8 exponentials for 16 products instead of 16.  On the
   // diagonal every pair has its own.
-  float* a_out = cell + walk_cell_a(P, false);
+  float* a_out = cell + walk_cell_a(P, 0);
   const int blocks = (n + 3) / 4;
   bool unsafe = false;
   for (int p = warp; p < blocks * (blocks + 1) / 2; p += kScoreThreads / 32) {
@@ -268,7 +268,7 @@ gla_chunk_kernel(GlaRows in, float* __restrict__ cells, const int* __restrict__ 
   }
   if (unsafe) unsafe_s = 1;
   __syncthreads();
-  if (tid == 0) *reinterpret_cast<float2*>(cell + walk_cell_decay(P, false) + P) = make_float2((float)unsafe_s, __int_as_float(n));
+  if (tid == 0) *reinterpret_cast<float2*>(cell + walk_cell_decay(P, 0) + P) = make_float2((float)unsafe_s, __int_as_float(n));
 }
 
 }  // namespace cie
@@ -306,7 +306,7 @@ extern "C" int cie_gla_scan(const float* proj, int proj_stride, int q_off, int k
 
 // Floats of scratch memory that the chunked form wants.
 extern "C" long long cie_gla_chunk_floats(int chunks, int heads, int dim) {
-  return (long long)chunks * heads * walk_cell_floats(walk_pad(dim), false);
+  return (long long)chunks * heads * walk_cell_floats(walk_pad(dim), 0);
 }
 
 // The chunked form.  cells: float32 scratch of cie_gla_chunk_floats, on 16 bytes.
@@ -334,7 +334,7 @@ extern "C" int cie_gla_chunked(const float* proj, int proj_stride, int q_off, in
   if (status != cudaSuccess) CIE_FAIL("gla_chunk: launch failed: %s", cudaGetErrorString(status));
   const WalkArgs walk{cells, proj + v_off, proj_stride, vdim, out, out_stride, state, (long long)heads * dim * vdim, chunk_row, chunk_count,
                       request_chunk_start, slots, request_active, heads, dim, vdim, max_slots, err};
-  const cudaError_t walked = launch_state_walk<false>(walk, P, requests, s);
+  const cudaError_t walked = launch_state_walk<0>(walk, P, requests, s);
   if (walked != cudaSuccess) CIE_FAIL("gla_walk: launch failed: %s", cudaGetErrorString(walked));
   return 0;
 }

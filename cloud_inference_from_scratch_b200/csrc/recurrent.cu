@@ -1171,7 +1171,7 @@ gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_
   pdl_trigger();
   const int chunk = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row0 = chunk_row[chunk], n = chunk_count[chunk], group = head / (heads / kv_heads), base = group * dim;
-  float* cell = cells + ((size_t)chunk * heads + head) * walk_cell_floats(P, true);
+  float* cell = cells + ((size_t)chunk * heads + head) * walk_cell_floats(P, 1);
   if (tid < C) {
     lg_s[tid] = tid < n ? gates[((size_t)(row0 + tid) * heads + head) * kMemGates + 1] : 0.f;
     beta_s[tid] = tid < n ? strength[(size_t)(row0 + tid) * heads + head] : 0.f;
@@ -1195,7 +1195,7 @@ gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_
       seen[j] = s <= t && t < n ? qv[j] * ratio : 0.f;
       unsafe |= tf32_unsafe(seen[j]);
     }
-    *reinterpret_cast<float4*>(cell + walk_cell_a(P, true) + t * kWalkA + s0) = make_float4(seen[0], seen[1], seen[2], seen[3]);
+    *reinterpret_cast<float4*>(cell + walk_cell_a(P, 1) + t * kWalkA + s0) = make_float4(seen[0], seen[1], seen[2], seen[3]);
   }
   const float lg_last = lg_s[n - 1];
 #pragma unroll
@@ -1212,11 +1212,11 @@ gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_
       const float k = in ? row[k_off + c] * inv.x : 0.f, q = in ? row[q_off + c] * inv.y * read : 0.f;
       k_s[t * kd + c] = k;
       cell[t * walk_q_row(P) + c] = q;
-      cell[walk_cell_k(P, true) + t * walk_k_row(P) + c] = k * write;
+      cell[walk_cell_k(P, 1) + t * walk_k_row(P) + c] = k * write;
       unsafe |= tf32_unsafe(q) || tf32_unsafe(k);
     }
   }
-  for (int d = tid; d < P; d += 256) cell[walk_cell_decay(P, true) + d] = expf(lg_last);
+  for (int d = tid; d < P; d += 256) cell[walk_cell_decay(P, 1) + d] = expf(lg_last);
   __syncthreads();
   if (tid < C) {            // column tid of T = (I + A)^-1: once a row is known it leaves all the rows below it
     float x[C];
@@ -1286,7 +1286,7 @@ gated_delta_solve_kernel(const float* __restrict__ conv, int conv_stride, int q_
   if (unsafe) unsafe_s = 1;
   __syncthreads();
   if (tid == 0)
-    *reinterpret_cast<float2*>(cell + walk_cell_decay(P, true) + P) = make_float2((float)unsafe_s, __int_as_float(n));
+    *reinterpret_cast<float2*>(cell + walk_cell_decay(P, 1) + P) = make_float2((float)unsafe_s, __int_as_float(n));
 }
 
 }  // namespace cie
@@ -1393,7 +1393,7 @@ extern "C" int cie_mlstm_chunked(const float* proj, int proj_stride, int q_off, 
 // Floats of scratch memory the gated delta rule in chunks wants: the cells, the products of unit rows, U' and the summed
 // log decays and strengths per token, and the rows' lengths.
 extern "C" long long cie_gated_delta_chunk_floats(int tokens, int chunks, int heads, int kv_heads, int dim, int vdim) {
-  return (long long)chunks * (heads * (long long)walk_cell_floats(walk_pad(dim), true) + kv_heads * 2ll * kScores) +
+  return (long long)chunks * (heads * (long long)walk_cell_floats(walk_pad(dim), 1) + kv_heads * 2ll * kScores) +
          (long long)tokens * (heads * (long long)(kMemGates + 1 + vdim) + 2ll * kv_heads);
 }
 
@@ -1415,7 +1415,7 @@ extern "C" int cie_gated_delta_chunked(const float* conv, int conv_stride, int q
   cudaStream_t s = (cudaStream_t)stream;
   const int P = walk_pad(dim);
   float* cells = scratch;
-  float* scores = cells + (size_t)chunks * heads * walk_cell_floats(P, true);
+  float* scores = cells + (size_t)chunks * heads * walk_cell_floats(P, 1);
   float* gates = scores + (size_t)chunks * kv_heads * 2 * kScores;
   float* u = gates + (size_t)tokens * heads * kMemGates;
   float2* inverse = reinterpret_cast<float2*>(u + (size_t)tokens * heads * vdim);
@@ -1432,7 +1432,7 @@ extern "C" int cie_gated_delta_chunked(const float* conv, int conv_stride, int q
              chunk_count, heads, kv_heads, dim, vdim);
   const WalkArgs walk{cells, u, (long long)heads * vdim, vdim, out, out_stride, state, state_stride, chunk_row, chunk_count,
                       request_chunk_start, slots, request_active, heads, dim, vdim, max_slots, err};
-  const cudaError_t walked = launch_state_walk<true>(walk, P, requests, s);
+  const cudaError_t walked = launch_state_walk<1>(walk, P, requests, s);
   if (walked != cudaSuccess) CIE_FAIL("gated_delta_walk: launch failed: %s", cudaGetErrorString(walked));
   return 0;
 }

@@ -162,3 +162,49 @@ def test_writes_that_are_not_finite_reach_the_tokens_behind_them_only(bad, heads
     close(got[calm], want[calm], "float32", tight=2e-5)
     close(state[1], final[1], "float32", tight=2e-5)
     assert not torch.isfinite(got[at:lengths[0], 0, 5]).any() and not torch.isfinite(state[0, 0, :, 5]).any()
+
+
+@pytest.mark.parametrize("lengths,heads,dim", [([31, 32, 33, 65, 8], 2, 64), ([40, 24], 80, 33), ([64, 2, 97], 30, 128), ([70], 3, 100)])
+@pytest.mark.parametrize("bad", [None, float("nan"), float("inf")])
+def test_generalized_delta_rule_at_the_edges_and_with_values_that_are_not_finite(lengths, heads, dim, bad):
+    """Narrow and wide blocks, one stage and several; a value that is not finite reaches the tokens behind it only."""
+    rt = runtime("float32")
+    tokens, inner = sum(lengths), heads * dim
+    proj, decay = rand(tokens, 4 * inner + 3, seed=1), rand(tokens, inner, seed=2)
+    w0, a0, start = rand(inner, seed=3) - 2, rand(inner, seed=4), rand(len(lengths), heads, dim, dim, scale=0.5, seed=5)
+    at, column = 20, 5
+    if bad is not None:
+        proj[at, 2 * inner + column] = bad
+    ctx, _ = fake_step(lengths, [0] * len(lengths), 16, torch.float32, 1, 8, 8)
+    ctx.slots = torch.arange(len(lengths), dtype=torch.int32).cuda()
+    ctx.request_active = torch.ones(len(lengths), dtype=torch.int32).cuda()
+    rt.ops.require_delta()
+    plan = {name: torch.from_numpy(a).cuda() for name, a in rt.ops._plan_chunks(ctx.host, rt.ops.delta_chunk_tokens).items()}
+    state, out = start.clone().cuda(), torch.empty(tokens, inner).cuda()
+    rt.ops.delta_scan(proj.cuda(), (0, inner, 2 * inner, 3 * inner), decay.cuda(), w0.cuda(), a0.cuda(), out, state, ctx, heads,
+                      dim, plan=plan)
+    rt.ops.check_errors()
+    r, k, v, a = (proj[:, i * inner:(i + 1) * inner].to(F).view(tokens, heads, dim) for i in range(4))
+    rate = torch.sigmoid(a + a0.to(F).view(heads, dim))
+    kept = torch.exp(-0.6065306597126334 * torch.sigmoid(decay.to(F) + w0.to(F))).view(tokens, heads, dim)
+    unit = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+    want, final, t = [], start.to(F).clone(), 0
+    for q, count in enumerate(lengths):
+        for _ in range(count):
+            seen = torch.einsum("hk,hkv->hv", unit[t], final[q])
+            final[q] = (kept[t].unsqueeze(-1) * final[q] - (rate[t] * unit[t]).unsqueeze(-1) * seen.unsqueeze(-2)
+                        + k[t].unsqueeze(-1) * v[t].unsqueeze(-2))
+            want.append(torch.einsum("hkv,hk->hv", final[q], r[t]))
+            t += 1
+    want, got, state = torch.stack(want), out.view(tokens, heads, dim).cpu(), state.cpu()
+    ends = [sum(lengths[:q + 1]) for q in range(len(lengths))]
+    owner = next(q for q, end in enumerate(ends) if at < end)
+    calm = torch.ones(want.shape, dtype=torch.bool)
+    if bad is not None:
+        calm[at:ends[owner], 0, column] = False
+        assert not torch.isfinite(got[at:ends[owner], 0, column]).any()
+    # sums of 32-bit products whose terms are up to exp(0.6 * 32) apart before they are scaled back
+    close(got[calm], want[calm], "float32", tight=4e-5)
+    others = [q for q in range(len(lengths)) if q != owner or bad is None]
+    if others:
+        close(state[others], final[others], "float32", tight=4e-5)
