@@ -11,7 +11,7 @@
 //
 //     U   = V2 - W S,   o_t = S^T q_t + sum_(s <= t) A_ts v_s + A2_ts u_s,   S <- diag(d) S + sum_s k_s v_s^T + k2_s u_s^T
 //
-// grid (requests, heads, blocks of 16 MT value columns).  A walk is a chain, and a prompt of one request has no more blocks
+// grid (blocks of 16 MT value columns, heads, requests: those with the most chunks first).  A walk is a chain, and a prompt of one request has no more blocks
 // than multiprocessors: what bounds it is the instructions of a chunk one after the other, so a block has many warps with
 // little to do each.
 //   * P / 16 warps own 16 keys of S^T each, in the layout in which mma.sync leaves a sum; with the keys of an operand named
@@ -33,6 +33,7 @@
 namespace cie {
 
 constexpr int kChunkTokens = 32;
+constexpr int kRanked = 64;                   // requests whose walks are ordered by length at most
 constexpr int kWalkHelpers = 4;               // warps of eight tokens each
 constexpr int kWalkA = kChunkTokens + 4;      // row of A in shared memory
 
@@ -112,10 +113,24 @@ state_walk_kernel(WalkArgs a) {
     for (int s = 0; s < 2; ++s) { mbar_init(&u_full[s], kWalkHelpers); mbar_init(&v_full[s], kWalkHelpers); }      // the tokens' warps may be a chunk ahead
     mbar_init_fence();
   }
+  // The blocks that start first take the longest walks (ranked while the kernel before runs; more requests than kRanked, whose
+  // blocks are many, come as they are): four portions of 7 to 15 chunks, 16 heads of 128, the layer 205 -> 188 us.
+  __shared__ int chunks_s[kRanked], request_s;
+  const int requests = gridDim.z;
+  if (tid == 0) request_s = blockIdx.z;
+  if (requests <= kRanked)
+    for (int r = tid; r < requests; r += Shape::THREADS) chunks_s[r] = a.request_chunk_start[r + 1] - a.request_chunk_start[r];
+  __syncthreads();
+  if (requests <= kRanked)
+    for (int r = tid; r < requests; r += Shape::THREADS) {
+      int before = 0;
+      for (int other = 0; other < requests; ++other) before += chunks_s[other] > chunks_s[r] || (chunks_s[other] == chunks_s[r] && other < r);
+      if (before == (int)blockIdx.z) request_s = r;
+    }
   __syncthreads();
   pdl_wait();
   pdl_trigger();
-  const int request = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * COLS, columns = min(COLS, a.vdim - col0);
+  const int request = request_s, head = blockIdx.y, col0 = blockIdx.x * COLS, columns = min(COLS, a.vdim - col0);
   const int slot = a.slots[request];
   if (slot < 0 || slot >= a.max_slots) {
     if (tid == 0) atomicOr(a.err, kErrBadRequest);
@@ -518,7 +533,7 @@ inline cudaError_t launch_state_walk(const WalkArgs& a, int P, int requests, cud
   auto go = [&](auto kernel, int MT, int threads, int floats) {
     const cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, floats * (int)sizeof(float));
     if (status != cudaSuccess) return status;
-    return launch(kernel, dim3(requests, a.heads, (a.vdim + 16 * MT - 1) / (16 * MT)), dim3(threads), (size_t)floats * sizeof(float), stream, a);
+    return launch(kernel, dim3((a.vdim + 16 * MT - 1) / (16 * MT), a.heads, requests), dim3(threads), (size_t)floats * sizeof(float), stream, a);
   };
 #define CIE_WALK(p)                                                                                                        \
   if (P == p)                                                                                                              \

@@ -1718,7 +1718,10 @@ class Ops:
         need = int(floats(rows, k))
         if held is None or held.numel() < need:
             if held is not None and self.scratch_frozen:
-                rows = max(1, min(rows, held.numel() // int(floats(1, k) + 4)))
+                rows = min(rows, held.numel() // int(floats(1, k) + 4))
+                if rows == 0:         # not even one: the CUDA cores, which need none
+                    self._gemm_simt(x, weight, bias, out, m, n, k, F32, F32, 0, stream)
+                    return
                 need = int(floats(rows, k))
             held = self.scratch("gemm_f32.terms", need, reserve=max(int(floats(min(max(m, self.max_rows), F32_BLOCK), k)), 1 << 19))
         for first in range(0, m, rows):

@@ -25,5 +25,9 @@ def test_rows_in_blocks_change_no_bit(monkeypatch):
     frozen.freeze_scratch()
     generation = frozen.scratch_generation
     assert torch.equal(frozen.linear(x, w, None, torch.empty(m, n).cuda()).nan_to_num(7.0), want.nan_to_num(7.0))
+    frozen._partial_buffers["gemm_f32.terms"] = torch.empty(9).cuda()
+    plain = frozen.linear(x, w, None, torch.empty(m, n).cuda())
+    rows = torch.arange(m) != 7
+    assert float((plain.cpu()[rows].double() - x.cpu()[rows].double() @ w.cpu().double().T).abs().max()) < 1e-3
     frozen.check_errors()
     assert frozen.scratch_generation == generation
