@@ -244,7 +244,7 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
 // ---------------------------------------------------------------- plan
 // One block.  counts[e]: pairs of expert e; offsets[e] = its first place (offsets[experts] = pairs); place_to_pair[p] =
 // the (token, choice) pair at place p; tiles: (expert, first place, rows) per tile, tile_count[0]; behind room for the most of
-// those there can be (`token_list`: the buffer has that room), how many tiles of up to kTokenTile rows there are and the same of them, the rows of an expert divided
+// those there can be, how many tiles of up to kTokenTile rows there are and the same of them, the rows of an expert divided
 // evenly among them (in sixteens).  Pairs of an expert that
 // a warp meets together are counted by one of its lanes, in shared memory.  8,192 pairs of 16 experts: 12 us (cold), whose
 // choices a thread at a time, one expert after the other in the sums and with counters in global memory, took as long; it also
@@ -252,7 +252,7 @@ moe_route_kernel(const T* __restrict__ x, const float* __restrict__ router,
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ ids, int* __restrict__ counts, int* __restrict__ offsets,
                 int* __restrict__ place_to_pair, int* __restrict__ tiles, int* __restrict__ tile_count, int pairs,
-                int experts, bool token_list) {
+                int experts) {
   __shared__ int count_s[kMaxExperts], off_s[kMaxExperts], tile_s[kMaxExperts], token_tile_s[kMaxExperts];
   int* token_tiles = tiles + 3 * ((pairs + kRowTile - 1) / kRowTile + experts);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -304,7 +304,7 @@ moe_plan_kernel(const int* __restrict__ ids, int* __restrict__ counts, int* __re
     if (lane == 0) {
       offsets[experts] = total;
       tile_count[0] = tile_total;
-      if (token_list) token_tiles[0] = token_total;
+      token_tiles[0] = token_total;
     }
   }
   __syncthreads();
@@ -317,7 +317,7 @@ moe_plan_kernel(const int* __restrict__ ids, int* __restrict__ counts, int* __re
       tiles[3 * tile + 1] = off_s[e] + j;
       tiles[3 * tile + 2] = min(kRowTile, n - j);
     }
-    if (token_list && n > 0) {
+    if (n > 0) {
       const int parts = (n + kTokenTile - 1) / kTokenTile, rows = ((n + parts - 1) / parts + 15) & ~15;
       int* to = token_tiles + 1 + 3 * token_tile_s[e];
       for (int i = 0; i < parts; ++i, to += 3) {
@@ -617,10 +617,11 @@ __global__ void moe_combine_kernel(const float* __restrict__ rows, const float* 
 using namespace cie;
 
 extern "C" int cie_moe_row_tile() { return kRowTile; }
+extern "C" int cie_moe_token_tile() { return kTokenTile; }
 
-// counts, offsets (experts + 1), cursors (not used), tile_count (1) and tiles (3 * (pairs / 128 + experts) and 3 * (pairs / 256
-// + experts) + 1 more with two tokens and more, both rounded up) are
-// int32 scratch of the caller; counts is zeroed here.  counts null: only the choices and their weights are wanted.
+// counts, offsets (experts + 1), tile_count (1) and tiles (3 * (pairs / kRowTile + experts), then 1 + 3 * (pairs / kTokenTile +
+// experts), both quotients rounded up) are int32 scratch of the caller, all written here; cursors is not read.  counts
+// null: only the choices and their weights are wanted.
 extern "C" int cie_moe_route(const void* x, const float* router, const float* correction, int* ids,
                              float* weights, int* counts, int* offsets, int* cursors, int* place_to_pair,
                              int* tiles, int* tile_count, int tokens, int hidden, int experts, int top,
@@ -663,7 +664,7 @@ extern "C" int cie_moe_route(const void* x, const float* router, const float* co
 #undef CIE_MOE_ROUTE
   if (!counts) return 0;
   CIE_LAUNCH("moe_plan", moe_plan_kernel, dim3(1), dim3(1024), 0, s, (const int*)ids, counts, offsets, place_to_pair, tiles,
-             tile_count, tokens * top, experts, tokens > 1);
+             tile_count, tokens * top, experts);
   return 0;
 }
 

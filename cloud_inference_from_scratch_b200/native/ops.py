@@ -51,6 +51,17 @@ LATENT_PROMPT_KEYS = 1 << 17
 LATENT_PROMPT_BYTES = 1 << 28
 
 
+def moe_plan_room(tokens: int, top: int, experts: int, row_tile: int, token_tile: int) -> tuple[int, int]:
+    """(integers a token of the buffer that the plan of a step's routed experts lies in, integers of its tile lists).  The
+    buffer holds a count and an offset an expert (and the last offset), the number of tiles, and two lists of three numbers
+    a tile: tiles of ``row_tile`` rows and, behind one number more, of up to ``token_tile``; an expert's last tile may be
+    short.  A token's share holds everything that does not grow with the tokens, so that one token is room enough."""
+    pairs = tokens * top
+    listed = 3 * (-(-pairs // row_tile) + experts) + 1 + 3 * (-(-pairs // token_tile) + experts)
+    width = 2 * experts + 2 + 1 + 6 * experts + 6 - (-3 * top // row_tile) - (-3 * top // token_tile)
+    return width, listed
+
+
 class _Lib:
     """A loaded library whose entry points return 0 or set ``cie_last_error``."""
 
@@ -1460,6 +1471,7 @@ class Ops:
             self._moe_gate_up_tc = lib.function("cie_moe_gate_up_tc", [v, v, v, v, v, v, v, i, i, i, i, i, i, f, f, f, v, v])
             self._moe_down_tc = lib.function("cie_moe_down_tc", [v, v, v, v, v, v, i, i, i, i, i, v])
             self.moe_row_tile = int(lib.handle.cie_moe_row_tile())
+            self.moe_token_tile = int(lib.handle.cie_moe_token_tile())
             self._moe_lib = lib
             self._moe_tcgen05_lib = None
             self.moe_few_pairs = 0
@@ -1518,15 +1530,12 @@ class Ops:
         ids = workspace.get("moe.ids", tokens, top, torch.int32)
         weights = workspace.get("moe.weights", tokens, top, torch.float32)
         place_to_pair = workspace.get("moe.places", tokens, top, torch.int32)
-        # counts, offsets, cursors, the tile count and the tile list (three numbers a tile; at most one
-        # tile per 64 pairs plus one per expert) share one integer buffer that holds them for any
-        # number of tokens
-        plan = workspace.get("moe.plan", tokens, 6 * experts + 8 + (3 * top + 63) // 64, torch.int32).view(-1)
-        counts, offsets, cursors = plan[:experts], plan[experts:2 * experts + 1], plan[2 * experts + 1:3 * experts + 1]
-        tile_count, tiles = plan[3 * experts + 1:3 * experts + 2], plan[3 * experts + 2:]
-        # (tiles of 128 rows and, behind them, tiles of up to 256)
-        listed = 3 * (-(-pairs // self.moe_row_tile) + experts) + 1 + 3 * (-(-pairs // 256) + experts)
-        assert tiles.numel() >= listed or tokens == 1
+        # counts, offsets, the tile count and the two tile lists share one integer buffer
+        width, listed = moe_plan_room(tokens, top, experts, self.moe_row_tile, self.moe_token_tile)
+        plan = workspace.get("moe.plan", tokens, width, torch.int32).view(-1)
+        counts, offsets = plan[:experts], plan[experts:2 * experts + 1]
+        tile_count, tiles = plan[2 * experts + 1:2 * experts + 2], plan[2 * experts + 2:]
+        assert tiles.numel() >= listed
         act = workspace.get("moe.act", tokens, top * ff, self.dtype)
         rows = workspace.get("moe.rows", tokens, top * hidden, torch.float32)
         code = self._code_of(x)
@@ -1534,7 +1543,7 @@ class Ops:
         few = w_up is None and pairs <= self.moe_few_pairs
         self.launches += 4 if few else 5
         self._moe_route(_ptr(x), _ptr(router), _ptr(correction), _ptr(ids), _ptr(weights), None if few else _ptr(counts),
-                        _ptr(offsets), _ptr(cursors), _ptr(place_to_pair), _ptr(tiles), _ptr(tile_count), tokens,
+                        _ptr(offsets), None, _ptr(place_to_pair), _ptr(tiles), _ptr(tile_count), tokens,
                         hidden, experts, top, 1 if renormalize else 0, _ptr(router_bias), 1 if chosen_softmax else 0,
                         1 if sigmoid else 0, groups[0], groups[1], float(norm_floor), code, self.stream)
         glu = (*glu, _ptr(weights) if weight_inputs else None)

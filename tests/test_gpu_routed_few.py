@@ -1,5 +1,7 @@
 """Routed experts of few pairs: the products that stream the chosen experts' weights."""
 
+import os
+
 import pytest
 import torch
 
@@ -15,6 +17,20 @@ def test_few_pairs(tokens, hidden, ff, weight_inputs):
     """An expert that every token chooses (units of eight pairs, one more, two and a half), one that none does; k that ends
     inside a block of 32, with fewer blocks than warps and with several steps a warp; weight rows that end inside a unit.  A
     token alone gives the same bits.  The activation is rounded to bfloat16 once, the sums are float32: 2^-7 of the largest."""
+    check_few(tokens, hidden, ff, weight_inputs)
+
+
+@pytest.mark.parametrize("hidden,ff", [(72, 16), (264, 144)])
+@pytest.mark.parametrize("tokens", [1, 2, 21])
+@pytest.mark.parametrize("tcgen05", ["0", "1"])
+def test_few_pairs_on_the_grouped_products(monkeypatch, tokens, hidden, ff, tcgen05):
+    """The same with the kernel for few pairs off: a plan for a single token, too, alone and among others (as above)."""
+    monkeypatch.setenv("CIE_MOE_FEW", "0")
+    monkeypatch.setenv("CIE_MOE_TCGEN05", tcgen05)
+    check_few(tokens, hidden, ff, False)
+
+
+def check_few(tokens, hidden, ff, weight_inputs):
     from cloud_inference_from_scratch_b200.engine.runtime import Runtime
 
     rt = Runtime("cuda:0", "bfloat16")
@@ -24,7 +40,7 @@ def test_few_pairs(tokens, hidden, ff, weight_inputs):
     router, bias = rand(experts, hidden, seed=2, scale=0.3), torch.tensor([0.0, 90.0, -90.0, 0.5, 0.0, -1.0])
     gate, up = (rand(experts, ff, hidden, seed=s, scale=hidden ** -0.5).bfloat16() for s in (3, 4))
     down = rand(experts, hidden, ff, seed=5, scale=ff ** -0.5).bfloat16()
-    assert rt.ops.moe_interleaves(hidden, ff) and tokens * top <= rt.ops.moe_few_pairs
+    assert rt.ops.moe_interleaves(hidden, ff) and (tokens * top <= rt.ops.moe_few_pairs or os.environ.get("CIE_MOE_FEW") == "0")
     both = rt.ops.interleave_gate_up(gate.cuda(), up.cuda())
 
     def run(rows):

@@ -155,3 +155,53 @@ def test_prompt_attention_key_ranges():
         for keys in (128, 4096, 1 << 20):
             ranges = key_ranges(ctas, keys, 148, 128)
             assert 1 <= ranges <= ta.MAX_KEY_RANGES and (ranges == 1 or ctas * ranges <= 148)
+
+
+def routed_plan(monkeypatch, tokens, top, experts, hidden=8, ff=16):
+    """What the router is given for a step of routed experts that goes to the grouped products: how many integers there are
+    from the list of tiles to the end of the buffer that it lies in."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from cloud_inference_from_scratch_b200.engine.runtime import Workspace
+    from cloud_inference_from_scratch_b200.native.ops import BF16, Ops
+
+    monkeypatch.delenv("CIE_MOE_TCGEN05", raising=False)
+    workspace, seen = Workspace("cpu"), {}
+
+    def route(x, router, correction, ids, weights, counts, offsets, cursors, places, tiles, tile_count, *sizes):
+        seen.update(counts=counts, offsets=offsets, tiles=tiles, tile_count=tile_count)
+
+    nothing = lambda *args: None  # noqa: E731
+    ops = SimpleNamespace(
+        torch=torch, dtype=torch.bfloat16, launches=0, stream=0, error_word=torch.zeros(1, dtype=torch.int32), _flush=nothing,
+        moe_few_pairs=0, moe_row_tile=128, moe_token_tile=256, _load_moe=nothing, _load_moe_tcgen05=nothing, _moe_route=route,
+        _moe_gate_up_tcgen05=nothing, _moe_down_tcgen05=nothing, _moe_combine=nothing, _code_of=lambda t: BF16)
+    x, router = torch.zeros(tokens, hidden, dtype=torch.bfloat16), torch.zeros(experts, hidden)
+    # (only the shapes and the addresses of the weights are looked at)
+    gate_up = torch.zeros(1, dtype=torch.bfloat16).expand(experts, 2 * ff, hidden)
+    down = torch.zeros(1, dtype=torch.bfloat16).expand(experts, hidden, ff)
+    Ops.routed_experts(ops, x, router, None, gate_up, None, down, top, False, torch.zeros(tokens, hidden), workspace)
+    (plan,) = [buffer for (tag, *_), buffer in workspace._buffers.items() if tag == "moe.plan"]
+    assert plan.data_ptr() == seen["counts"] and seen["offsets"] == seen["counts"] + 4 * experts
+    assert seen["tile_count"] >= seen["offsets"] + 4 * (experts + 1) and seen["tiles"] == seen["tile_count"] + 4
+    return plan.numel() - (seen["tiles"] - plan.data_ptr()) // 4
+
+
+@pytest.mark.parametrize("experts,top", [(1, 1), (2, 1), (16, 4), (32, 32), (64, 6), (1024, 8)])
+@pytest.mark.parametrize("tokens", [1, 2, 3, 17, 64, 257, 2048])
+def test_both_lists_of_tiles_fit_at_any_number_of_tokens(monkeypatch, tokens, experts, top):
+    """The grouped products read the second list alone, which lies behind room for the most tiles of the first: whatever
+    the choices (all of an expert, as even as can be, one pair too many for a tile), its last number lies in the buffer."""
+    pairs = tokens * top
+    room = routed_plan(monkeypatch, tokens, top, experts)
+    first = 3 * (-(-pairs // 128) + experts)
+    most = min(tokens, pairs)           # a token chooses an expert once
+    spread = [[most] * (pairs // most) + [pairs % most], [pairs // experts + (e < pairs % experts) for e in range(experts)],
+              [min(most, 129)] * (pairs // min(most, 129)) + [pairs % min(most, 129)],
+              [min(most, 257)] * (pairs // min(most, 257)) + [pairs % min(most, 257)]]
+    for counts in spread:
+        counts = [n for n in counts if n][:experts]
+        assert 3 * sum(-(-n // 128) for n in counts) <= first
+        assert first + 1 + 3 * sum(-(-n // 256) for n in counts) <= room
