@@ -173,10 +173,13 @@ state_walk_kernel(WalkArgs a) {
         if (pieces) {
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + row * (VL * 4)), "l"(in ? v_at + i * v_step : a.v),
                        "r"(in ? 16 : 0) : "memory");
-        } else {
-          float* dst = walk_smem + stage_to * Shape::STAGE + Shape::V + (piece_row + row) * VL + piece;
+        } else {      // the stage's barrier waits for a thread's copies, not for its plain stores: copies here, too
 #pragma unroll
-          for (int x = 0; x < 4; ++x) dst[x] = in && piece + x < columns ? v_at[i * v_step + x] : 0.f;
+          for (int x = 0; x < 4; ++x) {
+            const bool here = in && piece + x < columns;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + row * (VL * 4) + 4 * x),
+                         "l"(here ? v_at + i * v_step + x : a.v), "r"(here ? 4 : 0) : "memory");
+          }
         }
         if (kBoth)      // whole rows of P columns, zeros where there is nothing
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + Shape::VALUES * 4 + row * (VL * 4)),
