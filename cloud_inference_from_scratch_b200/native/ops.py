@@ -538,8 +538,7 @@ class Ops:
                 and os.environ.get("CIE_RECURRENT_CHUNKS", "1") != "0"):
             chunks = plan["chunk_row"].shape[0]
             floats = int(self._mlstm_chunk_floats(tokens, chunks, heads, dim, vdim))
-            rows = max(tokens, self.max_rows)
-            reserve = int(self._mlstm_chunk_floats(rows, -(-rows // self.mlstm_chunk_tokens) + ctx.num_requests,
+            reserve = int(self._mlstm_chunk_floats(max(tokens, self.max_rows), self._most_chunks(tokens, self.mlstm_chunk_tokens, ctx),
                                                    heads, dim, vdim))
             scratch = self.scratch(f"recurrent.chunks.{heads}x{dim}x{vdim}", floats, reserve=max(floats, reserve))
             self.launches += 5
@@ -602,10 +601,9 @@ class Ops:
                 and os.environ.get("CIE_RECURRENT_CHUNKS", "1") != "0"):
             chunks = plan["chunk_row"].shape[0]
             floats = int(self._gated_delta_chunk_floats(tokens, chunks, heads, kv_heads, dim, vdim))
-            rows = max(tokens, self.max_rows)
-            reserve = int(self._gated_delta_chunk_floats(rows, -(-rows // self.mlstm_chunk_tokens) + ctx.num_requests,
-                                                         heads, kv_heads, dim, vdim))
-            scratch = self.scratch(f"recurrent.delta_chunks.{heads}x{dim}x{vdim}", floats, reserve=max(floats, reserve))
+            reserve = int(self._gated_delta_chunk_floats(
+                max(tokens, self.max_rows), self._most_chunks(tokens, self.mlstm_chunk_tokens, ctx), heads, kv_heads, dim, vdim))
+            scratch = self.scratch(f"recurrent.delta_chunks.{heads}x{kv_heads}x{dim}x{vdim}", floats, reserve=max(floats, reserve))
             self.launches += 4
             self._gated_delta_chunked(_ptr(conv), conv.stride(0), q_off, k_off, v_off, _ptr(proj), proj.stride(0),
                                       b_off, a_off, _ptr(a_log), _ptr(dt_bias), float(q_scale), _ptr(scratch), _ptr(out),
@@ -872,9 +870,8 @@ class Ops:
         # under captured graphs the scratch memory keeps its place: a step of more chunks than it holds scans
         fits = not self.scratch_frozen or held is None or held.numel() >= floats
         if chunks and fits and tokens >= 8 * ctx.num_requests and os.environ.get("CIE_SSD_CHUNKS", "1") != "0":
-            # room for the chunks of the largest step the runtime knows of (and a partial chunk for many requests)
-            most = max(tokens, self.max_rows)
-            reserve = int(self._ssd_chunk_floats(most, -(-most // self.ssd_chunk_tokens) + 64, heads, groups, dim, vdim))
+            reserve = int(self._ssd_chunk_floats(max(tokens, self.max_rows), self._most_chunks(tokens, self.ssd_chunk_tokens, ctx),
+                                                 heads, groups, dim, vdim))
             scratch = self.scratch(tag, floats, reserve=max(floats, reserve))
             # 16-bit runs: the chunk products on the tensor cores, float32 operands as two bfloat16 terms each
             tensor = self.code == BF16 and os.environ.get("CIE_SSD_TENSOR", "1") != "0"
@@ -1010,6 +1007,13 @@ class Ops:
         return {"chunk_row": np.asarray(rows, dtype=np.int32), "chunk_count": np.asarray(counts, dtype=np.int32),
                 "request_chunk_start": np.asarray(starts, dtype=np.int32)}
 
+    def _most_chunks(self, tokens: int, size: int, ctx: Any) -> int:
+        """Most chunks of ``size`` tokens that a step can be cut into, by what the runtime knows of its steps (a step of
+        ``tokens`` now): whole chunks of all its tokens and one that is not whole for every request.  Scratch memory is made for
+        them at first use, so that no later step has to grow it under a captured graph.  Without a number of requests to go by,
+        64 are expected."""
+        return -(-max(tokens, self.max_rows) // size) + max(ctx.num_requests, self.max_requests or 64)
+
     def lightning_chunked(self, proj: Any, out: Any, state: Any, decay: Any, ctx: Any, plan: dict[str, Any],
                           heads: int, dim: int, vdim: int) -> None:
         """The same recurrence as ``lightning_scan`` for a step with prompt portions, in chunks (see
@@ -1018,7 +1022,8 @@ class Ops:
         self._flush()
         self._load_lightning()
         chunks = plan["chunk_row"].shape[0]
-        scratch = self.scratch("lightning.chunks", chunks * heads * dim * vdim)
+        most = self._most_chunks(proj.shape[0], self.lightning_chunk_tokens, ctx)
+        scratch = self.scratch(f"lightning.chunks.{heads}x{dim}x{vdim}", chunks * heads * dim * vdim, reserve=most * heads * dim * vdim)
         self.launches += 3
         self._lightning_chunked(_ptr(proj), proj.stride(0), _ptr(out), out.stride(0), _ptr(state), _ptr(scratch),
                                 _ptr(decay), _ptr(plan["chunk_row"]), _ptr(plan["chunk_count"]),
@@ -1098,9 +1103,7 @@ class Ops:
                    and os.environ.get("CIE_GLA_CHUNKS", "1") != "0")
         if chunked:
             chunks = plan["chunk_row"].shape[0]
-            # room for the chunks of the largest step the runtime knows of (and a partial chunk for many requests),
-            # so that a long prompt after captured steps does not have to grow the buffers
-            most = max(chunks, self.max_rows // self.gla_chunk_tokens + 64)
+            most = self._most_chunks(proj.shape[0], self.gla_chunk_tokens, ctx)
             cells = self.scratch(f"gla.chunks.{heads}x{dim}", int(self._gla_chunk_floats(chunks, heads, dim)),
                                  reserve=int(self._gla_chunk_floats(most, heads, dim)))
             self.launches += 2
@@ -1414,9 +1417,9 @@ class Ops:
         if plan:
             chunks = plan["chunk_row"].shape[0]
             floats = self._delta_lib.handle.cie_delta_chunk_floats
-            most = -(-max(tokens, self.max_rows) // self.delta_chunk_tokens) + max(ctx.num_requests, self.max_requests)
+            most = self._most_chunks(tokens, self.delta_chunk_tokens, ctx)
             cells = self.scratch(f"delta.cells.{heads}x{dim}", int(floats(chunks, heads, dim)),
-                                 reserve=int(floats(max(chunks, most), heads, dim)))
+                                 reserve=int(floats(most, heads, dim)))
             self.launches += 2
             self._delta_chunked(_ptr(proj), proj.stride(0), r_off, k_off, v_off, a_off, _ptr(decay), decay.stride(0),
                                 _ptr(decay_bias), _ptr(removal_bias), _ptr(cells), _ptr(out), out.stride(0), _ptr(state),
