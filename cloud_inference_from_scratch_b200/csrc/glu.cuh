@@ -23,9 +23,18 @@ __device__ __forceinline__ float glu(const GluAct& a, float g, float u, float we
   return g / (1.f + expf(-g)) * u;
 }
 
-// The same for a result that is rounded to 16 bits at once: the quotient within two units of its last place (float32), by
-// CUDA's fast division, which spares the branch that the exact one has (a denominator of infinity gives zero there too).
-__device__ __forceinline__ float glu_rounded(const GluAct& a, float g, float u, float weight) {
+// g / (1 + e), e >= 0, without the branches of the exact division: a quotient by the reciprocal within two units of its last
+// place, and one step of Markstein's correction (q + r (n - d q), IBM J. Res. Dev. 34, 1990), whose result is rounded as the exact
+// one is in all but one case in millions.  Both sides are taken four times smaller, because the fast reciprocal is
+// zero from 2^126 on; an infinity (of e: the quotient is zero; of g) makes the correction NaN, and stays without it.
+__device__ __forceinline__ float over_one_plus(float g, float e) {
+  const float n = 0.25f * g, d = fmaf(0.25f, e, 0.25f), r = __fdividef(1.f, d), q = n * r, whole = fmaf(fmaf(-d, q, n), r, q);
+  return whole == whole ? whole : q;
+}
+
+// The same activation where many values are worked out at one time: nothing in it branches.  The layer of moe_tcgen05.cu with 2,048
+// tokens: 229 us, 235 with the exact division, 227 with a fast one and no correction.
+__device__ __forceinline__ float glu_straight(const GluAct& a, float g, float u, float weight) {
   g *= weight;
   u *= weight;
   float slope = 1.f, shift = 0.f;
@@ -35,7 +44,7 @@ __device__ __forceinline__ float glu_rounded(const GluAct& a, float g, float u, 
     slope = a.slope;
     shift = a.shift;
   }
-  return __fdividef(g, 1.f + expf(-slope * g)) * (u + shift);
+  return over_one_plus(g, expf(-slope * g)) * (u + shift);
 }
 
 }  // namespace cie

@@ -99,7 +99,7 @@ __device__ __forceinline__ void write_tile(const GroupedArgs& a, uint32_t from, 
         const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(upper ? raw[c] : raw[c + 1]), 16);
         const float w = __shfl_sync(0xffffffffu, weight, c + upper);
         if (c0 + c + upper < rows && channel < a.n)
-          dst[(size_t)c * a.n] = __float2bfloat16_rn(glu_rounded(a.glu_act, upper ? other : mine, upper ? mine : other, w));
+          dst[(size_t)c * a.n] = __float2bfloat16_rn(glu_straight(a.glu_act, upper ? other : mine, upper ? mine : other, w));
       }
     } else {
       float* dst = reinterpret_cast<float*>(a.out) + row0 + lane;

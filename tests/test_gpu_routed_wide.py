@@ -52,6 +52,50 @@ def test_many_pairs(monkeypatch, tokens, hidden, ff, weight_inputs, columns):
     assert float((out[tokens] - 7.0).abs().max()) == 0
 
 
+@pytest.mark.parametrize("activation", [None, (130.0, 1.5, 1.0)])
+def test_gates_of_any_size(activation):
+    """The activation of the grouped products over gates from -136 to 136, most of all where the exponential is near the largest
+    float32 (1 + e^88 and the like), and gates that are infinite.  Float32 and rounded to bfloat16 once: 2^-8 and a little of
+    the value (an exponent of 136 is off by half a unit of its last place, 2^-18); where the exponential
+    is beyond the largest float32, 2^128, the quotient may be zero."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+
+    rt = Runtime("cuda:0", "bfloat16")
+    rt.ops._load_moe()
+    tokens, hidden, ff, experts = 130, 64, 272, 2
+    limit, slope, shift = activation or (float("inf"), 1.0, 0.0)
+    x = torch.zeros(tokens, hidden)
+    x[:, 0] = 1 + (torch.arange(tokens) % 64) / 128          # a token's gates are its one element times the weights
+    x[-1, 0] = 4.0
+    gates = torch.linspace(-90, 90, ff).bfloat16()
+    gates[7], gates[200] = 3e38, -3e38          # infinite for the last token
+    gate, up = torch.zeros(experts, ff, hidden), torch.zeros(experts, ff, hidden)
+    gate[:, :, 0], up[:, :, 1] = gates.float(), 2.0 ** 60
+    x[:, 1] = 1.0
+    x, down = x.bfloat16(), torch.zeros(experts, hidden, ff).bfloat16().cuda()
+    router = torch.zeros(experts, hidden)
+    router[0, 0], router[1, 0] = 1.0, -1.0          # all tokens to expert 0: places are in some order of the tokens
+    both = rt.ops.interleave_gate_up(gate.bfloat16().cuda(), up.bfloat16().cuda())
+    out = torch.empty(tokens, hidden).cuda()
+    rt.ops.routed_experts(x.cuda(), router.cuda(), None, both, None, down, 1, False, out, rt.workspace, chosen_softmax=True,
+                          activation=activation)
+    rt.ops.check_errors()
+    assert tokens > rt.ops.moe_few_pairs
+    places = rt.workspace.get("moe.places", tokens, 1, torch.int32).view(-1).long().cpu()
+    got = rt.workspace.get("moe.act", tokens, ff, torch.bfloat16).cpu()
+    got[places] = got.clone()
+    g = (x[:, :1].float() * gates.float()).double().clamp(max=limit)
+    u = min(2.0 ** 60, limit) + shift
+    want = g / (1 + torch.exp(-slope * g)) * u
+    whole = torch.isfinite(g) & (want.abs() < 3e38)
+    error = (got.double() - want).abs()[whole]
+    assert bool((error <= want.abs()[whole] * (2.0 ** -8 + 2.0 ** -16) + (2.0 ** -127 * g.abs() * u)[whole]).all())
+    large = whole & (-slope * g > 87.4) & (-slope * g < 88.7)          # the quotient is a normal float32, about 1e-36
+    assert int(large.sum()) > 50 and bool((got[large] != 0).all())
+    assert bool(((got[-1, 7] == float("inf")) if activation is None else torch.isfinite(got[-1, 7])).all())
+    assert bool(got[-1, 200].isnan())          # -inf / (1 + inf)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("hidden", [70, 72, 1032])          # single elements, pieces of four, several loads a lane
 @pytest.mark.parametrize("kind", ["softmax", "sigmoid", "grouped"])
