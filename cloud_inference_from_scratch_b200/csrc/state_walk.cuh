@@ -511,7 +511,7 @@ state_walk_kernel(WalkArgs a) {
         full_phase ^= 1;
       }
     }
-    if (alive && a.request_active[request]) {
+    if (alive && chunks > 0 && a.request_active[request]) {      // (whoever brings no tokens leaves the slot alone)
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll

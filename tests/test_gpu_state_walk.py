@@ -208,3 +208,52 @@ def test_generalized_delta_rule_at_the_edges_and_with_values_that_are_not_finite
     others = [q for q in range(len(lengths)) if q != owner or bad is None]
     if others:
         close(state[others], final[others], "float32", tight=4e-5)
+
+
+def general_case(lengths, heads, dim, seed=1):
+    tokens, inner = sum(lengths), heads * dim
+    return rand(tokens, 4 * inner, seed=seed), rand(tokens, inner, seed=seed + 1), rand(inner, seed=seed + 2) - 2, rand(inner, seed=seed + 3), \
+        rand(len(lengths), heads, dim, dim, scale=0.5, seed=seed + 4)
+
+
+def run_rule(rule, inputs, lengths, heads, dim, slots=None):
+    """Outputs and states of a step in chunks, by the rule's name, from inputs as the rule's case makes them."""
+    rt = runtime("float32")
+    tokens, inner, start = sum(lengths), heads * dim, inputs[-1]
+    ctx, _ = fake_step(lengths, [0] * len(lengths), 16, torch.float32, 1, 8, 8)
+    ctx.slots = (torch.arange(len(lengths)) if slots is None else torch.tensor(slots)).int().cuda()
+    ctx.request_active = torch.ones(len(lengths), dtype=torch.int32).cuda()
+    out, state = torch.empty(tokens, inner).cuda(), start.clone().cuda()
+    on = [t.cuda() for t in inputs[:-1]]
+    offsets = tuple(i * inner for i in range(4))
+    if rule == "gla":
+        rt.ops.require_gla()
+        rt.ops.gla(on[0], offsets[:3], on[1], on[2], 4.0, dim ** -0.5, out, state, ctx, heads, dim, dim, plan=plan_of(rt, ctx))
+    elif rule == "gated":
+        rt.ops._load_recurrent()
+        plan = {name: torch.from_numpy(a).cuda() for name, a in rt.ops._plan_chunks(ctx.host, rt.ops.mlstm_chunk_tokens).items()}
+        rt.ops.gated_delta_scan(on[0], offsets[:3], on[1], (0, heads), on[2], on[3], dim ** -0.5, out, state, ctx, heads, heads, dim,
+                                dim, plan=plan)
+    else:
+        rt.ops.require_delta()
+        plan = {name: torch.from_numpy(a).cuda() for name, a in rt.ops._plan_chunks(ctx.host, rt.ops.delta_chunk_tokens).items()}
+        rt.ops.delta_scan(on[0], offsets, on[1], on[2], on[3], out, state, ctx, heads, dim, plan=plan)
+    rt.ops.check_errors()
+    return out.cpu(), state.cpu()
+
+
+def inputs_of(rule, lengths, heads, dim):
+    if rule == "gla":
+        return gla_case(lengths, heads, dim, dim)
+    return delta_case(lengths, heads, heads, dim, dim) if rule == "gated" else general_case(lengths, heads, dim)
+
+
+@pytest.mark.parametrize("rule", ["gla", "gated", "general"])
+def test_a_request_without_tokens_leaves_its_slot_alone(rule):
+    """It names the slot of a request that brings some: what that one leaves there is what it leaves without the other."""
+    heads, dim = 3, 64
+    inputs = inputs_of(rule, [40, 33], heads, dim)
+    out, state = run_rule(rule, inputs, [40, 33], heads, dim)
+    more = [*inputs[:-1], torch.cat([inputs[-1], inputs[-1][:1]])]
+    beside, states = run_rule(rule, more, [40, 0, 33], heads, dim, slots=[0, 0, 1])
+    assert torch.equal(out, beside) and torch.equal(state, states[:2])
