@@ -366,8 +366,9 @@ norm_kv_pieces_kernel(const TI* __restrict__ src, const float* __restrict__ bias
     sin_s[i] = sn * magnitude;
     cos_s[i] = cs * magnitude;
   }
-  const int request = request_of_token[t], index = pos / page_size;
-  const int page = index < table_width ? table[(size_t)request * table_width + index] : -1;
+  // (whoever writes no pages need not have any)
+  const int request = write_cache ? request_of_token[t] : 0, index = pos / page_size;
+  const int page = write_cache && index < table_width ? table[(size_t)request * table_width + index] : -1;
   const bool kept = write_cache && !(extra.active && !extra.active[request]), bad = kept && (page < 0 || page >= num_pages);
   const size_t slot = (size_t)page * kv_heads * page_size + (size_t)(pos % page_size);   // + head * page_size
   pdl_wait();

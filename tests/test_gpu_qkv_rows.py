@@ -69,3 +69,35 @@ def test_rows_in_pieces(tokens, heads, kv_heads, dim, vdim, norm, v_norm, bias, 
     single = torch.tensor([t for p, t in last.items() if int((positions == p).sum()) == 1])
     assert float((k_pool.cpu()[page, :, place].double() - k)[single].abs().max()) < 2e-4
     assert float((v_pool.cpu()[page, :, place].double() - v)[single].abs().max()) < 2e-5
+
+
+def write_rows(ops, src, positions, requests, table, heads, kv_heads, dim, pools, norm=None, freq=None, extra=(None, 0.0, 0), active=None,
+               write=1, magnitude=1.25):
+    """One call with rows of ``src`` (a view of columns: its stride decides which kernel runs); q, and the pools are written."""
+    tokens, q_width = src.shape[0], heads * dim
+    pages = pools[0].shape[0] if pools else 0
+    out = torch.full((tokens, q_width), 7.0, dtype=ops.dtype).cuda()
+    pointer = lambda t: t.data_ptr() if t is not None else None  # noqa: E731
+    held = [pointer(t) for t in (pools or (None, None))]
+    q_gain, k_gain = norm or (None, None)
+    ops._norm_kv_write(src.data_ptr(), None, out.data_ptr(), q_width, positions.data_ptr(), pointer(requests), pointer(table),
+                       table.shape[1] if table is not None else 0, pages, *held, pointer(q_gain), pointer(k_gain), tokens, heads,
+                       kv_heads, dim, dim, 16, int(norm is not None), 0, 1e-6, write, src.stride(0), ops._code_of(src), pointer(freq),
+                       0 if freq is None else 2 * freq.numel(), magnitude, 0, pointer(extra[0]), extra[1], extra[2], None, 0, None,
+                       pointer(active), ops._code_of(out), ops.error_word.data_ptr(), ops.stream)
+    return out
+
+
+@pytest.mark.parametrize("shift", [0, 1])          # rows in pieces, and rows of any kind
+def test_queries_alone_need_no_pages(shift):
+    """A call that writes nothing to the cache reads no table and no requests."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+
+    ops = Runtime("cuda:0", "float32").ops
+    ops._load_streams()
+    tokens, heads, dim = 5, 4, 64
+    src = rand(tokens, 6 * dim + 4 + shift, seed=1).cuda()
+    positions = torch.arange(tokens, dtype=torch.int32).cuda() * 9
+    q = write_rows(ops, src, positions, None, None, heads, 1, dim, None, write=0)
+    ops.check_errors()
+    assert torch.equal(q, src[:, :heads * dim])
