@@ -257,3 +257,29 @@ def test_a_request_without_tokens_leaves_its_slot_alone(rule):
     more = [*inputs[:-1], torch.cat([inputs[-1], inputs[-1][:1]])]
     beside, states = run_rule(rule, more, [40, 0, 33], heads, dim, slots=[0, 0, 1])
     assert torch.equal(out, beside) and torch.equal(state, states[:2])
+
+
+@pytest.mark.parametrize("rule", ["gla", "gated", "general"])
+@pytest.mark.parametrize("count", [20, 64, 65, 90])
+def test_order_company_and_width_of_blocks_change_no_bit(rule, count):
+    """The longest walks start first among up to 64 requests and come as they are from 65 on; few blocks are 16 columns wide, many
+    32.  Requests in the reverse order, and each of a few alone, have the bits that they have among all."""
+    heads, dim = 3, 64
+    lengths = [8 + 37 * i % 61 for i in range(count)]
+    inputs = inputs_of(rule, lengths, heads, dim)
+    ends = [sum(lengths[:r + 1]) for r in range(count)]
+    tokens = [list(range(end - n, end)) for end, n in zip(ends, lengths)]
+    own = lambda requests: [t for r in requests for t in tokens[r]]  # noqa: E731
+
+    def part(requests):
+        """The inputs of some requests: rows of tokens, vectors of the layer, states."""
+        rows = own(requests)
+        return [t[rows] if t.shape[0] == ends[-1] else t for t in inputs[:-1]] + [inputs[-1][requests]]
+
+    out, state = run_rule(rule, inputs, lengths, heads, dim)
+    turned = list(range(count))[::-1]
+    beside, states = run_rule(rule, part(turned), [lengths[r] for r in turned], heads, dim)
+    assert torch.equal(beside, out[own(turned)]) and torch.equal(states, state[turned])
+    for r in (0, 5, count - 1):
+        alone, after = run_rule(rule, part([r]), [lengths[r]], heads, dim)
+        assert torch.equal(alone, out[tokens[r]]) and torch.equal(after[0], state[r])
