@@ -1709,12 +1709,11 @@ class Ops:
                 return Partials(out, 0, m, n, bias)   # the consumer adds the bias in float32
             self._cublas_linear(x, weight, bias, out)
             return out
-        self.launches += 1
-        # (the tensor cores' form: and one that splits the rows of x)
         if (self._gemm_f32 is not None and not few_rows and x.dtype == weight.dtype == out.dtype == self.torch.float32
                 and self._gemm_f32_takes(_ptr(x), _ptr(weight), k)):
             self._gemm_f32(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), m, n, k, 0, self.error_word.data_ptr(), self.stream)
             return out
+        self.launches += 1
         self._gemm_simt(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), m, n, k, self._code_of(x),
                         self._code_of(out), 0 if self.code == F32 else 1, self.stream)
         return out
@@ -1732,12 +1731,13 @@ class Ops:
             if held is not None and self.scratch_frozen:
                 rows = min(rows, held.numel() // int(floats(1, k) + 4))
                 if rows == 0:         # not even one: the CUDA cores, which need none
+                    self.launches += 1
                     self._gemm_simt(x, weight, bias, out, m, n, k, F32, F32, 0, stream)
                     return
                 need = int(floats(rows, k))
             held = self.scratch("gemm_f32.terms", need, reserve=max(int(floats(min(max(m, self.max_rows), F32_BLOCK), k)), 1 << 19))
         for first in range(0, m, rows):
-            self.launches += 1
+            self.launches += 2         # the terms, the product
             self._gemm_f32_tc(x + 4 * first * k, weight, bias, out + 4 * first * n, min(rows, m - first), n, k, columns,
                               held.data_ptr(), err, stream)
 

@@ -205,3 +205,33 @@ def test_both_lists_of_tiles_fit_at_any_number_of_tokens(monkeypatch, tokens, ex
         counts = [n for n in counts if n][:experts]
         assert 3 * sum(-(-n // 128) for n in counts) <= first
         assert first + 1 + 3 * sum(-(-n // 256) for n in counts) <= room
+
+
+@pytest.mark.parametrize("rows,held,few_rows,calls", [
+    (1, None, False, (1, 0)), (77, None, False, (1, 0)), (78, None, False, (2, 0)), (300, None, False, (4, 0)),      # blocks of 77
+    (300, 1440, False, (5, 0)), (300, 3, False, (0, 1)),          # frozen scratch for 60 rows, and for none
+    (300, None, True, (0, 1))])
+def test_float32_products_count_their_launches(monkeypatch, rows, held, few_rows, calls):
+    """A block of rows is two kernels, a product on the CUDA cores one."""
+    import types
+    from types import SimpleNamespace
+
+    import torch
+
+    from cloud_inference_from_scratch_b200.native import ops as module
+    from cloud_inference_from_scratch_b200.native.ops import F32, Ops
+
+    monkeypatch.setattr(module, "F32_BLOCK", 77)
+    n, k, made = 3, 512, {"tensor": 0, "plain": 0}
+    nothing = lambda *args: None  # noqa: E731
+    count = lambda name: lambda *args: made.__setitem__(name, made[name] + 1)  # noqa: E731
+    ops = SimpleNamespace(
+        torch=torch, device=torch.device("cpu"), dtype=torch.float32, code=F32, gemm_mode="simt", skinny_products="", _tensor_gemm=None,
+        fold_rows=0, launches=0, stream=0, max_rows=0, scratch_frozen=held is not None, scratch_generation=0, _flush=nothing,
+        error_word=torch.zeros(1, dtype=torch.int32), _code_of=lambda t: F32, _gemm_f32_takes=lambda *args: True,
+        _gemm_f32_floats=lambda m, k: 20 * m, _gemm_f32_tc=count("tensor"), _gemm_simt=count("plain"),
+        _partial_buffers={} if held is None else {"gemm_f32.terms": torch.empty(held)})
+    ops.scratch = types.MethodType(Ops.scratch, ops)
+    ops._gemm_f32 = types.MethodType(Ops._f32_product, ops)
+    Ops.linear(ops, torch.zeros(rows, k), torch.zeros(n, k), None, torch.zeros(rows, n), few_rows=few_rows)
+    assert (made["tensor"], made["plain"]) == calls and ops.launches == 2 * calls[0] + calls[1]
