@@ -1388,9 +1388,11 @@ class Ops:
         self._load_delta()
         if host.num_single == host.num_requests or dim > self.delta_stream_max_dim:
             return {}
-        # us on a B200 for heads padded to P: the walk follows its longest portion (2,048 tokens, P = 64: 1,790; P = 128:
-        # 3,945) until its blocks fill the device (32 portions of 64 tokens, 32 heads of 64: 187; 16 of 128: 360); the
-        # chunks cost what there are of them (the same four steps: 246, 515, 257, 612) and two launches
+        # us on a B200 for heads padded to P.  The stream follows its longest portion (2,048 tokens of 32 heads of 64: 1,844; 16 of
+        # 128: 4,078) until its blocks fill the device (32 portions of 64 tokens, the same heads: 191 and 361).  The chunks are
+        # charged what there is of them and two launches, at more than they take (the same four steps: 216, 368, 224, 308):
+        # where they win by little the stream runs, whose outputs are nearer to 64 bits (1.3e-7 of their norm, 2.4e-7 in chunks).  The
+        # furthest from the line that it leaves to the stream: four portions of 512, 32 heads of 128: 1,148 and 597.
         pad = 32 if dim <= 32 else 64 if dim <= 64 else 128
         lengths = host.query_lens
         walk = max(0.0135 * pad * int(lengths.max()), 7e-7 * pad * pad * heads * int(lengths.sum()))
@@ -1408,8 +1410,8 @@ class Ops:
         runs one kernel that works the rates out as it goes; a step with prompt portions (eight tokens a
         request or more on average) first works out, for all tokens at once, what the recurrence reads
         and then streams it through a ring of copies: the same additions in the same order.  With ``plan``
-        (``plan_delta``, on the device) the step runs in chunks: what a chunk does to any state in parallel, then a
-        walk over each request's chunks, with the additions in another order."""
+        (``plan_delta``, on the device) the step runs in chunks: what a chunk's tokens do to one another in parallel, then a
+        walk over each request's chunks that works outputs and states out, with the additions in another order."""
         self._flush()
         self._load_delta()
         r_off, k_off, v_off, a_off = offsets

@@ -1,5 +1,5 @@
-"""Norm, rotation and cache write of rows whose parts are whole pieces of four elements: the block sizes by row width and
-number of tokens, against the same in 64 bits."""
+"""Norm, rotation and cache write of rows whose parts are whole pieces of four elements, in both block sizes (by the row's width):
+against the same in 64 bits, and against the kernel for rows of any kind."""
 
 import pytest
 import torch
@@ -101,3 +101,44 @@ def test_queries_alone_need_no_pages(shift):
     q = write_rows(ops, src, positions, None, None, heads, 1, dim, None, write=0)
     ops.check_errors()
     assert torch.equal(q, src[:, :heads * dim])
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(16, 2), (40, 4)])          # blocks of 256 threads and of 512
+@pytest.mark.parametrize("source", ["float32", "bfloat16"])
+@pytest.mark.parametrize("norm", [False, True])
+def test_rows_in_pieces_as_rows_of_any_kind(heads, kv_heads, source, norm):
+    """bfloat16 queries and pages, factors a head, factors by position, a request that only pads and one whose page is missing:
+    the kernel for pieces writes what the other one writes (which an odd stride asks for), and leaves alone what it leaves."""
+    from cloud_inference_from_scratch_b200.engine.runtime import Runtime
+    from cloud_inference_from_scratch_b200.native.ops import KernelError
+
+    ops = Runtime("cuda:0", "bfloat16").ops
+    ops._load_streams()
+    tokens, dim, page_size = 48, 128, 16
+    width = (heads + 2 * kv_heads) * dim
+    rows = rand(tokens, width, seed=1).to(getattr(torch, source))
+    requests = (torch.arange(tokens) // 12).int().cuda()               # four of twelve tokens
+    positions = (torch.arange(tokens) % 12 + 10).int().cuda()          # over two pages each
+    table = torch.tensor([[0, 1], [2, 3], [4, -1], [6, 7]], dtype=torch.int32).cuda()
+    active = torch.tensor([1, 0, 1, 1], dtype=torch.int32).cuda()
+    factors, freq = (1 + rand(heads, seed=2, scale=0.3)).cuda(), (10000.0 ** (-torch.arange(32) / 32)).cuda()
+    gains = [(1 + rand(n * dim, seed=s, scale=0.2)).cuda() for n, s in ((heads, 3), (kv_heads, 4))] if norm else None
+    results = []
+    for extra in (4, 3):          # columns behind the row
+        src = torch.zeros(tokens, width + extra, dtype=rows.dtype).cuda()
+        src[:, :width] = rows.cuda()
+        pools = [torch.full((8, kv_heads, page_size, dim), 7.0, dtype=torch.bfloat16).cuda() for _ in range(2)]
+        q = write_rows(ops, src, positions, requests, table, heads, kv_heads, dim, pools, gains, freq, (factors, 0.4, 4), active)
+        with pytest.raises(KernelError, match="no valid cache page"):
+            ops.check_errors()
+        ops.check_errors()
+        results.append([t.float().cpu() for t in (q, *pools)])
+    for pieces, plain in zip(*results):
+        # float32 sums in another order, rounded to bfloat16: a unit of its last place where a value is near the middle of two
+        assert float((pieces - plain).abs().max()) <= 2.0 ** -7 * float(plain.abs().max())
+        assert float((pieces != plain).float().mean()) < 1e-2
+    k, v = results[0][1:]
+    for pool in (k, v):
+        assert bool((pool[2:4] == 7).all()) and bool((pool[5] == 7).all())          # the request that pads; no page
+        assert bool((pool[0, :, 10:] != 7).all()) and bool((pool[1, :, :6] != 7).all()) and bool((pool[4, :, 10:] != 7).all())
+        assert bool((pool[0, :, :10] == 7).all()) and bool((pool[1, :, 6:] == 7).all()) and bool((pool[4, :, :10] == 7).all())

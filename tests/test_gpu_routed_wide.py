@@ -1,5 +1,5 @@
-"""Routed experts of many pairs: the router that shares its matrix among tokens, and the grouped products in tiles of
-128 columns and of 256."""
+"""Routed experts of many pairs: the router that shares its matrix among tokens, and the grouped products in tiles of 128
+weight rows by up to 256 tokens of an expert."""
 
 import pytest
 import torch
@@ -12,17 +12,17 @@ def rand(*shape, seed, scale=1.0):
     return torch.randn(*shape, generator=generator) * scale
 
 
-@pytest.mark.parametrize("columns", ["128", "256"])
-@pytest.mark.parametrize("tokens", [342, 1185])          # one token more than whole blocks of four in the router
+# pairs of the expert that every token chooses: one short of a tile, a whole one, one more than one and two whole ones, some that
+# divide into even tiles, and one token more than whole blocks of four in the router
+@pytest.mark.parametrize("tokens", [255, 256, 257, 342, 513, 1185])
 @pytest.mark.parametrize("hidden,ff", [(72, 16), (256, 128), (264, 144), (512, 272)])
 @pytest.mark.parametrize("weight_inputs", [False, True])
-def test_many_pairs(monkeypatch, tokens, hidden, ff, weight_inputs, columns):
-    """An expert that every token chooses, one that none does, uneven others; columns that end inside a tile, at its edge
-    and one channel block behind it; K that ends inside a step.  The choice is the 32-bit logits' (no two are near a tie
+def test_many_pairs(tokens, hidden, ff, weight_inputs):
+    """An expert that every token chooses, one that none does, uneven others; weight rows that end inside a tile of 128, at its
+    edge and one channel block behind it; K that ends inside a step.  The choice is the 32-bit logits' (no two are near a tie
     here); the activation is rounded to bfloat16 once, the sums are float32: 2^-7 of the largest value."""
     from cloud_inference_from_scratch_b200.engine.runtime import Runtime
 
-    monkeypatch.setenv("CIE_MOE_TILE_COLUMNS", columns)
     rt = Runtime("cuda:0", "bfloat16")
     experts, top = 6, 3
     x = rand(tokens, hidden, seed=1).bfloat16()
