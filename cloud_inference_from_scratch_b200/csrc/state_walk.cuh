@@ -271,7 +271,7 @@ state_walk_kernel(WalkArgs a) {
       if (!__all_sync(0xffffffffu, mbar_wait(&u_full[i & 1], (i >> 1) & 1, a.err))) { alive = false; break; }
       float o[MT][4];
       {
-        Tf32Sum sum[MT];
+        Tf32Sum<!kBoth> sum[MT];
 #pragma unroll
         for (int kind = 0; kind < (kBoth ? 2 : 1); ++kind)
 #pragma unroll
@@ -446,7 +446,7 @@ state_walk_kernel(WalkArgs a) {
       float gained[MT][2][4];
       all = 0.f;
       auto gain_of = [&](const float* keys, const float* frags, bool more) {
-        Tf32Sum gain[2][MT];
+        Tf32Sum<!kBoth> gain[2][MT];
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
           const float* kt = keys + (8 * kk + t) * KL + warp * 16 + 2 * g;

@@ -283,3 +283,44 @@ def test_order_company_and_width_of_blocks_change_no_bit(rule, count):
     for r in (0, 5, count - 1):
         alone, after = run_rule(rule, part([r]), [lengths[r]], heads, dim)
         assert torch.equal(alone, out[tokens[r]]) and torch.equal(after[0], state[r])
+
+
+@pytest.mark.parametrize("rule,length,count,heads,dim,most", [
+    ("gla", 333, 4, 16, 128, 1.95e-7), ("gla", 500, 3, 8, 64, 1.82e-7), ("gated", 333, 4, 16, 128, 1.76e-7), ("gated", 500, 3, 8, 64, 1.88e-7)])
+def test_chunks_are_as_far_from_64_bits_as_float32_sums(rule, length, count, heads, dim, most):
+    """The error of a step's outputs, over their norm: 1.83e-7, 1.72e-7, 1.70e-7 and 1.81e-7.  On the CUDA cores the same
+    recurrences in chunks have 1.92e-7, 1.72e-7, 1.75e-7 and 1.75e-7; accumulators of the tensor cores that are cut at every step of
+    8 have 2.06e-7, 1.93e-7, 1.78e-7 and 1.93e-7."""
+    tokens, qk = count * length, heads * dim
+    generator = torch.Generator(device="cuda").manual_seed(1)
+    normal = lambda *shape: torch.empty(*shape, device="cuda").normal_(generator=generator)  # noqa: E731
+    uniform = lambda low, high, *shape: torch.empty(*shape, device="cuda").uniform_(low, high, generator=generator)  # noqa: E731
+    lengths, views = [length] * count, (count, length, heads, dim)
+    start = normal(count, heads, dim, dim) * 0.3
+    state, outs = start.to(F), []
+    if rule == "gla":
+        proj, z, bias = normal(tokens, 3 * qk), normal(tokens, qk), uniform(-1.0, 5.0, qk)
+        inputs = [proj, z, bias, start]
+        q, k, v = (proj[:, i * qk:(i + 1) * qk].to(F).view(views) for i in range(3))
+        decay = torch.sigmoid(z.to(F) + bias.to(F)).pow(0.25).view(views)
+        for t in range(length):
+            state = decay[:, t].unsqueeze(-1) * state + k[:, t].unsqueeze(-1) * v[:, t].unsqueeze(-2)
+            outs.append(torch.einsum("rhkv,rhk->rhv", state, q[:, t]) * dim ** -0.5)
+    else:
+        conv, gates = torch.nn.functional.silu(normal(tokens, 3 * qk)), normal(tokens, 2 * heads)
+        a_log, dt = torch.log(uniform(1.0, 16.0, heads)), torch.log(torch.expm1(torch.exp(uniform(-6.9, -2.3, heads))))
+        inputs = [conv, gates, a_log, dt, start.view(count, -1)]
+        q, k, v = (conv[:, i * qk:(i + 1) * qk].to(F).view(views) for i in range(3))
+        q, k = (x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6) for x in (q, k))
+        write = torch.sigmoid(gates[:, :heads].to(F)).view(views[:3])
+        decay = torch.exp(-torch.exp(a_log.to(F)) * torch.nn.functional.softplus(gates[:, heads:].to(F) + dt.to(F))).view(views[:3])
+        for t in range(length):
+            state = decay[:, t, :, None, None] * state
+            u = write[:, t].unsqueeze(-1) * (v[:, t] - torch.einsum("rhkv,rhk->rhv", state, k[:, t]))
+            state = state + k[:, t].unsqueeze(-1) * u.unsqueeze(-2)
+            outs.append(torch.einsum("rhkv,rhk->rhv", state, q[:, t]) * dim ** -0.5)
+    want = torch.stack(outs, 1).reshape(tokens, qk)
+    out, _ = run_rule(rule, inputs, lengths, heads, dim)
+    error = float((out.cuda().to(F) - want).norm() / want.norm())
+    print(f"{rule} {length} x {count}, {heads} heads of {dim}: {error:.3e}")
+    assert error <= most
