@@ -16,9 +16,9 @@
 // The rows of A are split once, by a kernel of their own, and come as terms by TMA; the rows of W, each of which one tile of
 // columns reads, are split on their way to shared memory.  What bounds it: shared memory, which the terms are written to (3 x 2
 // bytes an element) and which the tensor core reads both operands from (1,340 of the 1,870 cycles of a step), and the splitting
-// warps' instructions.  300 rows, 2,048 x 2,048: 37 us against 48 where every tile split its rows of A itself and 125 on the CUDA
-// cores; 22,016 x 2,048: 220, 279 and 690; 2,048 x 11,008: 165, 223 and 655; 17 rows of 2,048 x 11,008: 143 and 150, of 22,016 x
-// 2,048: 96 and 110.  Eight splitting warps, a step ahead: 16 warps, whose instructions get in each other's way, 233 (220 above),
+// warps' instructions.  300 rows, 2,048 x 2,048: 37 us against 47 where every tile split its rows of A itself and 124 on the CUDA
+// cores; 22,016 x 2,048: 223, 282 and 692; 2,048 x 11,008: 168, 226 and 656; one row, the same three: 31, 33 and 46; 97, 116 and 77;
+// 143, 157 and 240 (17 rows as one).  512 x 512 of one row: 12.0, 11.3 and 12.8.  Eight splitting warps, a step ahead: 16 warps, whose instructions get in each other's way, 233 (220 with eight),
 // two steps ahead 244 and four 255.
 #include "blackwell.cuh"
 #include "common.cuh"
@@ -363,8 +363,8 @@ extern "C" int cie_gemm_f32_tc(const float* a, const float* w, const float* bias
   CUtensorMap map_a;
   if (!tensor_map_bf16(terms, 3ll * m, padded_k(k), a_rows, &map_a)) CIE_FAIL("gemm_f32_tc: cuTensorMapEncodeTiled failed");
   CIE_LAUNCH("f32_terms", f32_terms_kernel, dim3(m, parts_of(k)), dim3(256), 0, (cudaStream_t)stream, a, terms, apart, m, k);
-  // narrow tiles while they do not make a second round: 64 x 2,048 results of 2,048 32 us against 37 with wide ones, 300 x
-  // 2,048 (192 narrow tiles, 96 wide ones) 67 against 48
+  // narrow tiles while they do not make a second round: 64 x 2,048 results of 2,048 31.5 us against 35 with wide ones, 300 x
+  // 2,048 (192 narrow tiles, 96 wide ones) 59 against 37
   const long long narrow = (long long)((m + kRows - 1) / kRows) * ((n + 31) / 32);
   if (columns != 32 && columns != 64) columns = narrow <= device_sms() ? 32 : 64;
   const cudaError_t status =

@@ -3,7 +3,7 @@
 // are the left operand of mma.sync, whose columns are the pairs, float32 sums; the eight warps share k and add their sums
 // up in shared memory.  The order of k inside 32 columns is chosen so that a lane's pieces of 16 bytes, straight from memory,
 // are its share of two products.  Every warp asks for the next 128 columns (or unit) before it multiplies the last.
-// 8 tokens, 4 of 16 experts of 1,376 channels, 2,048 wide (162 + 81 MB of weights): 33 and 21 us, the layer 48; with the
+// 8 tokens, 4 of 16 experts of 1,376 channels, 2,048 wide (162 + 81 MB of weights): 31 and 19 us, the layer 44; with the
 // multiplications on the CUDA cores, which then were the bound, 44 and 34, 68.
 //
 //   gate_up  W = [experts][2F][H], gate and up rows of an expert interleaved in blocks of 16 (moe_tcgen05.cu);

@@ -17,8 +17,8 @@
 // A tile's rows beyond the expert's last (they belong to the next expert, or lie outside the buffer and read as zero) are
 // computed and never stored.  Every wait on an mbarrier is bounded.
 // What bounds a large product: a stage's way through copy, products and back, 2 us of which four stages of 48 KB cover less
-// than the products would use up (85 us of the 98 below without the epilogue, 70 without loads), and the epilogue's
-// instructions.  2,048 tokens, 4 of 16 experts of 1,376 channels, 2,048 wide: 98 and 58 us, with token rows as the
+// than the products would use up (85 us of the 101 below without the epilogue, 70 without loads), and the epilogue's
+// instructions.  2,048 tokens, 4 of 16 experts of 1,376 channels, 2,048 wide: 101 and 58 us, with token rows as the
 // left operand in tiles of 128 by 256 119 and 66.  Tiles of 256 weight rows take up all of tensor memory, so that nothing hides
 // their epilogue: 100 and 61.  Asking L2 for later weights: 3 us more.  The layer of 17 tokens 94 -> 88, 512 tokens 123 -> 103,
 // 2,048 tokens of 32 experts of 2,048 channels, 4,096 wide, 689 -> 589.
@@ -252,7 +252,7 @@ using namespace cie;
 // and up rows interleaved in blocks of 16; act: [tokens * top][ff], rows by place.  All bfloat16,
 // 16-byte aligned; hidden a multiple of 8, ff a multiple of 16.  clamped, limit, slope, shift, input_weights: GluAct.
 extern "C" int cie_moe_gate_up_tcgen05(const void* x, void* sorted, const void* w_gate_up, void* act,
-                                       const int* place_to_pair, const int* tiles, const int* tile_count,
+                                       const int* place_to_pair, const int* tiles,
                                        int tokens, int top, int experts, int ff, int hidden, int row_tile, int clamped,
                                        float limit, float slope, float shift, const float* input_weights, int* err,
                                        void* stream) {
@@ -274,7 +274,7 @@ extern "C" int cie_moe_gate_up_tcgen05(const void* x, void* sorted, const void* 
 // act: [tokens * top][ff] by place; w_down: [experts][hidden][ff]; rows: float32 [tokens * top][hidden],
 // the row of pair (t, j) at t * top + j.
 extern "C" int cie_moe_down_tcgen05(const void* act, const void* w_down, float* rows, const int* place_to_pair,
-                                    const int* tiles, const int* tile_count, int tokens, int top, int experts,
+                                    const int* tiles, int tokens, int top, int experts,
                                     int ff, int hidden, int row_tile, int* err, void* stream) {
   if (tokens <= 0) return 0;
   if (hidden % 8 || ff % 8) CIE_FAIL("moe_down_tcgen05: sizes %d / %d", hidden, ff);

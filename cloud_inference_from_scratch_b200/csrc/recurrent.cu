@@ -898,8 +898,7 @@ mlstm_chunk_prefix_kernel(float* __restrict__ chunk_sums, float* __restrict__ st
 // grid (chunks, heads).  chunk_sums holds, after the walk, the state before each chunk.
 // q, k, v: where a head's rows are (see RowsOf).
 struct RowsOf {
-  const float* base;      // row t of head h starts at base + h * head_base + t * stride + col0 + h * head_col
-  long long head_base;
+  const float* base;      // row t of head h starts at base + t * stride + col0 + h * head_col
   int stride, col0, head_col;
 };
 
@@ -939,11 +938,11 @@ mlstm_chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_s
     gm_s[threadIdx.x] = g.z;
     if (threadIdx.x == 0) m_before = g.w;
   }
-  stage_rows(q_s, ld, q_rows.base + head * q_rows.head_base, q_rows.stride, row0, n, q_rows.col0 + head * q_rows.head_col,
+  stage_rows(q_s, ld, q_rows.base, q_rows.stride, row0, n, q_rows.col0 + head * q_rows.head_col,
              dim, [&](int) { return q_scale; });
-  stage_rows(k_s, ld, k_rows.base + head * k_rows.head_base, k_rows.stride, row0, n, k_rows.col0 + head * k_rows.head_col,
+  stage_rows(k_s, ld, k_rows.base, k_rows.stride, row0, n, k_rows.col0 + head * k_rows.head_col,
              dim, [](int) { return 1.f; });
-  stage_rows(v_s, vld, v_rows.base + head * v_rows.head_base, v_rows.stride, row0, n, v_rows.col0 + head * v_rows.head_col,
+  stage_rows(v_s, vld, v_rows.base, v_rows.stride, row0, n, v_rows.col0 + head * v_rows.head_col,
              vdim, [](int) { return 1.f; });
   if (padded != dim)
     for (int e = threadIdx.x; e < kMemChunk * (padded - dim); e += kOutThreads) {
@@ -1384,7 +1383,7 @@ extern "C" int cie_mlstm_chunked(const float* proj, int proj_stride, int q_off, 
   CIE_LAUNCH("mlstm_chunk_prefix", mlstm_chunk_prefix_kernel, dim3(requests, heads, (dim * vdim + dim + 1 + 255) / 256),
              dim3(256), 0, s, sums, state, state_stride, (const float*)gates, request_chunk_start, chunk_row, chunk_count,
              slots, request_active, heads, dim, vdim, max_slots, err);
-  const RowsOf q_rows{proj, 0, proj_stride, q_off, dim}, k_rows{proj, 0, proj_stride, k_off, dim}, v_rows{proj, 0, proj_stride, v_off, vdim};
+  const RowsOf q_rows{proj, proj_stride, q_off, dim}, k_rows{proj, proj_stride, k_off, dim}, v_rows{proj, proj_stride, v_off, vdim};
   CIE_LAUNCH("mlstm_chunk_output", mlstm_chunk_output_kernel, grid, block, smem4, s, q_rows, k_rows, v_rows, q_scale,
              (const float*)gates, (const float*)sums, out, out_stride, chunk_row, chunk_count, heads, dim, vdim);
   return 0;

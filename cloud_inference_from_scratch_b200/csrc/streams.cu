@@ -341,7 +341,7 @@ __global__ void norm_kv_write_kernel(const TI* __restrict__ src, const float* __
 // The same for rows whose parts are whole, aligned pieces of four elements, norms of whole projections or none, rotations of
 // halves that are whole pieces, and values that are not mixed: a thread keeps its pieces in registers, and the block meets
 // twice (the sums; the scaled row, whose other half the rotation reads).  What bounds it is how long a token's chain is and how
-// many tokens run at one time: angles, page and gains, which no kernel of the step writes, are there before the wait.  2,048
+// many tokens run at one time: angles and page, which no kernel of the step writes, are there before the wait.  2,048
 // tokens of 16 + 2 heads of 128, half of every head rotated: 17 us cold (its bytes 5), 22 on
 // the kernel above; the attention layer of 2,048 tokens 101.5 -> 97, of eight single tokens 34.5 -> 32.
 constexpr int kRowPieces = 3;      // pieces of a thread at most: six blocks of 256 threads an SM

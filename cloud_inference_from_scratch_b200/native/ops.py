@@ -1491,9 +1491,9 @@ class Ops:
             v, i, f = c_void_p, c_int, c_float
             lib = _Lib(load_library("moe_tcgen05.cu"))
             self._moe_gate_up_tcgen05 = lib.function(
-                "cie_moe_gate_up_tcgen05", [v, v, v, v, v, v, v, i, i, i, i, i, i, i, f, f, f, v, v, v])
+                "cie_moe_gate_up_tcgen05", [v, v, v, v, v, v, i, i, i, i, i, i, i, f, f, f, v, v, v])
             self._moe_down_tcgen05 = lib.function(
-                "cie_moe_down_tcgen05", [v, v, v, v, v, v, i, i, i, i, i, i, v, v])
+                "cie_moe_down_tcgen05", [v, v, v, v, v, i, i, i, i, i, i, v, v])
             self._moe_tcgen05_lib = lib
 
     def moe_interleaves(self, hidden: int, ff: int) -> bool:
@@ -1566,11 +1566,10 @@ class Ops:
             self._load_moe_tcgen05()
             gathered = workspace.get("moe.sorted", tokens, top * hidden, self.dtype)
             self._moe_gate_up_tcgen05(_ptr(x), _ptr(gathered), _ptr(w_gate), _ptr(act), _ptr(place_to_pair),
-                                      _ptr(tiles), _ptr(tile_count), tokens, top, experts, ff, hidden,
-                                      self.moe_row_tile, *glu, _ptr(self.error_word), self.stream)
-            self._moe_down_tcgen05(_ptr(act), _ptr(w_down), _ptr(rows), _ptr(place_to_pair), _ptr(tiles),
-                                   _ptr(tile_count), tokens, top, experts, ff, hidden, self.moe_row_tile,
-                                   _ptr(self.error_word), self.stream)
+                                      _ptr(tiles), tokens, top, experts, ff, hidden, self.moe_row_tile, *glu,
+                                      _ptr(self.error_word), self.stream)
+            self._moe_down_tcgen05(_ptr(act), _ptr(w_down), _ptr(rows), _ptr(place_to_pair), _ptr(tiles), tokens, top, experts,
+                                   ff, hidden, self.moe_row_tile, _ptr(self.error_word), self.stream)
             self.launches += 1
         elif (code == BF16 and hidden % 8 == 0 and ff % 8 == 0 and aligned
                 and (w_up is None or (os.environ.get("CIE_MOE_TC", "1") != "0" and w_up.data_ptr() % 16 == 0))):
@@ -1649,9 +1648,9 @@ class Ops:
 
         ``few_rows``: this product gets a row a request and never a whole prompt (the logits).  In 32-bit it then stays on
         the CUDA cores, whatever the number of rows, so that a row's bits do not depend on it: one row of 151,936 x 2,048
-        takes 313 us there and 580 on the tensor cores, which work on 128 rows at a time and are ahead from 17 rows on (582
-        against 665).  The layers' products go to the tensor cores at every number of rows, for the same reason; one row of
-        22,016 x 2,048 costs 108 us there (73 on the CUDA cores), of 2,048 x 11,008 139 (239), of 2,048 x 2,048 28 (46).
+        takes 307 us there and 496 on the tensor cores, which work on 128 rows at a time and are ahead from 17 rows on (498
+        against 666).  The layers' products go to the tensor cores at every number of rows, for the same reason; one row of
+        22,016 x 2,048 costs 97 us there (77 on the CUDA cores), of 2,048 x 11,008 143 (240), of 2,048 x 2,048 31 (46).
 
         Returns ``out``; or, when ``allow_partials`` and the product was cut along K, a
         ``Partials`` that a consuming kernel adds up (then ``out`` was not written); or, when the
