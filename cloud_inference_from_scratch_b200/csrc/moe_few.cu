@@ -3,7 +3,7 @@
 // are the left operand of mma.sync, whose columns are the pairs, float32 sums; the eight warps share k and add their sums
 // up in shared memory.  The order of k inside 32 columns is chosen so that a lane's pieces of 16 bytes, straight from memory,
 // are its share of two products.  Every warp asks for the next 128 columns (or unit) before it multiplies the last.
-// 8 tokens, 4 of 16 experts of 1,376 channels, 2,048 wide (162 + 81 MB of weights): 31 and 19 us, the layer 44; with the
+// 8 tokens, 4 of 16 experts of 1,376 channels, 2,048 wide (162 + 81 MB of weights): 31 and 20 us, the layer 45; with the
 // multiplications on the CUDA cores, which then were the bound, 44 and 34, 68.
 //
 //   gate_up  W = [experts][2F][H], gate and up rows of an expert interleaved in blocks of 16 (moe_tcgen05.cu);
@@ -33,6 +33,18 @@ __device__ __forceinline__ void few_mma(float (&d)[4], uint32_t a0, uint32_t a1,
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// From zero: the tensor core cuts what it adds to an accumulator.  Results that stay float32 (the down product's) add products of
+// 16 columns up in registers, where sums are rounded: 8.6e-8 of the rows' norm from 64 bits with 1,376 columns, 8.4e-8 as one
+// FMA after the other, 1.31e-7 with accumulators.  Those of gate_up are rounded to 16 bits.
+__device__ __forceinline__ void few_add(float (&sum)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  float d[4];
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) sum[i] += d[i];
 }
 
 // Two blocks an SM.  x: gate_up: token rows [tokens][k], the row of pair p is x[p / top]; down: rows by pair [pairs][k].  n:
@@ -129,8 +141,13 @@ moe_few_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, void* __r
   auto multiply = [&](const FewStep& s) {
 #pragma unroll
     for (int i = 0; i < kBlocks; ++i) {
-      few_mma(sum[0], s.low[i].x, s.high[i].x, s.low[i].y, s.high[i].y, s.x[i].x, s.x[i].y);
-      few_mma(sum[1], s.low[i].z, s.high[i].z, s.low[i].w, s.high[i].w, s.x[i].z, s.x[i].w);
+      if constexpr (kGateUp) {
+        few_mma(sum[0], s.low[i].x, s.high[i].x, s.low[i].y, s.high[i].y, s.x[i].x, s.x[i].y);
+        few_mma(sum[1], s.low[i].z, s.high[i].z, s.low[i].w, s.high[i].w, s.x[i].z, s.x[i].w);
+      } else {
+        few_add(sum[0], s.low[i].x, s.high[i].x, s.low[i].y, s.high[i].y, s.x[i].x, s.x[i].y);
+        few_add(sum[1], s.low[i].z, s.high[i].z, s.low[i].w, s.high[i].w, s.x[i].z, s.x[i].w);
+      }
     }
     if (++step < steps) return;
     step = 0;
