@@ -20,8 +20,8 @@
 // (2) per (request, head, block of value columns) a walk over the request's chunks that works out the
 // outputs and carries the state (state_walk.cuh).  Chunks come as a work list made on the host from the step's
 // portion lengths (first token row and token count of each chunk; where every request's chunks start).  2,048 tokens of 16
-// heads of 128 x 128: 39 and 88 us, 127 together; states of all chunks through memory (sums per chunk, a walk over them, outputs
-// per chunk, on the CUDA cores) took 184.  Eight portions of 287 tokens, 32 heads: 223 against 456.
+// heads of 128 x 128: 39 and 92 us, 131 together; states of all chunks through memory (sums per chunk, a walk over them, outputs
+// per chunk, on the CUDA cores) took 183.  Eight portions of 287 tokens, 32 heads: 223 against 457.
 //
 // A request's result depends on its own tokens and state only: the batch and the slot change nothing, the cut
 // of a prompt into portions only the order of additions.

@@ -1019,8 +1019,8 @@ mlstm_chunk_output_kernel(RowsOf q_rows, RowsOf k_rows, RowsOf v_rows, float q_s
 //                              S <- c_C S_0 + sum_s (c_C / c_s) k_s u_s^T
 // Ratios of decays are exponentials of differences of summed logarithms, never quotients.  1 and 2 work in float32 on the
 // CUDA cores, 3 as accurately on the tensor cores.  Keys up to kMemDim, values a multiple of 4.  Four portions of 333 tokens,
-// 16 heads of 128 x 128: 13 and 32 and 56 us, 104 in all; with the states of all chunks through memory and the walk and the
-// outputs on the CUDA cores 164; a prompt of 2,048 tokens 232 against 514.
+// 16 heads of 128 x 128: 121 us in all, half of them the walk; with the states of all chunks through memory and the walk and the
+// outputs on the CUDA cores 163; a prompt of 2,048 tokens 236 against 496.
 constexpr int kSolveRow = kMemChunk + 4;         // row of the solve's matrices, transposed: [earlier token][token]
 constexpr int kScores = kMemChunk * kMemChunk;   // floats of k_t . k_s of a chunk, and of q_t . k_s: row t, column s
 

@@ -23,7 +23,8 @@
 // that (lane 4 g + t reads keys 4 t .. 4 t + 3 of token g, and keys 2 g, 2 g + 1 of token t).
 //
 // Where an infinity, a NaN or a value near the largest one is met (in the cell, the warp's part of the state, or a sum), the
-// same is worked out on the CUDA cores, where a token's outputs read nothing of later tokens.
+// same is worked out on the CUDA cores, where a token's outputs read nothing of later tokens (for all columns of the block, whose
+// width follows the number of blocks: beside such a value, a finite one's last bits may depend on the company).
 #pragma once
 
 #include "blackwell.cuh"
